@@ -1881,12 +1881,13 @@ int trax_fit_prepare(trax_ctx* c, const trax_fit_opts* opts, uint64_t* n_fit) {
   }
   if (run > 0xffffffffull) return fail(c, TRAX_ERR_CAPACITY, "too many fit rows");
   c->nFit = run;
+  f.chunk = fit_chunk(run, sm_count());
   uint64_t base = 0, blk = 0;
   for (uint32_t k = 0; k < f.nLT; ++k) {
     f.ltBase[k] = (uint32_t)base;
     f.blkStart[k] = (uint32_t)blk;
     base += ltCount[k];
-    blk += (ltCount[k] + TRAX_FIT_CHUNK - 1) / TRAX_FIT_CHUNK;
+    blk += (ltCount[k] + f.chunk - 1) / f.chunk;
   }
   f.ltBase[f.nLT] = (uint32_t)base;
   f.blkStart[f.nLT] = (uint32_t)blk;

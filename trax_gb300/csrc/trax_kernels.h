@@ -306,15 +306,24 @@ cudaError_t ca_tracks(CABuffers b, const uint32_t* nTDev, uint64_t maxT, uint32_
 // ------------------------------------------- differentiable triplet fit
 // Fit rows are the selected triplets ordered by layer triplet; rows of layer
 // triplet k are [ltBase[k], ltBase[k+1]) and are reduced by the blocks
-// [blkStart[k], blkStart[k+1]), each taking FIT_CHUNK rows, so that every
-// FP64 sum is taken in a fixed order.
-#define TRAX_FIT_CHUNK 4096u
+// [blkStart[k], blkStart[k+1]), each taking `chunk` rows, so that every
+// sum is taken in a fixed order.
+// Rows per block: TRAX_FIT_CHUNK_MAX, or fewer (a power of two, at least one
+// row per thread) while that leaves fewer than eight blocks per SM -- 66 k
+// rows in blocks of 4096 kept 17 of 152 SMs busy.
+#define TRAX_FIT_CHUNK_MIN 256u
+#define TRAX_FIT_CHUNK_MAX 2048u
+inline uint32_t fit_chunk(uint64_t rows, int sms) {
+  uint32_t c = TRAX_FIT_CHUNK_MAX;
+  while (c > TRAX_FIT_CHUNK_MIN && rows / c < 8u * (uint64_t)sms) c >>= 1;
+  return c;
+}
 // per block: chi2, d chi2 / d(dr, dz, dphi) of the three hit layers, and an
 // approximate Gauss-Newton diagonal for the same nine (a preconditioner)
 #define TRAX_FIT_SLOTS 19
 
 struct FitConfig {
-  uint32_t L, nLT, nBlocks;
+  uint32_t L, nLT, nBlocks, chunk;
   uint32_t layer[3][TRAX_MAX_LT];  // 0-based layer of each hit slot of a layer triplet
   float wTip[TRAX_MAX_LT];         // 1 / sigma_tip^2 per layer triplet
   float wZ;                        // 1 / sigma_z^2
