@@ -328,8 +328,8 @@ typedef struct trax_tune_result {
 } trax_tune_result;
 int trax_autotune(trax_ctx* ctx, const char* cache_path, const trax_tune_opts* opts, trax_tune_result* result);
 
-/* Device time of the last run, from CUDA events on the context's stream
- * (RuntimeRecord's per-stage count/scan/store classes, RuntimeRecord.cpp:123-192):
+/* Device time of the last run, between the kernels' starts on the device's
+ * nanosecond clock (RuntimeRecord's per-stage count/scan/store classes, RuntimeRecord.cpp:123-192):
  * stage_ms[7] = grid, pairs, prediction, filter, connectivity, circle fit, CA;
  * kernel_ms[9] = grid build, pair count, pair store, prediction count,
  * prediction store, filter, filter store, connectivity count, connectivity

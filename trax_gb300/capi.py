@@ -474,7 +474,7 @@ class Context:
                "filter_store", "connectivity_count", "connectivity_store"]
 
     def timings(self):
-        """(stage ms, kernel ms) of the last run, from CUDA events; -1 = not run."""
+        """(stage ms, kernel ms) of the last run, from device time marks; -1 = not run."""
         s = np.zeros(len(self.STAGES), dtype=np.float32)
         k = np.zeros(len(self.KERNELS), dtype=np.float32)
         self._check(self._L.trax_get_timings(self._h, _p(s), _p(k)))

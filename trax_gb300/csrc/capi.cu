@@ -101,6 +101,7 @@ const uint64_t NO_CAP = 0xffffffffull;
 struct trax_ctx {
   int device = 0;
   cudaStream_t st = nullptr;
+  trax::Queue q;  // st, the launch count and the pending time marks
   std::string err;
   // configuration
   std::vector<trax_layer_triplet> lts;
@@ -154,7 +155,6 @@ struct trax_ctx {
   // chain's own filter output; checked for caller-provided triplets
   bool sortedSegments = true;
   bool identityHits = false;  // hit collection taken as uploaded (trax_set_tracklets)
-  uint32_t launches = 0;
   // DEVICE-mode capacities and the captured graph
   uint64_t capTasks = 0, capPairs = 0, capCands = 0, capT = 0, capLinks = 0, capTracks = 0;
   cudaGraph_t graph = nullptr;
@@ -166,7 +166,6 @@ struct trax_ctx {
   uint64_t graphCaptures = 0;  // calibrate-and-capture passes of the last trax_seed_batch
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   double lastMs = 0.0;
-  // per-stage and per-kernel timing events of the last run
   // differentiable fit: rows frozen by trax_fit_prepare for one triplet set
   DevBuf fitOk, fitSegCnt, fitSegDelta, fitRows, fitPartials, fitOut, fitParams, fitDHits, fitDHitsF;
   FitConfig fitCfg;
@@ -178,9 +177,6 @@ struct trax_ctx {
   uint64_t ptGen = 0, caGen = 0;
   bool caOnly = false;  // triplet count taken from the CA's caller input, no triplet arrays
   float fitSigmaTip[TRAX_MAX_LT] = {};
-  cudaEvent_t stageEv[N_STAGES + 1] = {};
-
-  cudaEvent_t kEv[2 * TK_N] = {};
   bool stageUsed[N_STAGES] = {};
   bool kUsed[TK_N] = {};
 };
@@ -276,23 +272,16 @@ struct NvtxRange {
   NvtxRange& operator=(const NvtxRange&) = delete;
 };
 
-// event marks around one kernel (recorded into the graph when capturing)
-// While the stream is being captured the record becomes an event-record node
-// of the graph (cudaEventRecordExternal); otherwise it is a plain record.
-cudaError_t record(trax_ctx* c, cudaEvent_t ev) {
-  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  cudaError_t e = cudaStreamIsCapturing(c->st, &cs);
-  if (e != cudaSuccess) return e;
-  if (cs == cudaStreamCaptureStatusActive) return cudaEventRecordWithFlags(ev, c->st, cudaEventRecordExternal);
-  return cudaEventRecord(ev, c->st);
-}
+// Time marks: the stage boundaries, then a begin and an end per timed
+// kernel.  A mark is written by the next kernel launched as it starts.
+enum { MARK_STAGE = 0, MARK_KERNEL = N_STAGES + 1, MARK_N = MARK_KERNEL + 2 * TK_N };
+static_assert(MARK_N <= 32, "the marks pending on a queue are one word");
+const size_t SLOT_WORDS = 64;  // the marks follow the slots
+const size_t SLOT_BYTES = SLOT_WORDS * sizeof(uint32_t) + MARK_N * sizeof(unsigned long long);
 
-void kmark(trax_ctx* c, int k, bool end) {
-  record(c, c->kEv[2 * k + (end ? 1 : 0)]);
-  if (end) c->kUsed[k] = true;
-}
-#define KBEG(k) kmark(c, k, false)
-#define KEND(k) kmark(c, k, true)
+void mark(trax_ctx* c, int k) { c->q.marks.which |= 1u << k; }
+#define KBEG(k) mark(c, MARK_KERNEL + 2 * (k))
+#define KEND(k) (mark(c, MARK_KERNEL + 2 * (k) + 1), c->kUsed[k] = true)
 uint32_t* dev_err(trax_ctx* c) { return slot(c, S_ERR); }
 
 float min_radius_curvature(float minPt) {
@@ -371,9 +360,10 @@ int build_config(trax_ctx* c, bool seeding = true) {
   return TRAX_OK;
 }
 
-// read all slots (error word, counters, totals) in one copy
+// read all slots (error word, counters, totals) and time marks: a kernel
+// writes them to the page-locked copy, which takes pending marks with it
 int read_slots(trax_ctx* c) {
-  CK(cudaMemcpyAsync(c->hSlots, c->slots.p, sizeof(uint32_t) * S_N, cudaMemcpyDeviceToHost, c->st));
+  CK(slots_to_host(ptr<uint32_t>(c->slots), c->hSlots, SLOT_BYTES / 4, c->q));
   CK(cudaStreamSynchronize(c->st));
   return TRAX_OK;
 }
@@ -383,9 +373,7 @@ int error_from_bits(trax_ctx* c, uint32_t bits);
 // a stage total read by the host in SYNCED mode; the error word comes along so
 // that an overflowed or timed-out scan stops the chain before its total is used
 int read_slot(trax_ctx* c, int k, uint64_t* out) {
-  CK(cudaMemcpyAsync(c->hSlots + k, slot(c, k), sizeof(uint32_t), cudaMemcpyDeviceToHost, c->st));
-  CK(cudaMemcpyAsync(c->hSlots + S_ERR, slot(c, S_ERR), sizeof(uint32_t), cudaMemcpyDeviceToHost, c->st));
-  CK(cudaStreamSynchronize(c->st));
+  RC(read_slots(c));
   *out = c->hSlots[k];
   return error_from_bits(c, c->hSlots[S_ERR] & (TRAX_EBIT_OVERFLOW | TRAX_EBIT_TIMEOUT));
 }
@@ -422,9 +410,9 @@ int scan_publish(trax_ctx* c, Mode mode, uint32_t* data, uint64_t nHost, const u
   if (mode == SYNCED) CK(ensure(c, c->scanScratch, scan_scratch_bytes(maxN)));
   else if (scan_scratch_bytes(maxN) > c->scanScratch.cap)
     return fail(c, TRAX_ERR_STATE, "device-mode scan scratch too small");
-  CK(scan_exclusive(data, data, nHost + 1, nDev, 1, maxN, c->scanScratch.p, dev_err(c), c->st, &c->launches,
+  CK(scan_exclusive(data, data, nHost + 1, nDev, 1, maxN, c->scanScratch.p, dev_err(c), c->q,
                     true, c->wait));
-  CK(publish_total(data, nDev, nHost, cap, slot(c, dst), dev_err(c), c->st, &c->launches));
+  CK(publish_total(data, nDev, nHost, cap, slot(c, dst), dev_err(c), c->q));
   return TRAX_OK;
 }
 
@@ -466,10 +454,8 @@ int stage_grid(trax_ctx* c, Mode mode) {
   sc.perm = ptr<uint32_t>(c->sc_perm);
   sc.counts = ptr<uint32_t>(c->sc_counts);
   KBEG(TK_GRID);
-  CK(grid_build(c->cfg, in, ptr<uint32_t>(c->grid), dev_hits(c), sc, c->maxLayerHits, dev_err(c), c->st,
-                &c->launches));
-  CK(fine_grid_build(c->cfg, ptr<uint32_t>(c->grid), ptr<float4>(c->pxyzp), fine_buffers(c), sc.counts, c->st,
-                     &c->launches));
+  CK(grid_build(c->cfg, in, ptr<uint32_t>(c->grid), dev_hits(c), sc, c->maxLayerHits, dev_err(c), c->q));
+  CK(fine_grid_build(c->cfg, ptr<uint32_t>(c->grid), ptr<float4>(c->pxyzp), fine_buffers(c), sc.counts, c->q));
   c->fineBuilt = c->cfg.fineRows;
   KEND(TK_GRID);
   return TRAX_OK;
@@ -482,7 +468,7 @@ int stage_pairs(trax_ctx* c, Mode mode) {
   ENSURE(taskBase, S + 1, 4);
   ENSURE(pairOffsets, S + 1, 4);
   uint32_t* taskBase = ptr<uint32_t>(c->taskBase);
-  CK(pair_segments(c->cfg, ptr<uint32_t>(c->grid), ptr<uint32_t>(c->segOuter), taskBase, c->st, &c->launches));
+  CK(pair_segments(c->cfg, ptr<uint32_t>(c->grid), ptr<uint32_t>(c->segOuter), taskBase, c->q));
   RC(scan_publish(c, mode, taskBase, S, nullptr, S, S_TASKS, mode == DEVICE ? c->capTasks : NO_CAP));
   const uint32_t* nTasksDev = slot(c, S_TASKS);
   uint64_t maxTasks = c->capTasks;
@@ -496,8 +482,7 @@ int stage_pairs(trax_ctx* c, Mode mode) {
   const PairTaskState taskState = pair_task_state(c->taskState.p, maxTasks);
   KBEG(TK_PAIR_COUNT);
   CK(pair_tasks(c->cfg, false, ptr<uint32_t>(c->grid), dev_hits(c), ptr<uint32_t>(c->segOuter), taskBase, nTasksDev,
-                maxTasks, taskCount, taskState, nullptr, 0, slot(c, S_PAIR_SENT), dev_err(c), c->st,
-                &c->launches));
+                maxTasks, taskCount, taskState, nullptr, 0, slot(c, S_PAIR_SENT), dev_err(c), c->q));
   KEND(TK_PAIR_COUNT);
   RC(scan_publish(c, mode, taskCount, c->nTasks, mode == DEVICE ? nTasksDev : nullptr, maxTasks, S_PAIRS,
                   mode == DEVICE ? c->capPairs : NO_CAP));
@@ -510,9 +495,9 @@ int stage_pairs(trax_ctx* c, Mode mode) {
   KBEG(TK_PAIR_EMIT);
   CK(pair_tasks(c->cfg, true, ptr<uint32_t>(c->grid), dev_hits(c), ptr<uint32_t>(c->segOuter), taskBase, nTasksDev,
                 maxTasks, taskCount, taskState, ptr<uint2>(c->pairs), maxPairs, slot(c, S_PAIR_SENT), dev_err(c),
-                c->st, &c->launches));
+                c->q));
   KEND(TK_PAIR_EMIT);
-  CK(pair_offsets(c->cfg, taskBase, taskCount, ptr<uint32_t>(c->pairOffsets), c->st, &c->launches));
+  CK(pair_offsets(c->cfg, taskBase, taskCount, ptr<uint32_t>(c->pairOffsets), c->q));
   return TRAX_OK;
 }
 
@@ -533,7 +518,7 @@ int stage_predict(trax_ctx* c, Mode mode) {
   KBEG(TK_PRED_COUNT);
   CK(predict_pairs(c->cfg, false, ptr<uint32_t>(c->grid), dev_hits(c), ptr<uint2>(c->pairs), nPairsDev, maxPairs,
                    candLocal, warpSums, slot(c, S_PRED_WARPS), ptr<uint32_t>(c->predKeep), nullptr, 0,
-                   slot(c, S_CAND_SENT), dev_err(c), c->st, &c->launches, fine_grid(c)));
+                   slot(c, S_CAND_SENT), dev_err(c), c->q, fine_grid(c)));
   KEND(TK_PRED_COUNT);
   // the prefix sum runs over the per-warp sums of the counts
   RC(scan_publish(c, mode, warpSums, (c->nPairs + 31) / 32, mode == DEVICE ? slot(c, S_PRED_WARPS) : nullptr,
@@ -547,10 +532,10 @@ int stage_predict(trax_ctx* c, Mode mode) {
   KBEG(TK_PRED_EMIT);
   CK(predict_pairs(c->cfg, true, ptr<uint32_t>(c->grid), dev_hits(c), ptr<uint2>(c->pairs), nPairsDev, maxPairs,
                    candLocal, warpSums, nullptr, ptr<uint32_t>(c->predKeep), ptr<uint2>(c->cands), maxCands,
-                   slot(c, S_CAND_SENT), dev_err(c), c->st, &c->launches, fine_grid(c)));
+                   slot(c, S_CAND_SENT), dev_err(c), c->q, fine_grid(c)));
   KEND(TK_PRED_EMIT);
   CK(predict_offsets(c->cfg, ptr<uint32_t>(c->pairOffsets), nPairsDev, candLocal, warpSums,
-                     ptr<uint32_t>(c->candOffsets), c->st, &c->launches));
+                     ptr<uint32_t>(c->candOffsets), c->q));
   return TRAX_OK;
 }
 
@@ -567,7 +552,7 @@ int stage_filter(trax_ctx* c, Mode mode) {
   uint32_t* sums = ptr<uint32_t>(c->flagSums);
   KBEG(TK_FILTER);
   CK(filter_candidates(c->cfg, dev_hits(c), ptr<uint2>(c->pairs), ptr<uint2>(c->cands), nCandsDev, maxCands, words,
-                       sums, slot(c, S_FLAG_WORDS), c->st, &c->launches));
+                       sums, slot(c, S_FLAG_WORDS), c->q));
   KEND(TK_FILTER);
   // the prefix sum runs over the numbers of flags per word of 32 candidates
   RC(scan_publish(c, mode, sums, (c->nCands + 31) / 32, mode == DEVICE ? slot(c, S_FLAG_WORDS) : nullptr, maxWords,
@@ -582,10 +567,10 @@ int stage_filter(trax_ctx* c, Mode mode) {
   ENSURE(h3, maxT, 4);
   KBEG(TK_FILTER_STORE);
   CK(filter_store(ptr<uint2>(c->pairs), ptr<uint2>(c->cands), nCandsDev, maxCands, words, sums, ptr<uint32_t>(c->h1),
-                  ptr<uint32_t>(c->h2), ptr<uint32_t>(c->h3), maxT, c->st, &c->launches));
+                  ptr<uint32_t>(c->h2), ptr<uint32_t>(c->h3), maxT, c->q));
   KEND(TK_FILTER_STORE);
   CK(triplet_offsets(c->cfg, dev_hits(c), ptr<uint32_t>(c->h1), slot(c, S_TRIPLETS), maxT,
-                     ptr<uint32_t>(c->tripOffsets), c->st, &c->launches));
+                     ptr<uint32_t>(c->tripOffsets), c->q));
   return TRAX_OK;
 }
 
@@ -623,13 +608,13 @@ int stage_connectivity(trax_ctx* c, Mode mode) {
   ENSURE(nonConnIdx, maxT, 4);
   TripletView tv = triplets(c, maxT);
   CK(cudaMemsetAsync(c->cflags.p, 0, (size_t)(maxT + 1) * 4, c->st));
-  CK(triplet_eta(c->cfg, dev_hits(c), tv, ptr<float>(c->eta), ptr<uint32_t>(c->segOf), c->st, &c->launches));
-  CK(segment_bounds(c->cfg, ptr<uint32_t>(c->segOf), nTDev, ptr<uint32_t>(c->segStart), c->st, &c->launches));
+  CK(triplet_eta(c->cfg, dev_hits(c), tv, ptr<float>(c->eta), ptr<uint32_t>(c->segOf), c->q));
+  CK(segment_bounds(c->cfg, ptr<uint32_t>(c->segOf), nTDev, ptr<uint32_t>(c->segStart), c->q));
   uint32_t* linkCount = ptr<uint32_t>(c->linkCount);
   KBEG(TK_CONN_COUNT);
   CK(connectivity_tasks(c->cfg, false, dev_hits(c), tv, ptr<float>(c->eta), ptr<uint32_t>(c->tripOffsets),
                         ptr<uint32_t>(c->segStart), linkCount, ptr<uint32_t>(c->cflags), ptr<uint32_t>(c->linkRun),
-                        nullptr, nullptr, 0, c->sortedSegments, c->st, &c->launches));
+                        nullptr, nullptr, 0, c->sortedSegments, c->q));
   KEND(TK_CONN_COUNT);
   RC(scan_publish(c, mode, linkCount, c->nT, mode == DEVICE ? nTDev : nullptr, maxT, S_LINKS,
                   mode == DEVICE ? c->capLinks : NO_CAP));
@@ -645,21 +630,19 @@ int stage_connectivity(trax_ctx* c, Mode mode) {
   KBEG(TK_CONN_EMIT);
   CK(connectivity_tasks(c->cfg, true, dev_hits(c), tv, ptr<float>(c->eta), ptr<uint32_t>(c->tripOffsets),
                         ptr<uint32_t>(c->segStart), linkCount, ptr<uint32_t>(c->cflags), ptr<uint32_t>(c->linkRun),
-                        ptr<uint32_t>(c->basis), ptr<uint32_t>(c->follower), maxLinks, c->sortedSegments, c->st,
-                        &c->launches));
+                        ptr<uint32_t>(c->basis), ptr<uint32_t>(c->follower), maxLinks, c->sortedSegments, c->q));
   KEND(TK_CONN_EMIT);
   // the two Q9 streams as words of 32 flags; the scans run over the words' counts
   CK(connectable_words(ptr<uint32_t>(c->cflags), nTDev, maxT, ptr<uint32_t>(c->connW), ptr<uint32_t>(c->connS),
-                       ptr<uint32_t>(c->nonConnW), ptr<uint32_t>(c->nonConnS), slot(c, S_CONN_WORDS), c->st,
-                       &c->launches));
+                       ptr<uint32_t>(c->nonConnW), ptr<uint32_t>(c->nonConnS), slot(c, S_CONN_WORDS), c->q));
   const uint64_t nTW = (c->nT + 31) / 32;
   const uint32_t* nTWDev = mode == DEVICE ? slot(c, S_CONN_WORDS) : nullptr;
   RC(scan_publish(c, mode, ptr<uint32_t>(c->connS), nTW, nTWDev, maxTW, S_CONN, NO_CAP));
   RC(scan_publish(c, mode, ptr<uint32_t>(c->nonConnS), nTW, nTWDev, maxTW, S_NONCONN, NO_CAP));
   CK(compact_words(ptr<uint32_t>(c->connW), ptr<uint32_t>(c->connS), nTDev, maxT, ptr<uint32_t>(c->connIdx), maxT,
-                   c->st, &c->launches));
+                   c->q));
   CK(compact_words(ptr<uint32_t>(c->nonConnW), ptr<uint32_t>(c->nonConnS), nTDev, maxT, ptr<uint32_t>(c->nonConnIdx),
-                   maxT, c->st, &c->launches));
+                   maxT, c->q));
   if (mode == SYNCED) {
     RC(read_slots(c));
     c->nConn = c->hSlots[S_CONN];
@@ -675,7 +658,7 @@ int stage_fit(trax_ctx* c, Mode mode) {
   CK(cudaMemsetAsync(c->pt.p, 0, (size_t)std::max<uint64_t>(maxT, 1) * 4, c->st));
   if (mode == SYNCED && c->noLinks) return TRAX_OK;
   CK(circle_fit(dev_hits(c), triplets(c, maxT), ptr<uint32_t>(c->connIdx), slot(c, S_CONN), maxT, ptr<float>(c->pt),
-                c->st, &c->launches));
+                c->q));
   return TRAX_OK;
 }
 
@@ -710,15 +693,14 @@ int stage_ca(trax_ctx* c, Mode mode) {
   ENSURE(isBest, maxT, 4);
   ENSURE(handlers, maxT + 1, 4);
   CABuffers b = ca_buffers(c);
-  CK(ca_in_degree(ptr<uint32_t>(c->follower), nLinksDev, maxLinks, b, nTDev, maxT, c->st, &c->launches));
+  CK(ca_in_degree(ptr<uint32_t>(c->follower), nLinksDev, maxLinks, b, nTDev, maxT, c->q));
   // in-degree prefix (its total is the number of links; not published)
   if (mode == SYNCED) CK(ensure(c, c->scanScratch, scan_scratch_bytes(maxT + 1)));
   CK(scan_exclusive(b.inStart, b.inStart, c->nT + 1, mode == DEVICE ? nTDev : nullptr, 1, maxT + 1,
-                    c->scanScratch.p, dev_err(c), c->st, &c->launches, true, c->wait));
-  CK(ca_fill(ptr<uint32_t>(c->basis), ptr<uint32_t>(c->follower), nLinksDev, maxLinks, b, nTDev, maxT, c->st,
-             &c->launches));
-  CK(ca_forward(c->cfg, b, nTDev, maxT, c->st, &c->launches));
-  CK(ca_backward(ptr<float>(c->pt), b, nTDev, maxT, nLinksDev, c->st, &c->launches));
+                    c->scanScratch.p, dev_err(c), c->q, true, c->wait));
+  CK(ca_fill(ptr<uint32_t>(c->basis), ptr<uint32_t>(c->follower), nLinksDev, maxLinks, b, nTDev, maxT, c->q));
+  CK(ca_forward(c->cfg, b, nTDev, maxT, c->q));
+  CK(ca_backward(ptr<float>(c->pt), b, nTDev, maxT, nLinksDev, c->q));
   RC(scan_publish(c, mode, b.handlers, c->nT, mode == DEVICE ? nTDev : nullptr, maxT, S_TRACKS,
                   mode == DEVICE ? c->capTracks : NO_CAP));
   uint64_t maxTracks = c->capTracks;
@@ -727,7 +709,7 @@ int stage_ca(trax_ctx* c, Mode mode) {
     maxTracks = c->nTracks;
   }
   ENSURE(tracks, maxTracks, 4);
-  CK(ca_tracks(b, nTDev, maxT, ptr<uint32_t>(c->tracks), maxTracks, dev_err(c), c->st, &c->launches));
+  CK(ca_tracks(b, nTDev, maxT, ptr<uint32_t>(c->tracks), maxTracks, dev_err(c), c->q));
   return TRAX_OK;
 }
 
@@ -748,7 +730,7 @@ int run_stage(trax_ctx* c, int stage) {
     for (bool& u : c->stageUsed) u = false;
     for (bool& u : c->kUsed) u = false;
   }
-  cudaEventRecord(c->stageEv[stage - 1], c->st);
+  mark(c, MARK_STAGE + stage - 1);
   switch (stage) {
     case 1: rc = begin_run(c, false); if (!rc) rc = stage_grid(c, SYNCED); break;
     case 2: rc = stage_pairs(c, SYNCED); break;
@@ -760,7 +742,7 @@ int run_stage(trax_ctx* c, int stage) {
     default: return fail(c, TRAX_ERR_ARG, "unknown stage");
   }
   if (rc) return rc;
-  cudaEventRecord(c->stageEv[stage], c->st);
+  mark(c, MARK_STAGE + stage);  // written by the read-back below, or again as the next stage starts
   c->stageUsed[stage - 1] = true;
   RC(check_device_error(c));
   c->stage = stage;
@@ -777,12 +759,14 @@ int chain_device(trax_ctx* c, bool linking) {
   int (*stages[N_STAGES])(trax_ctx*, Mode) = {stage_grid, stage_pairs, stage_predict, stage_filter,
                                               stage_connectivity, stage_fit, stage_ca};
   const int n = linking ? N_STAGES : 4;
-  CK(record(c, c->stageEv[0]));
+  mark(c, MARK_STAGE);
   for (int s = 0; s < n; ++s) {
     RC(stages[s](c, DEVICE));
-    CK(record(c, c->stageEv[s + 1]));
+    mark(c, MARK_STAGE + s + 1);
     c->stageUsed[s] = true;
   }
+  // the last node: slots and marks to the host
+  CK(slots_to_host(ptr<uint32_t>(c->slots), c->hSlots, SLOT_BYTES / 4, c->q));
   return TRAX_OK;
 }
 
@@ -914,7 +898,7 @@ void fill_stats(trax_ctx* c, trax_batch_stats* s) {
   s->n_track_entries = c->nTracks;
   s->n_pair_sentinels = c->pairSent;
   s->n_candidate_sentinels = c->candSent;
-  s->kernel_launches = c->launches;
+  s->kernel_launches = c->q.launches;
   s->device_ms = c->lastMs;
   s->graph_captures = c->graphCaptures;
 }
@@ -975,8 +959,8 @@ int fit_run(trax_ctx* c, const double* align, bool grad, bool params, bool hitsG
     dH = ptr<double>(c->fitDHits);
   }
   CK(fit_eval(f, grad, dev_hits(c), fit_triplets(c), ptr<uint32_t>(c->fitRows), ptr<double>(c->fitPartials),
-              params ? ptr<float>(c->fitParams) : nullptr, dH, c->st, &c->launches));
-  CK(fit_reduce(f, ptr<double>(c->fitPartials), ptr<double>(c->fitOut), c->st, &c->launches));
+              params ? ptr<float>(c->fitParams) : nullptr, dH, c->st, &c->q.launches));
+  CK(fit_reduce(f, ptr<double>(c->fitPartials), ptr<double>(c->fitOut), c->st, &c->q.launches));
   return TRAX_OK;
 }
 
@@ -994,13 +978,13 @@ int trax_create(trax_ctx** out, int device) {
   c->device = device;
   cudaError_t e = cudaSetDevice(device);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->st, cudaStreamNonBlocking);
-  if (e == cudaSuccess) e = cudaMallocHost(&c->hSlots, sizeof(uint32_t) * 64);
-  if (e == cudaSuccess) e = ensure(c, c->slots, sizeof(uint32_t) * 64);
-  if (e == cudaSuccess) e = cudaMemset(c->slots.p, 0, sizeof(uint32_t) * 64);
+  if (e == cudaSuccess) e = cudaMallocHost(&c->hSlots, SLOT_BYTES);
+  if (e == cudaSuccess) e = ensure(c, c->slots, SLOT_BYTES);
+  if (e == cudaSuccess) e = cudaMemset(c->slots.p, 0, SLOT_BYTES);
   if (e == cudaSuccess) e = cudaEventCreate(&c->ev0);
   if (e == cudaSuccess) e = cudaEventCreate(&c->ev1);
-  for (int i = 0; i <= N_STAGES && e == cudaSuccess; ++i) e = cudaEventCreate(&c->stageEv[i]);
-  for (int i = 0; i < 2 * TK_N && e == cudaSuccess; ++i) e = cudaEventCreate(&c->kEv[i]);
+  c->q.st = c->st;
+  c->q.marks.at = reinterpret_cast<unsigned long long*>(ptr<uint32_t>(c->slots) + SLOT_WORDS);
   if (e == cudaSuccess) e = grid_prepare(device);
   if (e != cudaSuccess) {
     trax_destroy(c);
@@ -1034,10 +1018,6 @@ void trax_destroy(trax_ctx* c) {
   if (c->hSlots) cudaFreeHost(c->hSlots);
   if (c->ev0) cudaEventDestroy(c->ev0);
   if (c->ev1) cudaEventDestroy(c->ev1);
-  for (cudaEvent_t& ev : c->stageEv)
-    if (ev) cudaEventDestroy(ev);
-  for (cudaEvent_t& ev : c->kEv)
-    if (ev) cudaEventDestroy(ev);
   if (c->st) cudaStreamDestroy(c->st);
   delete c;
 }
@@ -1309,7 +1289,7 @@ int trax_set_tracklets(trax_ctx* c, const uint32_t* h1, const uint32_t* h2, cons
   in.det = ptr<uint32_t>(c->in_det);
   in.hid = ptr<uint32_t>(c->in_hid);
   in.evt = ptr<uint32_t>(c->in_evt);
-  CK(identity_hits(in, (uint32_t)nh, dev_hits(c), c->st, &c->launches));
+  CK(identity_hits(in, (uint32_t)nh, dev_hits(c), c->q));
   c->fineBuilt = 0;  // the hit collection is no longer the grid's
   if (n) {
     CK(cudaMemcpyAsync(c->h1.p, h1, n * 4, cudaMemcpyHostToDevice, c->st));
@@ -1319,7 +1299,7 @@ int trax_set_tracklets(trax_ctx* c, const uint32_t* h1, const uint32_t* h2, cons
   c->hSlots[S_TRIPLETS] = (uint32_t)n;
   CK(cudaMemcpyAsync(slot(c, S_TRIPLETS), c->hSlots + S_TRIPLETS, 4, cudaMemcpyHostToDevice, c->st));
   CK(triplet_offsets(c->cfg, dev_hits(c), ptr<uint32_t>(c->h1), slot(c, S_TRIPLETS), n,
-                     ptr<uint32_t>(c->tripOffsets), c->st, &c->launches));
+                     ptr<uint32_t>(c->tripOffsets), c->q));
   c->nPairs = c->nCands = 0;
   c->nT = n;
   c->identityHits = true;
@@ -1384,7 +1364,7 @@ int trax_circle_fit_on(trax_ctx* c, const uint32_t* valid_idx, uint64_t n_valid)
   CK(cudaMemcpyAsync(slot(c, S_USER), c->hSlots + S_USER, 4, cudaMemcpyHostToDevice, c->st));
   CK(cudaMemsetAsync(c->pt.p, 0, (size_t)std::max<uint64_t>(nT, 1) * 4, c->st));
   CK(circle_fit(dev_hits(c), triplets(c, nT), ptr<uint32_t>(c->userIdx), slot(c, S_USER), n_valid,
-                ptr<float>(c->pt), c->st, &c->launches));
+                ptr<float>(c->pt), c->q));
   CK(cudaStreamSynchronize(c->st));
   RC(check_device_error(c));
   c->ptGen = c->tripGen;
@@ -1441,15 +1421,13 @@ int trax_cellular_automaton_on(trax_ctx* c, const uint32_t* basis, const uint32_
   const uint32_t* nLinksDev = slot(c, S_LINKS);
   CABuffers b = ca_buffers(c);
   // states 1, in-degrees, the incoming bases of every follower (ascending)
-  CK(ca_in_degree(ptr<uint32_t>(c->follower), nLinksDev, nL, b, nTDev, nT, c->st, &c->launches));
-  CK(scan_exclusive(b.inStart, b.inStart, nT + 1, nullptr, 0, nT + 1, c->scanScratch.p, dev_err(c), c->st,
-                    &c->launches, true, c->wait));
-  CK(ca_fill(ptr<uint32_t>(c->basis), ptr<uint32_t>(c->follower), nLinksDev, nL, b, nTDev, nT, c->st,
-             &c->launches));
+  CK(ca_in_degree(ptr<uint32_t>(c->follower), nLinksDev, nL, b, nTDev, nT, c->q));
+  CK(scan_exclusive(b.inStart, b.inStart, nT + 1, nullptr, 0, nT + 1, c->scanScratch.p, dev_err(c), c->q, true, c->wait));
+  CK(ca_fill(ptr<uint32_t>(c->basis), ptr<uint32_t>(c->follower), nLinksDev, nL, b, nTDev, nT, c->q));
   // forward phase: the reference's iteration (CellularAutomaton.cpp:37-98),
   // both state buffers starting at 1, swapped without copying; a link set
   // with a cycle never settles and is rejected after nT + 2 iterations
-  CK(fill_u32(ptr<uint32_t>(c->caNext), 1u, (uint32_t)nT, c->st, &c->launches));
+  CK(fill_u32(ptr<uint32_t>(c->caNext), 1u, (uint32_t)nT, c->q));
   uint32_t* cur = ptr<uint32_t>(c->states);
   uint32_t* next = ptr<uint32_t>(c->caNext);
   uint32_t* living = slot(c, S_LIVING);
@@ -1458,8 +1436,7 @@ int trax_cellular_automaton_on(trax_ctx* c, const uint32_t* basis, const uint32_
   do {
     ++iterations;
     CK(cudaMemsetAsync(living, 0, 4, c->st));
-    CK(ca_iteration(ptr<uint32_t>(c->basis), ptr<uint32_t>(c->follower), (uint32_t)nL, cur, next, living, c->st,
-                    &c->launches));
+    CK(ca_iteration(ptr<uint32_t>(c->basis), ptr<uint32_t>(c->follower), (uint32_t)nL, cur, next, living, c->q));
     CK(cudaMemcpyAsync(&alive, living, 4, cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));
     std::swap(cur, next);
@@ -1468,11 +1445,11 @@ int trax_cellular_automaton_on(trax_ctx* c, const uint32_t* basis, const uint32_
   if (cur != ptr<uint32_t>(c->states))
     CK(cudaMemcpyAsync(c->states.p, cur, nT * 4, cudaMemcpyDeviceToDevice, c->st));
   // backward phase, handlers and tracks as in the chain
-  CK(ca_backward(ptr<float>(c->pt), b, nTDev, nT, nLinksDev, c->st, &c->launches));
+  CK(ca_backward(ptr<float>(c->pt), b, nTDev, nT, nLinksDev, c->q));
   RC(scan_publish(c, SYNCED, b.handlers, nT, nullptr, nT, S_TRACKS, NO_CAP));
   RC(read_slot(c, S_TRACKS, &c->nTracks));
   ENSURE(tracks, c->nTracks, 4);
-  CK(ca_tracks(b, nTDev, nT, ptr<uint32_t>(c->tracks), c->nTracks, dev_err(c), c->st, &c->launches));
+  CK(ca_tracks(b, nTDev, nT, ptr<uint32_t>(c->tracks), c->nTracks, dev_err(c), c->q));
   CK(cudaStreamSynchronize(c->st));
   RC(check_device_error(c));
   c->nLinks = nL;
@@ -1494,8 +1471,7 @@ int trax_prefix_sum(trax_ctx* c, uint32_t* data, uint64_t n) {
   if (e == cudaSuccess) e = ensure(c, c->scanScratch, scan_scratch_bytes(n));
   if (e == cudaSuccess) e = cudaMemsetAsync(c->slots.p, 0, 4, c->st);
   if (e == cudaSuccess)
-    e = scan_exclusive(ptr<uint32_t>(tmp), ptr<uint32_t>(tmp), n, nullptr, 0, n, c->scanScratch.p, dev_err(c), c->st,
-                       &c->launches, false, c->wait);  // wraps like PrefixSum's uint arithmetic
+    e = scan_exclusive(ptr<uint32_t>(tmp), ptr<uint32_t>(tmp), n, nullptr, 0, n, c->scanScratch.p, dev_err(c), c->q, false, c->wait);  // wraps like PrefixSum's uint arithmetic
   if (e == cudaSuccess) e = cudaMemcpyAsync(data, tmp.p, n * 4, cudaMemcpyDeviceToHost, c->st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(c->st);
   if (e != cudaSuccess) rc = cuda_fail(c, e, "trax_prefix_sum");
@@ -1522,7 +1498,7 @@ int trax_seed_batch(trax_ctx* c, const trax_batch_opts* opts, trax_batch_stats* 
   const bool linking = opts ? opts->run_linking != 0 : true;
   const bool useGraph = opts ? opts->use_graph != 0 : false;
   if (opts && opts->d_eta_cut > 0.0f) c->dEtaCut = opts->d_eta_cut;
-  c->launches = 0;
+  c->q.launches = 0;
   c->graphCaptures = 0;
   c->identityHits = false;
   c->sortedSegments = true;
@@ -1551,7 +1527,7 @@ int trax_seed_batch(trax_ctx* c, const trax_batch_opts* opts, trax_batch_stats* 
         c->cfg.predKeep = c->keepAuto;
       }
       RC(size_device_buffers(c));
-      c->launches = 0;
+      c->q.launches = 0;
       CK(cudaStreamBeginCapture(c->st, cudaStreamCaptureModeThreadLocal));
       cudaMemsetAsync(c->slots.p, 0, sizeof(uint32_t) * S_N, c->st);
       int rc = chain_device(c, linking);
@@ -1564,18 +1540,18 @@ int trax_seed_batch(trax_ctx* c, const trax_batch_opts* opts, trax_batch_stats* 
       if (e != cudaSuccess) return cuda_fail(c, e, "cudaStreamEndCapture");
       c->graph = g;
       CK(cudaGraphInstantiate(&c->graphExec, g, 0));
-      c->graphLaunches = c->launches;
+      c->graphLaunches = c->q.launches;
       c->graphKey = shape_key(c, linking);
     }
     NvtxRange nvtxReplay("trax.replay");
     CK(cudaEventRecord(c->ev0, c->st));
     CK(cudaGraphLaunch(c->graphExec, c->st));
     CK(cudaEventRecord(c->ev1, c->st));
-    RC(read_slots(c));
+    CK(cudaStreamSynchronize(c->st));  // the graph's last node wrote the slots to the host
     float ms = 0;
     CK(cudaEventElapsedTime(&ms, c->ev0, c->ev1));
     c->lastMs = ms;
-    c->launches = c->graphLaunches;
+    c->q.launches = c->graphLaunches;
     const uint32_t bits = c->hSlots[S_ERR];
     c->nTasks = c->hSlots[S_TASKS];
     c->nPairs = c->hSlots[S_PAIRS];
@@ -1608,17 +1584,12 @@ int trax_seed_batch(trax_ctx* c, const trax_batch_opts* opts, trax_batch_stats* 
 int trax_get_timings(trax_ctx* c, float* stage_ms, float* kernel_ms) {
   if (!c) return TRAX_ERR_ARG;
   CK(cudaStreamSynchronize(c->st));
-  for (int s = 0; s < N_STAGES; ++s) {
-    float ms = -1.0f;
-    if (c->stageUsed[s] && cudaEventElapsedTime(&ms, c->stageEv[s], c->stageEv[s + 1]) != cudaSuccess) ms = -1.0f;
-    if (stage_ms) stage_ms[s] = ms;
-  }
-  for (int k = 0; k < TK_N; ++k) {
-    float ms = -1.0f;
-    if (c->kUsed[k] && cudaEventElapsedTime(&ms, c->kEv[2 * k], c->kEv[2 * k + 1]) != cudaSuccess) ms = -1.0f;
-    if (kernel_ms) kernel_ms[k] = ms;
-  }
-  cudaGetLastError();  // clear a "not ready"/"invalid handle" from unused events
+  const unsigned long long* at = reinterpret_cast<const unsigned long long*>(c->hSlots + SLOT_WORDS);
+  auto between = [at](int a, int b) { return (float)((double)(at[b] - at[a]) * 1e-6); };
+  for (int s = 0; s < N_STAGES; ++s)
+    if (stage_ms) stage_ms[s] = c->stageUsed[s] ? between(MARK_STAGE + s, MARK_STAGE + s + 1) : -1.0f;
+  for (int k = 0; k < TK_N; ++k)
+    if (kernel_ms) kernel_ms[k] = c->kUsed[k] ? between(MARK_KERNEL + 2 * k, MARK_KERNEL + 2 * k + 1) : -1.0f;
   return TRAX_OK;
 }
 
@@ -1718,9 +1689,9 @@ int trax_physics_tracks_device(trax_ctx* c, uint64_t total_tracks, trax_track_me
   const uint32_t* off = ptr<uint32_t>(c->handlers);
   CK(track_sizes(off, nT, isTrack, hitsOf, c->st));
   CK(scan_exclusive(isTrack, isTrack, (uint64_t)nT + 1, nullptr, 0, (uint64_t)nT + 1, c->scanScratch.p, dev_err(c),
-                    c->st, nullptr, true, c->wait));
+                    c->q, true, c->wait));
   CK(scan_exclusive(hitsOf, hitsOf, (uint64_t)nT + 1, nullptr, 0, (uint64_t)nT + 1, c->scanScratch.p, dev_err(c),
-                    c->st, nullptr, true, c->wait));
+                    c->q, true, c->wait));
   uint32_t totals[2];
   CK(cudaMemcpyAsync(&totals[0], isTrack + nT, 4, cudaMemcpyDeviceToHost, c->st));
   CK(cudaMemcpyAsync(&totals[1], hitsOf + nT, 4, cudaMemcpyDeviceToHost, c->st));
@@ -1763,7 +1734,7 @@ int trax_physics_tracks_device(trax_ctx* c, uint64_t total_tracks, trax_track_me
   if (!stable) return fail(c, TRAX_ERR_TIMEOUT, "track components did not settle in 64 rounds");
   CK(track_members(t, nTracks, false, c->st));
   CK(scan_exclusive(t.compSize, t.compStart, (uint64_t)nTracks + 1, nullptr, 0, (uint64_t)nTracks + 1,
-                    c->scanScratch.p, dev_err(c), c->st, nullptr, true, c->wait));
+                    c->scanScratch.p, dev_err(c), c->q, true, c->wait));
   CK(track_members(t, nTracks, true, c->st));
   unsigned long long* counts = ptr<unsigned long long>(c->trk_counts);
   CK(track_greedy(t, nTracks, ptr<unsigned long long>(c->trk_table), tableSize - 1, counts, c->st));
@@ -1862,10 +1833,9 @@ int trax_fit_prepare(trax_ctx* c, const trax_fit_opts* opts, uint64_t* n_fit) {
   CK(ensure(c, c->fitSegDelta, (size_t)S * 4));
   CK(cudaMemsetAsync(c->fitSegCnt.p, 0, (size_t)S * 4, c->st));
   uint32_t* ok = ptr<uint32_t>(c->fitOk);
-  CK(fit_select(f, c->cfg, dev_hits(c), fit_triplets(c), nT, truthOnly, ok, ptr<uint32_t>(c->fitSegCnt), c->st,
-                &c->launches));
+  CK(fit_select(f, c->cfg, dev_hits(c), fit_triplets(c), nT, truthOnly, ok, ptr<uint32_t>(c->fitSegCnt), c->st, &c->q.launches));
   CK(ensure(c, c->scanScratch, scan_scratch_bytes(nT + 1)));
-  CK(scan_exclusive(ok, ok, nT + 1, nullptr, 0, nT + 1, c->scanScratch.p, dev_err(c), c->st, &c->launches, true,
+  CK(scan_exclusive(ok, ok, nT + 1, nullptr, 0, nT + 1, c->scanScratch.p, dev_err(c), c->q, true,
                     c->wait));
   // 2. rows ordered by layer triplet, then by event (segment order inside a layer triplet)
   std::vector<uint32_t> cnt(S);
@@ -1902,7 +1872,7 @@ int trax_fit_prepare(trax_ctx* c, const trax_fit_opts* opts, uint64_t* n_fit) {
   if (S) CK(cudaMemcpyAsync(c->fitSegDelta.p, delta.data(), (size_t)S * 4, cudaMemcpyHostToDevice, c->st));
   CK(ensure(c, c->fitRows, std::max<uint64_t>(c->nFit, 1) * 4));
   CK(fit_scatter(c->cfg, dev_hits(c), fit_triplets(c), nT, ok, ptr<int32_t>(c->fitSegDelta),
-                 ptr<uint32_t>(c->fitRows), c->st, &c->launches));
+                 ptr<uint32_t>(c->fitRows), c->st, &c->q.launches));
   // 3. sigma_tip per layer triplet: given, or 1.4826 x median |d0| at zero alignment
   bool needD0 = false;
   for (uint32_t k = 0; k < f.nLT; ++k) {
@@ -1965,8 +1935,7 @@ int trax_fit_backward(trax_ctx* c, const double* align, double* chi2, double* d_
   CK(cudaMemcpyAsync(out.data(), c->fitOut.p, out.size() * sizeof(double), cudaMemcpyDeviceToHost, c->st));
   if (d_hits && c->nHits) {
     CK(ensure(c, c->fitDHitsF, (size_t)c->nHits * 3 * sizeof(float)));
-    CK(fit_hits_out(ptr<double>(c->fitDHits), ptr<uint32_t>(c->porig), c->nHits, ptr<float>(c->fitDHitsF), c->st,
-                    &c->launches));
+    CK(fit_hits_out(ptr<double>(c->fitDHits), ptr<uint32_t>(c->porig), c->nHits, ptr<float>(c->fitDHitsF), c->st, &c->q.launches));
     CK(cudaMemcpyAsync(d_hits, c->fitDHitsF.p, (size_t)c->nHits * 3 * sizeof(float), cudaMemcpyDeviceToHost,
                        c->st));
   }
@@ -1986,7 +1955,7 @@ int trax_apply_alignment(trax_ctx* c, const double* align) {
   c->fitCfg.L = c->L;
   RC(fit_set_alignment(c, align));
   CK(fit_apply(c->fitCfg, ptr<float>(c->in_x), ptr<float>(c->in_y), ptr<float>(c->in_z), ptr<uint32_t>(c->in_layer),
-               c->nHits, c->st, &c->launches));
+               c->nHits, c->st, &c->q.launches));
   CK(cudaStreamSynchronize(c->st));
   c->stage = 0;  // every stage output refers to the old positions
   c->fitReady = false;

@@ -90,8 +90,9 @@ __device__ __forceinline__ void cta_place_stable(uint32_t* cnt, uint32_t C, cons
 // counters when the layer has at most maxHits hits (the room the launch
 // gave them), otherwise in the global scratch arrays.
 __global__ void __launch_bounds__(GRID_THREADS)
-    grid_kernel(DevConfig cfg, GridInput in, uint32_t* __restrict__ grid, DevHits out, GridScratch sc,
+    grid_kernel(Stamp stamp, DevConfig cfg, GridInput in, uint32_t* __restrict__ grid, DevHits out, GridScratch sc,
                 uint32_t* err, int useSmem, uint32_t maxHits) {
+  stamp_begin(stamp);
   extern __shared__ uint32_t smem[];
   __shared__ uint32_t s_warpSum[GRID_WARPS];
   const uint32_t task = blockIdx.x;  // event * L + layer
@@ -171,8 +172,9 @@ __global__ void __launch_bounds__(GRID_THREADS)
 __device__ __forceinline__ uint32_t half_of(uint32_t word, uint32_t c) { return (word >> ((c & 1u) * 16u)) & 0xffffu; }
 
 __global__ void __launch_bounds__(GRID_THREADS)
-    grid_kernel16(DevConfig cfg, GridInput in, uint32_t* __restrict__ grid, DevHits out, GridScratch sc,
+    grid_kernel16(Stamp stamp, DevConfig cfg, GridInput in, uint32_t* __restrict__ grid, DevHits out, GridScratch sc,
                   uint32_t* err, uint32_t maxHits) {
+  stamp_begin(stamp);
   extern __shared__ uint32_t smem[];
   __shared__ uint32_t s_warpSum[GRID_WARPS];
   const uint32_t task = blockIdx.x;  // event * L + layer
@@ -350,8 +352,9 @@ __device__ __forceinline__ uint32_t fine_cell(const DevConfig& cfg, float4 h, ui
 }
 
 __global__ void __launch_bounds__(GRID_THREADS)
-    fine_grid_kernel(DevConfig cfg, const uint32_t* __restrict__ grid, const float4* __restrict__ xyzp,
+    fine_grid_kernel(Stamp stamp, DevConfig cfg, const uint32_t* __restrict__ grid, const float4* __restrict__ xyzp,
                      FineGrid fine, uint32_t* gcnt, uint32_t warpsPerBlock) {
+  stamp_begin(stamp);
   extern __shared__ uint32_t smem[];
   const uint32_t lane = threadIdx.x & 31u, wib = threadIdx.x >> 5;
   const uint32_t nZ = cfg.nZ, nP1 = cfg.nP + 1;
@@ -411,7 +414,8 @@ __global__ void __launch_bounds__(GRID_THREADS)
 
 // The uploaded hits taken as the hit collection as they are (identity
 // order), for the linking stages run on caller-provided triplets.
-__global__ void identity_hits_kernel(GridInput in, uint32_t n, DevHits out) {
+__global__ void identity_hits_kernel(Stamp stamp, GridInput in, uint32_t n, DevHits out) {
+  stamp_begin(stamp);
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const float x = in.x[i], y = in.y[i], z = in.z[i];
     out.x[i] = x;
@@ -428,10 +432,9 @@ __global__ void identity_hits_kernel(GridInput in, uint32_t n, DevHits out) {
 
 }  // namespace
 
-cudaError_t identity_hits(const GridInput& in, uint32_t n, DevHits out, cudaStream_t st, uint32_t* launches) {
+cudaError_t identity_hits(const GridInput& in, uint32_t n, DevHits out, Queue& q) {
   if (n == 0) return cudaSuccess;
-  identity_hits_kernel<<<(n + 255) / 256 < 4096 ? (n + 255) / 256 : 4096, 256, 0, st>>>(in, n, out);
-  if (launches) *launches += 1;
+  launch(q, identity_hits_kernel, (n + 255) / 256 < 4096 ? (n + 255) / 256 : 4096, 256, 0, in, n, out);
   return cudaGetLastError();
 }
 
@@ -444,7 +447,7 @@ cudaError_t grid_prepare(int) {
 }
 
 cudaError_t grid_build(const DevConfig& cfg, const GridInput& in, uint32_t* grid, DevHits out, GridScratch sc,
-                       uint32_t maxLayerHits, uint32_t* err, cudaStream_t st, uint32_t* launches) {
+                       uint32_t maxLayerHits, uint32_t* err, Queue& q) {
   const uint32_t tasks = cfg.E * cfg.L;
   if (tasks == 0) return cudaSuccess;
   const int useSmem = cfg.C <= GRID_SMEM_CELLS ? 1 : 0;
@@ -453,19 +456,17 @@ cudaError_t grid_build(const DevConfig& cfg, const GridInput& in, uint32_t* grid
   // 16-bit counters, cells and slots when every index fits
   const size_t bytes16 = (size_t)maxLayerHits * 8 + (size_t)(cfg.C + 1) / 2 * 4;
   if (useSmem && cfg.C < 65536u && maxLayerHits < 65536u && bytes16 <= GRID_SMEM_MAX) {
-    grid_kernel16<<<tasks, GRID_THREADS, bytes16, st>>>(cfg, in, grid, out, sc, err, maxLayerHits);
-    if (launches) *launches += 1;
+    launch(q, grid_kernel16, tasks, GRID_THREADS, bytes16, cfg, in, grid, out, sc, err, maxLayerHits);
     return cudaGetLastError();
   }
   const bool hitsFit = useSmem && counterBytes + hitBytes <= GRID_SMEM_MAX;
-  grid_kernel<<<tasks, GRID_THREADS, counterBytes + (hitsFit ? hitBytes : 0), st>>>(
-      cfg, in, grid, out, sc, err, useSmem, hitsFit ? maxLayerHits : 0u);
-  if (launches) *launches += 1;
+  launch(q, grid_kernel, tasks, GRID_THREADS, counterBytes + (hitsFit ? hitBytes : 0), cfg, in, grid, out, sc, err,
+         useSmem, hitsFit ? maxLayerHits : 0u);
   return cudaGetLastError();
 }
 
 cudaError_t fine_grid_build(const DevConfig& cfg, const uint32_t* grid, const float4* xyzp, FineGrid fine,
-                            uint32_t* counters, cudaStream_t st, uint32_t* launches) {
+                            uint32_t* counters, Queue& q) {
   const uint64_t tasks = (uint64_t)cfg.E * cfg.L * cfg.nZ;
   if (tasks == 0 || cfg.fineRows == 0) return cudaSuccess;
   const size_t rowBytes = (size_t)fine_row_cells(cfg) * sizeof(uint32_t);
@@ -473,9 +474,8 @@ cudaError_t fine_grid_build(const DevConfig& cfg, const uint32_t* grid, const fl
   const bool inSmem = wpb > 0;
   if (!inSmem) wpb = GRID_WARPS;
   const uint64_t blocks = (tasks + wpb - 1) / wpb;
-  fine_grid_kernel<<<(unsigned)blocks, wpb * 32, inSmem ? wpb * rowBytes : 0, st>>>(cfg, grid, xyzp, fine,
-                                                                                     inSmem ? nullptr : counters, wpb);
-  if (launches) *launches += 1;
+  launch(q, fine_grid_kernel, (unsigned)blocks, wpb * 32, inSmem ? wpb * rowBytes : 0, cfg, grid, xyzp, fine,
+         inSmem ? nullptr : counters, wpb);
   return cudaGetLastError();
 }
 

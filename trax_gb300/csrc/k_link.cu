@@ -41,9 +41,10 @@ int grid_for(uint64_t items, int threads) {
 
 #define GRID_STRIDE(i, n) for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < (n); i += gridDim.x * blockDim.x)
 
-__global__ void eta_kernel(DevConfig cfg, const float4* __restrict__ hits, const uint32_t* __restrict__ hitEvt,
+__global__ void eta_kernel(Stamp stamp, DevConfig cfg, const float4* __restrict__ hits, const uint32_t* __restrict__ hitEvt,
                            const uint32_t* __restrict__ hitLayer, const uint32_t* __restrict__ h1,
                            const uint32_t* __restrict__ h3, const uint32_t* nTDev, float* eta, uint32_t* seg) {
+  stamp_begin(stamp);
   const uint32_t nT = *nTDev;
   GRID_STRIDE(t, nT) {
     const uint32_t hi = trax_hit(h1[t], cfg), ho = trax_hit(h3[t], cfg);
@@ -56,8 +57,9 @@ __global__ void eta_kernel(DevConfig cfg, const float4* __restrict__ hits, const
 }
 
 // segStart[s] = first triplet of segment s (lower bound of s in seg[])
-__global__ void seg_bounds_kernel(DevConfig cfg, const uint32_t* __restrict__ seg, const uint32_t* nTDev,
+__global__ void seg_bounds_kernel(Stamp stamp, DevConfig cfg, const uint32_t* __restrict__ seg, const uint32_t* nTDev,
                                   uint32_t* segStart) {
+  stamp_begin(stamp);
   const uint32_t nT = *nTDev;
   const uint32_t S = cfg.E * cfg.nLT;
   GRID_STRIDE(s, S + 1) {
@@ -85,11 +87,12 @@ __device__ __forceinline__ uint32_t key_lower_bound(const uint32_t* h1, const ui
 
 template <bool EMIT>
 __global__ void __launch_bounds__(256)
-    conn_kernel(DevConfig cfg, const uint32_t* __restrict__ hitEvt, const uint32_t* __restrict__ hitLayer,
+    conn_kernel(Stamp stamp, DevConfig cfg, const uint32_t* __restrict__ hitEvt, const uint32_t* __restrict__ hitLayer,
                 const uint32_t* __restrict__ h1, const uint32_t* __restrict__ h2, const uint32_t* __restrict__ h3,
                 const uint32_t* nTDev, const float* __restrict__ eta, const uint32_t* __restrict__ offsets,
                 const uint32_t* __restrict__ segStart, uint32_t* linkCount, uint32_t* flags, uint32_t* runStart,
                 uint32_t* basis, uint32_t* follower, uint32_t capLinks, bool sortedSegments) {
+  stamp_begin(stamp);
   const uint32_t S = cfg.E * cfg.nLT;
   const uint32_t nT = S > 0 ? *nTDev : 0u;
   const float dEtaCut = cfg.dEtaCut;
@@ -165,8 +168,9 @@ __global__ void __launch_bounds__(256)
 // flags: connectable (flag set) and non-connectable (flag clear), with the
 // number set in each word (+1 slots zeroed; the number of words to
 // *nWordsOut), so that the two compactions scan one value per 32 triplets.
-__global__ void conn_words_kernel(const uint32_t* __restrict__ flags, const uint32_t* nTDev, uint32_t* connWords,
+__global__ void conn_words_kernel(Stamp stamp, const uint32_t* __restrict__ flags, const uint32_t* nTDev, uint32_t* connWords,
                                   uint32_t* connSums, uint32_t* nonWords, uint32_t* nonSums, uint32_t* nWordsOut) {
+  stamp_begin(stamp);
   const uint32_t nT = *nTDev;
   const uint32_t lane = threadIdx.x & 31u;
   for (uint32_t base = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); base < nT; base += gridDim.x * blockDim.x) {
@@ -190,8 +194,9 @@ __global__ void conn_words_kernel(const uint32_t* __restrict__ flags, const uint
 }
 
 // out[wordStart[k / 32] + (bits below k in its word)] = k for every set bit
-__global__ void compact_words_kernel(const uint32_t* __restrict__ words, const uint32_t* __restrict__ wordStart,
+__global__ void compact_words_kernel(Stamp stamp, const uint32_t* __restrict__ words, const uint32_t* __restrict__ wordStart,
                                      const uint32_t* nTDev, uint32_t* out, uint32_t capOut) {
+  stamp_begin(stamp);
   const uint32_t nT = *nTDev;
   GRID_STRIDE(k, nT) {
     const uint32_t w = words[k >> 5], bit = k & 31u;
@@ -202,9 +207,10 @@ __global__ void compact_words_kernel(const uint32_t* __restrict__ words, const u
   }
 }
 
-__global__ void circle_fit_kernel(const float4* __restrict__ hits, const uint32_t* __restrict__ h1,
+__global__ void circle_fit_kernel(Stamp stamp, const float4* __restrict__ hits, const uint32_t* __restrict__ h1,
                                   const uint32_t* __restrict__ h2, const uint32_t* __restrict__ h3,
                                   const uint32_t* __restrict__ conn, const uint32_t* nConnDev, float* pt) {
+  stamp_begin(stamp);
   const uint32_t n = *nConnDev;
   GRID_STRIDE(j, n) {
     const uint32_t t = conn[j];
@@ -220,7 +226,8 @@ __global__ void circle_fit_kernel(const float4* __restrict__ hits, const uint32_
   }
 }
 
-__global__ void in_degree_kernel(const uint32_t* __restrict__ follower, const uint32_t* nLinksDev, uint32_t* inDeg) {
+__global__ void in_degree_kernel(Stamp stamp, const uint32_t* __restrict__ follower, const uint32_t* nLinksDev, uint32_t* inDeg) {
+  stamp_begin(stamp);
   const uint32_t n = *nLinksDev;
   GRID_STRIDE(p, n) atomicAdd(&inDeg[follower[p]], 1u);
 }
@@ -228,9 +235,10 @@ __global__ void in_degree_kernel(const uint32_t* __restrict__ follower, const ui
 // The bases of each follower's incoming links.  Links are stored in basis
 // order, so the bases of one follower (all distinct) sort like the link
 // indices do.
-__global__ void in_fill_kernel(const uint32_t* __restrict__ basis, const uint32_t* __restrict__ follower,
+__global__ void in_fill_kernel(Stamp stamp, const uint32_t* __restrict__ basis, const uint32_t* __restrict__ follower,
                                const uint32_t* nLinksDev, const uint32_t* __restrict__ inStart, uint32_t* cursor,
                                uint32_t* inList) {
+  stamp_begin(stamp);
   const uint32_t n = *nLinksDev;
   GRID_STRIDE(p, n) {
     const uint32_t f = follower[p];
@@ -240,7 +248,8 @@ __global__ void in_fill_kernel(const uint32_t* __restrict__ basis, const uint32_
 
 // the incoming bases of each follower in ascending order, which is the
 // order of their links (insertion sort; lists are short)
-__global__ void in_sort_kernel(const uint32_t* __restrict__ inStart, const uint32_t* nTDev, uint32_t* inList) {
+__global__ void in_sort_kernel(Stamp stamp, const uint32_t* __restrict__ inStart, const uint32_t* nTDev, uint32_t* inList) {
+  stamp_begin(stamp);
   const uint32_t nT = *nTDev;
   GRID_STRIDE(t, nT) {
     const uint32_t a = inStart[t], b = inStart[t + 1];
@@ -258,7 +267,8 @@ __global__ void in_sort_kernel(const uint32_t* __restrict__ inStart, const uint3
 
 // the CA's per-triplet state before a run: in-degrees and cursors 0,
 // states 1, no best basis
-__global__ void ca_init_kernel(CABuffers b, const uint32_t* nTDev) {
+__global__ void ca_init_kernel(Stamp stamp, CABuffers b, const uint32_t* nTDev) {
+  stamp_begin(stamp);
   const uint32_t nT = *nTDev;
   GRID_STRIDE(i, nT + 1) {
     b.inStart[i] = 0u;
@@ -272,9 +282,10 @@ __global__ void ca_init_kernel(CABuffers b, const uint32_t* nTDev) {
 }
 
 // one layer-triplet level of the forward phase
-__global__ void ca_level_kernel(DevConfig cfg, uint32_t level, const uint32_t* __restrict__ segOf,
+__global__ void ca_level_kernel(Stamp stamp, DevConfig cfg, uint32_t level, const uint32_t* __restrict__ segOf,
                                 const uint32_t* __restrict__ inStart, const uint32_t* __restrict__ inList,
                                 const uint32_t* nTDev, uint32_t* states) {
+  stamp_begin(stamp);
   const uint32_t nT = *nTDev;
   GRID_STRIDE(t, nT) {
     if (segOf[t] % cfg.nLT != level) continue;
@@ -293,9 +304,10 @@ __global__ void ca_level_kernel(DevConfig cfg, uint32_t level, const uint32_t* _
 // copying (CellularAutomaton.cpp:52-98), until no cell lives.  Used for
 // caller-provided links, which need not go from one layer triplet to the
 // next as the chain's own do.
-__global__ void ca_iteration_kernel(const uint32_t* __restrict__ basis, const uint32_t* __restrict__ follower,
+__global__ void ca_iteration_kernel(Stamp stamp, const uint32_t* __restrict__ basis, const uint32_t* __restrict__ follower,
                                     uint32_t nLinks, const uint32_t* __restrict__ cur, uint32_t* next,
                                     uint32_t* living) {
+  stamp_begin(stamp);
   GRID_STRIDE(p, nLinks) {
     const uint32_t f = follower[p];
     const uint32_t fs = cur[f];
@@ -305,15 +317,17 @@ __global__ void ca_iteration_kernel(const uint32_t* __restrict__ basis, const ui
   }
 }
 
-__global__ void fill_u32_kernel(uint32_t* p, uint32_t v, uint32_t n) {
+__global__ void fill_u32_kernel(Stamp stamp, uint32_t* p, uint32_t v, uint32_t n) {
+  stamp_begin(stamp);
   GRID_STRIDE(i, n) p[i] = v;
 }
 
 // followerBestBasisStore semantics (CellularAutomaton.h:212-263)
-__global__ void ca_best_kernel(const float* __restrict__ pt,
+__global__ void ca_best_kernel(Stamp stamp, const float* __restrict__ pt,
                                const uint32_t* __restrict__ inStart, const uint32_t* __restrict__ inList,
                                const uint32_t* __restrict__ states, const uint32_t* nTDev, uint32_t* best,
                                uint32_t* isBest) {
+  stamp_begin(stamp);
   const uint32_t nT = *nTDev;
   GRID_STRIDE(t, nT) {
     const uint32_t a = inStart[t], b = inStart[t + 1];
@@ -344,15 +358,17 @@ __global__ void ca_best_kernel(const float* __restrict__ pt,
 
 // handlersStateStore (CellularAutomaton.h:270-288); no tracks at all when
 // there are no links (the reference skips the CA, TripletBuilder.cpp:414-421)
-__global__ void handlers_kernel(const uint32_t* __restrict__ states, const uint32_t* __restrict__ isBest,
+__global__ void handlers_kernel(Stamp stamp, const uint32_t* __restrict__ states, const uint32_t* __restrict__ isBest,
                                 const uint32_t* nTDev, const uint32_t* nLinksDev, uint32_t* handlers) {
+  stamp_begin(stamp);
   const uint32_t nT = *nTDev;
   const bool any = *nLinksDev != 0u;
   GRID_STRIDE(t, nT + 1) handlers[t] = (any && t < nT) ? (isBest[t] == 0u) * states[t] : 0u;
 }
 
-__global__ void tracks_kernel(const uint32_t* __restrict__ handlers, const uint32_t* __restrict__ best,
+__global__ void tracks_kernel(Stamp stamp, const uint32_t* __restrict__ handlers, const uint32_t* __restrict__ best,
                               const uint32_t* nTDev, uint32_t* tracks, uint64_t maxTracks, uint32_t* err) {
+  stamp_begin(stamp);
   const uint32_t nT = *nTDev;
   GRID_STRIDE(t, nT) {
     const uint32_t off = handlers[t];
@@ -371,127 +387,110 @@ __global__ void tracks_kernel(const uint32_t* __restrict__ handlers, const uint3
 
 }  // namespace
 
-cudaError_t triplet_eta(const DevConfig& cfg, DevHits hits, TripletView t, float* eta, uint32_t* seg, cudaStream_t st,
-                        uint32_t* launches) {
+cudaError_t triplet_eta(const DevConfig& cfg, DevHits hits, TripletView t, float* eta, uint32_t* seg, Queue& q) {
   if (t.maxN == 0) return cudaSuccess;
-  eta_kernel<<<grid_for(t.maxN, 256), 256, 0, st>>>(cfg, hits.xyzp, hits.evt, hits.layer, t.h1, t.h3, t.nDev, eta,
-                                                    seg);
-  if (launches) *launches += 1;
+  launch(q, eta_kernel, grid_for(t.maxN, 256), 256, 0, cfg, hits.xyzp, hits.evt, hits.layer, t.h1, t.h3, t.nDev,
+         eta, seg);
   return cudaGetLastError();
 }
 
 cudaError_t segment_bounds(const DevConfig& cfg, const uint32_t* seg, const uint32_t* nTDev, uint32_t* segStart,
-                           cudaStream_t st, uint32_t* launches) {
+                           Queue& q) {
   const uint32_t S = cfg.E * cfg.nLT;
-  seg_bounds_kernel<<<grid_for(S + 1, 256), 256, 0, st>>>(cfg, seg, nTDev, segStart);
-  if (launches) *launches += 1;
+  launch(q, seg_bounds_kernel, grid_for(S + 1, 256), 256, 0, cfg, seg, nTDev, segStart);
   return cudaGetLastError();
 }
 
 cudaError_t connectivity_tasks(const DevConfig& cfg, bool emit, DevHits hits, TripletView t, const float* eta,
                                const uint32_t* offsets, const uint32_t* segStart, uint32_t* linkCount,
                                uint32_t* flags, uint32_t* runStart, uint32_t* basis, uint32_t* follower,
-                               uint64_t capLinks, bool sortedSegments, cudaStream_t st, uint32_t* launches) {
+                               uint64_t capLinks, bool sortedSegments, Queue& q) {
   const int blocks = grid_for(t.maxN + 1, 256);
   const uint32_t cap = capLinks > 0xffffffffull ? 0xffffffffu : (uint32_t)capLinks;
   if (emit)
-    conn_kernel<true><<<blocks, 256, 0, st>>>(cfg, hits.evt, hits.layer, t.h1, t.h2, t.h3, t.nDev, eta, offsets,
-                                              segStart, linkCount, flags, runStart, basis, follower, cap,
-                                              sortedSegments);
+    launch(q, conn_kernel<true>, blocks, 256, 0, cfg, hits.evt, hits.layer, t.h1, t.h2, t.h3, t.nDev, eta, offsets,
+           segStart, linkCount, flags, runStart, basis, follower, cap, sortedSegments);
   else
-    conn_kernel<false><<<blocks, 256, 0, st>>>(cfg, hits.evt, hits.layer, t.h1, t.h2, t.h3, t.nDev, eta, offsets,
-                                               segStart, linkCount, flags, runStart, basis, follower, cap,
-                                               sortedSegments);
-  if (launches) *launches += 1;
+    launch(q, conn_kernel<false>, blocks, 256, 0, cfg, hits.evt, hits.layer, t.h1, t.h2, t.h3, t.nDev, eta, offsets,
+           segStart, linkCount, flags, runStart, basis, follower, cap, sortedSegments);
   return cudaGetLastError();
 }
 
 cudaError_t connectable_words(const uint32_t* flags, const uint32_t* nTDev, uint64_t maxT, uint32_t* connWords,
                               uint32_t* connSums, uint32_t* nonWords, uint32_t* nonSums, uint32_t* nWordsOut,
-                              cudaStream_t st, uint32_t* launches) {
-  conn_words_kernel<<<grid_for(maxT + 1, 256), 256, 0, st>>>(flags, nTDev, connWords, connSums, nonWords, nonSums,
-                                                             nWordsOut);
-  if (launches) *launches += 1;
+                              Queue& q) {
+  launch(q, conn_words_kernel, grid_for(maxT + 1, 256), 256, 0, flags, nTDev, connWords, connSums, nonWords,
+         nonSums, nWordsOut);
   return cudaGetLastError();
 }
 
 cudaError_t compact_words(const uint32_t* words, const uint32_t* wordStart, const uint32_t* nTDev, uint64_t maxT,
-                          uint32_t* outIdx, uint64_t capOut, cudaStream_t st, uint32_t* launches) {
+                          uint32_t* outIdx, uint64_t capOut, Queue& q) {
   if (maxT == 0) return cudaSuccess;
   const uint32_t cap = capOut > 0xffffffffull ? 0xffffffffu : (uint32_t)capOut;
-  compact_words_kernel<<<grid_for(maxT, 256), 256, 0, st>>>(words, wordStart, nTDev, outIdx, cap);
-  if (launches) *launches += 1;
+  launch(q, compact_words_kernel, grid_for(maxT, 256), 256, 0, words, wordStart, nTDev, outIdx, cap);
   return cudaGetLastError();
 }
 
 cudaError_t circle_fit(DevHits hits, TripletView t, const uint32_t* connectable, const uint32_t* nConnDev,
-                       uint64_t maxConn, float* pt, cudaStream_t st, uint32_t* launches) {
+                       uint64_t maxConn, float* pt, Queue& q) {
   if (maxConn == 0) return cudaSuccess;
-  circle_fit_kernel<<<grid_for(maxConn, 256), 256, 0, st>>>(hits.xyzp, t.h1, t.h2, t.h3, connectable, nConnDev, pt);
-  if (launches) *launches += 1;
+  launch(q, circle_fit_kernel, grid_for(maxConn, 256), 256, 0, hits.xyzp, t.h1, t.h2, t.h3, connectable, nConnDev,
+         pt);
   return cudaGetLastError();
 }
 
 cudaError_t ca_in_degree(const uint32_t* follower, const uint32_t* nLinksDev, uint64_t maxLinks, CABuffers b,
-                         const uint32_t* nTDev, uint64_t maxT, cudaStream_t st, uint32_t* launches) {
-  ca_init_kernel<<<grid_for(maxT + 1, 256), 256, 0, st>>>(b, nTDev);
-  if (launches) *launches += 1;
+                         const uint32_t* nTDev, uint64_t maxT, Queue& q) {
+  launch(q, ca_init_kernel, grid_for(maxT + 1, 256), 256, 0, b, nTDev);
   if (maxLinks > 0) {
-    in_degree_kernel<<<grid_for(maxLinks, 256), 256, 0, st>>>(follower, nLinksDev, b.inStart);
-    if (launches) *launches += 1;
+    launch(q, in_degree_kernel, grid_for(maxLinks, 256), 256, 0, follower, nLinksDev, b.inStart);
   }
   return cudaGetLastError();
 }
 
 cudaError_t ca_fill(const uint32_t* basis, const uint32_t* follower, const uint32_t* nLinksDev, uint64_t maxLinks,
-                    CABuffers b, const uint32_t* nTDev, uint64_t maxT, cudaStream_t st, uint32_t* launches) {
+                    CABuffers b, const uint32_t* nTDev, uint64_t maxT, Queue& q) {
   if (maxLinks > 0) {
-    in_fill_kernel<<<grid_for(maxLinks, 256), 256, 0, st>>>(basis, follower, nLinksDev, b.inStart, b.inCursor,
-                                                            b.inList);
-    if (launches) *launches += 1;
+    launch(q, in_fill_kernel, grid_for(maxLinks, 256), 256, 0, basis, follower, nLinksDev, b.inStart, b.inCursor,
+           b.inList);
   }
-  in_sort_kernel<<<grid_for(maxT, 256), 256, 0, st>>>(b.inStart, nTDev, b.inList);
-  if (launches) *launches += 1;
+  launch(q, in_sort_kernel, grid_for(maxT, 256), 256, 0, b.inStart, nTDev, b.inList);
   return cudaGetLastError();
 }
 
-cudaError_t ca_forward(const DevConfig& cfg, CABuffers b, const uint32_t* nTDev, uint64_t maxT, cudaStream_t st,
-                       uint32_t* launches) {
+cudaError_t ca_forward(const DevConfig& cfg, CABuffers b, const uint32_t* nTDev, uint64_t maxT, Queue& q) {
   for (uint32_t level = 1; level < cfg.nLT; ++level) {
-    ca_level_kernel<<<grid_for(maxT, 256), 256, 0, st>>>(cfg, level, b.segOf, b.inStart, b.inList, nTDev, b.states);
-    if (launches) *launches += 1;
+    launch(q, ca_level_kernel, grid_for(maxT, 256), 256, 0, cfg, level, b.segOf, b.inStart, b.inList, nTDev,
+           b.states);
   }
   return cudaGetLastError();
 }
 
 cudaError_t ca_iteration(const uint32_t* basis, const uint32_t* follower, uint32_t nLinks, const uint32_t* cur,
-                         uint32_t* next, uint32_t* living, cudaStream_t st, uint32_t* launches) {
+                         uint32_t* next, uint32_t* living, Queue& q) {
   if (nLinks == 0) return cudaSuccess;
-  ca_iteration_kernel<<<grid_for(nLinks, 256), 256, 0, st>>>(basis, follower, nLinks, cur, next, living);
-  if (launches) *launches += 1;
+  launch(q, ca_iteration_kernel, grid_for(nLinks, 256), 256, 0, basis, follower, nLinks, cur, next, living);
   return cudaGetLastError();
 }
 
-cudaError_t fill_u32(uint32_t* p, uint32_t v, uint32_t n, cudaStream_t st, uint32_t* launches) {
+cudaError_t fill_u32(uint32_t* p, uint32_t v, uint32_t n, Queue& q) {
   if (n == 0) return cudaSuccess;
-  fill_u32_kernel<<<grid_for(n, 256), 256, 0, st>>>(p, v, n);
-  if (launches) *launches += 1;
+  launch(q, fill_u32_kernel, grid_for(n, 256), 256, 0, p, v, n);
   return cudaGetLastError();
 }
 
 cudaError_t ca_backward(const float* pt, CABuffers b, const uint32_t* nTDev, uint64_t maxT,
-                        const uint32_t* nLinksDev, cudaStream_t st, uint32_t* launches) {
-  ca_best_kernel<<<grid_for(maxT, 256), 256, 0, st>>>(pt, b.inStart, b.inList, b.states, nTDev, b.best, b.isBest);
-  handlers_kernel<<<grid_for(maxT + 1, 256), 256, 0, st>>>(b.states, b.isBest, nTDev, nLinksDev, b.handlers);
-  if (launches) *launches += 2;
+                        const uint32_t* nLinksDev, Queue& q) {
+  launch(q, ca_best_kernel, grid_for(maxT, 256), 256, 0, pt, b.inStart, b.inList, b.states, nTDev, b.best, b.isBest);
+  launch(q, handlers_kernel, grid_for(maxT + 1, 256), 256, 0, b.states, b.isBest, nTDev, nLinksDev, b.handlers);
   return cudaGetLastError();
 }
 
 cudaError_t ca_tracks(CABuffers b, const uint32_t* nTDev, uint64_t maxT, uint32_t* tracks, uint64_t maxTracks,
-                      uint32_t* err, cudaStream_t st, uint32_t* launches) {
+                      uint32_t* err, Queue& q) {
   if (maxT == 0) return cudaSuccess;
-  tracks_kernel<<<grid_for(maxT, 256), 256, 0, st>>>(b.handlers, b.best, nTDev, tracks, maxTracks, err);
-  if (launches) *launches += 1;
+  launch(q, tracks_kernel, grid_for(maxT, 256), 256, 0, b.handlers, b.best, nTDev, tracks, maxTracks, err);
   return cudaGetLastError();
 }
 

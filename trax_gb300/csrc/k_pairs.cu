@@ -183,8 +183,9 @@ __device__ __forceinline__ uint32_t find_segment(const uint32_t* taskBase, uint3
   return lo;
 }
 
-__global__ void segments_kernel(DevConfig cfg, const uint32_t* __restrict__ grid, uint32_t* segOuter,
+__global__ void segments_kernel(Stamp stamp, DevConfig cfg, const uint32_t* __restrict__ grid, uint32_t* segOuter,
                                 uint32_t* segCount) {
+  stamp_begin(stamp);
   const uint32_t S = cfg.E * cfg.nLT;
   for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < S; s += gridDim.x * blockDim.x) {
     const uint32_t e = s / cfg.nLT, p = s % cfg.nLT;
@@ -198,10 +199,11 @@ __global__ void segments_kernel(DevConfig cfg, const uint32_t* __restrict__ grid
 
 template <bool EMIT>
 __global__ void __launch_bounds__(TRAX_MAX_TUNED_THREADS)
-    pair_kernel(DevConfig cfg, const uint32_t* __restrict__ grid, const float4* __restrict__ hits,
+    pair_kernel(Stamp stamp, DevConfig cfg, const uint32_t* __restrict__ grid, const float4* __restrict__ hits,
                 const uint32_t* __restrict__ segOuter, const uint32_t* __restrict__ taskBase,
                 const uint32_t* __restrict__ nTasksDev, uint32_t* taskCount, PairTaskState state, uint2* pairs,
                 uint32_t capPairs, uint32_t* sentinels, uint32_t* err) {
+  stamp_begin(stamp);
   const uint32_t S = cfg.E * cfg.nLT;
   const uint32_t nTasks = *nTasksDev;
   const uint32_t C = cfg.C, nP = cfg.nP;
@@ -305,8 +307,9 @@ __global__ void __launch_bounds__(TRAX_MAX_TUNED_THREADS)
   if (!EMIT && blockIdx.x == 0 && threadIdx.x == 0) taskCount[nTasks] = 0u;  // the scan's +1 slot
 }
 
-__global__ void pair_offsets_kernel(DevConfig cfg, const uint32_t* taskBase, const uint32_t* pairStart,
+__global__ void pair_offsets_kernel(Stamp stamp, DevConfig cfg, const uint32_t* taskBase, const uint32_t* pairStart,
                                     uint32_t* pairOffsets) {
+  stamp_begin(stamp);
   const uint32_t S = cfg.E * cfg.nLT;
   for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s <= S; s += gridDim.x * blockDim.x)
     pairOffsets[s] = s == 0 ? 0u : pairStart[taskBase[s]];
@@ -323,36 +326,33 @@ int grid_for(uint64_t items, int threads) {
 }  // namespace
 
 cudaError_t pair_segments(const DevConfig& cfg, const uint32_t* grid, uint32_t* segOuter, uint32_t* segCount,
-                          cudaStream_t st, uint32_t* launches) {
+                          Queue& q) {
   const uint32_t S = cfg.E * cfg.nLT;
-  segments_kernel<<<grid_for(S + 1, 256), 256, 0, st>>>(cfg, grid, segOuter, segCount);
-  if (launches) *launches += 1;
+  launch(q, segments_kernel, grid_for(S + 1, 256), 256, 0, cfg, grid, segOuter, segCount);
   return cudaGetLastError();
 }
 
 cudaError_t pair_tasks(const DevConfig& cfg, bool emit, const uint32_t* grid, DevHits hits, const uint32_t* segOuter,
                        const uint32_t* taskBase, const uint32_t* nTasksDev, uint64_t maxTasks, uint32_t* taskCount,
                        PairTaskState state, uint2* pairs, uint64_t capPairs, uint32_t* sentinels, uint32_t* err,
-                       cudaStream_t st, uint32_t* launches) {
+                       Queue& q) {
   const uint32_t cap = capPairs > 0xffffffffull ? 0xffffffffu : (uint32_t)capPairs;
   if (emit && maxTasks == 0) return cudaSuccess;
   const int threads = (int)cfg.pairThreads;
   const int blocks = grid_for(maxTasks + 1, threads);
   if (emit)
-    pair_kernel<true><<<blocks, threads, 0, st>>>(cfg, grid, hits.xyzp, segOuter, taskBase, nTasksDev,
-                                                       taskCount, state, pairs, cap, sentinels, err);
+    launch(q, pair_kernel<true>, blocks, threads, 0, cfg, grid, hits.xyzp, segOuter, taskBase, nTasksDev, taskCount,
+           state, pairs, cap, sentinels, err);
   else
-    pair_kernel<false><<<blocks, threads, 0, st>>>(cfg, grid, hits.xyzp, segOuter, taskBase, nTasksDev,
-                                                        taskCount, state, pairs, cap, sentinels, err);
-  if (launches) *launches += 1;
+    launch(q, pair_kernel<false>, blocks, threads, 0, cfg, grid, hits.xyzp, segOuter, taskBase, nTasksDev,
+           taskCount, state, pairs, cap, sentinels, err);
   return cudaGetLastError();
 }
 
 cudaError_t pair_offsets(const DevConfig& cfg, const uint32_t* taskBase, const uint32_t* pairStart,
-                         uint32_t* pairOffsets, cudaStream_t st, uint32_t* launches) {
+                         uint32_t* pairOffsets, Queue& q) {
   const uint32_t S = cfg.E * cfg.nLT;
-  pair_offsets_kernel<<<grid_for(S + 1, 256), 256, 0, st>>>(cfg, taskBase, pairStart, pairOffsets);
-  if (launches) *launches += 1;
+  launch(q, pair_offsets_kernel, grid_for(S + 1, 256), 256, 0, cfg, taskBase, pairStart, pairOffsets);
   return cudaGetLastError();
 }
 

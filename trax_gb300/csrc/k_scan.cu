@@ -21,9 +21,10 @@ constexpr int SCAN_ITEMS = 16;
 constexpr uint32_t SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
 
 __global__ void __launch_bounds__(SCAN_THREADS)
-    scan_kernel(const uint32_t* __restrict__ in, uint32_t* out, uint64_t nHost, const uint32_t* nDev,
+    scan_kernel(Stamp stamp, const uint32_t* __restrict__ in, uint32_t* out, uint64_t nHost, const uint32_t* nDev,
                 uint32_t nAdd, unsigned long long* status, uint32_t* ticket, uint32_t* err, uint32_t overflowBit,
                 WaitCtl ctl) {
+  stamp_begin(stamp);
   __shared__ uint32_t s_tile;
   __shared__ uint32_t s_warp[SCAN_THREADS / 32];
   __shared__ unsigned long long s_wide[SCAN_THREADS / 32];
@@ -109,7 +110,8 @@ __global__ void __launch_bounds__(SCAN_THREADS)
 
 // Inclusive running maximum, one CTA (the serial semantics of the offset
 // monotonize kernels, TripletThetaPhiFilter.h:267-280).
-__global__ void __launch_bounds__(1024) max_scan_kernel(uint32_t* data, uint32_t n) {
+__global__ void __launch_bounds__(1024) max_scan_kernel(Stamp stamp, uint32_t* data, uint32_t n) {
+  stamp_begin(stamp);
   __shared__ uint32_t s_w[32];
   __shared__ uint32_t s_carry;
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
@@ -145,8 +147,9 @@ __global__ void __launch_bounds__(1024) max_scan_kernel(uint32_t* data, uint32_t
 }
 
 // dst = data[n] with n = *nDev (or nHost), clamped to cap
-__global__ void publish_kernel(const uint32_t* data, const uint32_t* nDev, uint32_t nHost, uint32_t cap,
+__global__ void publish_kernel(Stamp stamp, const uint32_t* data, const uint32_t* nDev, uint32_t nHost, uint32_t cap,
                                uint32_t* dst, uint32_t* err) {
+  stamp_begin(stamp);
   const uint32_t n = nDev ? *nDev : nHost;
   uint32_t v = data[n];
   if (v > cap) {
@@ -156,13 +159,24 @@ __global__ void publish_kernel(const uint32_t* data, const uint32_t* nDev, uint3
   *dst = v;
 }
 
+// the context's slots and time marks to page-locked host memory
+__global__ void slots_to_host_kernel(Stamp stamp, const uint32_t* slots, uint32_t* host, uint32_t n) {
+  stamp_begin(stamp);
+  __syncthreads();
+  for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) host[i] = slots[i];
+}
+
 }  // namespace
 
+cudaError_t slots_to_host(const uint32_t* slots, uint32_t* host, uint32_t words, Queue& q) {
+  launch(q, slots_to_host_kernel, 1, 128, 0, slots, host, words);
+  return cudaGetLastError();
+}
+
 cudaError_t publish_total(const uint32_t* data, const uint32_t* nDev, uint64_t nHost, uint64_t cap, uint32_t* dst,
-                          uint32_t* err, cudaStream_t st, uint32_t* launches) {
+                          uint32_t* err, Queue& q) {
   const uint32_t c = cap > 0xffffffffull ? 0xffffffffu : (uint32_t)cap;
-  publish_kernel<<<1, 1, 0, st>>>(data, nDev, (uint32_t)nHost, c, dst, err);
-  if (launches) *launches += 1;
+  launch(q, publish_kernel, 1, 1, 0, data, nDev, (uint32_t)nHost, c, dst, err);
   return cudaGetLastError();
 }
 
@@ -172,26 +186,24 @@ size_t scan_scratch_bytes(uint64_t maxN) {
 }
 
 cudaError_t scan_exclusive(const uint32_t* in, uint32_t* out, uint64_t n, const uint32_t* nDev, uint32_t nAdd,
-                           uint64_t maxN, void* scratch, uint32_t* err, cudaStream_t st, uint32_t* launches,
+                           uint64_t maxN, void* scratch, uint32_t* err, Queue& q,
                            bool flagOverflow, WaitCtl ctl) {
   uint64_t cap = nDev ? maxN : n;
   if (cap == 0) return cudaSuccess;
   uint64_t tiles = (cap + SCAN_TILE - 1) / SCAN_TILE;
   size_t bytes = 256 + tiles * sizeof(unsigned long long);
-  cudaError_t e = cudaMemsetAsync(scratch, 0, bytes, st);
+  cudaError_t e = cudaMemsetAsync(scratch, 0, bytes, q.st);
   if (e != cudaSuccess) return e;
   uint32_t* ticket = reinterpret_cast<uint32_t*>(scratch);
   unsigned long long* status = reinterpret_cast<unsigned long long*>(static_cast<char*>(scratch) + 256);
-  scan_kernel<<<(unsigned)tiles, SCAN_THREADS, 0, st>>>(in, out, n, nDev, nAdd, status, ticket, err,
-                                                        flagOverflow ? TRAX_EBIT_OVERFLOW : 0u, ctl);
-  if (launches) *launches += 1;
+  launch(q, scan_kernel, (unsigned)tiles, SCAN_THREADS, 0, in, out, n, nDev, nAdd, status, ticket, err,
+         flagOverflow ? TRAX_EBIT_OVERFLOW : 0u, ctl);
   return cudaGetLastError();
 }
 
-cudaError_t max_scan_inclusive(uint32_t* data, uint32_t n, cudaStream_t st, uint32_t* launches) {
+cudaError_t max_scan_inclusive(uint32_t* data, uint32_t n, Queue& q) {
   if (n == 0) return cudaSuccess;
-  max_scan_kernel<<<1, 1024, 0, st>>>(data, n);
-  if (launches) *launches += 1;
+  launch(q, max_scan_kernel, 1, 1024, 0, data, n);
   return cudaGetLastError();
 }
 
@@ -278,7 +290,7 @@ extern "C" int trax_prefix_sum_noalloc(const uint32_t* d_in, uint32_t* d_out, ui
   // the ticket, the error word and the status words of this call start at zero
   e = cudaMemsetAsync(base, 0, NOALLOC_HEADER + tiles * sizeof(unsigned long long), st);
   if (e == cudaSuccess) {
-    trax::scan_kernel<<<(unsigned)tiles, trax::SCAN_THREADS, 0, st>>>(d_in, d_out, n, nullptr, 0, status, ticket,
+    trax::scan_kernel<<<(unsigned)tiles, trax::SCAN_THREADS, 0, st>>>(trax::Stamp{}, d_in, d_out, n, nullptr, 0, status, ticket,
                                                                       err, 0u, noalloc_wait());
     e = cudaGetLastError();
   }

@@ -154,10 +154,11 @@ __device__ __forceinline__ void fine_walk(const DevConfig& cfg, const PredUnionW
 // same counts and captured candidates.  IL: the slots' layout (keep_slots).
 template <bool FINE, bool IL>
 __global__ void __launch_bounds__(TRAX_MAX_TUNED_THREADS, 6)
-    predict_count_kernel(DevConfig cfg, const uint32_t* __restrict__ grid, const float4* __restrict__ hits,
+    predict_count_kernel(Stamp stamp, DevConfig cfg, const uint32_t* __restrict__ grid, const float4* __restrict__ hits,
                          const uint32_t* __restrict__ hitEvt, const uint32_t* __restrict__ hitLayer,
                          const uint2* __restrict__ pairs, const uint32_t* __restrict__ nPairsDev, uint32_t* candCount,
                          uint32_t* keep, uint32_t* warpSums, uint32_t* nWarpsOut, uint32_t* err, FineGrid fine) {
+  stamp_begin(stamp);
   const uint32_t nPairs = *nPairsDev;
   const uint32_t lane = threadIdx.x & 31u;
   // warp-uniform loop: each warp covers 32 consecutive pairs per step
@@ -269,11 +270,12 @@ struct PredStage {
 
 template <int K>
 __global__ void __launch_bounds__(TRAX_MAX_TUNED_THREADS, 4)
-    predict_count_k_kernel(DevConfig cfg, const uint32_t* __restrict__ grid, const float4* __restrict__ hits,
+    predict_count_k_kernel(Stamp stamp, DevConfig cfg, const uint32_t* __restrict__ grid, const float4* __restrict__ hits,
                            const uint32_t* __restrict__ hitEvt, const uint32_t* __restrict__ hitLayer,
                            const uint2* __restrict__ pairs, const uint32_t* __restrict__ nPairsDev,
                            uint32_t* candCount, uint32_t* keep, uint32_t* warpSums, uint32_t* nWarpsOut,
                            uint32_t* err) {
+  stamp_begin(stamp);
   extern __shared__ PredStage s_stage[];  // [warp][k][lane]
   const uint32_t nPairs = *nPairsDev;
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
@@ -446,12 +448,13 @@ __global__ void __launch_bounds__(TRAX_MAX_TUNED_THREADS, 4)
 // at 40).
 template <bool IL, bool FINE>
 __global__ void __launch_bounds__(TRAX_MAX_TUNED_THREADS, FINE ? 6 : 8)
-    predict_store_kernel(DevConfig cfg, const uint32_t* __restrict__ grid, const float4* __restrict__ hits,
+    predict_store_kernel(Stamp stamp, DevConfig cfg, const uint32_t* __restrict__ grid, const float4* __restrict__ hits,
                          const uint32_t* __restrict__ hitEvt, const uint32_t* __restrict__ hitLayer,
                          const uint2* __restrict__ pairs, const uint32_t* __restrict__ nPairsDev,
                          const uint32_t* __restrict__ local, const uint32_t* __restrict__ warpStart,
                          const uint32_t* __restrict__ keep, uint2* cands, uint32_t capCands, uint32_t* sentinels,
                          FineGrid fine) {
+  stamp_begin(stamp);
   const uint32_t nPairs = *nPairsDev;
   uint32_t sent = 0;
   for (uint32_t gid = blockIdx.x * blockDim.x + threadIdx.x; gid < nPairs; gid += gridDim.x * blockDim.x) {
@@ -517,9 +520,10 @@ __global__ void __launch_bounds__(TRAX_MAX_TUNED_THREADS, FINE ? 6 : 8)
 // pairs of a segment are contiguous and sentinel pairs count zero
 // candidates, so both come down to the candidate position at the segment's
 // pair end.
-__global__ void predict_offsets_kernel(uint32_t S, const uint32_t* __restrict__ pairOffsets,
+__global__ void predict_offsets_kernel(Stamp stamp, uint32_t S, const uint32_t* __restrict__ pairOffsets,
                                        const uint32_t* __restrict__ nPairsDev, const uint32_t* __restrict__ local,
                                        const uint32_t* __restrict__ warpStart, uint32_t* offsets) {
+  stamp_begin(stamp);
   const uint32_t nPairs = *nPairsDev;
   for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s <= S; s += gridDim.x * blockDim.x) {
     if (s == 0) {
@@ -549,9 +553,10 @@ __global__ void predict_offsets_kernel(uint32_t S, const uint32_t* __restrict__ 
 // At most 32 registers (eight 256-thread blocks per SM): full occupancy
 // outweighs the few spilled bytes (0.99 -> 0.86 ms on the 1000-event batch).
 __global__ void __launch_bounds__(TRAX_MAX_TUNED_THREADS, 8)
-    filter_kernel(DevConfig cfg, const float4* __restrict__ hits, const uint32_t* __restrict__ hitLayer,
+    filter_kernel(Stamp stamp, DevConfig cfg, const float4* __restrict__ hits, const uint32_t* __restrict__ hitLayer,
                   const uint2* __restrict__ pairs, const uint2* __restrict__ cands, const uint32_t* nCandsDev,
                   uint32_t* masks, uint32_t* warpSums, uint32_t* nWordsOut) {
+  stamp_begin(stamp);
   constexpr uint32_t WORDS = 32;  // a warp takes 32 words = 1024 candidates at a time
   __shared__ uint32_t s_queue[TRAX_MAX_TUNED_THREADS / 32][64];
   __shared__ uint32_t s_queue2[TRAX_MAX_TUNED_THREADS / 32][64];
@@ -662,10 +667,11 @@ __global__ void __launch_bounds__(TRAX_MAX_TUNED_THREADS, 8)
 // step, finding its word by a 5-step search over the words' running counts
 // and its candidate by the rank of the bit in the word (0.21 -> 0.15 ms on
 // the 1000-event batch against one thread per candidate).
-__global__ void filter_store_kernel(const uint2* __restrict__ pairs, const uint2* __restrict__ cands,
+__global__ void filter_store_kernel(Stamp stamp, const uint2* __restrict__ pairs, const uint2* __restrict__ cands,
                                     const uint32_t* nCandsDev, const uint32_t* __restrict__ masks,
                                     const uint32_t* __restrict__ wordStart, uint32_t* h1, uint32_t* h2, uint32_t* h3,
                                     uint32_t capT) {
+  stamp_begin(stamp);
   const uint32_t n = *nCandsDev;
   const uint32_t nW = (n + 31u) >> 5;
   const uint32_t lane = threadIdx.x & 31u;
@@ -708,9 +714,10 @@ __global__ void filter_store_kernel(const uint2* __restrict__ pairs, const uint2
 }
 
 // filterOffsetStore (TripletThetaPhiFilter.h:221-257)
-__global__ void triplet_offsets_kernel(DevConfig cfg, const uint32_t* __restrict__ hitEvt,
+__global__ void triplet_offsets_kernel(Stamp stamp, DevConfig cfg, const uint32_t* __restrict__ hitEvt,
                                        const uint32_t* __restrict__ hitLayer, const uint32_t* __restrict__ h1,
                                        const uint32_t* nTDev, uint32_t* offsets) {
+  stamp_begin(stamp);
   const uint32_t nT = *nTDev;
   for (uint32_t gid = blockIdx.x * blockDim.x + threadIdx.x; gid < nT; gid += gridDim.x * blockDim.x) {
     const uint32_t hitId = trax_hit(h1[gid], cfg);
@@ -738,7 +745,7 @@ bool pred_k_fits(const DevConfig& cfg) {
 cudaError_t predict_pairs(const DevConfig& cfg, bool emit, const uint32_t* grid, DevHits hits, const uint2* pairs,
                           const uint32_t* nPairsDev, uint64_t maxPairs, uint32_t* candCount, uint32_t* warpSums,
                           uint32_t* nWarpsOut, uint32_t* keep, uint2* cands, uint64_t capCands, uint32_t* sentinels,
-                          uint32_t* err, cudaStream_t st, uint32_t* launches, FineGrid fine) {
+                          uint32_t* err, Queue& q, FineGrid fine) {
   const uint32_t cap = capCands > 0xffffffffull ? 0xffffffffu : (uint32_t)capCands;
   const int threads = (int)cfg.predThreads;
   const int blocks = grid_for(maxPairs + 1, threads);
@@ -746,87 +753,76 @@ cudaError_t predict_pairs(const DevConfig& cfg, bool emit, const uint32_t* grid,
   if (emit) {
     if (maxPairs == 0) return cudaSuccess;
     if (cfg.fineRows > 0 && fine.grid)
-      predict_store_kernel<true, true><<<blocks, threads, 0, st>>>(cfg, grid, hits.xyzp, hits.evt, hits.layer,
-                                                                   pairs, nPairsDev, candCount, warpSums, keep,
-                                                                   cands, cap, sentinels, fine);
+      launch(q, (predict_store_kernel<true, true>), blocks, threads, 0, cfg, grid, hits.xyzp, hits.evt, hits.layer,
+             pairs, nPairsDev, candCount, warpSums, keep, cands, cap, sentinels, fine);
     else if (il)
-      predict_store_kernel<true, false><<<blocks, threads, 0, st>>>(cfg, grid, hits.xyzp, hits.evt, hits.layer,
-                                                                    pairs, nPairsDev, candCount, warpSums, keep,
-                                                                    cands, cap, sentinels, fine);
+      launch(q, (predict_store_kernel<true, false>), blocks, threads, 0, cfg, grid, hits.xyzp, hits.evt, hits.layer,
+             pairs, nPairsDev, candCount, warpSums, keep, cands, cap, sentinels, fine);
     else
-      predict_store_kernel<false, false><<<blocks, threads, 0, st>>>(cfg, grid, hits.xyzp, hits.evt, hits.layer,
-                                                                     pairs, nPairsDev, candCount, warpSums, keep,
-                                                                     cands, cap, sentinels, fine);
+      launch(q, (predict_store_kernel<false, false>), blocks, threads, 0, cfg, grid, hits.xyzp, hits.evt,
+             hits.layer, pairs, nPairsDev, candCount, warpSums, keep, cands, cap, sentinels, fine);
   } else if (cfg.fineRows > 0 && fine.grid) {
-    predict_count_kernel<true, true><<<blocks, threads, 0, st>>>(cfg, grid, hits.xyzp, hits.evt, hits.layer, pairs,
-                                                                 nPairsDev, candCount, keep, warpSums, nWarpsOut,
-                                                                 err, fine);
+    launch(q, (predict_count_kernel<true, true>), blocks, threads, 0, cfg, grid, hits.xyzp, hits.evt, hits.layer,
+           pairs, nPairsDev, candCount, keep, warpSums, nWarpsOut, err, fine);
   } else if (il) {  // the K-pairs kernel keeps the consecutive layout
-    predict_count_kernel<false, true><<<blocks, threads, 0, st>>>(cfg, grid, hits.xyzp, hits.evt, hits.layer, pairs,
-                                                                  nPairsDev, candCount, keep, warpSums, nWarpsOut,
-                                                                  err, fine);
+    launch(q, (predict_count_kernel<false, true>), blocks, threads, 0, cfg, grid, hits.xyzp, hits.evt, hits.layer,
+           pairs, nPairsDev, candCount, keep, warpSums, nWarpsOut, err, fine);
   } else if (cfg.predPairsPerThread <= 1 || !pred_k_fits(cfg)) {
-    predict_count_kernel<false, false><<<blocks, threads, 0, st>>>(cfg, grid, hits.xyzp, hits.evt, hits.layer,
-                                                                   pairs, nPairsDev, candCount, keep, warpSums,
-                                                                   nWarpsOut, err, fine);
+    launch(q, (predict_count_kernel<false, false>), blocks, threads, 0, cfg, grid, hits.xyzp, hits.evt, hits.layer,
+           pairs, nPairsDev, candCount, keep, warpSums, nWarpsOut, err, fine);
   } else {
     const int K = cfg.predPairsPerThread;
     const size_t smem = (size_t)threads * K * sizeof(PredStage);
     const int kb = grid_for((maxPairs + K - 1) / K + 1, threads);
     if (K == 2)
-      predict_count_k_kernel<2><<<kb, threads, smem, st>>>(cfg, grid, hits.xyzp, hits.evt, hits.layer, pairs,
-                                                           nPairsDev, candCount, keep, warpSums, nWarpsOut, err);
+      launch(q, predict_count_k_kernel<2>, kb, threads, smem, cfg, grid, hits.xyzp, hits.evt, hits.layer, pairs,
+             nPairsDev, candCount, keep, warpSums, nWarpsOut, err);
     else
-      predict_count_k_kernel<4><<<kb, threads, smem, st>>>(cfg, grid, hits.xyzp, hits.evt, hits.layer, pairs,
-                                                           nPairsDev, candCount, keep, warpSums, nWarpsOut, err);
+      launch(q, predict_count_k_kernel<4>, kb, threads, smem, cfg, grid, hits.xyzp, hits.evt, hits.layer, pairs,
+             nPairsDev, candCount, keep, warpSums, nWarpsOut, err);
   }
-  if (launches) *launches += 1;
   return cudaGetLastError();
 }
 
 cudaError_t predict_offsets(const DevConfig& cfg, const uint32_t* pairOffsets, const uint32_t* nPairsDev,
                             const uint32_t* candCount, const uint32_t* warpStart, uint32_t* candOffsets,
-                            cudaStream_t st, uint32_t* launches) {
+                            Queue& q) {
   const uint32_t S = cfg.E * cfg.nLT;
-  predict_offsets_kernel<<<grid_for(S + 1, 256), 256, 0, st>>>(S, pairOffsets, nPairsDev, candCount, warpStart,
-                                                               candOffsets);
-  if (launches) *launches += 1;
+  launch(q, predict_offsets_kernel, grid_for(S + 1, 256), 256, 0, S, pairOffsets, nPairsDev, candCount, warpStart,
+         candOffsets);
   return cudaGetLastError();
 }
 
 cudaError_t filter_candidates(const DevConfig& cfg, DevHits hits, const uint2* pairs, const uint2* cands,
                               const uint32_t* nCandsDev, uint64_t maxCands, uint32_t* masks, uint32_t* warpSums,
-                              uint32_t* nWordsOut, cudaStream_t st, uint32_t* launches) {
+                              uint32_t* nWordsOut, Queue& q) {
   const int threads = (int)cfg.filterThreads;
-  filter_kernel<<<grid_for(maxCands + 1, threads), threads, 0, st>>>(cfg, hits.xyzp, hits.layer, pairs, cands,
-                                                                     nCandsDev, masks, warpSums, nWordsOut);
-  if (launches) *launches += 1;
+  launch(q, filter_kernel, grid_for(maxCands + 1, threads), threads, 0, cfg, hits.xyzp, hits.layer, pairs, cands,
+         nCandsDev, masks, warpSums, nWordsOut);
   return cudaGetLastError();
 }
 
 cudaError_t filter_store(const uint2* pairs, const uint2* cands, const uint32_t* nCandsDev, uint64_t maxCands,
                          const uint32_t* masks, const uint32_t* wordStart, uint32_t* h1, uint32_t* h2, uint32_t* h3,
-                         uint64_t capT, cudaStream_t st, uint32_t* launches) {
+                         uint64_t capT, Queue& q) {
   if (maxCands == 0) return cudaSuccess;
   const uint32_t cap = capT > 0xffffffffull ? 0xffffffffu : (uint32_t)capT;
-  filter_store_kernel<<<grid_for((maxCands + 1023) / 1024 * 32, 256), 256, 0, st>>>(pairs, cands, nCandsDev, masks,
-                                                                                    wordStart, h1, h2, h3, cap);
-  if (launches) *launches += 1;
+  launch(q, filter_store_kernel, grid_for((maxCands + 1023) / 1024 * 32, 256), 256, 0, pairs, cands, nCandsDev,
+         masks, wordStart, h1, h2, h3, cap);
   return cudaGetLastError();
 }
 
 cudaError_t triplet_offsets(const DevConfig& cfg, DevHits hits, const uint32_t* h1, const uint32_t* nTDev,
-                            uint64_t maxT, uint32_t* offsets, cudaStream_t st, uint32_t* launches) {
+                            uint64_t maxT, uint32_t* offsets, Queue& q) {
   const uint32_t S = cfg.E * cfg.nLT;
-  cudaError_t e = cudaMemsetAsync(offsets, 0, (S + 1) * sizeof(uint32_t), st);
+  cudaError_t e = cudaMemsetAsync(offsets, 0, (S + 1) * sizeof(uint32_t), q.st);
   if (e != cudaSuccess) return e;
   if (maxT > 0) {
-    triplet_offsets_kernel<<<grid_for(maxT, 256), 256, 0, st>>>(cfg, hits.evt, hits.layer, h1, nTDev, offsets);
-    if (launches) *launches += 1;
+    launch(q, triplet_offsets_kernel, grid_for(maxT, 256), 256, 0, cfg, hits.evt, hits.layer, h1, nTDev, offsets);
   }
   e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  return max_scan_inclusive(offsets, S + 1, st, launches);
+  return max_scan_inclusive(offsets, S + 1, q);
 }
 
 }  // namespace trax

@@ -1,6 +1,6 @@
 // trax_kernels.h -- host-side launchers of the sm_103a kernels.  Each
-// launcher enqueues work on `st` and adds the number of kernels it launched
-// to *launches.  Counts that are only known on the device are passed as
+// launcher enqueues work on its Queue's stream (or `st`) and counts the
+// kernels it launched.  Counts that are only known on the device are passed as
 // device pointers together with a host-side capacity that sizes the grid.
 #pragma once
 
@@ -13,6 +13,29 @@ struct trax_ctx;
 
 namespace trax {
 
+// Where the launchers enqueue: a stream, the number of kernels launched so
+// far, and the time marks the next kernel writes as it starts.
+struct Queue {
+  cudaStream_t st = nullptr;
+  uint32_t launches = 0;
+  Stamp marks;
+};
+
+// Every kernel of the chain takes its Stamp first.
+template <class... P, class... A>
+cudaError_t launch(Queue& q, void (*kernel)(Stamp, P...), unsigned blocks, unsigned threads, size_t smem,
+                   A&&... args) {
+  cudaLaunchConfig_t c = {};
+  c.gridDim = dim3(blocks);
+  c.blockDim = dim3(threads);
+  c.dynamicSmemBytes = smem;
+  c.stream = q.st;
+  const Stamp marks = q.marks;
+  q.marks.which = 0;
+  ++q.launches;
+  return cudaLaunchKernelEx(&c, kernel, marks, static_cast<P>(args)...);
+}
+
 // ---------------------------------------------------------------- scans
 size_t scan_scratch_bytes(uint64_t maxN);
 // Exclusive scan of n elements (or *nDev + nAdd when nDev != nullptr, with
@@ -20,9 +43,9 @@ size_t scan_scratch_bytes(uint64_t maxN);
 // with flagOverflow a total of 2^32 or more sets TRAX_EBIT_OVERFLOW.  `ctl`
 // bounds the look-back waits (and may name a tile that never publishes).
 cudaError_t scan_exclusive(const uint32_t* in, uint32_t* out, uint64_t n, const uint32_t* nDev, uint32_t nAdd,
-                           uint64_t maxN, void* scratch, uint32_t* err, cudaStream_t st, uint32_t* launches,
+                           uint64_t maxN, void* scratch, uint32_t* err, Queue& q,
                            bool flagOverflow, WaitCtl ctl);
-cudaError_t max_scan_inclusive(uint32_t* data, uint32_t n, cudaStream_t st, uint32_t* launches);
+cudaError_t max_scan_inclusive(uint32_t* data, uint32_t n, Queue& q);
 
 // ------------------------------------------------------ event bucketing
 // The hits of a group of events as their file holds them, with the host's
@@ -126,8 +149,7 @@ struct GridScratch {
 };
 
 cudaError_t grid_build(const DevConfig& cfg, const GridInput& in, uint32_t* grid, DevHits out,
-                       GridScratch scratch, uint32_t maxLayerHits, uint32_t* err, cudaStream_t st,
-                       uint32_t* launches);
+                       GridScratch scratch, uint32_t maxLayerHits, uint32_t* err, Queue& q);
 cudaError_t grid_prepare(int device);  // one-time kernel attributes
 
 // The fine z grid the prediction count walks when cfg.fineRows > 0: the
@@ -153,14 +175,14 @@ inline uint64_t fine_counter_cells(const DevConfig& cfg) {
              : 0;
 }
 cudaError_t fine_grid_build(const DevConfig& cfg, const uint32_t* grid, const float4* xyzp, FineGrid fine,
-                            uint32_t* counters, cudaStream_t st, uint32_t* launches);
+                            uint32_t* counters, Queue& q);
 // hit collection = uploaded hits in input order (plus the packed xyz-phi array)
-cudaError_t identity_hits(const GridInput& in, uint32_t n, DevHits out, cudaStream_t st, uint32_t* launches);
+cudaError_t identity_hits(const GridInput& in, uint32_t n, DevHits out, Queue& q);
 
 // ----------------------------------------------------------------- pairs
 // Per (event, layer triplet) segment: first outer hit and number of outer hits.
 cudaError_t pair_segments(const DevConfig& cfg, const uint32_t* grid, uint32_t* segOuter, uint32_t* segCount,
-                          cudaStream_t st, uint32_t* launches);
+                          Queue& q);
 // What the count pass leaves for the store pass per outer-hit task k, so
 // that the store pass neither searches the task's segment nor recomputes
 // its window: bounds[k] = (zLow, zHigh, phiLow, phiHigh);
@@ -186,11 +208,10 @@ inline PairTaskState pair_task_state(void* base, uint64_t n) {
 cudaError_t pair_tasks(const DevConfig& cfg, bool emit, const uint32_t* grid, DevHits hits,
                        const uint32_t* segOuter, const uint32_t* taskBase, const uint32_t* nTasksDev,
                        uint64_t maxTasks, uint32_t* taskCount, PairTaskState state, uint2* pairs,
-                       uint64_t capPairs, uint32_t* sentinelCount, uint32_t* err, cudaStream_t st,
-                       uint32_t* launches);
+                       uint64_t capPairs, uint32_t* sentinelCount, uint32_t* err, Queue& q);
 // pairOffsets[s+1] = first pair of segment s+1 (Pairing::pairingOffsets)
 cudaError_t pair_offsets(const DevConfig& cfg, const uint32_t* taskBase, const uint32_t* pairStart,
-                         uint32_t* pairOffsets, cudaStream_t st, uint32_t* launches);
+                         uint32_t* pairOffsets, Queue& q);
 
 // ------------------------------------------------------------ prediction
 // Count pass (emit == false): per pair the exclusive offset of its
@@ -217,11 +238,11 @@ inline bool keep_interleaved(const DevConfig& cfg) { return cfg.predKeep >= 16u 
 cudaError_t predict_pairs(const DevConfig& cfg, bool emit, const uint32_t* grid, DevHits hits, const uint2* pairs,
                           const uint32_t* nPairsDev, uint64_t maxPairs, uint32_t* candCount, uint32_t* warpSums,
                           uint32_t* nWarpsOut, uint32_t* keep, uint2* cands, uint64_t capCands,
-                          uint32_t* sentinelCount, uint32_t* err, cudaStream_t st, uint32_t* launches,
+                          uint32_t* sentinelCount, uint32_t* err, Queue& q,
                           FineGrid fine = FineGrid{nullptr, nullptr});
 cudaError_t predict_offsets(const DevConfig& cfg, const uint32_t* pairOffsets, const uint32_t* nPairsDev,
                             const uint32_t* candCount, const uint32_t* warpStart, uint32_t* candOffsets,
-                            cudaStream_t st, uint32_t* launches);
+                            Queue& q);
 
 // ---------------------------------------------------------------- filter
 // the flags of 32 consecutive candidates as one word masks[g / 32] (bit
@@ -229,15 +250,15 @@ cudaError_t predict_offsets(const DevConfig& cfg, const uint32_t* pairOffsets, c
 // (+1 slot zeroed; the number of words goes to *nWordsOut)
 cudaError_t filter_candidates(const DevConfig& cfg, DevHits hits, const uint2* pairs, const uint2* cands,
                               const uint32_t* nCandsDev, uint64_t maxCands, uint32_t* masks, uint32_t* warpSums,
-                              uint32_t* nWordsOut, cudaStream_t st, uint32_t* launches);
+                              uint32_t* nWordsOut, Queue& q);
 // with warpSums exclusively scanned into wordStart: the triplets of the
 // flagged candidates at wordStart[g / 32] + (flags below g in its word)
 cudaError_t filter_store(const uint2* pairs, const uint2* cands, const uint32_t* nCandsDev, uint64_t maxCands,
                          const uint32_t* masks, const uint32_t* wordStart, uint32_t* h1, uint32_t* h2, uint32_t* h3,
-                         uint64_t capT, cudaStream_t st, uint32_t* launches);
+                         uint64_t capT, Queue& q);
 // trackletOffsets with the reference's filterOffsetStore + monotonize semantics
 cudaError_t triplet_offsets(const DevConfig& cfg, DevHits hits, const uint32_t* h1, const uint32_t* nTDev,
-                            uint64_t maxT, uint32_t* offsets, cudaStream_t st, uint32_t* launches);
+                            uint64_t maxT, uint32_t* offsets, Queue& q);
 
 // ---------------------------------------------------------- connectivity
 struct TripletView {
@@ -249,32 +270,35 @@ struct TripletView {
 };
 
 cudaError_t triplet_eta(const DevConfig& cfg, DevHits hits, TripletView t, float* eta, uint32_t* seg,
-                        cudaStream_t st, uint32_t* launches);
+                        Queue& q);
 cudaError_t segment_bounds(const DevConfig& cfg, const uint32_t* seg, const uint32_t* nTDev, uint32_t* segStart,
-                           cudaStream_t st, uint32_t* launches);
+                           Queue& q);
 // runStart[t]: where the count pass found the (h2, h1) run of t's
 // followers in sorted segments; the store pass starts there
 cudaError_t connectivity_tasks(const DevConfig& cfg, bool emit, DevHits hits, TripletView t, const float* eta,
                                const uint32_t* offsets, const uint32_t* segStart, uint32_t* linkCount,
                                uint32_t* flags, uint32_t* runStart, uint32_t* basis, uint32_t* follower,
-                               uint64_t capLinks, bool sortedSegments, cudaStream_t st, uint32_t* launches);
+                               uint64_t capLinks, bool sortedSegments, Queue& q);
 // flags[k] for k < n-1 -> words of 32 (flag) and (!flag) bits with the number
 // set per word (+1 slots zeroed, the number of words to *nWordsOut)
 cudaError_t connectable_words(const uint32_t* flags, const uint32_t* nTDev, uint64_t maxT, uint32_t* connWords,
                               uint32_t* connSums, uint32_t* nonWords, uint32_t* nonSums, uint32_t* nWordsOut,
-                              cudaStream_t st, uint32_t* launches);
+                              Queue& q);
 // with the sums scanned into wordStart: outIdx[wordStart[k / 32] + (bits
 // below k in its word)] = k for every set bit k < *nTDev
 cudaError_t compact_words(const uint32_t* words, const uint32_t* wordStart, const uint32_t* nTDev, uint64_t maxT,
-                          uint32_t* outIdx, uint64_t capOut, cudaStream_t st, uint32_t* launches);
+                          uint32_t* outIdx, uint64_t capOut, Queue& q);
 // *dst = data[n] (n = *nDev, or nHost when nDev is null): the total a scan of
 // n+1 elements left in its last slot, clamped to cap (TRAX_EBIT_CAPACITY)
 cudaError_t publish_total(const uint32_t* data, const uint32_t* nDev, uint64_t nHost, uint64_t cap, uint32_t* dst,
-                          uint32_t* err, cudaStream_t st, uint32_t* launches);
+                          uint32_t* err, Queue& q);
+
+// the context's slots and the time marks after them to page-locked host memory
+cudaError_t slots_to_host(const uint32_t* slots, uint32_t* host, uint32_t words, Queue& q);
 
 // ---------------------------------------------------- circle fit and CA
 cudaError_t circle_fit(DevHits hits, TripletView t, const uint32_t* connectable, const uint32_t* nConnDev,
-                       uint64_t maxConn, float* pt, cudaStream_t st, uint32_t* launches);
+                       uint64_t maxConn, float* pt, Queue& q);
 
 struct CABuffers {
   uint32_t* states;    // [nT]
@@ -288,20 +312,19 @@ struct CABuffers {
 };
 
 cudaError_t ca_in_degree(const uint32_t* follower, const uint32_t* nLinksDev, uint64_t maxLinks, CABuffers b,
-                         const uint32_t* nTDev, uint64_t maxT, cudaStream_t st, uint32_t* launches);
+                         const uint32_t* nTDev, uint64_t maxT, Queue& q);
 cudaError_t ca_fill(const uint32_t* basis, const uint32_t* follower, const uint32_t* nLinksDev, uint64_t maxLinks,
-                    CABuffers b, const uint32_t* nTDev, uint64_t maxT, cudaStream_t st, uint32_t* launches);
-cudaError_t ca_forward(const DevConfig& cfg, CABuffers b, const uint32_t* nTDev, uint64_t maxT, cudaStream_t st,
-                       uint32_t* launches);
+                    CABuffers b, const uint32_t* nTDev, uint64_t maxT, Queue& q);
+cudaError_t ca_forward(const DevConfig& cfg, CABuffers b, const uint32_t* nTDev, uint64_t maxT, Queue& q);
 // One forward iteration of the reference's CA over any link set
 // (CellularAutomaton.h:52-100); *living is set when a cell lives.
 cudaError_t ca_iteration(const uint32_t* basis, const uint32_t* follower, uint32_t nLinks, const uint32_t* cur,
-                         uint32_t* next, uint32_t* living, cudaStream_t st, uint32_t* launches);
-cudaError_t fill_u32(uint32_t* p, uint32_t v, uint32_t n, cudaStream_t st, uint32_t* launches);
+                         uint32_t* next, uint32_t* living, Queue& q);
+cudaError_t fill_u32(uint32_t* p, uint32_t v, uint32_t n, Queue& q);
 cudaError_t ca_backward(const float* pt, CABuffers b, const uint32_t* nTDev, uint64_t maxT,
-                        const uint32_t* nLinksDev, cudaStream_t st, uint32_t* launches);
+                        const uint32_t* nLinksDev, Queue& q);
 cudaError_t ca_tracks(CABuffers b, const uint32_t* nTDev, uint64_t maxT, uint32_t* tracks, uint64_t maxTracks,
-                      uint32_t* err, cudaStream_t st, uint32_t* launches);
+                      uint32_t* err, Queue& q);
 
 // ------------------------------------------- differentiable triplet fit
 // Fit rows are the selected triplets ordered by layer triplet; rows of layer
