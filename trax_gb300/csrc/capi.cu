@@ -144,6 +144,7 @@ struct trax_ctx {
   DevBuf userIdx, caNext;  // caller-provided fit list; second state buffer of the caller-link CA
   // bookkeeping
   DevBuf scanScratch, slots;
+  size_t scanUsed = 0;  // scan scratch taken by the chain being captured
   uint32_t* hSlots = nullptr;  // pinned copy of the slots
   uint32_t maxLayerHits = 0;   // most hits of one (event, layer) in the uploaded batch
   // sizes of the last run
@@ -402,18 +403,36 @@ int check_device_error(trax_ctx* c) {
       return fail(c, TRAX_ERR_STATE, "device-mode buffer " #buf " too small");  \
   } while (0)
 
-// exclusive scan of (count + 1) elements in place, count = nHost or *nDev;
-// the total is published into slot `dst` (clamped to cap)
-int scan_publish(trax_ctx* c, Mode mode, uint32_t* data, uint64_t nHost, const uint32_t* nDev, uint64_t maxCount,
-                 int dst, uint64_t cap) {
+// Exclusive scan of (count + 1) elements, count = nHost or *nDev; the total
+// goes to slot `dst` (clamped to cap; -1: nowhere).  In DEVICE mode every
+// scan of the chain has its own part of the scratch, cleared by the grid
+// build; in SYNCED mode the scratch is cleared by each scan.
+int scan_publish(trax_ctx* c, Mode mode, const uint32_t* in, uint32_t* out, uint64_t nHost, const uint32_t* nDev,
+                 uint64_t maxCount, int dst, uint64_t cap) {
   const uint64_t maxN = maxCount + 1;
-  if (mode == SYNCED) CK(ensure(c, c->scanScratch, scan_scratch_bytes(maxN)));
-  else if (scan_scratch_bytes(maxN) > c->scanScratch.cap)
+  const size_t bytes = scan_scratch_bytes(maxN);
+  if (mode == SYNCED) {
+    CK(ensure(c, c->scanScratch, bytes));
+    c->scanUsed = 0;
+  } else if (c->scanUsed + bytes > c->scanScratch.cap) {
     return fail(c, TRAX_ERR_STATE, "device-mode scan scratch too small");
-  CK(scan_exclusive(data, data, nHost + 1, nDev, 1, maxN, c->scanScratch.p, dev_err(c), c->q,
-                    true, c->wait));
-  CK(publish_total(data, nDev, nHost, cap, slot(c, dst), dev_err(c), c->q));
+  }
+  char* scratch = static_cast<char*>(c->scanScratch.p) + c->scanUsed;
+  if (mode == DEVICE) c->scanUsed += bytes;
+  ScanTotal total;
+  if (dst >= 0) total = ScanTotal{slot(c, dst), cap > 0xffffffffull ? 0xffffffffu : (uint32_t)cap};
+  CK(scan_exclusive(in, out, nHost + 1, nDev, 1, maxN, scratch, mode == DEVICE, dev_err(c), c->q, true, c->wait,
+                    total));
   return TRAX_OK;
+}
+
+// scratch of all the scans of one chain in DEVICE mode: segments, tasks,
+// pairs and candidates by 32, and the linking stages' per-triplet scans
+size_t chain_scan_bytes(trax_ctx* c) {
+  const uint64_t maxTW = (c->capT + 31) / 32;
+  return scan_scratch_bytes((uint64_t)c->cfg.E * c->cfg.nLT + 1) + scan_scratch_bytes(c->capTasks + 1) +
+         scan_scratch_bytes((c->capPairs + 31) / 32 + 1) + scan_scratch_bytes((c->capCands + 31) / 32 + 1) +
+         3 * scan_scratch_bytes(c->capT + 1) + 2 * scan_scratch_bytes(maxTW + 1);
 }
 
 // ------------------------------------------------------------------ stages
@@ -453,6 +472,9 @@ int stage_grid(trax_ctx* c, Mode mode) {
   sc.phi = ptr<float>(c->sc_phi);
   sc.perm = ptr<uint32_t>(c->sc_perm);
   sc.counts = ptr<uint32_t>(c->sc_counts);
+  sc.clear = ptr<uint4>(c->scanScratch);
+  sc.clearWords = mode == DEVICE ? (uint32_t)(chain_scan_bytes(c) / 16) : 0u;
+  c->scanUsed = 0;
   KBEG(TK_GRID);
   CK(grid_build(c->cfg, in, ptr<uint32_t>(c->grid), dev_hits(c), sc, c->maxLayerHits, dev_err(c), c->q));
   CK(fine_grid_build(c->cfg, ptr<uint32_t>(c->grid), ptr<float4>(c->pxyzp), fine_buffers(c), sc.counts, c->q));
@@ -469,7 +491,7 @@ int stage_pairs(trax_ctx* c, Mode mode) {
   ENSURE(pairOffsets, S + 1, 4);
   uint32_t* taskBase = ptr<uint32_t>(c->taskBase);
   CK(pair_segments(c->cfg, ptr<uint32_t>(c->grid), ptr<uint32_t>(c->segOuter), taskBase, c->q));
-  RC(scan_publish(c, mode, taskBase, S, nullptr, S, S_TASKS, mode == DEVICE ? c->capTasks : NO_CAP));
+  RC(scan_publish(c, mode, taskBase, taskBase, S, nullptr, S, S_TASKS, mode == DEVICE ? c->capTasks : NO_CAP));
   const uint32_t* nTasksDev = slot(c, S_TASKS);
   uint64_t maxTasks = c->capTasks;
   if (mode == SYNCED) {
@@ -484,7 +506,7 @@ int stage_pairs(trax_ctx* c, Mode mode) {
   CK(pair_tasks(c->cfg, false, ptr<uint32_t>(c->grid), dev_hits(c), ptr<uint32_t>(c->segOuter), taskBase, nTasksDev,
                 maxTasks, taskCount, taskState, nullptr, 0, slot(c, S_PAIR_SENT), dev_err(c), c->q));
   KEND(TK_PAIR_COUNT);
-  RC(scan_publish(c, mode, taskCount, c->nTasks, mode == DEVICE ? nTasksDev : nullptr, maxTasks, S_PAIRS,
+  RC(scan_publish(c, mode, taskCount, taskCount, c->nTasks, mode == DEVICE ? nTasksDev : nullptr, maxTasks, S_PAIRS,
                   mode == DEVICE ? c->capPairs : NO_CAP));
   uint64_t maxPairs = c->capPairs;
   if (mode == SYNCED) {
@@ -521,7 +543,7 @@ int stage_predict(trax_ctx* c, Mode mode) {
                    slot(c, S_CAND_SENT), dev_err(c), c->q, fine_grid(c)));
   KEND(TK_PRED_COUNT);
   // the prefix sum runs over the per-warp sums of the counts
-  RC(scan_publish(c, mode, warpSums, (c->nPairs + 31) / 32, mode == DEVICE ? slot(c, S_PRED_WARPS) : nullptr,
+  RC(scan_publish(c, mode, warpSums, warpSums, (c->nPairs + 31) / 32, mode == DEVICE ? slot(c, S_PRED_WARPS) : nullptr,
                   maxWarps, S_CANDS, mode == DEVICE ? c->capCands : NO_CAP));
   uint64_t maxCands = c->capCands;
   if (mode == SYNCED) {
@@ -555,7 +577,7 @@ int stage_filter(trax_ctx* c, Mode mode) {
                        sums, slot(c, S_FLAG_WORDS), c->q));
   KEND(TK_FILTER);
   // the prefix sum runs over the numbers of flags per word of 32 candidates
-  RC(scan_publish(c, mode, sums, (c->nCands + 31) / 32, mode == DEVICE ? slot(c, S_FLAG_WORDS) : nullptr, maxWords,
+  RC(scan_publish(c, mode, sums, sums, (c->nCands + 31) / 32, mode == DEVICE ? slot(c, S_FLAG_WORDS) : nullptr, maxWords,
                   S_TRIPLETS, mode == DEVICE ? c->capT : NO_CAP));
   uint64_t maxT = c->capT;
   if (mode == SYNCED) {
@@ -616,7 +638,7 @@ int stage_connectivity(trax_ctx* c, Mode mode) {
                         ptr<uint32_t>(c->segStart), linkCount, ptr<uint32_t>(c->cflags), ptr<uint32_t>(c->linkRun),
                         nullptr, nullptr, 0, c->sortedSegments, c->q));
   KEND(TK_CONN_COUNT);
-  RC(scan_publish(c, mode, linkCount, c->nT, mode == DEVICE ? nTDev : nullptr, maxT, S_LINKS,
+  RC(scan_publish(c, mode, linkCount, linkCount, c->nT, mode == DEVICE ? nTDev : nullptr, maxT, S_LINKS,
                   mode == DEVICE ? c->capLinks : NO_CAP));
   uint64_t maxLinks = c->capLinks;
   if (mode == SYNCED) {
@@ -637,8 +659,8 @@ int stage_connectivity(trax_ctx* c, Mode mode) {
                        ptr<uint32_t>(c->nonConnW), ptr<uint32_t>(c->nonConnS), slot(c, S_CONN_WORDS), c->q));
   const uint64_t nTW = (c->nT + 31) / 32;
   const uint32_t* nTWDev = mode == DEVICE ? slot(c, S_CONN_WORDS) : nullptr;
-  RC(scan_publish(c, mode, ptr<uint32_t>(c->connS), nTW, nTWDev, maxTW, S_CONN, NO_CAP));
-  RC(scan_publish(c, mode, ptr<uint32_t>(c->nonConnS), nTW, nTWDev, maxTW, S_NONCONN, NO_CAP));
+  RC(scan_publish(c, mode, ptr<uint32_t>(c->connS), ptr<uint32_t>(c->connS), nTW, nTWDev, maxTW, S_CONN, NO_CAP));
+  RC(scan_publish(c, mode, ptr<uint32_t>(c->nonConnS), ptr<uint32_t>(c->nonConnS), nTW, nTWDev, maxTW, S_NONCONN, NO_CAP));
   CK(compact_words(ptr<uint32_t>(c->connW), ptr<uint32_t>(c->connS), nTDev, maxT, ptr<uint32_t>(c->connIdx), maxT,
                    c->q));
   CK(compact_words(ptr<uint32_t>(c->nonConnW), ptr<uint32_t>(c->nonConnS), nTDev, maxT, ptr<uint32_t>(c->nonConnIdx),
@@ -695,13 +717,11 @@ int stage_ca(trax_ctx* c, Mode mode) {
   CABuffers b = ca_buffers(c);
   CK(ca_in_degree(ptr<uint32_t>(c->follower), nLinksDev, maxLinks, b, nTDev, maxT, c->q));
   // in-degree prefix (its total is the number of links; not published)
-  if (mode == SYNCED) CK(ensure(c, c->scanScratch, scan_scratch_bytes(maxT + 1)));
-  CK(scan_exclusive(b.inStart, b.inStart, c->nT + 1, mode == DEVICE ? nTDev : nullptr, 1, maxT + 1,
-                    c->scanScratch.p, dev_err(c), c->q, true, c->wait));
+  RC(scan_publish(c, mode, b.inStart, b.inStart, c->nT, mode == DEVICE ? nTDev : nullptr, maxT, -1, NO_CAP));
   CK(ca_fill(ptr<uint32_t>(c->basis), ptr<uint32_t>(c->follower), nLinksDev, maxLinks, b, nTDev, maxT, c->q));
   CK(ca_forward(c->cfg, b, nTDev, maxT, c->q));
   CK(ca_backward(ptr<float>(c->pt), b, nTDev, maxT, nLinksDev, c->q));
-  RC(scan_publish(c, mode, b.handlers, c->nT, mode == DEVICE ? nTDev : nullptr, maxT, S_TRACKS,
+  RC(scan_publish(c, mode, b.handlers, b.handlers, c->nT, mode == DEVICE ? nTDev : nullptr, maxT, S_TRACKS,
                   mode == DEVICE ? c->capTracks : NO_CAP));
   uint64_t maxTracks = c->capTracks;
   if (mode == SYNCED) {
@@ -801,8 +821,7 @@ int size_device_buffers(trax_ctx* c) {
   ENSURE(states, c->capT, 4); ENSURE(inStart, c->capT + 1, 4); ENSURE(inCursor, c->capT, 4);
   ENSURE(inList, c->capLinks, 4); ENSURE(best, c->capT, 4); ENSURE(isBest, c->capT, 4);
   ENSURE(handlers, c->capT + 1, 4); ENSURE(tracks, c->capTracks, 4);
-  uint64_t maxScan = std::max({c->capTasks, c->capPairs, c->capCands, c->capT, (uint64_t)S}) + 1;
-  CK(ensure(c, c->scanScratch, scan_scratch_bytes(maxScan)));
+  CK(ensure(c, c->scanScratch, chain_scan_bytes(c)));
   return TRAX_OK;
 }
 
@@ -1422,7 +1441,8 @@ int trax_cellular_automaton_on(trax_ctx* c, const uint32_t* basis, const uint32_
   CABuffers b = ca_buffers(c);
   // states 1, in-degrees, the incoming bases of every follower (ascending)
   CK(ca_in_degree(ptr<uint32_t>(c->follower), nLinksDev, nL, b, nTDev, nT, c->q));
-  CK(scan_exclusive(b.inStart, b.inStart, nT + 1, nullptr, 0, nT + 1, c->scanScratch.p, dev_err(c), c->q, true, c->wait));
+  CK(scan_exclusive(b.inStart, b.inStart, nT + 1, nullptr, 0, nT + 1, c->scanScratch.p, false, dev_err(c), c->q, true,
+                    c->wait));
   CK(ca_fill(ptr<uint32_t>(c->basis), ptr<uint32_t>(c->follower), nLinksDev, nL, b, nTDev, nT, c->q));
   // forward phase: the reference's iteration (CellularAutomaton.cpp:37-98),
   // both state buffers starting at 1, swapped without copying; a link set
@@ -1446,7 +1466,7 @@ int trax_cellular_automaton_on(trax_ctx* c, const uint32_t* basis, const uint32_
     CK(cudaMemcpyAsync(c->states.p, cur, nT * 4, cudaMemcpyDeviceToDevice, c->st));
   // backward phase, handlers and tracks as in the chain
   CK(ca_backward(ptr<float>(c->pt), b, nTDev, nT, nLinksDev, c->q));
-  RC(scan_publish(c, SYNCED, b.handlers, nT, nullptr, nT, S_TRACKS, NO_CAP));
+  RC(scan_publish(c, SYNCED, b.handlers, b.handlers, nT, nullptr, nT, S_TRACKS, NO_CAP));
   RC(read_slot(c, S_TRACKS, &c->nTracks));
   ENSURE(tracks, c->nTracks, 4);
   CK(ca_tracks(b, nTDev, nT, ptr<uint32_t>(c->tracks), c->nTracks, dev_err(c), c->q));
@@ -1471,7 +1491,8 @@ int trax_prefix_sum(trax_ctx* c, uint32_t* data, uint64_t n) {
   if (e == cudaSuccess) e = ensure(c, c->scanScratch, scan_scratch_bytes(n));
   if (e == cudaSuccess) e = cudaMemsetAsync(c->slots.p, 0, 4, c->st);
   if (e == cudaSuccess)
-    e = scan_exclusive(ptr<uint32_t>(tmp), ptr<uint32_t>(tmp), n, nullptr, 0, n, c->scanScratch.p, dev_err(c), c->q, false, c->wait);  // wraps like PrefixSum's uint arithmetic
+    e = scan_exclusive(ptr<uint32_t>(tmp), ptr<uint32_t>(tmp), n, nullptr, 0, n, c->scanScratch.p, false, dev_err(c),
+                       c->q, false, c->wait);  // wraps like PrefixSum's uint arithmetic
   if (e == cudaSuccess) e = cudaMemcpyAsync(data, tmp.p, n * 4, cudaMemcpyDeviceToHost, c->st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(c->st);
   if (e != cudaSuccess) rc = cuda_fail(c, e, "trax_prefix_sum");
@@ -1688,10 +1709,10 @@ int trax_physics_tracks_device(trax_ctx* c, uint64_t total_tracks, trax_track_me
   uint32_t* hitsOf = ptr<uint32_t>(c->trk_hitsOf);
   const uint32_t* off = ptr<uint32_t>(c->handlers);
   CK(track_sizes(off, nT, isTrack, hitsOf, c->st));
-  CK(scan_exclusive(isTrack, isTrack, (uint64_t)nT + 1, nullptr, 0, (uint64_t)nT + 1, c->scanScratch.p, dev_err(c),
-                    c->q, true, c->wait));
-  CK(scan_exclusive(hitsOf, hitsOf, (uint64_t)nT + 1, nullptr, 0, (uint64_t)nT + 1, c->scanScratch.p, dev_err(c),
-                    c->q, true, c->wait));
+  CK(scan_exclusive(isTrack, isTrack, (uint64_t)nT + 1, nullptr, 0, (uint64_t)nT + 1, c->scanScratch.p, false,
+                    dev_err(c), c->q, true, c->wait));
+  CK(scan_exclusive(hitsOf, hitsOf, (uint64_t)nT + 1, nullptr, 0, (uint64_t)nT + 1, c->scanScratch.p, false,
+                    dev_err(c), c->q, true, c->wait));
   uint32_t totals[2];
   CK(cudaMemcpyAsync(&totals[0], isTrack + nT, 4, cudaMemcpyDeviceToHost, c->st));
   CK(cudaMemcpyAsync(&totals[1], hitsOf + nT, 4, cudaMemcpyDeviceToHost, c->st));
@@ -1734,7 +1755,7 @@ int trax_physics_tracks_device(trax_ctx* c, uint64_t total_tracks, trax_track_me
   if (!stable) return fail(c, TRAX_ERR_TIMEOUT, "track components did not settle in 64 rounds");
   CK(track_members(t, nTracks, false, c->st));
   CK(scan_exclusive(t.compSize, t.compStart, (uint64_t)nTracks + 1, nullptr, 0, (uint64_t)nTracks + 1,
-                    c->scanScratch.p, dev_err(c), c->q, true, c->wait));
+                    c->scanScratch.p, false, dev_err(c), c->q, true, c->wait));
   CK(track_members(t, nTracks, true, c->st));
   unsigned long long* counts = ptr<unsigned long long>(c->trk_counts);
   CK(track_greedy(t, nTracks, ptr<unsigned long long>(c->trk_table), tableSize - 1, counts, c->st));
@@ -1835,7 +1856,7 @@ int trax_fit_prepare(trax_ctx* c, const trax_fit_opts* opts, uint64_t* n_fit) {
   uint32_t* ok = ptr<uint32_t>(c->fitOk);
   CK(fit_select(f, c->cfg, dev_hits(c), fit_triplets(c), nT, truthOnly, ok, ptr<uint32_t>(c->fitSegCnt), c->st, &c->q.launches));
   CK(ensure(c, c->scanScratch, scan_scratch_bytes(nT + 1)));
-  CK(scan_exclusive(ok, ok, nT + 1, nullptr, 0, nT + 1, c->scanScratch.p, dev_err(c), c->q, true,
+  CK(scan_exclusive(ok, ok, nT + 1, nullptr, 0, nT + 1, c->scanScratch.p, false, dev_err(c), c->q, true,
                     c->wait));
   // 2. rows ordered by layer triplet, then by event (segment order inside a layer triplet)
   std::vector<uint32_t> cnt(S);

@@ -32,6 +32,12 @@ constexpr uint32_t GRID_SMEM_CELLS = TRAX_GRID_SMEM_CELLS;
 // cell, phi and slot of each of the layer's hits (12 bytes per hit)
 constexpr size_t GRID_SMEM_MAX = TRAX_GRID_SMEM_BYTES;
 
+// the scan scratch of the chain's compactions, all of which run after the grid
+__device__ __forceinline__ void clear_scan_scratch(const GridScratch& sc) {
+  for (uint32_t i = blockIdx.x * GRID_THREADS + threadIdx.x; i < sc.clearWords; i += gridDim.x * GRID_THREADS)
+    sc.clear[i] = make_uint4(0u, 0u, 0u, 0u);
+}
+
 // The CTA's exclusive scan of C cell counters in place: cnt[c] becomes the
 // first slot of cell c.  Each thread sums a chunk of consecutive cells,
 // warps scan the sums with shuffles, and the chunks are rewritten.
@@ -93,6 +99,7 @@ __global__ void __launch_bounds__(GRID_THREADS)
     grid_kernel(Stamp stamp, DevConfig cfg, GridInput in, uint32_t* __restrict__ grid, DevHits out, GridScratch sc,
                 uint32_t* err, int useSmem, uint32_t maxHits) {
   stamp_begin(stamp);
+  clear_scan_scratch(sc);
   extern __shared__ uint32_t smem[];
   __shared__ uint32_t s_warpSum[GRID_WARPS];
   const uint32_t task = blockIdx.x;  // event * L + layer
@@ -175,6 +182,7 @@ __global__ void __launch_bounds__(GRID_THREADS)
     grid_kernel16(Stamp stamp, DevConfig cfg, GridInput in, uint32_t* __restrict__ grid, DevHits out, GridScratch sc,
                   uint32_t* err, uint32_t maxHits) {
   stamp_begin(stamp);
+  clear_scan_scratch(sc);
   extern __shared__ uint32_t smem[];
   __shared__ uint32_t s_warpSum[GRID_WARPS];
   const uint32_t task = blockIdx.x;  // event * L + layer
@@ -449,7 +457,7 @@ cudaError_t grid_prepare(int) {
 cudaError_t grid_build(const DevConfig& cfg, const GridInput& in, uint32_t* grid, DevHits out, GridScratch sc,
                        uint32_t maxLayerHits, uint32_t* err, Queue& q) {
   const uint32_t tasks = cfg.E * cfg.L;
-  if (tasks == 0) return cudaSuccess;
+  if (tasks == 0) return cudaMemsetAsync(sc.clear, 0, (size_t)sc.clearWords * 16, q.st);
   const int useSmem = cfg.C <= GRID_SMEM_CELLS ? 1 : 0;
   const size_t counterBytes = useSmem ? (size_t)cfg.C * sizeof(uint32_t) : 0;
   const size_t hitBytes = (size_t)maxLayerHits * 3 * sizeof(uint32_t);

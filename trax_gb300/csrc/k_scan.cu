@@ -8,7 +8,13 @@
 // one with an inclusive prefix is found.  Every wait is bounded: after
 // TRAX_SPIN_LIMIT polls the tile records TRAX_EBIT_TIMEOUT, treats the
 // missing predecessor as zero and finishes, so a lost tile can never hang
-// the GPU.
+// the GPU.  A launch of one tile needs no ticket, status or cleared scratch.
+//
+// A compaction scans count + 1 elements; the tile holding the last one also
+// publishes the total (ScanTotal), clamped to the capacity of what follows.
+// With the scratch of a whole chain cleared by its first kernel, a
+// compaction is one launch instead of three nodes (clear, scan, publish),
+// each of them 2 to 3 us in a serial graph.
 #include "trax_kernels.h"
 #include "trax_lookback.cuh"
 
@@ -23,14 +29,14 @@ constexpr uint32_t SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
 __global__ void __launch_bounds__(SCAN_THREADS)
     scan_kernel(Stamp stamp, const uint32_t* __restrict__ in, uint32_t* out, uint64_t nHost, const uint32_t* nDev,
                 uint32_t nAdd, unsigned long long* status, uint32_t* ticket, uint32_t* err, uint32_t overflowBit,
-                WaitCtl ctl) {
+                WaitCtl ctl, ScanTotal total) {
   stamp_begin(stamp);
   __shared__ uint32_t s_tile;
   __shared__ uint32_t s_warp[SCAN_THREADS / 32];
   __shared__ unsigned long long s_wide[SCAN_THREADS / 32];
   __shared__ uint32_t s_prefix;
   const uint64_t n = nDev ? (uint64_t)(*nDev) + nAdd : nHost;
-  if (threadIdx.x == 0) s_tile = atomicAdd(ticket, 1u);
+  if (threadIdx.x == 0) s_tile = gridDim.x > 1 ? atomicAdd(ticket, 1u) : 0u;
   __syncthreads();
   const uint32_t tile = s_tile;
   const uint64_t base = (uint64_t)tile * SCAN_TILE;
@@ -88,7 +94,7 @@ __global__ void __launch_bounds__(SCAN_THREADS)
     agg = __shfl_sync(0xffffffffu, agg, 0);
     // publish and look back (bounded waits); the 32-bit outputs wrap like the
     // reference's uint scan, the exact total flags a count past 2^32
-    const unsigned long long excl = lb_exclusive_prefix(status, tile, agg, err, ctl);
+    const unsigned long long excl = gridDim.x > 1 ? lb_exclusive_prefix(status, tile, agg, err, ctl) : 0ull;
     if (lane == 0) {
       s_prefix = (uint32_t)excl;
       if (overflowBit && excl + agg > 0xffffffffull) raise_error(err, overflowBit);
@@ -105,6 +111,17 @@ __global__ void __launch_bounds__(SCAN_THREADS)
 #pragma unroll
     for (int k = 0; k < SCAN_ITEMS; ++k)
       if (i0 + k < n) out[i0 + k] = off + v[k];
+  }
+  if (total.dst && i0 < n && i0 + SCAN_ITEMS >= n) {  // holds element n - 1
+    uint32_t t = 0;
+#pragma unroll
+    for (int k = 0; k < SCAN_ITEMS; ++k)
+      if (i0 + k + 1 == n) t = off + v[k];
+    if (t > total.cap) {
+      t = total.cap;
+      raise_error(err, TRAX_EBIT_CAPACITY);
+    }
+    *total.dst = t;
   }
 }
 
@@ -146,19 +163,6 @@ __global__ void __launch_bounds__(1024) max_scan_kernel(Stamp stamp, uint32_t* d
   }
 }
 
-// dst = data[n] with n = *nDev (or nHost), clamped to cap
-__global__ void publish_kernel(Stamp stamp, const uint32_t* data, const uint32_t* nDev, uint32_t nHost, uint32_t cap,
-                               uint32_t* dst, uint32_t* err) {
-  stamp_begin(stamp);
-  const uint32_t n = nDev ? *nDev : nHost;
-  uint32_t v = data[n];
-  if (v > cap) {
-    v = cap;
-    raise_error(err, TRAX_EBIT_CAPACITY);
-  }
-  *dst = v;
-}
-
 // the context's slots and time marks to page-locked host memory
 __global__ void slots_to_host_kernel(Stamp stamp, const uint32_t* slots, uint32_t* host, uint32_t n) {
   stamp_begin(stamp);
@@ -173,31 +177,25 @@ cudaError_t slots_to_host(const uint32_t* slots, uint32_t* host, uint32_t words,
   return cudaGetLastError();
 }
 
-cudaError_t publish_total(const uint32_t* data, const uint32_t* nDev, uint64_t nHost, uint64_t cap, uint32_t* dst,
-                          uint32_t* err, Queue& q) {
-  const uint32_t c = cap > 0xffffffffull ? 0xffffffffu : (uint32_t)cap;
-  launch(q, publish_kernel, 1, 1, 0, data, nDev, (uint32_t)nHost, c, dst, err);
-  return cudaGetLastError();
-}
-
 size_t scan_scratch_bytes(uint64_t maxN) {
   uint64_t tiles = (maxN + SCAN_TILE - 1) / SCAN_TILE + 1;
-  return 256 + tiles * sizeof(unsigned long long);
+  return (256 + tiles * sizeof(unsigned long long) + 255) / 256 * 256;
 }
 
 cudaError_t scan_exclusive(const uint32_t* in, uint32_t* out, uint64_t n, const uint32_t* nDev, uint32_t nAdd,
-                           uint64_t maxN, void* scratch, uint32_t* err, Queue& q,
-                           bool flagOverflow, WaitCtl ctl) {
+                           uint64_t maxN, void* scratch, bool cleared, uint32_t* err, Queue& q, bool flagOverflow,
+                           WaitCtl ctl, ScanTotal total) {
   uint64_t cap = nDev ? maxN : n;
   if (cap == 0) return cudaSuccess;
   uint64_t tiles = (cap + SCAN_TILE - 1) / SCAN_TILE;
-  size_t bytes = 256 + tiles * sizeof(unsigned long long);
-  cudaError_t e = cudaMemsetAsync(scratch, 0, bytes, q.st);
-  if (e != cudaSuccess) return e;
+  if (tiles > 1 && !cleared) {
+    cudaError_t e = cudaMemsetAsync(scratch, 0, 256 + tiles * sizeof(unsigned long long), q.st);
+    if (e != cudaSuccess) return e;
+  }
   uint32_t* ticket = reinterpret_cast<uint32_t*>(scratch);
   unsigned long long* status = reinterpret_cast<unsigned long long*>(static_cast<char*>(scratch) + 256);
   launch(q, scan_kernel, (unsigned)tiles, SCAN_THREADS, 0, in, out, n, nDev, nAdd, status, ticket, err,
-         flagOverflow ? TRAX_EBIT_OVERFLOW : 0u, ctl);
+         flagOverflow ? TRAX_EBIT_OVERFLOW : 0u, ctl, total);
   return cudaGetLastError();
 }
 
@@ -291,7 +289,8 @@ extern "C" int trax_prefix_sum_noalloc(const uint32_t* d_in, uint32_t* d_out, ui
   e = cudaMemsetAsync(base, 0, NOALLOC_HEADER + tiles * sizeof(unsigned long long), st);
   if (e == cudaSuccess) {
     trax::scan_kernel<<<(unsigned)tiles, trax::SCAN_THREADS, 0, st>>>(trax::Stamp{}, d_in, d_out, n, nullptr, 0, status, ticket,
-                                                                      err, 0u, noalloc_wait());
+                                                                      err, 0u, noalloc_wait(),
+                                                                      trax::ScanTotal{});
     e = cudaGetLastError();
   }
   uint32_t hostErr = 0;

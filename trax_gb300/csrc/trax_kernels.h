@@ -38,13 +38,21 @@ cudaError_t launch(Queue& q, void (*kernel)(Stamp, P...), unsigned blocks, unsig
 
 // ---------------------------------------------------------------- scans
 size_t scan_scratch_bytes(uint64_t maxN);
+// Where a scan of count + 1 elements leaves its total (the last output),
+// clamped to cap (TRAX_EBIT_CAPACITY); dst null: nowhere.
+struct ScanTotal {
+  uint32_t* dst = nullptr;
+  uint32_t cap = 0xffffffffu;
+};
 // Exclusive scan of n elements (or *nDev + nAdd when nDev != nullptr, with
 // maxN bounding the launch), in place allowed.  Outputs wrap modulo 2^32;
 // with flagOverflow a total of 2^32 or more sets TRAX_EBIT_OVERFLOW.  `ctl`
 // bounds the look-back waits (and may name a tile that never publishes).
+// `scratch` holds scan_scratch_bytes(maxN), `cleared`: zero already and used
+// by no other scan since (otherwise it is cleared here).
 cudaError_t scan_exclusive(const uint32_t* in, uint32_t* out, uint64_t n, const uint32_t* nDev, uint32_t nAdd,
-                           uint64_t maxN, void* scratch, uint32_t* err, Queue& q,
-                           bool flagOverflow, WaitCtl ctl);
+                           uint64_t maxN, void* scratch, bool cleared, uint32_t* err, Queue& q, bool flagOverflow,
+                           WaitCtl ctl, ScanTotal total = ScanTotal{});
 cudaError_t max_scan_inclusive(uint32_t* data, uint32_t n, Queue& q);
 
 // ------------------------------------------------------ event bucketing
@@ -146,6 +154,8 @@ struct GridScratch {
   float* phi;        // [n]
   uint32_t* perm;    // [n]
   uint32_t* counts;  // [E*L*C] used when the cell counters do not fit in shared memory
+  uint4* clear;      // scan scratch of the chain, zeroed by the grid build (clearWords of 16 bytes)
+  uint32_t clearWords;
 };
 
 cudaError_t grid_build(const DevConfig& cfg, const GridInput& in, uint32_t* grid, DevHits out,
@@ -288,11 +298,6 @@ cudaError_t connectable_words(const uint32_t* flags, const uint32_t* nTDev, uint
 // below k in its word)] = k for every set bit k < *nTDev
 cudaError_t compact_words(const uint32_t* words, const uint32_t* wordStart, const uint32_t* nTDev, uint64_t maxT,
                           uint32_t* outIdx, uint64_t capOut, Queue& q);
-// *dst = data[n] (n = *nDev, or nHost when nDev is null): the total a scan of
-// n+1 elements left in its last slot, clamped to cap (TRAX_EBIT_CAPACITY)
-cudaError_t publish_total(const uint32_t* data, const uint32_t* nDev, uint64_t nHost, uint64_t cap, uint32_t* dst,
-                          uint32_t* err, Queue& q);
-
 // the context's slots and the time marks after them to page-locked host memory
 cudaError_t slots_to_host(const uint32_t* slots, uint32_t* host, uint32_t words, Queue& q);
 
