@@ -536,14 +536,14 @@ __global__ void predict_offsets_kernel(Stamp stamp, uint32_t S, const uint32_t* 
 }
 
 // The flags in two steps, each warp on its own (no block barriers): a warp
-// takes 1024 consecutive candidates, 32 at a time; every candidate takes the
+// takes up to 1024 consecutive candidates, 32 at a time; every candidate takes the
 // dphi test, which rejects most of them, and the survivors go to the warp's
 // queue in shared memory.  The dphi test is decided from the cross and dot
 // products of the two transverse segments wherever the angle is more than
 // 1e-4 rad from the cut, which leaves the two atan2 to a few candidates in
 // ten thousand (0.87 -> 0.55 ms on the 1000-event batch).  Whenever the queue holds 32 the warp
 // runs the dtheta / TIP / curvature tests on them with every lane busy, and
-// it empties the queue at the end of its 1024.  The flag is the AND of
+// it empties the queue at the end of its candidates.  The flag is the AND of
 // filterCount's four predicates (TripletThetaPhiFilter.h:65-154).
 // filterPopCount + PrefixSum run on words of 32 flags: the flags of 32
 // consecutive candidates are one word of masks, the number set goes to
@@ -555,15 +555,21 @@ __global__ void predict_offsets_kernel(Stamp stamp, uint32_t S, const uint32_t* 
 __global__ void __launch_bounds__(TRAX_MAX_TUNED_THREADS, 8)
     filter_kernel(Stamp stamp, DevConfig cfg, const float4* __restrict__ hits, const uint32_t* __restrict__ hitLayer,
                   const uint2* __restrict__ pairs, const uint2* __restrict__ cands, const uint32_t* nCandsDev,
-                  uint32_t* masks, uint32_t* warpSums, uint32_t* nWordsOut) {
+                  uint32_t* masks, uint32_t* warpSums, uint32_t* nWordsOut, uint32_t residentWarps) {
   stamp_begin(stamp);
-  constexpr uint32_t WORDS = 32;  // a warp takes 32 words = 1024 candidates at a time
+  constexpr uint32_t WORDS = 32;
   __shared__ uint32_t s_queue[TRAX_MAX_TUNED_THREADS / 32][64];
   __shared__ uint32_t s_queue2[TRAX_MAX_TUNED_THREADS / 32][64];
   __shared__ uint32_t s_bits[TRAX_MAX_TUNED_THREADS / 32][WORDS];
   const uint32_t n = *nCandsDev;
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+  // A warp takes `words` words of 32 candidates at a time: 32 of them when
+  // that fills the chip, fewer (down to one) while warps would stay idle.
+  // Longer runs keep the queues' rounds full, shorter ones share the work:
+  // always 32 took 63 us for 57 k candidates (56 warps on the chip; 5 us
+  // now) and 92 us for 1.9 M (30 us now); the 49 M of 1000 events keep 32.
+  const uint32_t words = min(WORDS, n / (32u * residentWarps) + 1u);
   uint32_t* queue = s_queue[warp];
   uint32_t* queue2 = s_queue2[warp];
   uint32_t* bits = s_bits[warp];
@@ -614,17 +620,19 @@ __global__ void __launch_bounds__(TRAX_MAX_TUNED_THREADS, 8)
       __syncwarp();
     }
   };
-  for (uint32_t g0 = (blockIdx.x * (blockDim.x >> 5) + warp) * (WORDS * 32); g0 < n; g0 += warps * WORDS * 32) {
+  for (uint64_t g64 = (uint64_t)(blockIdx.x * (blockDim.x >> 5) + warp) * (words * 32); g64 < n;
+       g64 += (uint64_t)warps * words * 32) {
+    const uint32_t g0 = (uint32_t)g64;
     bits[lane] = 0u;
     uint32_t queued = 0;  // warp-uniform
     __syncwarp();
     // each lane's next candidate is loaded one step ahead (0.499 -> 0.482 ms
     // on the ttbar-like batch; its pair as well, or 40 registers, were slower)
     uint2 cN = g0 + lane < n ? cands[g0 + lane] : make_uint2(0u, TRAX_SENTINEL);
-    for (uint32_t k = 0; k < WORDS; ++k) {
+    for (uint32_t k = 0; k < words; ++k) {
       const uint32_t g = g0 + k * 32 + lane;
       const uint2 c = cN;
-      if (k + 1 < WORDS) cN = g + 32 < n ? cands[g + 32] : make_uint2(0u, TRAX_SENTINEL);
+      if (k + 1 < words) cN = g + 32 < n ? cands[g + 32] : make_uint2(0u, TRAX_SENTINEL);
       bool pass = false;
       if (c.y != TRAX_SENTINEL) {  // a slot the reference never wrote fails
         const uint2 pr = pairs[c.x];
@@ -647,7 +655,7 @@ __global__ void __launch_bounds__(TRAX_MAX_TUNED_THREADS, 8)
     dtheta_round(g0, queued2);
     queued2 = 0;
     const uint32_t word = (g0 >> 5) + lane;
-    if (g0 + lane * 32 < n) {
+    if (lane < words && g64 + lane * 32 < n) {
       const uint32_t b = bits[lane];
       masks[word] = b;
       warpSums[word] = (uint32_t)__popc(b);
@@ -798,7 +806,7 @@ cudaError_t filter_candidates(const DevConfig& cfg, DevHits hits, const uint2* p
                               uint32_t* nWordsOut, Queue& q) {
   const int threads = (int)cfg.filterThreads;
   launch(q, filter_kernel, grid_for(maxCands + 1, threads), threads, 0, cfg, hits.xyzp, hits.layer, pairs, cands,
-         nCandsDev, masks, warpSums, nWordsOut);
+         nCandsDev, masks, warpSums, nWordsOut, (uint32_t)sm_count() * 64u);
   return cudaGetLastError();
 }
 
