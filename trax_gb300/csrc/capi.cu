@@ -490,8 +490,10 @@ int stage_pairs(trax_ctx* c, Mode mode) {
   ENSURE(taskBase, S + 1, 4);
   ENSURE(pairOffsets, S + 1, 4);
   uint32_t* taskBase = ptr<uint32_t>(c->taskBase);
-  CK(pair_segments(c->cfg, ptr<uint32_t>(c->grid), ptr<uint32_t>(c->segOuter), taskBase, c->q));
-  RC(scan_publish(c, mode, taskBase, taskBase, S, nullptr, S, S_TASKS, mode == DEVICE ? c->capTasks : NO_CAP));
+  const uint64_t capTasks = mode == DEVICE ? c->capTasks : NO_CAP;
+  CK(pair_segments(c->cfg, ptr<uint32_t>(c->grid), ptr<uint32_t>(c->segOuter), taskBase,
+                   ScanTotal{slot(c, S_TASKS), (uint32_t)std::min(capTasks, NO_CAP)}, dev_err(c), c->q));
+  if (S > TRAX_SEGMENT_SCAN) RC(scan_publish(c, mode, taskBase, taskBase, S, nullptr, S, S_TASKS, capTasks));
   const uint32_t* nTasksDev = slot(c, S_TASKS);
   uint64_t maxTasks = c->capTasks;
   if (mode == SYNCED) {
@@ -504,7 +506,7 @@ int stage_pairs(trax_ctx* c, Mode mode) {
   const PairTaskState taskState = pair_task_state(c->taskState.p, maxTasks);
   KBEG(TK_PAIR_COUNT);
   CK(pair_tasks(c->cfg, false, ptr<uint32_t>(c->grid), dev_hits(c), ptr<uint32_t>(c->segOuter), taskBase, nTasksDev,
-                maxTasks, taskCount, taskState, nullptr, 0, slot(c, S_PAIR_SENT), dev_err(c), c->q));
+                maxTasks, taskCount, taskState, nullptr, 0, nullptr, slot(c, S_PAIR_SENT), dev_err(c), c->q));
   KEND(TK_PAIR_COUNT);
   RC(scan_publish(c, mode, taskCount, taskCount, c->nTasks, mode == DEVICE ? nTasksDev : nullptr, maxTasks, S_PAIRS,
                   mode == DEVICE ? c->capPairs : NO_CAP));
@@ -516,10 +518,9 @@ int stage_pairs(trax_ctx* c, Mode mode) {
   ENSURE(pairs, maxPairs, 8);
   KBEG(TK_PAIR_EMIT);
   CK(pair_tasks(c->cfg, true, ptr<uint32_t>(c->grid), dev_hits(c), ptr<uint32_t>(c->segOuter), taskBase, nTasksDev,
-                maxTasks, taskCount, taskState, ptr<uint2>(c->pairs), maxPairs, slot(c, S_PAIR_SENT), dev_err(c),
+                maxTasks, taskCount, taskState, ptr<uint2>(c->pairs), maxPairs, ptr<uint32_t>(c->pairOffsets), slot(c, S_PAIR_SENT), dev_err(c),
                 c->q));
   KEND(TK_PAIR_EMIT);
-  CK(pair_offsets(c->cfg, taskBase, taskCount, ptr<uint32_t>(c->pairOffsets), c->q));
   return TRAX_OK;
 }
 
@@ -540,7 +541,7 @@ int stage_predict(trax_ctx* c, Mode mode) {
   KBEG(TK_PRED_COUNT);
   CK(predict_pairs(c->cfg, false, ptr<uint32_t>(c->grid), dev_hits(c), ptr<uint2>(c->pairs), nPairsDev, maxPairs,
                    candLocal, warpSums, slot(c, S_PRED_WARPS), ptr<uint32_t>(c->predKeep), nullptr, 0,
-                   slot(c, S_CAND_SENT), dev_err(c), c->q, fine_grid(c)));
+                   slot(c, S_CAND_SENT), dev_err(c), c->q, fine_grid(c), nullptr, nullptr));
   KEND(TK_PRED_COUNT);
   // the prefix sum runs over the per-warp sums of the counts
   RC(scan_publish(c, mode, warpSums, warpSums, (c->nPairs + 31) / 32, mode == DEVICE ? slot(c, S_PRED_WARPS) : nullptr,
@@ -554,10 +555,9 @@ int stage_predict(trax_ctx* c, Mode mode) {
   KBEG(TK_PRED_EMIT);
   CK(predict_pairs(c->cfg, true, ptr<uint32_t>(c->grid), dev_hits(c), ptr<uint2>(c->pairs), nPairsDev, maxPairs,
                    candLocal, warpSums, nullptr, ptr<uint32_t>(c->predKeep), ptr<uint2>(c->cands), maxCands,
-                   slot(c, S_CAND_SENT), dev_err(c), c->q, fine_grid(c)));
+                   slot(c, S_CAND_SENT), dev_err(c), c->q, fine_grid(c), ptr<uint32_t>(c->pairOffsets),
+                   ptr<uint32_t>(c->candOffsets)));
   KEND(TK_PRED_EMIT);
-  CK(predict_offsets(c->cfg, ptr<uint32_t>(c->pairOffsets), nPairsDev, candLocal, warpSums,
-                     ptr<uint32_t>(c->candOffsets), c->q));
   return TRAX_OK;
 }
 

@@ -197,15 +197,84 @@ __global__ void segments_kernel(Stamp stamp, DevConfig cfg, const uint32_t* __re
   if (blockIdx.x == 0 && threadIdx.x == 0) segCount[S] = 0u;
 }
 
+// segments_kernel and the scan of its counts in one CTA, SEG_ITEMS
+// consecutive segments per thread and step: one launch instead of two where
+// a few steps cover the segments (6000 of them: one).
+constexpr int SEG_THREADS = 1024, SEG_ITEMS = 8;
+__global__ void __launch_bounds__(SEG_THREADS)
+    segments_scan_kernel(Stamp stamp, DevConfig cfg, const uint32_t* __restrict__ grid, uint32_t* segOuter,
+                         uint32_t* taskBase, ScanTotal total, uint32_t* err) {
+  stamp_begin(stamp);
+  __shared__ unsigned long long s_warp[SEG_THREADS / 32];
+  const uint32_t S = cfg.E * cfg.nLT;
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  unsigned long long carry = 0;
+  for (uint32_t s0 = 0; s0 <= S; s0 += SEG_THREADS * SEG_ITEMS) {
+    const uint32_t a = s0 + threadIdx.x * SEG_ITEMS;
+    uint32_t n[SEG_ITEMS];
+    unsigned long long sum = 0;
+#pragma unroll
+    for (int k = 0; k < SEG_ITEMS; ++k) {
+      const uint32_t s = a + k;
+      n[k] = 0u;
+      if (s < S) {
+        const uint32_t* lG2 = grid + ((size_t)(s / cfg.nLT) * cfg.L + (cfg.layer2[s % cfg.nLT] - 1)) * cfg.C;
+        const uint32_t l2off = lG2[0];
+        segOuter[s] = l2off;
+        n[k] = lG2[cfg.C - 1] - l2off;  // PairGeneratorBeamspot.h:70-73
+      }
+      sum += n[k];
+    }
+    unsigned long long incl = sum;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const unsigned long long t = __shfl_up_sync(0xffffffffu, incl, d);
+      if (lane >= (uint32_t)d) incl += t;
+    }
+    if (lane == 31) s_warp[warp] = incl;
+    __syncthreads();
+    if (warp == 0) {
+      unsigned long long w = s_warp[lane];
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const unsigned long long t = __shfl_up_sync(0xffffffffu, w, d);
+        if (lane >= (uint32_t)d) w += t;
+      }
+      s_warp[lane] = w;  // inclusive over the warps
+    }
+    __syncthreads();
+    unsigned long long run = carry + (warp ? s_warp[warp - 1] : 0ull) + incl - sum;
+#pragma unroll
+    for (int k = 0; k < SEG_ITEMS; ++k) {
+      if (a + k <= S) taskBase[a + k] = (uint32_t)run;
+      if (a + k == S) {  // the total
+        if (run > 0xffffffffull) raise_error(err, TRAX_EBIT_OVERFLOW);
+        uint32_t t = (uint32_t)run;
+        if (t > total.cap) {
+          t = total.cap;
+          raise_error(err, TRAX_EBIT_CAPACITY);
+        }
+        *total.dst = t;
+      }
+      run += n[k];
+    }
+    carry += s_warp[SEG_THREADS / 32 - 1];
+    __syncthreads();
+  }
+}
+
 template <bool EMIT>
 __global__ void __launch_bounds__(TRAX_MAX_TUNED_THREADS)
     pair_kernel(Stamp stamp, DevConfig cfg, const uint32_t* __restrict__ grid, const float4* __restrict__ hits,
                 const uint32_t* __restrict__ segOuter, const uint32_t* __restrict__ taskBase,
                 const uint32_t* __restrict__ nTasksDev, uint32_t* taskCount, PairTaskState state, uint2* pairs,
-                uint32_t capPairs, uint32_t* sentinels, uint32_t* err) {
+                uint32_t capPairs, uint32_t* pairOffsets, uint32_t* sentinels, uint32_t* err) {
   stamp_begin(stamp);
   const uint32_t S = cfg.E * cfg.nLT;
   const uint32_t nTasks = *nTasksDev;
+  if (EMIT)  // taskCount is scanned: the first pair of every segment
+    for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s <= S; s += gridDim.x * blockDim.x)
+      pairOffsets[s] = s == 0 ? 0u : taskCount[min(taskBase[s], nTasks)];
   const uint32_t C = cfg.C, nP = cfg.nP;
   for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < nTasks; k += gridDim.x * blockDim.x) {
     uint32_t s, i;
@@ -307,14 +376,6 @@ __global__ void __launch_bounds__(TRAX_MAX_TUNED_THREADS)
   if (!EMIT && blockIdx.x == 0 && threadIdx.x == 0) taskCount[nTasks] = 0u;  // the scan's +1 slot
 }
 
-__global__ void pair_offsets_kernel(Stamp stamp, DevConfig cfg, const uint32_t* taskBase, const uint32_t* pairStart,
-                                    uint32_t* pairOffsets) {
-  stamp_begin(stamp);
-  const uint32_t S = cfg.E * cfg.nLT;
-  for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s <= S; s += gridDim.x * blockDim.x)
-    pairOffsets[s] = s == 0 ? 0u : pairStart[taskBase[s]];
-}
-
 int grid_for(uint64_t items, int threads) {
   uint64_t blocks = (items + threads - 1) / threads;
   uint64_t cap = (uint64_t)sm_count() * (4096 / threads);  // two waves at full occupancy
@@ -325,34 +386,29 @@ int grid_for(uint64_t items, int threads) {
 
 }  // namespace
 
-cudaError_t pair_segments(const DevConfig& cfg, const uint32_t* grid, uint32_t* segOuter, uint32_t* segCount,
-                          Queue& q) {
+cudaError_t pair_segments(const DevConfig& cfg, const uint32_t* grid, uint32_t* segOuter, uint32_t* taskBase,
+                          ScanTotal total, uint32_t* err, Queue& q) {
   const uint32_t S = cfg.E * cfg.nLT;
-  launch(q, segments_kernel, grid_for(S + 1, 256), 256, 0, cfg, grid, segOuter, segCount);
+  if (S <= TRAX_SEGMENT_SCAN)
+    launch(q, segments_scan_kernel, 1, SEG_THREADS, 0, cfg, grid, segOuter, taskBase, total, err);
+  else
+    launch(q, segments_kernel, grid_for(S + 1, 256), 256, 0, cfg, grid, segOuter, taskBase);
   return cudaGetLastError();
 }
 
 cudaError_t pair_tasks(const DevConfig& cfg, bool emit, const uint32_t* grid, DevHits hits, const uint32_t* segOuter,
                        const uint32_t* taskBase, const uint32_t* nTasksDev, uint64_t maxTasks, uint32_t* taskCount,
-                       PairTaskState state, uint2* pairs, uint64_t capPairs, uint32_t* sentinels, uint32_t* err,
-                       Queue& q) {
+                       PairTaskState state, uint2* pairs, uint64_t capPairs, uint32_t* pairOffsets,
+                       uint32_t* sentinels, uint32_t* err, Queue& q) {
   const uint32_t cap = capPairs > 0xffffffffull ? 0xffffffffu : (uint32_t)capPairs;
-  if (emit && maxTasks == 0) return cudaSuccess;
   const int threads = (int)cfg.pairThreads;
   const int blocks = grid_for(maxTasks + 1, threads);
   if (emit)
     launch(q, pair_kernel<true>, blocks, threads, 0, cfg, grid, hits.xyzp, segOuter, taskBase, nTasksDev, taskCount,
-           state, pairs, cap, sentinels, err);
+           state, pairs, cap, pairOffsets, sentinels, err);
   else
     launch(q, pair_kernel<false>, blocks, threads, 0, cfg, grid, hits.xyzp, segOuter, taskBase, nTasksDev,
-           taskCount, state, pairs, cap, sentinels, err);
-  return cudaGetLastError();
-}
-
-cudaError_t pair_offsets(const DevConfig& cfg, const uint32_t* taskBase, const uint32_t* pairStart,
-                         uint32_t* pairOffsets, Queue& q) {
-  const uint32_t S = cfg.E * cfg.nLT;
-  launch(q, pair_offsets_kernel, grid_for(S + 1, 256), 256, 0, cfg, taskBase, pairStart, pairOffsets);
+           taskCount, state, pairs, cap, pairOffsets, sentinels, err);
   return cudaGetLastError();
 }
 

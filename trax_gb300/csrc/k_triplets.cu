@@ -453,9 +453,21 @@ __global__ void __launch_bounds__(TRAX_MAX_TUNED_THREADS, FINE ? 6 : 8)
                          const uint2* __restrict__ pairs, const uint32_t* __restrict__ nPairsDev,
                          const uint32_t* __restrict__ local, const uint32_t* __restrict__ warpStart,
                          const uint32_t* __restrict__ keep, uint2* cands, uint32_t capCands, uint32_t* sentinels,
-                         FineGrid fine) {
+                         FineGrid fine, const uint32_t* __restrict__ pairOffsets, uint32_t* candOffsets) {
   stamp_begin(stamp);
   const uint32_t nPairs = *nPairsDev;
+  // tripletOffsets of predictStore (:404-418) + predictOffsetMonotonizeStore
+  // (:432-447).  The last non-sentinel pair of a segment stores the candidate
+  // position after it, and empty segments inherit their predecessor's value;
+  // pairs of a segment are contiguous and sentinel pairs count zero
+  // candidates, so both come down to the candidate position at the segment's
+  // pair end.
+  for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s <= cfg.E * cfg.nLT; s += gridDim.x * blockDim.x) {
+    const uint32_t p = min(pairOffsets[s], nPairs);
+    candOffsets[s] = s == 0      ? 0u
+                     : p == nPairs ? warpStart[(nPairs + 31u) >> 5]
+                                   : warpStart[p >> 5] + local[p];
+  }
   uint32_t sent = 0;
   for (uint32_t gid = blockIdx.x * blockDim.x + threadIdx.x; gid < nPairs; gid += gridDim.x * blockDim.x) {
     const uint32_t wi = gid >> 5;
@@ -512,27 +524,6 @@ __global__ void __launch_bounds__(TRAX_MAX_TUNED_THREADS, FINE ? 6 : 8)
   }
   for (int d = 16; d > 0; d >>= 1) sent += __shfl_down_sync(0xffffffffu, sent, d);
   if ((threadIdx.x & 31u) == 0 && sent) atomicAdd(sentinels, sent);
-}
-
-// tripletOffsets of predictStore (:404-418) + predictOffsetMonotonizeStore
-// (:432-447).  The last non-sentinel pair of a segment stores the candidate
-// position after it, and empty segments inherit their predecessor's value;
-// pairs of a segment are contiguous and sentinel pairs count zero
-// candidates, so both come down to the candidate position at the segment's
-// pair end.
-__global__ void predict_offsets_kernel(Stamp stamp, uint32_t S, const uint32_t* __restrict__ pairOffsets,
-                                       const uint32_t* __restrict__ nPairsDev, const uint32_t* __restrict__ local,
-                                       const uint32_t* __restrict__ warpStart, uint32_t* offsets) {
-  stamp_begin(stamp);
-  const uint32_t nPairs = *nPairsDev;
-  for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s <= S; s += gridDim.x * blockDim.x) {
-    if (s == 0) {
-      offsets[0] = 0u;
-      continue;
-    }
-    const uint32_t p = min(pairOffsets[s], nPairs);
-    offsets[s] = p == nPairs ? warpStart[(nPairs + 31u) >> 5] : warpStart[p >> 5] + local[p];
-  }
 }
 
 // The flags in two steps, each warp on its own (no block barriers): a warp
@@ -670,7 +661,8 @@ __global__ void __launch_bounds__(TRAX_MAX_TUNED_THREADS, 8)
 }
 
 // filterStore: (h1, h2, h3) of every flagged candidate, in candidate order.
-// A warp takes 32 flag words (1024 candidates), whose triplets occupy the
+// A warp takes 32 flag words (1024 candidates; fewer while warps would stay
+// idle, as in filter_kernel), whose triplets occupy the
 // positions wordStart[w0] + 0, 1, ...: each lane writes one of them per
 // step, finding its word by a 5-step search over the words' running counts
 // and its candidate by the rank of the bit in the word (0.21 -> 0.15 ms on
@@ -678,14 +670,15 @@ __global__ void __launch_bounds__(TRAX_MAX_TUNED_THREADS, 8)
 __global__ void filter_store_kernel(Stamp stamp, const uint2* __restrict__ pairs, const uint2* __restrict__ cands,
                                     const uint32_t* nCandsDev, const uint32_t* __restrict__ masks,
                                     const uint32_t* __restrict__ wordStart, uint32_t* h1, uint32_t* h2, uint32_t* h3,
-                                    uint32_t capT) {
+                                    uint32_t capT, uint32_t residentWarps) {
   stamp_begin(stamp);
   const uint32_t n = *nCandsDev;
   const uint32_t nW = (n + 31u) >> 5;
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t warps = gridDim.x * (blockDim.x >> 5);
-  for (uint32_t w0 = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * 32u; w0 < nW; w0 += warps * 32u) {
-    const uint32_t word = w0 + lane < nW ? masks[w0 + lane] : 0u;
+  const uint32_t words = min(32u, nW / residentWarps + 1u);
+  for (uint32_t w0 = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * words; w0 < nW; w0 += warps * words) {
+    const uint32_t word = lane < words && w0 + lane < nW ? masks[w0 + lane] : 0u;
     const uint32_t base = wordStart[w0];
     uint32_t incl = (uint32_t)__popc(word);
 #pragma unroll
@@ -753,22 +746,23 @@ bool pred_k_fits(const DevConfig& cfg) {
 cudaError_t predict_pairs(const DevConfig& cfg, bool emit, const uint32_t* grid, DevHits hits, const uint2* pairs,
                           const uint32_t* nPairsDev, uint64_t maxPairs, uint32_t* candCount, uint32_t* warpSums,
                           uint32_t* nWarpsOut, uint32_t* keep, uint2* cands, uint64_t capCands, uint32_t* sentinels,
-                          uint32_t* err, Queue& q, FineGrid fine) {
+                          uint32_t* err, Queue& q, FineGrid fine,
+                          const uint32_t* pairOffsets, uint32_t* candOffsets) {
   const uint32_t cap = capCands > 0xffffffffull ? 0xffffffffu : (uint32_t)capCands;
   const int threads = (int)cfg.predThreads;
   const int blocks = grid_for(maxPairs + 1, threads);
   const bool il = keep_interleaved(cfg);
   if (emit) {
-    if (maxPairs == 0) return cudaSuccess;
     if (cfg.fineRows > 0 && fine.grid)
       launch(q, (predict_store_kernel<true, true>), blocks, threads, 0, cfg, grid, hits.xyzp, hits.evt, hits.layer,
-             pairs, nPairsDev, candCount, warpSums, keep, cands, cap, sentinels, fine);
+             pairs, nPairsDev, candCount, warpSums, keep, cands, cap, sentinels, fine, pairOffsets, candOffsets);
     else if (il)
       launch(q, (predict_store_kernel<true, false>), blocks, threads, 0, cfg, grid, hits.xyzp, hits.evt, hits.layer,
-             pairs, nPairsDev, candCount, warpSums, keep, cands, cap, sentinels, fine);
+             pairs, nPairsDev, candCount, warpSums, keep, cands, cap, sentinels, fine, pairOffsets, candOffsets);
     else
       launch(q, (predict_store_kernel<false, false>), blocks, threads, 0, cfg, grid, hits.xyzp, hits.evt,
-             hits.layer, pairs, nPairsDev, candCount, warpSums, keep, cands, cap, sentinels, fine);
+             hits.layer, pairs, nPairsDev, candCount, warpSums, keep, cands, cap, sentinels, fine, pairOffsets,
+             candOffsets);
   } else if (cfg.fineRows > 0 && fine.grid) {
     launch(q, (predict_count_kernel<true, true>), blocks, threads, 0, cfg, grid, hits.xyzp, hits.evt, hits.layer,
            pairs, nPairsDev, candCount, keep, warpSums, nWarpsOut, err, fine);
@@ -792,15 +786,6 @@ cudaError_t predict_pairs(const DevConfig& cfg, bool emit, const uint32_t* grid,
   return cudaGetLastError();
 }
 
-cudaError_t predict_offsets(const DevConfig& cfg, const uint32_t* pairOffsets, const uint32_t* nPairsDev,
-                            const uint32_t* candCount, const uint32_t* warpStart, uint32_t* candOffsets,
-                            Queue& q) {
-  const uint32_t S = cfg.E * cfg.nLT;
-  launch(q, predict_offsets_kernel, grid_for(S + 1, 256), 256, 0, S, pairOffsets, nPairsDev, candCount, warpStart,
-         candOffsets);
-  return cudaGetLastError();
-}
-
 cudaError_t filter_candidates(const DevConfig& cfg, DevHits hits, const uint2* pairs, const uint2* cands,
                               const uint32_t* nCandsDev, uint64_t maxCands, uint32_t* masks, uint32_t* warpSums,
                               uint32_t* nWordsOut, Queue& q) {
@@ -815,8 +800,8 @@ cudaError_t filter_store(const uint2* pairs, const uint2* cands, const uint32_t*
                          uint64_t capT, Queue& q) {
   if (maxCands == 0) return cudaSuccess;
   const uint32_t cap = capT > 0xffffffffull ? 0xffffffffu : (uint32_t)capT;
-  launch(q, filter_store_kernel, grid_for((maxCands + 1023) / 1024 * 32, 256), 256, 0, pairs, cands, nCandsDev,
-         masks, wordStart, h1, h2, h3, cap);
+  launch(q, filter_store_kernel, grid_for(maxCands, 256), 256, 0, pairs, cands, nCandsDev, masks, wordStart, h1, h2,
+         h3, cap, (uint32_t)sm_count() * 64u);
   return cudaGetLastError();
 }
 

@@ -190,9 +190,12 @@ cudaError_t fine_grid_build(const DevConfig& cfg, const uint32_t* grid, const fl
 cudaError_t identity_hits(const GridInput& in, uint32_t n, DevHits out, Queue& q);
 
 // ----------------------------------------------------------------- pairs
-// Per (event, layer triplet) segment: first outer hit and number of outer hits.
-cudaError_t pair_segments(const DevConfig& cfg, const uint32_t* grid, uint32_t* segOuter, uint32_t* segCount,
-                          Queue& q);
+// Per (event, layer triplet) segment: its first outer hit, and the exclusive
+// scan of the segments' outer hits in taskBase[S+1] with its total published
+// (S up to TRAX_SEGMENT_SCAN; above, the counts are left for scan_exclusive).
+#define TRAX_SEGMENT_SCAN 32767u
+cudaError_t pair_segments(const DevConfig& cfg, const uint32_t* grid, uint32_t* segOuter, uint32_t* taskBase,
+                          ScanTotal total, uint32_t* err, Queue& q);
 // What the count pass leaves for the store pass per outer-hit task k, so
 // that the store pass neither searches the task's segment nor recomputes
 // its window: bounds[k] = (zLow, zHigh, phiLow, phiHigh);
@@ -214,14 +217,12 @@ inline PairTaskState pair_task_state(void* base, uint64_t n) {
 
 // Count (emit == false) or store (emit == true) pairs of every outer-hit task.
 // taskBase[S+1] is the exclusive scan of segCount; nTasksDev = &taskBase[S].
-// The count pass writes `state`, the store pass reads it.
+// The count pass writes `state`, the store pass reads it and also writes
+// pairOffsets[s] = first pair of segment s (Pairing::pairingOffsets).
 cudaError_t pair_tasks(const DevConfig& cfg, bool emit, const uint32_t* grid, DevHits hits,
                        const uint32_t* segOuter, const uint32_t* taskBase, const uint32_t* nTasksDev,
                        uint64_t maxTasks, uint32_t* taskCount, PairTaskState state, uint2* pairs,
-                       uint64_t capPairs, uint32_t* sentinelCount, uint32_t* err, Queue& q);
-// pairOffsets[s+1] = first pair of segment s+1 (Pairing::pairingOffsets)
-cudaError_t pair_offsets(const DevConfig& cfg, const uint32_t* taskBase, const uint32_t* pairStart,
-                         uint32_t* pairOffsets, Queue& q);
+                       uint64_t capPairs, uint32_t* pairOffsets, uint32_t* sentinelCount, uint32_t* err, Queue& q);
 
 // ------------------------------------------------------------ prediction
 // Count pass (emit == false): per pair the exclusive offset of its
@@ -244,15 +245,13 @@ inline bool keep_interleaved(const DevConfig& cfg) { return cfg.predKeep >= 16u 
 // counters (4 bytes per cell)
 #define TRAX_GRID_SMEM_CELLS 53248u
 // With cfg.fineRows > 0 the count pass, and the store pass's re-walks of
-// pairs with more candidates than slots, walk `fine` (same outputs).
+// pairs with more candidates than slots, walk `fine` (same outputs).  The
+// store pass also writes candOffsets[s] = first candidate of segment s.
 cudaError_t predict_pairs(const DevConfig& cfg, bool emit, const uint32_t* grid, DevHits hits, const uint2* pairs,
                           const uint32_t* nPairsDev, uint64_t maxPairs, uint32_t* candCount, uint32_t* warpSums,
                           uint32_t* nWarpsOut, uint32_t* keep, uint2* cands, uint64_t capCands,
                           uint32_t* sentinelCount, uint32_t* err, Queue& q,
-                          FineGrid fine = FineGrid{nullptr, nullptr});
-cudaError_t predict_offsets(const DevConfig& cfg, const uint32_t* pairOffsets, const uint32_t* nPairsDev,
-                            const uint32_t* candCount, const uint32_t* warpStart, uint32_t* candOffsets,
-                            Queue& q);
+                          FineGrid fine, const uint32_t* pairOffsets, uint32_t* candOffsets);
 
 // ---------------------------------------------------------------- filter
 // the flags of 32 consecutive candidates as one word masks[g / 32] (bit
