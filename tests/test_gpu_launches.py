@@ -57,3 +57,46 @@ def test_segment_scan_sizes(trax_lib, n_events):
             alone = few.event[h1] == last % 7
             shift = int(starts[last]) - int(few.event_offsets[last % 7])
             assert np.array_equal(k1[e == last], h1[alone] + shift)
+
+
+@pytest.mark.parametrize("where", [(0, 1, 2), (5, 40, 299), (0, 150, 298), (297, 298, 299)])
+@pytest.mark.parametrize("graph", [True, False])
+def test_segments_between_empty_events(trax_lib, oracle_lib, where, graph):
+    """Triplet segments and offsets with runs of empty segments before, between and after the ones that hold triplets
+    (gaps shorter and longer than a warp), and the CA's event blocks without triplets: every array as the oracle's."""
+    few = events.generate(1, n_events=3)
+    layer_hits = np.zeros((300, few.n_layers), dtype=np.uint32)
+    layer_hits[list(where)] = few.layer_hits
+    cols = {k: getattr(few, k) for k in ("x", "y", "z", "layer", "det_id", "hit_id")}
+    cols["event"] = np.asarray(where, dtype=np.uint32)[few.event]
+    batch = events._assemble(cols, layer_hits, few)
+    want = oracle_lib.run(batch)[0]
+    with trax_lib.Context(0) as ctx:
+        ctx.upload(batch)
+        ctx.seed_batch(use_graph=graph)
+        got = ctx.results()
+    for name in ("pair_offsets", "cand_offsets", "trip_offsets", "trip_h1", "trip_h2", "trip_h3", "link_basis",
+                 "link_follower", "connectable", "non_connectable", "ca_states", "tracks", "track_offsets"):
+        assert np.array_equal(got[name], want[name]), name
+
+
+def test_linking_after_a_callers_links(trax_lib):
+    """trax_cellular_automaton_on takes the incoming-link lists for its own links; the chain's linking stages run
+    again on the context give what they gave before."""
+    batch = events.generate(1, n_events=6)
+    with trax_lib.Context(0) as ctx:
+        ctx.upload(batch)
+        ctx.seed_batch(use_graph=False)
+        first = ctx.results()
+        n = first["trip_h1"].size
+        ctx.cellular_automaton_on([0, 1], [n - 1, n - 1], np.ones(n, np.float32))
+        assert ctx.connectivity(batch.d_eta_cut) == first["link_basis"].size
+        ctx.circle_fit()
+        ctx.cellular_automaton()
+        again = ctx.results()
+        b, f = first["link_basis"], first["link_follower"]
+        by_caller = ctx.cellular_automaton_on(b, f, first["pt"])  # the chain's links as a caller's
+    for k, v in first.items():
+        assert np.array_equal(v, again[k]), k
+    for v, k in zip(by_caller, ("ca_states", "tracks", "track_offsets")):
+        assert np.array_equal(v, first[k]), k

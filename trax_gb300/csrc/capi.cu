@@ -19,6 +19,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <initializer_list>
 #include <string>
 #include <vector>
 
@@ -66,7 +67,6 @@ enum Slot {
   S_TRIPLETS,
   S_LINKS,
   S_CONN,
-  S_NONCONN,
   S_TRACKS,
   S_PRED_WARPS,
   S_FLAG_WORDS,
@@ -139,7 +139,7 @@ struct trax_ctx {
   // prediction / filter
   DevBuf candLocal, predWarps, predKeep, cands, candOffsets, flagWords, flagSums, h1, h2, h3, tripOffsets;
   // connectivity / fit / CA
-  DevBuf eta, segOf, segStart, linkCount, linkRun, cflags, basis, follower, connS, nonConnS, connW, nonConnW, connIdx, nonConnIdx, pt;
+  DevBuf eta, segOf, segStart, linkCount, linkRun, inDeg, basis, follower, connS, connW, connIdx, nonConnIdx, pt;
   DevBuf states, inStart, inCursor, inList, best, isBest, handlers, tracks;
   DevBuf userIdx, caNext;  // caller-provided fit list; second state buffer of the caller-link CA
   // bookkeeping
@@ -155,6 +155,8 @@ struct trax_ctx {
   // triplets of every segment ordered by (second hit, first hit): true for the
   // chain's own filter output; checked for caller-provided triplets
   bool sortedSegments = true;
+  bool chainLinking = false;  // the chain being captured includes the linking stages
+  bool inListOwn = false;     // inStart / inList hold the incoming links of the last connectivity run
   bool identityHits = false;  // hit collection taken as uploaded (trax_set_tracklets)
   // DEVICE-mode capacities and the captured graph
   uint64_t capTasks = 0, capPairs = 0, capCands = 0, capT = 0, capLinks = 0, capTracks = 0;
@@ -403,27 +405,40 @@ int check_device_error(trax_ctx* c) {
       return fail(c, TRAX_ERR_STATE, "device-mode buffer " #buf " too small");  \
   } while (0)
 
-// Exclusive scan of (count + 1) elements, count = nHost or *nDev; the total
-// goes to slot `dst` (clamped to cap; -1: nowhere).  In DEVICE mode every
-// scan of the chain has its own part of the scratch, cleared by the grid
-// build; in SYNCED mode the scratch is cleared by each scan.
-int scan_publish(trax_ctx* c, Mode mode, const uint32_t* in, uint32_t* out, uint64_t nHost, const uint32_t* nDev,
+// Exclusive scans of one or two arrays of (count + 1) elements, count =
+// nHost or *nDev; the first one's total goes to slot `dst` (clamped to cap;
+// -1: nowhere).  In DEVICE mode every scan of the chain has its own part of
+// the scratch, cleared by the grid build; in SYNCED mode the scratch is
+// cleared by each scan.
+struct ScanArray {
+  const uint32_t* in;
+  uint32_t* out;
+};
+int scan_publish(trax_ctx* c, Mode mode, std::initializer_list<ScanArray> arrays, uint64_t nHost, const uint32_t* nDev,
                  uint64_t maxCount, int dst, uint64_t cap) {
   const uint64_t maxN = maxCount + 1;
-  const size_t bytes = scan_scratch_bytes(maxN);
+  const size_t bytes = scan_scratch_bytes(maxN), all = bytes * arrays.size();
   if (mode == SYNCED) {
-    CK(ensure(c, c->scanScratch, bytes));
+    CK(ensure(c, c->scanScratch, all));
     c->scanUsed = 0;
-  } else if (c->scanUsed + bytes > c->scanScratch.cap) {
+  } else if (c->scanUsed + all > c->scanScratch.cap) {
     return fail(c, TRAX_ERR_STATE, "device-mode scan scratch too small");
   }
   char* scratch = static_cast<char*>(c->scanScratch.p) + c->scanUsed;
-  if (mode == DEVICE) c->scanUsed += bytes;
-  ScanTotal total;
-  if (dst >= 0) total = ScanTotal{slot(c, dst), cap > 0xffffffffull ? 0xffffffffu : (uint32_t)cap};
-  CK(scan_exclusive(in, out, nHost + 1, nDev, 1, maxN, scratch, mode == DEVICE, dev_err(c), c->q, true, c->wait,
-                    total));
+  if (mode == DEVICE) c->scanUsed += all;
+  ScanJob jobs[2];
+  int n = 0;
+  for (const ScanArray& a : arrays) {
+    jobs[n] = ScanJob{a.in, a.out, scratch + n * bytes, ScanTotal{}};
+    ++n;
+  }
+  if (dst >= 0) jobs[0].total = ScanTotal{slot(c, dst), cap > 0xffffffffull ? 0xffffffffu : (uint32_t)cap};
+  CK(scan_exclusive(jobs, n, nHost + 1, nDev, 1, maxN, mode == DEVICE, dev_err(c), c->q, true, c->wait));
   return TRAX_OK;
+}
+int scan_publish(trax_ctx* c, Mode mode, uint32_t* data, uint64_t nHost, const uint32_t* nDev, uint64_t maxCount,
+                 int dst, uint64_t cap) {
+  return scan_publish(c, mode, {ScanArray{data, data}}, nHost, nDev, maxCount, dst, cap);
 }
 
 // scratch of all the scans of one chain in DEVICE mode: segments, tasks,
@@ -432,7 +447,7 @@ size_t chain_scan_bytes(trax_ctx* c) {
   const uint64_t maxTW = (c->capT + 31) / 32;
   return scan_scratch_bytes((uint64_t)c->cfg.E * c->cfg.nLT + 1) + scan_scratch_bytes(c->capTasks + 1) +
          scan_scratch_bytes((c->capPairs + 31) / 32 + 1) + scan_scratch_bytes((c->capCands + 31) / 32 + 1) +
-         3 * scan_scratch_bytes(c->capT + 1) + 2 * scan_scratch_bytes(maxTW + 1);
+         3 * scan_scratch_bytes(c->capT + 1) + scan_scratch_bytes(maxTW + 1);
 }
 
 // ------------------------------------------------------------------ stages
@@ -493,7 +508,7 @@ int stage_pairs(trax_ctx* c, Mode mode) {
   const uint64_t capTasks = mode == DEVICE ? c->capTasks : NO_CAP;
   CK(pair_segments(c->cfg, ptr<uint32_t>(c->grid), ptr<uint32_t>(c->segOuter), taskBase,
                    ScanTotal{slot(c, S_TASKS), (uint32_t)std::min(capTasks, NO_CAP)}, dev_err(c), c->q));
-  if (S > TRAX_SEGMENT_SCAN) RC(scan_publish(c, mode, taskBase, taskBase, S, nullptr, S, S_TASKS, capTasks));
+  if (S > TRAX_SEGMENT_SCAN) RC(scan_publish(c, mode, taskBase, S, nullptr, S, S_TASKS, capTasks));
   const uint32_t* nTasksDev = slot(c, S_TASKS);
   uint64_t maxTasks = c->capTasks;
   if (mode == SYNCED) {
@@ -508,7 +523,7 @@ int stage_pairs(trax_ctx* c, Mode mode) {
   CK(pair_tasks(c->cfg, false, ptr<uint32_t>(c->grid), dev_hits(c), ptr<uint32_t>(c->segOuter), taskBase, nTasksDev,
                 maxTasks, taskCount, taskState, nullptr, 0, nullptr, slot(c, S_PAIR_SENT), dev_err(c), c->q));
   KEND(TK_PAIR_COUNT);
-  RC(scan_publish(c, mode, taskCount, taskCount, c->nTasks, mode == DEVICE ? nTasksDev : nullptr, maxTasks, S_PAIRS,
+  RC(scan_publish(c, mode, taskCount, c->nTasks, mode == DEVICE ? nTasksDev : nullptr, maxTasks, S_PAIRS,
                   mode == DEVICE ? c->capPairs : NO_CAP));
   uint64_t maxPairs = c->capPairs;
   if (mode == SYNCED) {
@@ -544,7 +559,7 @@ int stage_predict(trax_ctx* c, Mode mode) {
                    slot(c, S_CAND_SENT), dev_err(c), c->q, fine_grid(c), nullptr, nullptr));
   KEND(TK_PRED_COUNT);
   // the prefix sum runs over the per-warp sums of the counts
-  RC(scan_publish(c, mode, warpSums, warpSums, (c->nPairs + 31) / 32, mode == DEVICE ? slot(c, S_PRED_WARPS) : nullptr,
+  RC(scan_publish(c, mode, warpSums, (c->nPairs + 31) / 32, mode == DEVICE ? slot(c, S_PRED_WARPS) : nullptr,
                   maxWarps, S_CANDS, mode == DEVICE ? c->capCands : NO_CAP));
   uint64_t maxCands = c->capCands;
   if (mode == SYNCED) {
@@ -561,6 +576,27 @@ int stage_predict(trax_ctx* c, Mode mode) {
   return TRAX_OK;
 }
 
+TripletView triplets(trax_ctx* c, uint64_t maxT) {
+  TripletView t;
+  t.h1 = ptr<uint32_t>(c->h1);
+  t.h2 = ptr<uint32_t>(c->h2);
+  t.h3 = ptr<uint32_t>(c->h3);
+  t.nDev = slot(c, S_TRIPLETS);
+  t.maxN = maxT;
+  return t;
+}
+
+// what the link part of triplet_segments writes
+int link_buffers(trax_ctx* c, Mode mode, uint64_t maxT) {
+  ENSURE(eta, maxT, 4);
+  ENSURE(inDeg, maxT + 1, 4);
+  ENSURE(inCursor, maxT, 4);
+  return TRAX_OK;
+}
+LinkStart link_start(trax_ctx* c) {
+  return LinkStart{ptr<float>(c->eta), ptr<uint32_t>(c->inDeg), ptr<uint32_t>(c->inCursor)};
+}
+
 int stage_filter(trax_ctx* c, Mode mode) {
   NvtxRange nvtx("trax.filter");
   const uint32_t S = c->cfg.E * c->cfg.nLT;
@@ -570,6 +606,7 @@ int stage_filter(trax_ctx* c, Mode mode) {
   ENSURE(flagWords, maxWords + 1, 4);
   ENSURE(flagSums, maxWords + 1, 4);
   ENSURE(tripOffsets, S + 1, 4);
+  ENSURE(segStart, S + 1, 4);
   uint32_t* words = ptr<uint32_t>(c->flagWords);
   uint32_t* sums = ptr<uint32_t>(c->flagSums);
   KBEG(TK_FILTER);
@@ -577,7 +614,7 @@ int stage_filter(trax_ctx* c, Mode mode) {
                        sums, slot(c, S_FLAG_WORDS), c->q));
   KEND(TK_FILTER);
   // the prefix sum runs over the numbers of flags per word of 32 candidates
-  RC(scan_publish(c, mode, sums, sums, (c->nCands + 31) / 32, mode == DEVICE ? slot(c, S_FLAG_WORDS) : nullptr, maxWords,
+  RC(scan_publish(c, mode, sums, (c->nCands + 31) / 32, mode == DEVICE ? slot(c, S_FLAG_WORDS) : nullptr, maxWords,
                   S_TRIPLETS, mode == DEVICE ? c->capT : NO_CAP));
   uint64_t maxT = c->capT;
   if (mode == SYNCED) {
@@ -591,19 +628,13 @@ int stage_filter(trax_ctx* c, Mode mode) {
   CK(filter_store(ptr<uint2>(c->pairs), ptr<uint2>(c->cands), nCandsDev, maxCands, words, sums, ptr<uint32_t>(c->h1),
                   ptr<uint32_t>(c->h2), ptr<uint32_t>(c->h3), maxT, c->q));
   KEND(TK_FILTER_STORE);
-  CK(triplet_offsets(c->cfg, dev_hits(c), ptr<uint32_t>(c->h1), slot(c, S_TRIPLETS), maxT,
-                     ptr<uint32_t>(c->tripOffsets), c->q));
+  // a captured chain that goes on to the linking prepares it in the same pass
+  const bool link = mode == DEVICE && c->chainLinking;
+  if (link) RC(link_buffers(c, mode, maxT));
+  const LinkStart ls = link_start(c);
+  CK(triplet_segments(c->cfg, dev_hits(c), triplets(c, maxT), ptr<uint32_t>(c->segStart), nullptr,
+                      ptr<uint32_t>(c->tripOffsets), link ? &ls : nullptr, c->q));
   return TRAX_OK;
-}
-
-TripletView triplets(trax_ctx* c, uint64_t maxT) {
-  TripletView t;
-  t.h1 = ptr<uint32_t>(c->h1);
-  t.h2 = ptr<uint32_t>(c->h2);
-  t.h3 = ptr<uint32_t>(c->h3);
-  t.nDev = slot(c, S_TRIPLETS);
-  t.maxN = maxT;
-  return t;
 }
 
 int stage_connectivity(trax_ctx* c, Mode mode) {
@@ -615,31 +646,26 @@ int stage_connectivity(trax_ctx* c, Mode mode) {
     c->nLinks = c->nConn = c->nNonConn = c->nTracks = 0;
     c->noLinks = true;
   }
-  ENSURE(eta, maxT, 4);
-  ENSURE(segOf, maxT, 4);
-  ENSURE(segStart, S + 1, 4);
+  RC(link_buffers(c, mode, maxT));
   ENSURE(linkCount, maxT + 1, 4);
   ENSURE(linkRun, maxT + 1, 4);
-  ENSURE(cflags, maxT + 1, 4);
+  ENSURE(inStart, maxT + 1, 4);
   const uint64_t maxTW = (maxT + 31) / 32;
   ENSURE(connS, maxTW + 1, 4);
-  ENSURE(nonConnS, maxTW + 1, 4);
   ENSURE(connW, maxTW + 1, 4);
-  ENSURE(nonConnW, maxTW + 1, 4);
   ENSURE(connIdx, maxT, 4);
   ENSURE(nonConnIdx, maxT, 4);
   TripletView tv = triplets(c, maxT);
-  CK(cudaMemsetAsync(c->cflags.p, 0, (size_t)(maxT + 1) * 4, c->st));
-  CK(triplet_eta(c->cfg, dev_hits(c), tv, ptr<float>(c->eta), ptr<uint32_t>(c->segOf), c->q));
-  CK(segment_bounds(c->cfg, ptr<uint32_t>(c->segOf), nTDev, ptr<uint32_t>(c->segStart), c->q));
+  if (mode == SYNCED) CK(triplet_link_start(c->cfg, dev_hits(c), tv, link_start(c), c->q));
   uint32_t* linkCount = ptr<uint32_t>(c->linkCount);
   KBEG(TK_CONN_COUNT);
-  CK(connectivity_tasks(c->cfg, false, dev_hits(c), tv, ptr<float>(c->eta), ptr<uint32_t>(c->tripOffsets),
-                        ptr<uint32_t>(c->segStart), linkCount, ptr<uint32_t>(c->cflags), ptr<uint32_t>(c->linkRun),
-                        nullptr, nullptr, 0, c->sortedSegments, c->q));
+  CK(connectivity_count(c->cfg, dev_hits(c), tv, ptr<float>(c->eta), ptr<uint32_t>(c->tripOffsets),
+                        ptr<uint32_t>(c->segStart), linkCount, ptr<uint32_t>(c->inDeg), ptr<uint32_t>(c->linkRun),
+                        c->sortedSegments, c->q));
   KEND(TK_CONN_COUNT);
-  RC(scan_publish(c, mode, linkCount, linkCount, c->nT, mode == DEVICE ? nTDev : nullptr, maxT, S_LINKS,
-                  mode == DEVICE ? c->capLinks : NO_CAP));
+  // the links' places, and the places of the incoming links of every follower
+  RC(scan_publish(c, mode, {ScanArray{linkCount, linkCount}, ScanArray{ptr<uint32_t>(c->inDeg), ptr<uint32_t>(c->inStart)}},
+                  c->nT, mode == DEVICE ? nTDev : nullptr, maxT, S_LINKS, mode == DEVICE ? c->capLinks : NO_CAP));
   uint64_t maxLinks = c->capLinks;
   if (mode == SYNCED) {
     RC(read_slot(c, S_LINKS, &c->nLinks));
@@ -649,26 +675,25 @@ int stage_connectivity(trax_ctx* c, Mode mode) {
   }
   ENSURE(basis, maxLinks, 4);
   ENSURE(follower, maxLinks, 4);
+  ENSURE(inList, maxLinks, 4);
   KBEG(TK_CONN_EMIT);
-  CK(connectivity_tasks(c->cfg, true, dev_hits(c), tv, ptr<float>(c->eta), ptr<uint32_t>(c->tripOffsets),
-                        ptr<uint32_t>(c->segStart), linkCount, ptr<uint32_t>(c->cflags), ptr<uint32_t>(c->linkRun),
-                        ptr<uint32_t>(c->basis), ptr<uint32_t>(c->follower), maxLinks, c->sortedSegments, c->q));
+  const LinkStore store{linkCount, ptr<uint32_t>(c->linkRun), ptr<uint32_t>(c->inStart), ptr<uint32_t>(c->inCursor),
+                        ptr<uint32_t>(c->basis), ptr<uint32_t>(c->follower), ptr<uint32_t>(c->inList),
+                        (uint32_t)std::min(maxLinks, NO_CAP), c->sortedSegments, ptr<uint32_t>(c->connW),
+                        ptr<uint32_t>(c->connS), slot(c, S_CONN_WORDS)};
+  CK(connectivity_store(c->cfg, tv, ptr<float>(c->eta), store, c->q));
   KEND(TK_CONN_EMIT);
-  // the two Q9 streams as words of 32 flags; the scans run over the words' counts
-  CK(connectable_words(ptr<uint32_t>(c->cflags), nTDev, maxT, ptr<uint32_t>(c->connW), ptr<uint32_t>(c->connS),
-                       ptr<uint32_t>(c->nonConnW), ptr<uint32_t>(c->nonConnS), slot(c, S_CONN_WORDS), c->q));
-  const uint64_t nTW = (c->nT + 31) / 32;
-  const uint32_t* nTWDev = mode == DEVICE ? slot(c, S_CONN_WORDS) : nullptr;
-  RC(scan_publish(c, mode, ptr<uint32_t>(c->connS), ptr<uint32_t>(c->connS), nTW, nTWDev, maxTW, S_CONN, NO_CAP));
-  RC(scan_publish(c, mode, ptr<uint32_t>(c->nonConnS), ptr<uint32_t>(c->nonConnS), nTW, nTWDev, maxTW, S_NONCONN, NO_CAP));
-  CK(compact_words(ptr<uint32_t>(c->connW), ptr<uint32_t>(c->connS), nTDev, maxT, ptr<uint32_t>(c->connIdx), maxT,
-                   c->q));
-  CK(compact_words(ptr<uint32_t>(c->nonConnW), ptr<uint32_t>(c->nonConnS), nTDev, maxT, ptr<uint32_t>(c->nonConnIdx),
-                   maxT, c->q));
+  c->inListOwn = true;
+  // the Q9 streams: the scan runs over the words' counts; the second stream
+  // is what the first leaves of the triplets but the last
+  RC(scan_publish(c, mode, ptr<uint32_t>(c->connS), (c->nT + 31) / 32, mode == DEVICE ? slot(c, S_CONN_WORDS) : nullptr,
+                  maxTW, S_CONN, NO_CAP));
+  CK(connectable_lists(tv, ptr<uint32_t>(c->connW), ptr<uint32_t>(c->connS), ptr<uint32_t>(c->connIdx),
+                       ptr<uint32_t>(c->nonConnIdx), c->q));
   if (mode == SYNCED) {
     RC(read_slots(c));
     c->nConn = c->hSlots[S_CONN];
-    c->nNonConn = c->hSlots[S_NONCONN];
+    c->nNonConn = c->nT - 1 - c->nConn;  // with links there are at least two triplets
   }
   return TRAX_OK;
 }
@@ -677,10 +702,11 @@ int stage_fit(trax_ctx* c, Mode mode) {
   NvtxRange nvtx("trax.circle_fit");
   const uint64_t maxT = mode == SYNCED ? c->nT : c->capT;
   ENSURE(pt, maxT, 4);
-  CK(cudaMemsetAsync(c->pt.p, 0, (size_t)std::max<uint64_t>(maxT, 1) * 4, c->st));
-  if (mode == SYNCED && c->noLinks) return TRAX_OK;
-  CK(circle_fit(dev_hits(c), triplets(c, maxT), ptr<uint32_t>(c->connIdx), slot(c, S_CONN), maxT, ptr<float>(c->pt),
-                c->q));
+  if (mode == SYNCED && c->noLinks) {
+    CK(cudaMemsetAsync(c->pt.p, 0, (size_t)std::max<uint64_t>(maxT, 1) * 4, c->st));
+    return TRAX_OK;
+  }
+  CK(circle_fit_words(dev_hits(c), triplets(c, maxT), ptr<uint32_t>(c->connW), ptr<float>(c->pt), c->q));
   return TRAX_OK;
 }
 
@@ -708,20 +734,22 @@ int stage_ca(trax_ctx* c, Mode mode) {
   const uint32_t* nTDev = slot(c, S_TRIPLETS);
   const uint32_t* nLinksDev = slot(c, S_LINKS);
   ENSURE(states, maxT, 4);
-  ENSURE(inStart, maxT + 1, 4);
-  ENSURE(inCursor, maxT, 4);
-  ENSURE(inList, maxLinks, 4);
   ENSURE(best, maxT, 4);
   ENSURE(isBest, maxT, 4);
   ENSURE(handlers, maxT + 1, 4);
   CABuffers b = ca_buffers(c);
-  CK(ca_in_degree(ptr<uint32_t>(c->follower), nLinksDev, maxLinks, b, nTDev, maxT, c->q));
-  // in-degree prefix (its total is the number of links; not published)
-  RC(scan_publish(c, mode, b.inStart, b.inStart, c->nT, mode == DEVICE ? nTDev : nullptr, maxT, -1, NO_CAP));
-  CK(ca_fill(ptr<uint32_t>(c->basis), ptr<uint32_t>(c->follower), nLinksDev, maxLinks, b, nTDev, maxT, c->q));
-  CK(ca_forward(c->cfg, b, nTDev, maxT, c->q));
-  CK(ca_backward(ptr<float>(c->pt), b, nTDev, maxT, nLinksDev, c->q));
-  RC(scan_publish(c, mode, b.handlers, b.handlers, c->nT, mode == DEVICE ? nTDev : nullptr, maxT, S_TRACKS,
+  if (!c->inListOwn) {  // a caller's links took the lists (trax_cellular_automaton_on): fill them again
+    CK(ca_in_degree(ptr<uint32_t>(c->follower), nLinksDev, maxLinks, b, nTDev, maxT, c->q));
+    RC(scan_publish(c, mode, b.inStart, c->nT, nullptr, maxT, -1, NO_CAP));
+    CK(ca_fill(ptr<uint32_t>(c->basis), ptr<uint32_t>(c->follower), nLinksDev, maxLinks, b, c->q));
+    c->inListOwn = true;
+  }
+  // one CTA per event while that fills the CTAs evenly enough; the chain's
+  // own triplets only: a caller's may link across events
+  const bool perEvent = !c->identityHits && c->cfg.E > 0 && maxT <= (uint64_t)c->cfg.E * TRAX_CA_EVENT_TRIPLETS;
+  CK(ca_chain(c->cfg, ptr<float>(c->pt), b, c->identityHits ? nullptr : ptr<uint32_t>(c->segStart), perEvent, nTDev,
+              maxT, nLinksDev, c->q));
+  RC(scan_publish(c, mode, b.handlers, c->nT, mode == DEVICE ? nTDev : nullptr, maxT, S_TRACKS,
                   mode == DEVICE ? c->capTracks : NO_CAP));
   uint64_t maxTracks = c->capTracks;
   if (mode == SYNCED) {
@@ -779,6 +807,7 @@ int chain_device(trax_ctx* c, bool linking) {
   int (*stages[N_STAGES])(trax_ctx*, Mode) = {stage_grid, stage_pairs, stage_predict, stage_filter,
                                               stage_connectivity, stage_fit, stage_ca};
   const int n = linking ? N_STAGES : 4;
+  c->chainLinking = linking;
   mark(c, MARK_STAGE);
   for (int s = 0; s < n; ++s) {
     RC(stages[s](c, DEVICE));
@@ -812,10 +841,9 @@ int size_device_buffers(trax_ctx* c) {
   ENSURE(flagWords, (c->capCands + 31) / 32 + 1, 4);
   ENSURE(flagSums, (c->capCands + 31) / 32 + 1, 4);
   ENSURE(h1, c->capT, 4); ENSURE(h2, c->capT, 4); ENSURE(h3, c->capT, 4);
-  ENSURE(eta, c->capT, 4); ENSURE(segOf, c->capT, 4); ENSURE(segStart, S + 1, 4);
-  ENSURE(linkCount, c->capT + 1, 4); ENSURE(linkRun, c->capT + 1, 4); ENSURE(cflags, c->capT + 1, 4);
-  ENSURE(connS, (c->capT + 31) / 32 + 1, 4); ENSURE(nonConnS, (c->capT + 31) / 32 + 1, 4);
-  ENSURE(connW, (c->capT + 31) / 32 + 1, 4); ENSURE(nonConnW, (c->capT + 31) / 32 + 1, 4);
+  ENSURE(eta, c->capT, 4); ENSURE(segStart, S + 1, 4);
+  ENSURE(linkCount, c->capT + 1, 4); ENSURE(linkRun, c->capT + 1, 4); ENSURE(inDeg, c->capT + 1, 4);
+  ENSURE(connS, (c->capT + 31) / 32 + 1, 4); ENSURE(connW, (c->capT + 31) / 32 + 1, 4);
   ENSURE(connIdx, c->capT, 4); ENSURE(nonConnIdx, c->capT, 4); ENSURE(pt, c->capT, 4);
   ENSURE(basis, c->capLinks, 4); ENSURE(follower, c->capLinks, 4);
   ENSURE(states, c->capT, 4); ENSURE(inStart, c->capT + 1, 4); ENSURE(inCursor, c->capT, 4);
@@ -1028,7 +1056,7 @@ void trax_destroy(trax_ctx* c) {
                     &c->pevt, &c->porig, &c->pxyzp, &c->sc_cell, &c->sc_phi, &c->sc_perm, &c->sc_counts,
                     &c->fineGrid, &c->fineHits, &c->segOuter, &c->taskBase, &c->taskCount, &c->taskState, &c->pairs, &c->pairOffsets, &c->candLocal, &c->predWarps, &c->predKeep, &c->cands,
                     &c->candOffsets, &c->flagWords, &c->flagSums, &c->h1, &c->h2, &c->h3, &c->tripOffsets, &c->eta, &c->segOf,
-                    &c->segStart, &c->linkCount, &c->linkRun, &c->cflags, &c->basis, &c->follower, &c->connS, &c->nonConnS, &c->connW, &c->nonConnW,
+                    &c->segStart, &c->linkCount, &c->linkRun, &c->inDeg, &c->basis, &c->follower, &c->connS, &c->connW,
                     &c->connIdx, &c->nonConnIdx, &c->pt, &c->states, &c->inStart, &c->inCursor, &c->inList, &c->best,
                     &c->isBest, &c->handlers, &c->tracks, &c->scanScratch, &c->slots, &c->fitOk, &c->fitSegCnt,
                     &c->fitSegDelta, &c->fitRows, &c->fitPartials, &c->fitOut, &c->fitParams, &c->fitDHits,
@@ -1299,6 +1327,8 @@ int trax_set_tracklets(trax_ctx* c, const uint32_t* h1, const uint32_t* h2, cons
   ENSURE(h2, n, 4);
   ENSURE(h3, n, 4);
   ENSURE(tripOffsets, (size_t)c->cfg.E * c->cfg.nLT + 1, 4);
+  ENSURE(segStart, (size_t)c->cfg.E * c->cfg.nLT + 1, 4);
+  ENSURE(segOf, n, 4);
   GridInput in;
   memset(&in, 0, sizeof(in));
   in.x = ptr<float>(c->in_x);
@@ -1317,8 +1347,8 @@ int trax_set_tracklets(trax_ctx* c, const uint32_t* h1, const uint32_t* h2, cons
   }
   c->hSlots[S_TRIPLETS] = (uint32_t)n;
   CK(cudaMemcpyAsync(slot(c, S_TRIPLETS), c->hSlots + S_TRIPLETS, 4, cudaMemcpyHostToDevice, c->st));
-  CK(triplet_offsets(c->cfg, dev_hits(c), ptr<uint32_t>(c->h1), slot(c, S_TRIPLETS), n,
-                     ptr<uint32_t>(c->tripOffsets), c->q));
+  CK(triplet_segments(c->cfg, dev_hits(c), triplets(c, n), ptr<uint32_t>(c->segStart), ptr<uint32_t>(c->segOf),
+                      ptr<uint32_t>(c->tripOffsets), nullptr, c->q));
   c->nPairs = c->nCands = 0;
   c->nT = n;
   c->identityHits = true;
@@ -1441,9 +1471,9 @@ int trax_cellular_automaton_on(trax_ctx* c, const uint32_t* basis, const uint32_
   CABuffers b = ca_buffers(c);
   // states 1, in-degrees, the incoming bases of every follower (ascending)
   CK(ca_in_degree(ptr<uint32_t>(c->follower), nLinksDev, nL, b, nTDev, nT, c->q));
-  CK(scan_exclusive(b.inStart, b.inStart, nT + 1, nullptr, 0, nT + 1, c->scanScratch.p, false, dev_err(c), c->q, true,
-                    c->wait));
-  CK(ca_fill(ptr<uint32_t>(c->basis), ptr<uint32_t>(c->follower), nLinksDev, nL, b, nTDev, nT, c->q));
+  CK(scan_exclusive(b.inStart, b.inStart, nT + 1, c->scanScratch.p, dev_err(c), c->q, true, c->wait));
+  c->inListOwn = false;
+  CK(ca_fill(ptr<uint32_t>(c->basis), ptr<uint32_t>(c->follower), nLinksDev, nL, b, c->q));
   // forward phase: the reference's iteration (CellularAutomaton.cpp:37-98),
   // both state buffers starting at 1, swapped without copying; a link set
   // with a cycle never settles and is rejected after nT + 2 iterations
@@ -1465,8 +1495,8 @@ int trax_cellular_automaton_on(trax_ctx* c, const uint32_t* basis, const uint32_
   if (cur != ptr<uint32_t>(c->states))
     CK(cudaMemcpyAsync(c->states.p, cur, nT * 4, cudaMemcpyDeviceToDevice, c->st));
   // backward phase, handlers and tracks as in the chain
-  CK(ca_backward(ptr<float>(c->pt), b, nTDev, nT, nLinksDev, c->q));
-  RC(scan_publish(c, SYNCED, b.handlers, b.handlers, nT, nullptr, nT, S_TRACKS, NO_CAP));
+  CK(ca_backward(ptr<float>(c->pt), b, nTDev, nT, nLinksDev, dev_err(c), c->q));
+  RC(scan_publish(c, SYNCED, b.handlers, nT, nullptr, nT, S_TRACKS, NO_CAP));
   RC(read_slot(c, S_TRACKS, &c->nTracks));
   ENSURE(tracks, c->nTracks, 4);
   CK(ca_tracks(b, nTDev, nT, ptr<uint32_t>(c->tracks), c->nTracks, dev_err(c), c->q));
@@ -1491,8 +1521,8 @@ int trax_prefix_sum(trax_ctx* c, uint32_t* data, uint64_t n) {
   if (e == cudaSuccess) e = ensure(c, c->scanScratch, scan_scratch_bytes(n));
   if (e == cudaSuccess) e = cudaMemsetAsync(c->slots.p, 0, 4, c->st);
   if (e == cudaSuccess)
-    e = scan_exclusive(ptr<uint32_t>(tmp), ptr<uint32_t>(tmp), n, nullptr, 0, n, c->scanScratch.p, false, dev_err(c),
-                       c->q, false, c->wait);  // wraps like PrefixSum's uint arithmetic
+    e = scan_exclusive(ptr<uint32_t>(tmp), ptr<uint32_t>(tmp), n, c->scanScratch.p, dev_err(c), c->q, false,
+                       c->wait);  // wraps like PrefixSum's uint arithmetic
   if (e == cudaSuccess) e = cudaMemcpyAsync(data, tmp.p, n * 4, cudaMemcpyDeviceToHost, c->st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(c->st);
   if (e != cudaSuccess) rc = cuda_fail(c, e, "trax_prefix_sum");
@@ -1580,7 +1610,7 @@ int trax_seed_batch(trax_ctx* c, const trax_batch_opts* opts, trax_batch_stats* 
     c->nT = c->hSlots[S_TRIPLETS];
     c->nLinks = linking ? c->hSlots[S_LINKS] : 0;
     c->nConn = linking ? c->hSlots[S_CONN] : 0;
-    c->nNonConn = linking ? c->hSlots[S_NONCONN] : 0;
+    c->nNonConn = linking && c->nT ? c->nT - 1 - c->nConn : 0;
     c->nTracks = linking ? c->hSlots[S_TRACKS] : 0;
     c->noLinks = c->nLinks == 0;
     if (c->noLinks) c->nConn = c->nNonConn = c->nTracks = 0;  // the reference returns no lists then
@@ -1595,6 +1625,7 @@ int trax_seed_batch(trax_ctx* c, const trax_batch_opts* opts, trax_batch_stats* 
     c->stage = linking ? 7 : 4;
     ++c->tripGen;
     if (linking) c->ptGen = c->caGen = c->tripGen;
+    if (linking) c->inListOwn = true;
     c->caOnly = false;
     fill_stats(c, stats);
     return TRAX_OK;
@@ -1709,10 +1740,8 @@ int trax_physics_tracks_device(trax_ctx* c, uint64_t total_tracks, trax_track_me
   uint32_t* hitsOf = ptr<uint32_t>(c->trk_hitsOf);
   const uint32_t* off = ptr<uint32_t>(c->handlers);
   CK(track_sizes(off, nT, isTrack, hitsOf, c->st));
-  CK(scan_exclusive(isTrack, isTrack, (uint64_t)nT + 1, nullptr, 0, (uint64_t)nT + 1, c->scanScratch.p, false,
-                    dev_err(c), c->q, true, c->wait));
-  CK(scan_exclusive(hitsOf, hitsOf, (uint64_t)nT + 1, nullptr, 0, (uint64_t)nT + 1, c->scanScratch.p, false,
-                    dev_err(c), c->q, true, c->wait));
+  CK(scan_exclusive(isTrack, isTrack, (uint64_t)nT + 1, c->scanScratch.p, dev_err(c), c->q, true, c->wait));
+  CK(scan_exclusive(hitsOf, hitsOf, (uint64_t)nT + 1, c->scanScratch.p, dev_err(c), c->q, true, c->wait));
   uint32_t totals[2];
   CK(cudaMemcpyAsync(&totals[0], isTrack + nT, 4, cudaMemcpyDeviceToHost, c->st));
   CK(cudaMemcpyAsync(&totals[1], hitsOf + nT, 4, cudaMemcpyDeviceToHost, c->st));
@@ -1754,8 +1783,8 @@ int trax_physics_tracks_device(trax_ctx* c, uint64_t total_tracks, trax_track_me
   }
   if (!stable) return fail(c, TRAX_ERR_TIMEOUT, "track components did not settle in 64 rounds");
   CK(track_members(t, nTracks, false, c->st));
-  CK(scan_exclusive(t.compSize, t.compStart, (uint64_t)nTracks + 1, nullptr, 0, (uint64_t)nTracks + 1,
-                    c->scanScratch.p, false, dev_err(c), c->q, true, c->wait));
+  CK(scan_exclusive(t.compSize, t.compStart, (uint64_t)nTracks + 1, c->scanScratch.p, dev_err(c), c->q, true,
+                    c->wait));
   CK(track_members(t, nTracks, true, c->st));
   unsigned long long* counts = ptr<unsigned long long>(c->trk_counts);
   CK(track_greedy(t, nTracks, ptr<unsigned long long>(c->trk_table), tableSize - 1, counts, c->st));
@@ -1856,8 +1885,7 @@ int trax_fit_prepare(trax_ctx* c, const trax_fit_opts* opts, uint64_t* n_fit) {
   uint32_t* ok = ptr<uint32_t>(c->fitOk);
   CK(fit_select(f, c->cfg, dev_hits(c), fit_triplets(c), nT, truthOnly, ok, ptr<uint32_t>(c->fitSegCnt), c->st, &c->q.launches));
   CK(ensure(c, c->scanScratch, scan_scratch_bytes(nT + 1)));
-  CK(scan_exclusive(ok, ok, nT + 1, nullptr, 0, nT + 1, c->scanScratch.p, false, dev_err(c), c->q, true,
-                    c->wait));
+  CK(scan_exclusive(ok, ok, nT + 1, c->scanScratch.p, dev_err(c), c->q, true, c->wait));
   // 2. rows ordered by layer triplet, then by event (segment order inside a layer triplet)
   std::vector<uint32_t> cnt(S);
   if (S) CK(cudaMemcpyAsync(cnt.data(), c->fitSegCnt.p, (size_t)S * 4, cudaMemcpyDeviceToHost, c->st));

@@ -27,14 +27,20 @@ constexpr int SCAN_ITEMS = 16;
 constexpr uint32_t SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
 
 __global__ void __launch_bounds__(SCAN_THREADS)
-    scan_kernel(Stamp stamp, const uint32_t* __restrict__ in, uint32_t* out, uint64_t nHost, const uint32_t* nDev,
-                uint32_t nAdd, unsigned long long* status, uint32_t* ticket, uint32_t* err, uint32_t overflowBit,
-                WaitCtl ctl, ScanTotal total) {
+    scan_kernel(Stamp stamp, ScanJob job0, ScanJob job1, uint64_t nHost, const uint32_t* nDev, uint32_t nAdd,
+                uint32_t* err, uint32_t overflowBit, WaitCtl ctl) {
   stamp_begin(stamp);
   __shared__ uint32_t s_tile;
   __shared__ uint32_t s_warp[SCAN_THREADS / 32];
   __shared__ unsigned long long s_wide[SCAN_THREADS / 32];
   __shared__ uint32_t s_prefix;
+  // two arrays of one length may share a launch (blockIdx.y), each with its own tickets
+  const ScanJob& job = blockIdx.y ? job1 : job0;
+  const uint32_t* __restrict__ in = job.in;
+  uint32_t* out = job.out;
+  uint32_t* ticket = static_cast<uint32_t*>(job.scratch);
+  unsigned long long* status = reinterpret_cast<unsigned long long*>(static_cast<char*>(job.scratch) + 256);
+  const ScanTotal total = job.total;
   const uint64_t n = nDev ? (uint64_t)(*nDev) + nAdd : nHost;
   if (threadIdx.x == 0) s_tile = gridDim.x > 1 ? atomicAdd(ticket, 1u) : 0u;
   __syncthreads();
@@ -125,44 +131,6 @@ __global__ void __launch_bounds__(SCAN_THREADS)
   }
 }
 
-// Inclusive running maximum, one CTA (the serial semantics of the offset
-// monotonize kernels, TripletThetaPhiFilter.h:267-280).
-__global__ void __launch_bounds__(1024) max_scan_kernel(Stamp stamp, uint32_t* data, uint32_t n) {
-  stamp_begin(stamp);
-  __shared__ uint32_t s_w[32];
-  __shared__ uint32_t s_carry;
-  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-  if (threadIdx.x == 0) s_carry = 0;
-  __syncthreads();
-  for (uint32_t b = 0; b < n; b += blockDim.x) {
-    uint32_t i = b + threadIdx.x;
-    uint32_t v = i < n ? data[i] : 0u;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      uint32_t t = __shfl_up_sync(0xffffffffu, v, d);
-      if (lane >= (uint32_t)d) v = max(v, t);
-    }
-    if (lane == 31) s_w[warp] = v;
-    __syncthreads();
-    if (warp == 0) {
-      uint32_t w = (lane < blockDim.x / 32) ? s_w[lane] : 0u;
-#pragma unroll
-      for (int d = 1; d < 32; d <<= 1) {
-        uint32_t t = __shfl_up_sync(0xffffffffu, w, d);
-        if (lane >= (uint32_t)d) w = max(w, t);
-      }
-      s_w[lane] = w;
-    }
-    __syncthreads();
-    uint32_t pre = (warp > 0) ? s_w[warp - 1] : 0u;
-    uint32_t r = max(max(v, pre), s_carry);
-    if (i < n) data[i] = r;
-    __syncthreads();
-    if (threadIdx.x == blockDim.x - 1) s_carry = r;
-    __syncthreads();
-  }
-}
-
 // the context's slots and time marks to page-locked host memory
 __global__ void slots_to_host_kernel(Stamp stamp, const uint32_t* slots, uint32_t* host, uint32_t n) {
   stamp_begin(stamp);
@@ -182,27 +150,26 @@ size_t scan_scratch_bytes(uint64_t maxN) {
   return (256 + tiles * sizeof(unsigned long long) + 255) / 256 * 256;
 }
 
-cudaError_t scan_exclusive(const uint32_t* in, uint32_t* out, uint64_t n, const uint32_t* nDev, uint32_t nAdd,
-                           uint64_t maxN, void* scratch, bool cleared, uint32_t* err, Queue& q, bool flagOverflow,
-                           WaitCtl ctl, ScanTotal total) {
+cudaError_t scan_exclusive(const ScanJob* jobs, int nJobs, uint64_t n, const uint32_t* nDev, uint32_t nAdd,
+                           uint64_t maxN, bool cleared, uint32_t* err, Queue& q, bool flagOverflow, WaitCtl ctl) {
   uint64_t cap = nDev ? maxN : n;
   if (cap == 0) return cudaSuccess;
   uint64_t tiles = (cap + SCAN_TILE - 1) / SCAN_TILE;
   if (tiles > 1 && !cleared) {
-    cudaError_t e = cudaMemsetAsync(scratch, 0, 256 + tiles * sizeof(unsigned long long), q.st);
-    if (e != cudaSuccess) return e;
+    for (int j = 0; j < nJobs; ++j) {
+      cudaError_t e = cudaMemsetAsync(jobs[j].scratch, 0, 256 + tiles * sizeof(unsigned long long), q.st);
+      if (e != cudaSuccess) return e;
+    }
   }
-  uint32_t* ticket = reinterpret_cast<uint32_t*>(scratch);
-  unsigned long long* status = reinterpret_cast<unsigned long long*>(static_cast<char*>(scratch) + 256);
-  launch(q, scan_kernel, (unsigned)tiles, SCAN_THREADS, 0, in, out, n, nDev, nAdd, status, ticket, err,
-         flagOverflow ? TRAX_EBIT_OVERFLOW : 0u, ctl, total);
+  launch(q, scan_kernel, dim3((unsigned)tiles, nJobs), SCAN_THREADS, 0, jobs[0], jobs[nJobs - 1], n, nDev, nAdd, err,
+         flagOverflow ? TRAX_EBIT_OVERFLOW : 0u, ctl);
   return cudaGetLastError();
 }
 
-cudaError_t max_scan_inclusive(uint32_t* data, uint32_t n, Queue& q) {
-  if (n == 0) return cudaSuccess;
-  launch(q, max_scan_kernel, 1, 1024, 0, data, n);
-  return cudaGetLastError();
+cudaError_t scan_exclusive(const uint32_t* in, uint32_t* out, uint64_t n, void* scratch, uint32_t* err, Queue& q,
+                           bool flagOverflow, WaitCtl ctl) {
+  const ScanJob job{in, out, scratch, ScanTotal{}};
+  return scan_exclusive(&job, 1, n, nullptr, 0, n, false, err, q, flagOverflow, ctl);
 }
 
 }  // namespace trax
@@ -227,7 +194,7 @@ cudaError_t max_scan_inclusive(uint32_t* data, uint32_t n, Queue& q) {
 namespace {
 
 constexpr uint64_t NOALLOC_TILES = (TRAX_NOALLOC_SCAN_MAX + trax::SCAN_TILE - 1) / trax::SCAN_TILE;
-constexpr size_t NOALLOC_HEADER = 256;  // ticket at byte 0, error word at byte 4
+constexpr size_t NOALLOC_HEADER = 256;  // ticket at byte 0, error word at byte 4 (ScanJob::scratch)
 constexpr size_t NOALLOC_BYTES = NOALLOC_HEADER + NOALLOC_TILES * sizeof(unsigned long long);
 
 static __device__ __align__(256) unsigned char g_noalloc_scan_scratch[NOALLOC_BYTES];
@@ -282,15 +249,13 @@ extern "C" int trax_prefix_sum_noalloc(const uint32_t* d_in, uint32_t* d_out, ui
   }
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const uint64_t tiles = (n + trax::SCAN_TILE - 1) / trax::SCAN_TILE;
-  uint32_t* ticket = static_cast<uint32_t*>(base);
-  uint32_t* err = ticket + 1;
-  unsigned long long* status = reinterpret_cast<unsigned long long*>(static_cast<char*>(base) + NOALLOC_HEADER);
+  uint32_t* err = static_cast<uint32_t*>(base) + 1;  // behind the ticket
   // the ticket, the error word and the status words of this call start at zero
   e = cudaMemsetAsync(base, 0, NOALLOC_HEADER + tiles * sizeof(unsigned long long), st);
   if (e == cudaSuccess) {
-    trax::scan_kernel<<<(unsigned)tiles, trax::SCAN_THREADS, 0, st>>>(trax::Stamp{}, d_in, d_out, n, nullptr, 0, status, ticket,
-                                                                      err, 0u, noalloc_wait(),
-                                                                      trax::ScanTotal{});
+    const trax::ScanJob job{d_in, d_out, base, trax::ScanTotal{}};
+    trax::scan_kernel<<<(unsigned)tiles, trax::SCAN_THREADS, 0, st>>>(trax::Stamp{}, job, job, n, nullptr, 0, err, 0u,
+                                                                      noalloc_wait());
     e = cudaGetLastError();
   }
   uint32_t hostErr = 0;

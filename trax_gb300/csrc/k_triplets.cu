@@ -714,27 +714,6 @@ __global__ void filter_store_kernel(Stamp stamp, const uint2* __restrict__ pairs
   }
 }
 
-// filterOffsetStore (TripletThetaPhiFilter.h:221-257)
-__global__ void triplet_offsets_kernel(Stamp stamp, DevConfig cfg, const uint32_t* __restrict__ hitEvt,
-                                       const uint32_t* __restrict__ hitLayer, const uint32_t* __restrict__ h1,
-                                       const uint32_t* nTDev, uint32_t* offsets) {
-  stamp_begin(stamp);
-  const uint32_t nT = *nTDev;
-  for (uint32_t gid = blockIdx.x * blockDim.x + threadIdx.x; gid < nT; gid += gridDim.x * blockDim.x) {
-    const uint32_t hitId = trax_hit(h1[gid], cfg);
-    const uint32_t layerTriplet = hitLayer[hitId];
-    const uint32_t event = hitEvt[hitId];
-    if (gid > 0) {
-      const uint32_t prev = h1[gid - 1];
-      if (layerTriplet != hitLayer[prev] || event != hitEvt[prev])
-        offsets[(size_t)event * cfg.nLT + layerTriplet - 1] = gid;
-      if ((gid + 1) == nT) offsets[(size_t)event * cfg.nLT + layerTriplet] = gid;
-    } else {
-      offsets[(size_t)event * cfg.nLT + layerTriplet - 1] = gid;
-    }
-  }
-}
-
 // The staged windows pack the z rows and phi columns into 16 bits and the
 // third layer's first cell into 32 bits.
 bool pred_k_fits(const DevConfig& cfg) {
@@ -803,19 +782,6 @@ cudaError_t filter_store(const uint2* pairs, const uint2* cands, const uint32_t*
   launch(q, filter_store_kernel, grid_for(maxCands, 256), 256, 0, pairs, cands, nCandsDev, masks, wordStart, h1, h2,
          h3, cap, (uint32_t)sm_count() * 64u);
   return cudaGetLastError();
-}
-
-cudaError_t triplet_offsets(const DevConfig& cfg, DevHits hits, const uint32_t* h1, const uint32_t* nTDev,
-                            uint64_t maxT, uint32_t* offsets, Queue& q) {
-  const uint32_t S = cfg.E * cfg.nLT;
-  cudaError_t e = cudaMemsetAsync(offsets, 0, (S + 1) * sizeof(uint32_t), q.st);
-  if (e != cudaSuccess) return e;
-  if (maxT > 0) {
-    launch(q, triplet_offsets_kernel, grid_for(maxT, 256), 256, 0, cfg, hits.evt, hits.layer, h1, nTDev, offsets);
-  }
-  e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  return max_scan_inclusive(offsets, S + 1, q);
 }
 
 }  // namespace trax

@@ -23,10 +23,10 @@ struct Queue {
 
 // Every kernel of the chain takes its Stamp first.
 template <class... P, class... A>
-cudaError_t launch(Queue& q, void (*kernel)(Stamp, P...), unsigned blocks, unsigned threads, size_t smem,
+cudaError_t launch(Queue& q, void (*kernel)(Stamp, P...), dim3 blocks, unsigned threads, size_t smem,
                    A&&... args) {
   cudaLaunchConfig_t c = {};
-  c.gridDim = dim3(blocks);
+  c.gridDim = blocks;
   c.blockDim = dim3(threads);
   c.dynamicSmemBytes = smem;
   c.stream = q.st;
@@ -44,16 +44,24 @@ struct ScanTotal {
   uint32_t* dst = nullptr;
   uint32_t cap = 0xffffffffu;
 };
-// Exclusive scan of n elements (or *nDev + nAdd when nDev != nullptr, with
-// maxN bounding the launch), in place allowed.  Outputs wrap modulo 2^32;
+// One array to scan, in place allowed; scratch holds scan_scratch_bytes.
+struct ScanJob {
+  const uint32_t* in;
+  uint32_t* out;
+  void* scratch;
+  ScanTotal total;
+};
+// Exclusive scans of one or two arrays of n elements (or *nDev + nAdd when
+// nDev != nullptr, with maxN bounding the launch).  Outputs wrap modulo 2^32;
 // with flagOverflow a total of 2^32 or more sets TRAX_EBIT_OVERFLOW.  `ctl`
 // bounds the look-back waits (and may name a tile that never publishes).
-// `scratch` holds scan_scratch_bytes(maxN), `cleared`: zero already and used
-// by no other scan since (otherwise it is cleared here).
-cudaError_t scan_exclusive(const uint32_t* in, uint32_t* out, uint64_t n, const uint32_t* nDev, uint32_t nAdd,
-                           uint64_t maxN, void* scratch, bool cleared, uint32_t* err, Queue& q, bool flagOverflow,
-                           WaitCtl ctl, ScanTotal total = ScanTotal{});
-cudaError_t max_scan_inclusive(uint32_t* data, uint32_t n, Queue& q);
+// `cleared`: the scratch is zero already and used by no other scan since
+// (otherwise it is cleared here).
+cudaError_t scan_exclusive(const ScanJob* jobs, int nJobs, uint64_t n, const uint32_t* nDev, uint32_t nAdd,
+                           uint64_t maxN, bool cleared, uint32_t* err, Queue& q, bool flagOverflow, WaitCtl ctl);
+// one array of n elements
+cudaError_t scan_exclusive(const uint32_t* in, uint32_t* out, uint64_t n, void* scratch, uint32_t* err, Queue& q,
+                           bool flagOverflow, WaitCtl ctl);
 
 // ------------------------------------------------------ event bucketing
 // The hits of a group of events as their file holds them, with the host's
@@ -265,10 +273,6 @@ cudaError_t filter_candidates(const DevConfig& cfg, DevHits hits, const uint2* p
 cudaError_t filter_store(const uint2* pairs, const uint2* cands, const uint32_t* nCandsDev, uint64_t maxCands,
                          const uint32_t* masks, const uint32_t* wordStart, uint32_t* h1, uint32_t* h2, uint32_t* h3,
                          uint64_t capT, Queue& q);
-// trackletOffsets with the reference's filterOffsetStore + monotonize semantics
-cudaError_t triplet_offsets(const DevConfig& cfg, DevHits hits, const uint32_t* h1, const uint32_t* nTDev,
-                            uint64_t maxT, uint32_t* offsets, Queue& q);
-
 // ---------------------------------------------------------- connectivity
 struct TripletView {
   const uint32_t* h1;
@@ -278,25 +282,47 @@ struct TripletView {
   uint64_t maxN;
 };
 
-cudaError_t triplet_eta(const DevConfig& cfg, DevHits hits, TripletView t, float* eta, uint32_t* seg,
-                        Queue& q);
-cudaError_t segment_bounds(const DevConfig& cfg, const uint32_t* seg, const uint32_t* nTDev, uint32_t* segStart,
-                           Queue& q);
-// runStart[t]: where the count pass found the (h2, h1) run of t's
-// followers in sorted segments; the store pass starts there
-cudaError_t connectivity_tasks(const DevConfig& cfg, bool emit, DevHits hits, TripletView t, const float* eta,
+// Segments of the triplets: segStart[s] = first triplet of segment s or
+// later (S + 1 entries), offsets = trackletOffsets with the reference's
+// filterOffsetStore + monotonize semantics, segOf[t] (unless null).  With
+// `link` also what connectivity starts from: eta, and inDeg / inCursor zeroed.
+struct LinkStart {
+  float* eta;
+  uint32_t* inDeg;     // [nT+1]
+  uint32_t* inCursor;  // [nT]
+};
+cudaError_t triplet_segments(const DevConfig& cfg, DevHits hits, TripletView t, uint32_t* segStart, uint32_t* segOf,
+                             uint32_t* offsets, const LinkStart* link, Queue& q);
+// the link part alone
+cudaError_t triplet_link_start(const DevConfig& cfg, DevHits hits, TripletView t, LinkStart link, Queue& q);
+// links per basis triplet (linkCount, +1 slot zeroed) and per follower
+// (inDeg); runStart[t]: where the store pass starts looking for t's followers
+cudaError_t connectivity_count(const DevConfig& cfg, DevHits hits, TripletView t, const float* eta,
                                const uint32_t* offsets, const uint32_t* segStart, uint32_t* linkCount,
-                               uint32_t* flags, uint32_t* runStart, uint32_t* basis, uint32_t* follower,
-                               uint64_t capLinks, bool sortedSegments, Queue& q);
-// flags[k] for k < n-1 -> words of 32 (flag) and (!flag) bits with the number
-// set per word (+1 slots zeroed, the number of words to *nWordsOut)
-cudaError_t connectable_words(const uint32_t* flags, const uint32_t* nTDev, uint64_t maxT, uint32_t* connWords,
-                              uint32_t* connSums, uint32_t* nonWords, uint32_t* nonSums, uint32_t* nWordsOut,
-                              Queue& q);
-// with the sums scanned into wordStart: outIdx[wordStart[k / 32] + (bits
-// below k in its word)] = k for every set bit k < *nTDev
-cudaError_t compact_words(const uint32_t* words, const uint32_t* wordStart, const uint32_t* nTDev, uint64_t maxT,
-                          uint32_t* outIdx, uint64_t capOut, Queue& q);
+                               uint32_t* inDeg, uint32_t* runStart, bool sortedSegments, Queue& q);
+// With linkCount and inDeg scanned (the latter into inStart): the links, the
+// bases of each follower's links in inList (any order), and the words of 32
+// connectable flags with the number set per word (+1 slot zeroed, the number
+// of words to *nWordsOut)
+struct LinkStore {
+  const uint32_t* linkStart;
+  const uint32_t* runStart;
+  const uint32_t* inStart;
+  uint32_t* inCursor;
+  uint32_t* basis;
+  uint32_t* follower;
+  uint32_t* inList;
+  uint32_t capLinks;
+  bool sortedSegments;
+  uint32_t* connWords;
+  uint32_t* connSums;
+  uint32_t* nWordsOut;
+};
+cudaError_t connectivity_store(const DevConfig& cfg, TripletView t, const float* eta, LinkStore ls, Queue& q);
+// With connSums scanned into wordStart: the connectable and non-connectable
+// triplets among the first nT - 1
+cudaError_t connectable_lists(TripletView t, const uint32_t* connWords, const uint32_t* wordStart, uint32_t* connIdx,
+                              uint32_t* nonConnIdx, Queue& q);
 // the context's slots and the time marks after them to page-locked host memory
 cudaError_t slots_to_host(const uint32_t* slots, uint32_t* host, uint32_t words, Queue& q);
 
@@ -304,11 +330,14 @@ cudaError_t slots_to_host(const uint32_t* slots, uint32_t* host, uint32_t words,
 cudaError_t circle_fit(DevHits hits, TripletView t, const uint32_t* connectable, const uint32_t* nConnDev,
                        uint64_t maxConn, float* pt, Queue& q);
 
+// pt[t] of every triplet: the circle fit of the connectable ones, 0 for the others
+cudaError_t circle_fit_words(DevHits hits, TripletView t, const uint32_t* connWords, float* pt, Queue& q);
+
 struct CABuffers {
   uint32_t* states;    // [nT]
   uint32_t* inStart;   // [nT+1]
   uint32_t* inCursor;  // [nT]
-  uint32_t* inList;    // [nLinks] bases of the incoming links, grouped by follower
+  uint32_t* inList;    // [nLinks] bases of the incoming links, grouped by follower, any order
   uint32_t* best;      // [nT]
   uint32_t* isBest;    // [nT]
   uint32_t* handlers;  // [nT+1]
@@ -318,15 +347,22 @@ struct CABuffers {
 cudaError_t ca_in_degree(const uint32_t* follower, const uint32_t* nLinksDev, uint64_t maxLinks, CABuffers b,
                          const uint32_t* nTDev, uint64_t maxT, Queue& q);
 cudaError_t ca_fill(const uint32_t* basis, const uint32_t* follower, const uint32_t* nLinksDev, uint64_t maxLinks,
-                    CABuffers b, const uint32_t* nTDev, uint64_t maxT, Queue& q);
-cudaError_t ca_forward(const DevConfig& cfg, CABuffers b, const uint32_t* nTDev, uint64_t maxT, Queue& q);
+                    CABuffers b, Queue& q);
+// Triplets per event (on average) up to which one CTA per event runs the
+// chain's CA (ca_event_kernel); above, a CTA would take too many steps and a
+// launch per level over the whole chip is faster.
+#define TRAX_CA_EVENT_TRIPLETS 16384u
+// The chain's forward and backward phases and handlers (inStart and inList
+// given).  perEvent: one CTA per event; segStart null: levels by segOf.
+cudaError_t ca_chain(const DevConfig& cfg, const float* pt, CABuffers b, const uint32_t* segStart, bool perEvent,
+                     const uint32_t* nTDev, uint64_t maxT, const uint32_t* nLinksDev, Queue& q);
 // One forward iteration of the reference's CA over any link set
 // (CellularAutomaton.h:52-100); *living is set when a cell lives.
 cudaError_t ca_iteration(const uint32_t* basis, const uint32_t* follower, uint32_t nLinks, const uint32_t* cur,
                          uint32_t* next, uint32_t* living, Queue& q);
 cudaError_t fill_u32(uint32_t* p, uint32_t v, uint32_t n, Queue& q);
 cudaError_t ca_backward(const float* pt, CABuffers b, const uint32_t* nTDev, uint64_t maxT,
-                        const uint32_t* nLinksDev, Queue& q);
+                        const uint32_t* nLinksDev, const uint32_t* err, Queue& q);
 cudaError_t ca_tracks(CABuffers b, const uint32_t* nTDev, uint64_t maxT, uint32_t* tracks, uint64_t maxTracks,
                       uint32_t* err, Queue& q);
 
