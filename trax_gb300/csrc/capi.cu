@@ -373,12 +373,26 @@ int read_slots(trax_ctx* c) {
 
 int error_from_bits(trax_ctx* c, uint32_t bits);
 
-// a stage total read by the host in SYNCED mode; the error word comes along so
-// that an overflowed or timed-out scan stops the chain before its total is used
-int read_slot(trax_ctx* c, int k, uint64_t* out) {
-  RC(read_slots(c));
+// a stage total the host waits for in SYNCED mode: the scan wrote it to the
+// page-locked slots (scan_total), the error word with it, so that an
+// overflowed or timed-out scan stops the chain before its total is used
+int read_total(trax_ctx* c, int k, uint64_t* out) {
+  CK(cudaStreamSynchronize(c->st));
   *out = c->hSlots[k];
   return error_from_bits(c, c->hSlots[S_ERR] & (TRAX_EBIT_OVERFLOW | TRAX_EBIT_TIMEOUT));
+}
+
+// where a scan's total goes: slot k, clamped to cap; in SYNCED mode also to
+// the host's copy of the slot (read_total)
+ScanTotal scan_total(trax_ctx* c, Mode mode, int k, uint64_t cap) {
+  ScanTotal t;
+  t.dst = slot(c, k);
+  t.cap = (uint32_t)std::min(cap, NO_CAP);
+  if (mode == SYNCED) {
+    t.host = c->hSlots + k;
+    t.hostErr = c->hSlots + S_ERR;
+  }
+  return t;
 }
 
 int error_from_bits(trax_ctx* c, uint32_t bits) {
@@ -432,7 +446,7 @@ int scan_publish(trax_ctx* c, Mode mode, std::initializer_list<ScanArray> arrays
     jobs[n] = ScanJob{a.in, a.out, scratch + n * bytes, ScanTotal{}};
     ++n;
   }
-  if (dst >= 0) jobs[0].total = ScanTotal{slot(c, dst), cap > 0xffffffffull ? 0xffffffffu : (uint32_t)cap};
+  if (dst >= 0) jobs[0].total = scan_total(c, mode, dst, cap);
   CK(scan_exclusive(jobs, n, nHost + 1, nDev, 1, maxN, mode == DEVICE, dev_err(c), c->q, true, c->wait));
   return TRAX_OK;
 }
@@ -507,12 +521,12 @@ int stage_pairs(trax_ctx* c, Mode mode) {
   uint32_t* taskBase = ptr<uint32_t>(c->taskBase);
   const uint64_t capTasks = mode == DEVICE ? c->capTasks : NO_CAP;
   CK(pair_segments(c->cfg, ptr<uint32_t>(c->grid), ptr<uint32_t>(c->segOuter), taskBase,
-                   ScanTotal{slot(c, S_TASKS), (uint32_t)std::min(capTasks, NO_CAP)}, dev_err(c), c->q));
+                   scan_total(c, mode, S_TASKS, capTasks), dev_err(c), c->q));
   if (S > TRAX_SEGMENT_SCAN) RC(scan_publish(c, mode, taskBase, S, nullptr, S, S_TASKS, capTasks));
   const uint32_t* nTasksDev = slot(c, S_TASKS);
   uint64_t maxTasks = c->capTasks;
   if (mode == SYNCED) {
-    RC(read_slot(c, S_TASKS, &c->nTasks));
+    RC(read_total(c, S_TASKS, &c->nTasks));
     maxTasks = c->nTasks;
   }
   ENSURE(taskCount, maxTasks + 1, 4);
@@ -527,7 +541,7 @@ int stage_pairs(trax_ctx* c, Mode mode) {
                   mode == DEVICE ? c->capPairs : NO_CAP));
   uint64_t maxPairs = c->capPairs;
   if (mode == SYNCED) {
-    RC(read_slot(c, S_PAIRS, &c->nPairs));
+    RC(read_total(c, S_PAIRS, &c->nPairs));
     maxPairs = c->nPairs;
   }
   ENSURE(pairs, maxPairs, 8);
@@ -563,7 +577,7 @@ int stage_predict(trax_ctx* c, Mode mode) {
                   maxWarps, S_CANDS, mode == DEVICE ? c->capCands : NO_CAP));
   uint64_t maxCands = c->capCands;
   if (mode == SYNCED) {
-    RC(read_slot(c, S_CANDS, &c->nCands));
+    RC(read_total(c, S_CANDS, &c->nCands));
     maxCands = c->nCands;
   }
   ENSURE(cands, maxCands, 8);
@@ -618,7 +632,7 @@ int stage_filter(trax_ctx* c, Mode mode) {
                   S_TRIPLETS, mode == DEVICE ? c->capT : NO_CAP));
   uint64_t maxT = c->capT;
   if (mode == SYNCED) {
-    RC(read_slot(c, S_TRIPLETS, &c->nT));
+    RC(read_total(c, S_TRIPLETS, &c->nT));
     maxT = c->nT;
   }
   ENSURE(h1, maxT, 4);
@@ -668,7 +682,7 @@ int stage_connectivity(trax_ctx* c, Mode mode) {
                   c->nT, mode == DEVICE ? nTDev : nullptr, maxT, S_LINKS, mode == DEVICE ? c->capLinks : NO_CAP));
   uint64_t maxLinks = c->capLinks;
   if (mode == SYNCED) {
-    RC(read_slot(c, S_LINKS, &c->nLinks));
+    RC(read_total(c, S_LINKS, &c->nLinks));
     maxLinks = c->nLinks;
     c->noLinks = c->nLinks == 0;
     if (c->noLinks) return TRAX_OK;  // TripletConnectivityTight.cpp:127-129
@@ -691,8 +705,7 @@ int stage_connectivity(trax_ctx* c, Mode mode) {
   CK(connectable_lists(tv, ptr<uint32_t>(c->connW), ptr<uint32_t>(c->connS), ptr<uint32_t>(c->connIdx),
                        ptr<uint32_t>(c->nonConnIdx), c->q));
   if (mode == SYNCED) {
-    RC(read_slots(c));
-    c->nConn = c->hSlots[S_CONN];
+    RC(read_total(c, S_CONN, &c->nConn));
     c->nNonConn = c->nT - 1 - c->nConn;  // with links there are at least two triplets
   }
   return TRAX_OK;
@@ -753,7 +766,7 @@ int stage_ca(trax_ctx* c, Mode mode) {
                   mode == DEVICE ? c->capTracks : NO_CAP));
   uint64_t maxTracks = c->capTracks;
   if (mode == SYNCED) {
-    RC(read_slot(c, S_TRACKS, &c->nTracks));
+    RC(read_total(c, S_TRACKS, &c->nTracks));
     maxTracks = c->nTracks;
   }
   ENSURE(tracks, maxTracks, 4);
@@ -1497,7 +1510,7 @@ int trax_cellular_automaton_on(trax_ctx* c, const uint32_t* basis, const uint32_
   // backward phase, handlers and tracks as in the chain
   CK(ca_backward(ptr<float>(c->pt), b, nTDev, nT, nLinksDev, dev_err(c), c->q));
   RC(scan_publish(c, SYNCED, b.handlers, nT, nullptr, nT, S_TRACKS, NO_CAP));
-  RC(read_slot(c, S_TRACKS, &c->nTracks));
+  RC(read_total(c, S_TRACKS, &c->nTracks));
   ENSURE(tracks, c->nTracks, 4);
   CK(ca_tracks(b, nTDev, nT, ptr<uint32_t>(c->tracks), c->nTracks, dev_err(c), c->q));
   CK(cudaStreamSynchronize(c->st));

@@ -249,12 +249,7 @@ __global__ void __launch_bounds__(SEG_THREADS)
       if (a + k <= S) taskBase[a + k] = (uint32_t)run;
       if (a + k == S) {  // the total
         if (run > 0xffffffffull) raise_error(err, TRAX_EBIT_OVERFLOW);
-        uint32_t t = (uint32_t)run;
-        if (t > total.cap) {
-          t = total.cap;
-          raise_error(err, TRAX_EBIT_CAPACITY);
-        }
-        *total.dst = t;
+        publish_total(total, (uint32_t)run, err);
       }
       run += n[k];
     }

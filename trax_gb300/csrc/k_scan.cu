@@ -123,11 +123,7 @@ __global__ void __launch_bounds__(SCAN_THREADS)
 #pragma unroll
     for (int k = 0; k < SCAN_ITEMS; ++k)
       if (i0 + k + 1 == n) t = off + v[k];
-    if (t > total.cap) {
-      t = total.cap;
-      raise_error(err, TRAX_EBIT_CAPACITY);
-    }
-    *total.dst = t;
+    publish_total(total, t, err);
   }
 }
 

@@ -117,6 +117,29 @@ __device__ __forceinline__ void stamp_begin(Stamp s) {
 // up, records TRAX_EBIT_TIMEOUT and carries on with what it has.
 #define TRAX_SPIN_LIMIT (1u << 22)
 
+// Where a scan of count + 1 elements leaves its total (the last output),
+// clamped to cap (TRAX_EBIT_CAPACITY): dst on the device (null: nowhere), and
+// on the host too when it waits for the total before it goes on (host, with
+// the error word in hostErr; page-locked memory).
+struct ScanTotal {
+  uint32_t* dst = nullptr;
+  uint32_t cap = 0xffffffffu;
+  uint32_t* host = nullptr;
+  uint32_t* hostErr = nullptr;
+};
+
+__device__ __forceinline__ void publish_total(const ScanTotal& total, uint32_t t, uint32_t* err) {
+  if (t > total.cap) {
+    t = total.cap;
+    raise_error(err, TRAX_EBIT_CAPACITY);
+  }
+  *total.dst = t;
+  if (total.host) {
+    *total.host = t;
+    *total.hostErr = atomicOr(err, 0u);
+  }
+}
+
 // Settings of the scans' bounded waits, passed to every scan launch:
 // spinLimit polls before a wait gives up (0: TRAX_SPIN_LIMIT), and a tile
 // that publishes nothing (0xffffffff: none) -- a host-set fault that makes

@@ -38,12 +38,6 @@ cudaError_t launch(Queue& q, void (*kernel)(Stamp, P...), dim3 blocks, unsigned 
 
 // ---------------------------------------------------------------- scans
 size_t scan_scratch_bytes(uint64_t maxN);
-// Where a scan of count + 1 elements leaves its total (the last output),
-// clamped to cap (TRAX_EBIT_CAPACITY); dst null: nowhere.
-struct ScanTotal {
-  uint32_t* dst = nullptr;
-  uint32_t cap = 0xffffffffu;
-};
 // One array to scan, in place allowed; scratch holds scan_scratch_bytes.
 struct ScanJob {
   const uint32_t* in;
