@@ -23,7 +23,10 @@ namespace trax {
 
 namespace {
 
+// Threads of a grid CTA: 256 while the (event, layer) tasks alone fill the
+// chip, 512 and 1024 for fewer (grid_threads); the fine grid's CTAs have 256.
 constexpr int GRID_THREADS = 256;
+constexpr int GRID_MAX_THREADS = 1024;
 constexpr int GRID_WARPS = GRID_THREADS / 32;
 // cell counters live in shared memory up to TRAX_GRID_SMEM_CELLS cells (208 KB,
 // one CTA per SM at the largest grids); larger grids count in global memory
@@ -34,7 +37,7 @@ constexpr size_t GRID_SMEM_MAX = TRAX_GRID_SMEM_BYTES;
 
 // the scan scratch of the chain's compactions, all of which run after the grid
 __device__ __forceinline__ void clear_scan_scratch(const GridScratch& sc) {
-  for (uint32_t i = blockIdx.x * GRID_THREADS + threadIdx.x; i < sc.clearWords; i += gridDim.x * GRID_THREADS)
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < sc.clearWords; i += gridDim.x * blockDim.x)
     sc.clear[i] = make_uint4(0u, 0u, 0u, 0u);
 }
 
@@ -43,7 +46,9 @@ __device__ __forceinline__ void clear_scan_scratch(const GridScratch& sc) {
 // warps scan the sums with shuffles, and the chunks are rewritten.
 __device__ __forceinline__ void cta_cell_scan(uint32_t* cnt, uint32_t C, uint32_t* s_warpSum) {
   const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-  const uint32_t chunk = (C + GRID_THREADS - 1) / GRID_THREADS;
+  // consecutive cells per thread, an odd number of them: threads a multiple
+  // of the 32 banks apart would read the same banks
+  const uint32_t chunk = ((C + blockDim.x - 1) / blockDim.x) | 1u;
   const uint32_t c0 = min(tid * chunk, C), c1 = min(c0 + chunk, C);
   uint32_t local = 0;
   for (uint32_t c = c0; c < c1; ++c) local += cnt[c];
@@ -74,9 +79,9 @@ __device__ __forceinline__ void cta_cell_scan(uint32_t* cnt, uint32_t C, uint32_
 __device__ __forceinline__ void cta_place_stable(uint32_t* cnt, uint32_t C, const uint32_t* cellOf, uint32_t* perm,
                                                  uint32_t n) {
   const uint32_t tid = threadIdx.x;
-  for (uint32_t i = tid; i < n; i += GRID_THREADS) perm[atomicAdd(&cnt[cellOf[i]], 1u)] = i;
+  for (uint32_t i = tid; i < n; i += blockDim.x) perm[atomicAdd(&cnt[cellOf[i]], 1u)] = i;
   __syncthreads();
-  for (uint32_t c = tid; c < C; c += GRID_THREADS) {
+  for (uint32_t c = tid; c < C; c += blockDim.x) {
     const uint32_t lo = c ? cnt[c - 1] : 0u, hi = cnt[c];
     if (hi - lo < 2) continue;
     for (uint32_t a = lo + 1; a < hi; ++a) {  // insertion sort: cells hold a few hits
@@ -95,13 +100,13 @@ __device__ __forceinline__ void cta_place_stable(uint32_t* cnt, uint32_t C, cons
 // The per-hit cell, phi and slot arrays are in shared memory after the
 // counters when the layer has at most maxHits hits (the room the launch
 // gave them), otherwise in the global scratch arrays.
-__global__ void __launch_bounds__(GRID_THREADS)
+__global__ void __launch_bounds__(GRID_MAX_THREADS)
     grid_kernel(Stamp stamp, DevConfig cfg, GridInput in, uint32_t* __restrict__ grid, DevHits out, GridScratch sc,
                 uint32_t* err, int useSmem, uint32_t maxHits) {
   stamp_begin(stamp);
   clear_scan_scratch(sc);
   extern __shared__ uint32_t smem[];
-  __shared__ uint32_t s_warpSum[GRID_WARPS];
+  __shared__ uint32_t s_warpSum[GRID_MAX_THREADS / 32];
   const uint32_t task = blockIdx.x;  // event * L + layer
   const uint32_t e = task / cfg.L;
   const uint32_t C = cfg.C;
@@ -115,11 +120,11 @@ __global__ void __launch_bounds__(GRID_THREADS)
   uint32_t* perm = inSmem ? smem + C + 2 * maxHits : sc.perm + base;
   const uint32_t tid = threadIdx.x;
 
-  for (uint32_t c = tid; c < C; c += GRID_THREADS) cnt[c] = 0u;
+  for (uint32_t c = tid; c < C; c += blockDim.x) cnt[c] = 0u;
   __syncthreads();
 
   // 1. cells (gridCount, GridBuilder.h:80-87)
-  for (uint32_t i = tid; i < n; i += GRID_THREADS) {
+  for (uint32_t i = tid; i < n; i += blockDim.x) {
     const uint32_t k = base + i;
     const float x = in.x[k], y = in.y[k], z = in.z[k];
     uint32_t zSector = f2u_sat(floor_(div_(z - cfg.minZ, cfg.sZ)));
@@ -141,7 +146,7 @@ __global__ void __launch_bounds__(GRID_THREADS)
   cta_cell_scan(cnt, C, s_warpSum);
   // the boundaries, written with consecutive threads on consecutive cells
   uint32_t* gl = grid + (size_t)task * C;
-  for (uint32_t c = tid; c < C; c += GRID_THREADS) gl[c] = base + cnt[c];
+  for (uint32_t c = tid; c < C; c += blockDim.x) gl[c] = base + cnt[c];
   __syncthreads();
 
   // 3. placement: a slot per hit from the cell cursors (shared-memory
@@ -151,7 +156,7 @@ __global__ void __launch_bounds__(GRID_THREADS)
   cta_place_stable(cnt, C, cellOf, perm, n);
 
   // 4. gather into cell order (gridStore, GridBuilder.h:243-253)
-  for (uint32_t s = tid; s < n; s += GRID_THREADS) {
+  for (uint32_t s = tid; s < n; s += blockDim.x) {
     const uint32_t dst = base + s;
     const uint32_t i = perm[s];
     const uint32_t src = base + i;
@@ -178,13 +183,13 @@ __global__ void __launch_bounds__(GRID_THREADS)
 // arrays in global scratch.
 __device__ __forceinline__ uint32_t half_of(uint32_t word, uint32_t c) { return (word >> ((c & 1u) * 16u)) & 0xffffu; }
 
-__global__ void __launch_bounds__(GRID_THREADS)
+__global__ void __launch_bounds__(GRID_MAX_THREADS)
     grid_kernel16(Stamp stamp, DevConfig cfg, GridInput in, uint32_t* __restrict__ grid, DevHits out, GridScratch sc,
                   uint32_t* err, uint32_t maxHits) {
   stamp_begin(stamp);
   clear_scan_scratch(sc);
   extern __shared__ uint32_t smem[];
-  __shared__ uint32_t s_warpSum[GRID_WARPS];
+  __shared__ uint32_t s_warpSum[GRID_MAX_THREADS / 32];
   const uint32_t task = blockIdx.x;  // event * L + layer
   const uint32_t e = task / cfg.L;
   const uint32_t C = cfg.C, W = (C + 1) / 2;
@@ -202,8 +207,8 @@ __global__ void __launch_bounds__(GRID_THREADS)
     // no cell holds a hit, the hits in input order
     if (tid == 0) raise_error(err, TRAX_EBIT_BOUNDS);
     uint32_t* gl = grid + (size_t)task * C;
-    for (uint32_t c = tid; c < C; c += GRID_THREADS) gl[c] = base;
-    for (uint32_t s = tid; s < n; s += GRID_THREADS) {
+    for (uint32_t c = tid; c < C; c += blockDim.x) gl[c] = base;
+    for (uint32_t s = tid; s < n; s += blockDim.x) {
       const uint32_t k = base + s;
       const float x = in.x[k], y = in.y[k], z = in.z[k];
       out.x[k] = x;
@@ -219,11 +224,11 @@ __global__ void __launch_bounds__(GRID_THREADS)
     return;
   }
 
-  for (uint32_t w = tid; w < W; w += GRID_THREADS) cnt[w] = 0u;
+  for (uint32_t w = tid; w < W; w += blockDim.x) cnt[w] = 0u;
   __syncthreads();
 
   // 1. cells (gridCount, GridBuilder.h:80-87)
-  for (uint32_t i = tid; i < n; i += GRID_THREADS) {
+  for (uint32_t i = tid; i < n; i += blockDim.x) {
     const uint32_t k = base + i;
     const float x = in.x[k], y = in.y[k], z = in.z[k];
     uint32_t zSector = f2u_sat(floor_(div_(z - cfg.minZ, cfg.sZ)));
@@ -248,7 +253,8 @@ __global__ void __launch_bounds__(GRID_THREADS)
 
   // 2. CTA exclusive scan of the counters over whole words per thread;
   //    write the grid boundaries
-  const uint32_t chunkW = (W + GRID_THREADS - 1) / GRID_THREADS;
+  // (an odd number of words: no two threads of a warp in the same bank)
+  const uint32_t chunkW = ((W + blockDim.x - 1) / blockDim.x) | 1u;
   const uint32_t w0 = min(tid * chunkW, W), w1 = min(w0 + chunkW, W);
   uint32_t local = 0;
   for (uint32_t w = w0; w < w1; ++w) {
@@ -276,26 +282,26 @@ __global__ void __launch_bounds__(GRID_THREADS)
   __syncthreads();
   // the boundaries, written with consecutive threads on consecutive cells
   uint32_t* gl = grid + (size_t)task * C;
-  for (uint32_t c = tid; c < C; c += GRID_THREADS) gl[c] = base + half_of(cnt[c >> 1], c);
+  for (uint32_t c = tid; c < C; c += blockDim.x) gl[c] = base + half_of(cnt[c >> 1], c);
   __syncthreads();
 
   // 3. placement by the cell cursors, then the stable order inside each cell
   //    (as in grid_kernel); afterwards cursor c is the end of cell c
   if (inSmem) {
-    for (uint32_t i = tid; i < n; i += GRID_THREADS) {
+    for (uint32_t i = tid; i < n; i += blockDim.x) {
       const uint32_t cell = cellS[i];
       const uint32_t sh = (cell & 1u) * 16u;
       permS[(atomicAdd(&cnt[cell >> 1], 1u << sh) >> sh) & 0xffffu] = (uint16_t)i;
     }
   } else {
-    for (uint32_t i = tid; i < n; i += GRID_THREADS) {
+    for (uint32_t i = tid; i < n; i += blockDim.x) {
       const uint32_t cell = sc.cell[base + i];
       const uint32_t sh = (cell & 1u) * 16u;
       sc.perm[base + ((atomicAdd(&cnt[cell >> 1], 1u << sh) >> sh) & 0xffffu)] = i;
     }
   }
   __syncthreads();
-  for (uint32_t c = tid; c < C; c += GRID_THREADS) {
+  for (uint32_t c = tid; c < C; c += blockDim.x) {
     const uint32_t lo = c ? half_of(cnt[(c - 1) >> 1], c - 1) : 0u, hi = half_of(cnt[c >> 1], c);
     if (hi - lo < 2) continue;
     if (inSmem) {
@@ -324,7 +330,7 @@ __global__ void __launch_bounds__(GRID_THREADS)
   __syncthreads();
 
   // 4. gather into cell order (gridStore, GridBuilder.h:243-253)
-  for (uint32_t s = tid; s < n; s += GRID_THREADS) {
+  for (uint32_t s = tid; s < n; s += blockDim.x) {
     const uint32_t dst = base + s;
     const uint32_t i = inSmem ? (uint32_t)permS[s] : sc.perm[dst];
     const uint32_t src = base + i;
@@ -454,6 +460,13 @@ cudaError_t grid_prepare(int) {
   return cudaFuncSetAttribute(fine_grid_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GRID_SMEM_MAX);
 }
 
+// More threads per CTA while that many CTAs still fit the chip at once: with
+// few tasks the latency of one CTA's phases is the whole build.
+static unsigned grid_threads(uint32_t tasks) {
+  const uint32_t sms = (uint32_t)sm_count();
+  return tasks <= sms ? 1024u : tasks <= 4u * sms ? 512u : 256u;
+}
+
 cudaError_t grid_build(const DevConfig& cfg, const GridInput& in, uint32_t* grid, DevHits out, GridScratch sc,
                        uint32_t maxLayerHits, uint32_t* err, Queue& q) {
   const uint32_t tasks = cfg.E * cfg.L;
@@ -464,11 +477,12 @@ cudaError_t grid_build(const DevConfig& cfg, const GridInput& in, uint32_t* grid
   // 16-bit counters, cells and slots when every index fits
   const size_t bytes16 = (size_t)maxLayerHits * 8 + (size_t)(cfg.C + 1) / 2 * 4;
   if (useSmem && cfg.C < 65536u && maxLayerHits < 65536u && bytes16 <= GRID_SMEM_MAX) {
-    launch(q, grid_kernel16, tasks, GRID_THREADS, bytes16, cfg, in, grid, out, sc, err, maxLayerHits);
+    launch(q, grid_kernel16, tasks, grid_threads(tasks), bytes16, cfg, in, grid, out, sc, err, maxLayerHits);
     return cudaGetLastError();
   }
   const bool hitsFit = useSmem && counterBytes + hitBytes <= GRID_SMEM_MAX;
-  launch(q, grid_kernel, tasks, GRID_THREADS, counterBytes + (hitsFit ? hitBytes : 0), cfg, in, grid, out, sc, err,
+  launch(q, grid_kernel, tasks, grid_threads(tasks), counterBytes + (hitsFit ? hitBytes : 0), cfg, in, grid, out,
+         sc, err,
          useSmem, hitsFit ? maxLayerHits : 0u);
   return cudaGetLastError();
 }
