@@ -104,14 +104,14 @@ def test_linking_after_a_callers_links(trax_lib):
 
 @pytest.mark.parametrize("n_z, n_phi", [(80, 256), (4, 8), (1, 1), (3, 40)])
 def test_mask_walk_range_lengths(trax_lib, oracle_lib, n_z, n_phi):
-    """The prediction's walk by masks (16 or more captured candidates) over visit ranges from none to far more than
+    """The prediction's walk by masks (8 or more captured candidates) over visit ranges from none to far more than
     the 32 hits of a mask, the last layer's hits at the end of the hit arrays included: every array as the oracle's."""
     batch = events.generate(1, n_events=5)
     batch.n_z, batch.n_phi = n_z, n_phi
     want = oracle_lib.run(batch)[0]
     with trax_lib.Context(0) as ctx:
         ctx.upload(batch)
-        for slots in (16, 32, 4):
+        for slots in (16, 32, 8, 4):
             ctx.set_candidate_slots(slots)
             ctx.seed_batch(use_graph=False)
             got = ctx.results()

@@ -138,28 +138,18 @@ __device__ __forceinline__ void fine_walk(const DevConfig& cfg, const PredUnionW
   }
 }
 
-// The test of one visited hit in walk_range: z within the union
-// of both variants' bounds, and phi in the window.  The phi test
+// The hits of a walk whose z lies in the union of both variants' bounds, taken
+// in grid order: the phi test and each variant's own z test, the count, and
+// the first nKeep of the store variant in the slots.  The phi test
 // (TripletThetaPhiPredictor.h:211-214) on hit angles from atan2_, which lie
 // in [-pi, pi] or are NaN: the wrapped window's `phi <= pi` and `-pi <= phi`
-// always hold, so it is lo || hi, the plain one lo && hi -- the majority of
-// (lo, hi, wrap) (NaN fails both, as in the reference's form).
-struct VisitTest {
-  float zLow, zHigh, phiLow, phiHigh;
-  bool wrap;
-  __device__ __forceinline__ bool operator()(float z, float phi) const {
-    const bool lo = phiLow <= phi, hi = phi <= phiHigh;
-    return zLow <= z && z <= zHigh && ((lo && hi) || (wrap && (lo || hi)));
-  }
-};
-
-// The hits of a walk that passed the visit test, taken in grid order: each
-// variant's own z test, the count, and the first nKeep of the store
-// variant in the slots.
+// always hold, so it is lo || hi, the plain one lo && hi (NaN fails both, as
+// in the reference's form).
 template <class Slots>
 struct Taker {
   const float2* zphi;  // (z, phi) of grid-ordered hit j at zphi[2 j]
-  float zl0, zh0, zl1, zh1;
+  float zl0, zh0, zl1, zh1, phiLow, phiHigh;
+  bool wrap;
   Slots slot;
   uint32_t nKeep;
   uint32_t count = 0, nStore = 0;
@@ -168,9 +158,11 @@ struct Taker {
     while (m) {
       const uint32_t j = j0 + (uint32_t)__ffs(m) - 1u;
       m &= m - 1u;
-      const float z = __ldg(&zphi[2 * (size_t)j].x);
-      count += (zl0 <= z && z <= zh0);
-      if (zl1 <= z && z <= zh1) {
+      const float2 h = __ldg(zphi + 2 * (size_t)j);
+      const bool lo = phiLow <= h.y, hi = h.y <= phiHigh;
+      if (!(wrap ? (lo || hi) : (lo && hi))) continue;
+      count += (zl0 <= h.x && h.x <= zh0);
+      if (zl1 <= h.x && h.x <= zh1) {
         if (nStore < nKeep) slot[nStore] = j;
         ++nStore;
       }
@@ -178,34 +170,39 @@ struct Taker {
   }
 };
 
-// The walk over one visit range [a, b) of the grid, the tests first and the
-// passing hits after them: 32 hits give one mask, tested four at a time
-// (independent loads; up to three hits past b are read and dropped, the
-// array has that many more), and only the bits set are then taken.  A visit
-// costs the tests alone, and the few passing hits of a warp's lanes are taken
-// in as many steps as its busiest lane has, not in as many as the lanes
-// visit.  What bounds the walk is instruction issue.  It is the walk of pairs
-// with 16 or more captured candidates (IL): three pileup events, about 30
-// visits per pair, 4.33 -> 2.72 ms; with the 4 visits per pair of the
-// ttbar-like batch the plain loop is as fast (2.39 against 2.42 ms) and
-// stays.
+// The walk over one visit range [a, b) of the grid, z first and the rest on
+// the hits that pass it: 32 hits give one mask, tested against the union's z
+// bounds four at a time (one 16-byte load of the z column; up to three hits
+// before a and past b are read and dropped, the column has that many more),
+// and only the bits set are then taken.  A visit costs a quarter of a load
+// and the z test, which nine in ten fail where rows are long against the
+// window, and the passing hits of a warp's lanes are taken in as many steps
+// as its busiest lane has, not in as many as the lanes visit.  What bounds
+// it is instruction issue.  Three pileup events, about 30 visits per pair:
+// 4.33 ms with a plain loop over the visits, 2.73 ms with z and phi tested in
+// the first step (wider groups were slower: eight hits 3.15 ms), 2.25 ms so.
+// It is the walk of pairs with 8 or more captured candidates; with the 4
+// visits per pair of the ttbar-like batch the plain loop is faster (2.39
+// against 2.61 ms) and stays.
 template <class Slots>
-__device__ __forceinline__ void walk_range(Taker<Slots>& t, const VisitTest& test, uint32_t a, uint32_t b,
-                                           const DevConfig& cfg) {
-  for (uint32_t base = a; base < b; base += 32u) {
+__device__ __forceinline__ void walk_range(Taker<Slots>& t, const float* __restrict__ hitZ, float zLow, float zHigh,
+                                           uint32_t a, uint32_t b, const DevConfig& cfg) {
+  if (a >= b || trax_hit(b - 1u, cfg) != b - 1u) return;
+  for (uint32_t base = a & ~3u; base < b; base += 32u) {
     const uint32_t len = min(b - base, 32u);
     uint32_t m = 0;
     for (uint32_t q = 0; q < len; q += 4u) {
-      const float2* p = t.zphi + 2 * (size_t)trax_hit(base + q, cfg);
-      const float2 h0 = __ldg(p), h1 = __ldg(p + 2), h2 = __ldg(p + 4), h3 = __ldg(p + 6);
+      const float4 z = __ldg(reinterpret_cast<const float4*>(hitZ + base + q));
       uint32_t n = 0;
-      if (test(h0.x, h0.y)) n |= 1u;
-      if (test(h1.x, h1.y)) n |= 2u;
-      if (test(h2.x, h2.y)) n |= 4u;
-      if (test(h3.x, h3.y)) n |= 8u;
+      if (zLow <= z.x && z.x <= zHigh) n |= 1u;
+      if (zLow <= z.y && z.y <= zHigh) n |= 2u;
+      if (zLow <= z.z && z.z <= zHigh) n |= 4u;
+      if (zLow <= z.w && z.w <= zHigh) n |= 8u;
       m |= n << q;
     }
-    t.take(base, m & (0xffffffffu >> (32u - len)));
+    m &= 0xffffffffu >> (32u - len);
+    if (base < a) m &= 0xffffffffu << (a - base);
+    t.take(base, m);
   }
 }
 
@@ -223,9 +220,11 @@ __device__ __forceinline__ void walk_range(Taker<Slots>& t, const VisitTest& tes
 //
 // FINE: the walk goes over the fine z grid instead (fine_walk), with the
 // same counts and captured candidates.  IL: the slots' layout (keep_slots).
-template <bool FINE, bool IL>
+// MASK: the grid walk by masks (walk_range).
+template <bool FINE, bool IL, bool MASK>
 __global__ void __launch_bounds__(TRAX_MAX_TUNED_THREADS, 6)
     predict_count_kernel(Stamp stamp, DevConfig cfg, const uint32_t* __restrict__ grid, const float4* __restrict__ hits,
+                         const float* __restrict__ hitZ,
                          const uint32_t* __restrict__ hitEvt, const uint32_t* __restrict__ hitLayer,
                          const uint2* __restrict__ pairs, const uint32_t* __restrict__ nPairsDev, uint32_t* candCount,
                          uint32_t* keep, uint32_t* warpSums, uint32_t* nWarpsOut, uint32_t* err, FineGrid fine) {
@@ -262,20 +261,20 @@ __global__ void __launch_bounds__(TRAX_MAX_TUNED_THREADS, 6)
       const float2* zphi = reinterpret_cast<const float2*>(hits) + 1;  // (z, phi) of hit j at zphi[2 j]
       if (FINE && w.pL <= nP) {
         fine_walk<true>(cfg, w, fine, event, layer, slot, nKeep, count, nStore);
-      } else if (IL && !FINE) {
+      } else if (MASK) {
         // a switched-off variant's bounds are (+inf, -inf)
-        const VisitTest test{fminf(zl0, zl1), fmaxf(zh0, zh1), w.phiLow, w.phiHigh, wrap};
-        Taker<KeepSlots<IL, uint32_t>> t{zphi, zl0, zh0, zl1, zh1, slot, nKeep};
+        const float zLow = fminf(zl0, zl1), zHigh = fmaxf(zh0, zh1);
+        Taker<KeepSlots<IL, uint32_t>> t{zphi, zl0, zh0, zl1, zh1, w.phiLow, w.phiHigh, wrap, slot, nKeep};
         for (uint32_t zs = w.zLo; zs < w.zHi; ++zs) {
           if (!wrap && w.pL <= nP) {  // one range, as below
             const uint32_t row = zs * (nP + 1);
-            walk_range(t, test, cell_at(lG3, row + w.pL, C), cell_at(lG3, row + w.pH, C), cfg);
+            walk_range(t, hitZ, zLow, zHigh, cell_at(lG3, row + w.pL, C), cell_at(lG3, row + w.pH, C), cfg);
           } else {
             uint32_t a[2], b[2];
             pred_row_parts(w, lG3, C, nP, zs, a[0], b[0], a[1], b[1]);
 #pragma unroll 1
             for (int part = 0; part < 2; ++part)
-              walk_range(t, test, part ? a[1] : a[0], part ? b[1] : b[0], cfg);
+              walk_range(t, hitZ, zLow, zHigh, part ? a[1] : a[0], part ? b[1] : b[0], cfg);
           }
         }
         count = t.count;
@@ -832,14 +831,18 @@ cudaError_t predict_pairs(const DevConfig& cfg, bool emit, const uint32_t* grid,
              hits.layer, pairs, nPairsDev, candCount, warpSums, keep, cands, cap, sentinels, fine, pairOffsets,
              candOffsets);
   } else if (cfg.fineRows > 0 && fine.grid) {
-    launch(q, (predict_count_kernel<true, true>), blocks, threads, 0, cfg, grid, hits.xyzp, hits.evt, hits.layer,
-           pairs, nPairsDev, candCount, keep, warpSums, nWarpsOut, err, fine);
+    launch(q, (predict_count_kernel<true, true, false>), blocks, threads, 0, cfg, grid, hits.xyzp, hits.z, hits.evt,
+           hits.layer, pairs, nPairsDev, candCount, keep, warpSums, nWarpsOut, err, fine);
   } else if (il) {  // the K-pairs kernel keeps the consecutive layout
-    launch(q, (predict_count_kernel<false, true>), blocks, threads, 0, cfg, grid, hits.xyzp, hits.evt, hits.layer,
-           pairs, nPairsDev, candCount, keep, warpSums, nWarpsOut, err, fine);
+    launch(q, (predict_count_kernel<false, true, true>), blocks, threads, 0, cfg, grid, hits.xyzp, hits.z, hits.evt,
+           hits.layer, pairs, nPairsDev, candCount, keep, warpSums, nWarpsOut, err, fine);
   } else if (cfg.predPairsPerThread <= 1 || !pred_k_fits(cfg)) {
-    launch(q, (predict_count_kernel<false, false>), blocks, threads, 0, cfg, grid, hits.xyzp, hits.evt, hits.layer,
-           pairs, nPairsDev, candCount, keep, warpSums, nWarpsOut, err, fine);
+    if (cfg.predKeep >= 8u)
+      launch(q, (predict_count_kernel<false, false, true>), blocks, threads, 0, cfg, grid, hits.xyzp, hits.z, hits.evt,
+             hits.layer, pairs, nPairsDev, candCount, keep, warpSums, nWarpsOut, err, fine);
+    else
+      launch(q, (predict_count_kernel<false, false, false>), blocks, threads, 0, cfg, grid, hits.xyzp, hits.z,
+             hits.evt, hits.layer, pairs, nPairsDev, candCount, keep, warpSums, nWarpsOut, err, fine);
   } else {
     const int K = cfg.predPairsPerThread;
     const size_t smem = (size_t)threads * K * sizeof(PredStage);
