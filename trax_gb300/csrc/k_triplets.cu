@@ -63,18 +63,20 @@ struct CandSlots {
 //    and keeps it in its grid row's block, so its fine row is among them.
 //    Hits outside those rows fail both z tests, as in the grid walk.
 // The captured candidates are the first nKeep store-valid visits in the
-// grid walk's order, (row, part, grid index): the visits of one (row, part)
-// come here in fine order, so the slots of the current (row, part) are kept
-// sorted by grid index -- appended while they come in order (the largest
+// grid walk's order, (row, part, grid index).  The visits of one (row, part)
+// come here in fine order.  ORDERED: the slots of the current (row, part) are
+// kept sorted by grid index -- appended while they come in order (the largest
 // is kept in a register), inserted otherwise -- and a visit past the last
-// slot replaces the largest of them when it is smaller.  COUNT: count the
-// count variant's valid visits too (the count pass); otherwise (the store
-// pass's re-walk, both variants the store variant) stop at the first
-// (row, part) after nKeep captures, which can add nothing.
-template <bool COUNT, class Slots>
+// slot replaces the largest of them when it is smaller.  Otherwise they are
+// appended as they come and `last` turns TRAX_SENTINEL when they are not in
+// ascending order, for the caller to sort.  COUNT: count the count variant's
+// valid visits too (the count pass); otherwise (the store pass's re-walk, both
+// variants the store variant) stop at the first (row, part) after nKeep
+// captures, which can add nothing.
+template <bool COUNT, bool ORDERED, class Slots>
 __device__ __forceinline__ void fine_walk(const DevConfig& cfg, const PredUnionWindow& w, const FineGrid& fine,
                                           uint32_t event, uint32_t layer, Slots slot, uint32_t nKeep,
-                                          uint32_t& count, uint32_t& nStore) {
+                                          uint32_t& count, uint32_t& nStore, uint32_t& last) {
   const uint32_t F = cfg.fineRows, Cf = cfg.fineC, nP = cfg.nP;
   const uint32_t* lG = fine.grid + ((size_t)event * cfg.L + layer) * Cf;
   // zl, zh as pred_union_window (a switched-off variant holds +inf, -inf);
@@ -89,7 +91,7 @@ __device__ __forceinline__ void fine_walk(const DevConfig& cfg, const PredUnionW
     for (uint32_t part = 0; part <= w.wrap; ++part) {
       if (!COUNT && nStore >= nKeep) return;
       const uint32_t cs = nStore;  // the first visit of this (row, part)
-      uint32_t last = 0u;          // the largest kept of this (row, part), at min(nStore, nKeep) - 1
+      if (ORDERED) last = 0u;      // the largest kept of this (row, part), at min(nStore, nKeep) - 1
       // part 0: columns [pL, pH), or [pL, nP] under wrap; part 1: [0, pH)
       const uint32_t ca = part ? 0u : w.pL;
       const uint32_t cb = (wrap && !part) ? nP + 1u : w.pH;
@@ -105,7 +107,10 @@ __device__ __forceinline__ void fine_walk(const DevConfig& cfg, const PredUnionW
           if (COUNT) count += (phiOk && zl0 <= h.x && h.x <= zh0);
           if (phiOk && zl1 <= h.x && h.x <= zh1) {
             const uint32_t j = __float_as_uint(h.z);
-            if (nStore < nKeep) {
+            if (!ORDERED) {
+              if (nStore < nKeep) slot[nStore] = j;
+              last = j >= last ? j : TRAX_SENTINEL;
+            } else if (nStore < nKeep) {
               if (nStore == cs || j > last) {  // in grid order: append
                 slot[nStore] = j;
                 last = j;
@@ -206,6 +211,48 @@ __device__ __forceinline__ void walk_range(Taker<Slots>& t, const float* __restr
   }
 }
 
+// fine_walk in order for the pairs that need it (below), out of line so that
+// its registers do not weigh on the others.
+struct FineCaptures {
+  uint32_t count, nStore;
+};
+template <class Slots>
+__device__ __noinline__ FineCaptures fine_walk_ordered(const DevConfig& cfg, PredUnionWindow w, FineGrid fine,
+                                                       uint32_t event, uint32_t layer, Slots slot, uint32_t nKeep) {
+  FineCaptures c{0u, 0u};
+  uint32_t last = 0u;
+  fine_walk<true, true>(cfg, w, fine, event, layer, slot, nKeep, c.count, c.nStore, last);
+  return c;
+}
+
+// Sorts the first n <= N values of the slots (n of this lane; 0: none).  A
+// sorting network (Batcher's odd-even merge) over N registers, missing
+// values as TRAX_SENTINEL: the same steps for every lane, where sorting by
+// insertion as the visits came took the lanes of a warp through one
+// another's branches.
+template <int N, class Slots>
+__device__ __forceinline__ void sort_slots(Slots slot, uint32_t n) {
+  uint32_t v[N];
+#pragma unroll
+  for (int k = 0; k < N; ++k) v[k] = (uint32_t)k < n ? slot[k] : TRAX_SENTINEL;
+#pragma unroll
+  for (int p = 1; p < N; p *= 2)
+#pragma unroll
+    for (int k = p; k >= 1; k /= 2)
+#pragma unroll
+      for (int j = k % p; j + k < N; j += 2 * k)
+#pragma unroll
+        for (int i = 0; i < k; ++i)
+          if (i + j + k < N && (i + j) / (2 * p) == (i + j + k) / (2 * p)) {
+            const uint32_t a = v[i + j], b = v[i + j + k];
+            v[i + j] = min(a, b);
+            v[i + j + k] = max(a, b);
+          }
+#pragma unroll
+  for (int k = 0; k < N; ++k)
+    if ((uint32_t)k < n) slot[k] = v[k];
+}
+
 // Count pass (predictCount, :190-219) that also captures the first
 // min(count, cfg.predKeep) candidates the store pass would write (the store
 // variant's valid hits, capped at the count; slots it would leave unwritten
@@ -237,6 +284,7 @@ __global__ void __launch_bounds__(TRAX_MAX_TUNED_THREADS, 6)
     const uint32_t gid = base + lane;
     const uint2 pr = gid < nPairs ? pairs[gid] : make_uint2(TRAX_SENTINEL, TRAX_SENTINEL);
     uint32_t count = 0;
+    uint32_t nSort = 0;  // FINE: captured slots to be sorted
     if (pr.x != TRAX_SENTINEL) {
       const uint32_t hx = trax_hit(pr.x, cfg), hy = trax_hit(pr.y, cfg);
       const uint32_t event = hitEvt[hx];
@@ -260,7 +308,25 @@ __global__ void __launch_bounds__(TRAX_MAX_TUNED_THREADS, 6)
       const float zl0 = w.zLow[0], zh0 = w.zHigh[0], zl1 = w.zLow[1], zh1 = w.zHigh[1];
       const float2* zphi = reinterpret_cast<const float2*>(hits) + 1;  // (z, phi) of hit j at zphi[2 j]
       if (FINE && w.pL <= nP) {
-        fine_walk<true>(cfg, w, fine, event, layer, slot, nKeep, count, nStore);
+        // Rows follow one another in grid order, so a window that does not
+        // wrap captures in ascending order of grid index all in all: its
+        // captures are appended as they come and sorted below.  In order
+        // from the start: windows that wrap (their second part comes first
+        // in the grid), more than 16 slots, and a pair with more store-valid
+        // visits than slots but no more candidates than slots (Q4's two
+        // roundings), whose first captures in order must be found.
+        bool ordered = wrap || nKeep > 16u;
+        if (!ordered) {
+          uint32_t last = 0u;
+          fine_walk<true, false>(cfg, w, fine, event, layer, slot, nKeep, count, nStore, last);
+          ordered = nStore > nKeep && count <= nKeep;
+          if (last == TRAX_SENTINEL && nStore <= nKeep) nSort = nStore;
+        }
+        if (ordered) {
+          const FineCaptures c = fine_walk_ordered(cfg, w, fine, event, layer, slot, nKeep);
+          count = c.count;
+          nStore = c.nStore;
+        }
       } else if (MASK) {
         // a switched-off variant's bounds are (+inf, -inf)
         const float zLow = fminf(zl0, zl1), zHigh = fmaxf(zh0, zh1);
@@ -312,6 +378,12 @@ __global__ void __launch_bounds__(TRAX_MAX_TUNED_THREADS, 6)
       // slots the reference leaves unwritten
       const uint32_t k = min(count, nKeep);
       for (uint32_t q = nStore; q < k; ++q) slot[q] = TRAX_SENTINEL;
+    }
+    if (FINE) {  // warp-uniform: the lanes' captures sorted together
+      const uint32_t most = __reduce_max_sync(0xffffffffu, nSort);
+      const KeepSlots<IL, uint32_t> slot = keep_slots<IL>(keep, gid, cfg.predKeep);
+      if (most > 8u) sort_slots<16>(slot, nSort);
+      else if (most > 0u) sort_slots<8>(slot, nSort);
     }
     uint32_t incl = count;
 #pragma unroll
@@ -596,8 +668,8 @@ __global__ void __launch_bounds__(TRAX_MAX_TUNED_THREADS, FINE ? 6 : 8)
       u.pL = w.pL;
       u.pH = w.pH;
       u.wrap = w.wrap;
-      uint32_t unused = 0;
-      fine_walk<false>(cfg, u, fine, event, layer, CandSlots{out, gid}, limit, unused, n);
+      uint32_t unused = 0, last = 0;
+      fine_walk<false, true>(cfg, u, fine, event, layer, CandSlots{out, gid}, limit, unused, n, last);
       n = min(n, limit);
     } else
     for (uint32_t zs = w.zLoSec[1]; zs < w.zHiSec[1] && n < limit; ++zs) {
