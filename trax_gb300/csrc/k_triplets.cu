@@ -640,11 +640,28 @@ __global__ void __launch_bounds__(TRAX_MAX_TUNED_THREADS, FINE ? 6 : 8)
     if (limit == 0) continue;
     uint2* out = cands + pos;
     if (limit <= cfg.predKeep) {
+      // the slots are read in groups before any of them is written: one
+      // at a time, every read waited for the one before it
       const KeepSlots<IL, const uint32_t> slot = keep_slots<IL>(keep, gid, cfg.predKeep);
-      for (uint32_t q = 0; q < limit; ++q) {
-        const uint32_t h = slot[q];
-        sent += h == TRAX_SENTINEL;
-        out[q] = make_uint2(gid, h);
+      constexpr uint32_t GROUP = IL ? 8u : 4u;
+      for (uint32_t q0 = 0; q0 < limit; q0 += GROUP) {
+        uint32_t h[GROUP];
+        if (IL) {
+#pragma unroll
+          for (uint32_t k = 0; k < GROUP; ++k) h[k] = q0 + k < limit ? slot[q0 + k] : 0u;
+        } else {  // four or eight consecutive slots, 16-byte aligned
+          const uint4 v = __ldg(reinterpret_cast<const uint4*>(slot.p + q0));
+          h[0] = v.x;
+          h[1] = v.y;
+          h[2] = v.z;
+          h[3] = v.w;
+        }
+#pragma unroll
+        for (uint32_t k = 0; k < GROUP; ++k)
+          if (q0 + k < limit) {
+            sent += h[k] == TRAX_SENTINEL;
+            out[q0 + k] = make_uint2(gid, h[k]);
+          }
       }
       continue;
     }
