@@ -470,9 +470,10 @@ int stage_grid(trax_ctx* c, Mode mode) {
   const uint64_t n = c->nHits;
   const uint64_t cells = (uint64_t)c->E * c->L * c->cfg.C;
   ENSURE(grid, cells, 4);
-  ENSURE(px, n, 4); ENSURE(py, n, 4); ENSURE(pz, n, 4);
+  ENSURE(px, n, 4); ENSURE(py, n, 4);
+  ENSURE(pz, n + 4, 4);  // walk_range reads up to 3 hits past a range
   ENSURE(player, n, 4); ENSURE(pdet, n, 4); ENSURE(phid, n, 4); ENSURE(pevt, n, 4); ENSURE(porig, n, 4);
-  ENSURE(pxyzp, n + 4, 16);  // walk_range reads up to 3 hits past a range
+  ENSURE(pxyzp, n, 16);
   ENSURE(sc_cell, n, 4); ENSURE(sc_phi, n, 4); ENSURE(sc_perm, n, 4);
   uint64_t counters = c->cfg.C > TRAX_GRID_SMEM_CELLS ? cells : 0;
   if (fine_counter_cells(c->cfg) > counters) counters = fine_counter_cells(c->cfg);
@@ -1335,7 +1336,7 @@ int trax_set_tracklets(trax_ctx* c, const uint32_t* h1, const uint32_t* h2, cons
   }
   ENSURE(px, nh, 4); ENSURE(py, nh, 4); ENSURE(pz, nh, 4);
   ENSURE(player, nh, 4); ENSURE(pdet, nh, 4); ENSURE(phid, nh, 4); ENSURE(pevt, nh, 4); ENSURE(porig, nh, 4);
-  ENSURE(pxyzp, nh + 4, 16);
+  ENSURE(pxyzp, nh, 16);
   ENSURE(h1, n, 4);
   ENSURE(h2, n, 4);
   ENSURE(h3, n, 4);
