@@ -1,4 +1,6 @@
 """Launch structure of the chain: time marks."""
+import dataclasses
+
 import numpy as np
 import pytest
 
@@ -117,3 +119,25 @@ def test_mask_walk_range_lengths(trax_lib, oracle_lib, n_z, n_phi):
             got = ctx.results()
             for name in ("pairs", "cands", "cand_offsets", "trip_h1", "trip_h2", "trip_h3"):
                 assert np.array_equal(got[name], want[name]), (slots, name)
+
+
+def test_one_graph_serves_a_stream_of_unequal_batches(trax_lib, oracle_lib):
+    """Groups of one shape replay one captured graph whatever their number of hits, as long as they fit: more hits than
+    the captured buffers, a larger layer than the captured grid layout or more pairs than the capacities capture anew.
+    Every group's results are the oracle's."""
+    groups = [events.generate(1, n_events=6, seed=s) for s in (3, 4, 5)]
+    dense = events.generate_workload(dataclasses.replace(events.workload(1, 6), n_tracks=420), seed=6)
+    want = [oracle_lib.run(b)[0] for b in groups + [dense]]
+    names = ("pairs", "cands", "trip_offsets", "trip_h1", "trip_h3", "link_basis", "connectable", "tracks")
+    with trax_lib.Context(0) as ctx:
+        ctx.upload(groups[0])
+        captures = []
+        for k in (0, 1, 2, 0, 3, 1, 2, 3):
+            b = (groups + [dense])[k]
+            ctx.upload_hits(b)
+            captures.append(ctx.seed_batch(use_graph=True).graph_captures)
+            got = ctx.results()
+            for name in names:
+                assert np.array_equal(got[name], want[k][name]), (k, name)
+    assert captures[0] == 1 and captures[3] == 0 and captures[4] >= 1
+    assert captures[5:] == [0, 0, 0]  # the dense group's graph holds the others too

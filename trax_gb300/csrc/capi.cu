@@ -147,6 +147,7 @@ struct trax_ctx {
   size_t scanUsed = 0;  // scan scratch taken by the chain being captured
   uint32_t* hSlots = nullptr;  // pinned copy of the slots
   uint32_t maxLayerHits = 0;   // most hits of one (event, layer) in the uploaded batch
+  uint32_t capLayerHits = 0;   // the same the captured grid build is laid out for
   // sizes of the last run
   uint64_t nTasks = 0, nPairs = 0, nCands = 0, nT = 0, nLinks = 0, nConn = 0, nNonConn = 0, nTracks = 0;
   uint64_t pairSent = 0, candSent = 0;
@@ -163,6 +164,7 @@ struct trax_ctx {
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t graphExec = nullptr;
   uint64_t graphKey = 0;
+  uint64_t capShape = 0;  // batch shape the capacities were calibrated for
   uint64_t bufGeneration = 0;
   trax::WaitCtl wait;  // bounded-wait settings of every scan (trax_set_wait_limit, trax_debug_skip_publish)
   uint32_t graphLaunches = 0;
@@ -506,7 +508,8 @@ int stage_grid(trax_ctx* c, Mode mode) {
   sc.clearWords = mode == DEVICE ? (uint32_t)(chain_scan_bytes(c) / 16) : 0u;
   c->scanUsed = 0;
   KBEG(TK_GRID);
-  CK(grid_build(c->cfg, in, ptr<uint32_t>(c->grid), dev_hits(c), sc, c->maxLayerHits, dev_err(c), c->q));
+  CK(grid_build(c->cfg, in, ptr<uint32_t>(c->grid), dev_hits(c), sc,
+                mode == DEVICE ? c->capLayerHits : c->maxLayerHits, dev_err(c), c->q));
   CK(fine_grid_build(c->cfg, ptr<uint32_t>(c->grid), ptr<float4>(c->pxyzp), fine_buffers(c), sc.counts, c->q));
   c->fineBuilt = c->cfg.fineRows;
   KEND(TK_GRID);
@@ -836,14 +839,22 @@ int chain_device(trax_ctx* c, bool linking) {
 uint64_t with_headroom(uint64_t n) { return n + n / 4 + 4096; }
 
 // Size every buffer for DEVICE mode from the sizes of the last SYNCED run.
+// Capacities calibrated on earlier batches of the same shape are not given
+// up: a stream of unequal batches settles on one graph.
 int size_device_buffers(trax_ctx* c) {
   const Mode mode = SYNCED;
-  c->capTasks = with_headroom(c->nTasks);
-  c->capPairs = with_headroom(c->nPairs);
-  c->capCands = with_headroom(c->nCands);
-  c->capT = with_headroom(c->nT);
-  c->capLinks = with_headroom(c->nLinks);
-  c->capTracks = with_headroom(c->nTracks);
+  const uint64_t shape = ((uint64_t)c->E * TRAX_MAX_LAYERS + c->L) * (1ull << 22) * TRAX_MAX_LT +
+                         (uint64_t)c->cfg.C * TRAX_MAX_LT + c->cfg.nLT;
+  const bool same = c->capShape == shape;
+  c->capShape = shape;
+  auto cap = [same](uint64_t& cap, uint64_t n) { cap = same ? std::max(cap, with_headroom(n)) : with_headroom(n); };
+  cap(c->capTasks, c->nTasks);
+  cap(c->capPairs, c->nPairs);
+  cap(c->capCands, c->nCands);
+  cap(c->capT, c->nT);
+  cap(c->capLinks, c->nLinks);
+  cap(c->capTracks, c->nTracks);
+  c->capLayerHits = grid_layer_room(c->cfg, c->maxLayerHits);
   const uint32_t S = c->cfg.E * c->cfg.nLT;
   ENSURE(taskCount, c->capTasks + 1, 4);
   ENSURE(taskState, pair_task_state_bytes(c->capTasks) + 16, 1);
@@ -890,20 +901,41 @@ uint32_t auto_keep_slots(uint64_t nCands, uint64_t nPairs) {
   return 32u;
 }
 
+// What a captured graph depends on.  Not the number of hits: the kernels take
+// their counts from the supplements and device slots, so a graph serves every
+// batch of its shape whose hits fit the captured buffers (graph_fits) and
+// whose pairs, candidates, triplets and links stay within the capacities.  A
+// stream of groups of unequal size replays one graph, where keying on the
+// hits had every group calibrated by a host-synced run and captured anew.
 uint64_t shape_key(trax_ctx* c, bool linking) {
   uint64_t k = 1469598103934665603ull;
   auto mix = [&k](uint64_t v) {
     k ^= v;
     k *= 1099511628211ull;
   };
-  mix(c->E); mix(c->L); mix(c->nHits); mix(c->cfg.C); mix(c->cfg.nLT); mix(linking ? 1 : 0);
-  mix(c->maxLayerHits > 0xffffu ? 1 : 0);  // the grid build's 16-bit counters hold layers below 65 536 hits
+  mix(c->E); mix(c->L); mix(c->cfg.C); mix(c->cfg.nLT); mix(linking ? 1 : 0);
   mix(c->bufGeneration); mix(c->capTasks); mix(c->capPairs); mix(c->capCands); mix(c->capT); mix(c->capLinks);
-  mix(c->capTracks);
+  mix(c->capTracks); mix(c->capLayerHits);
   mix(c->wait.spinLimit); mix(c->wait.skipTile);  // captured into the scans' launch arguments
-  const unsigned char* b = reinterpret_cast<const unsigned char*>(&c->cfg);
+  DevConfig g = c->cfg;
+#if !defined(TRAX_BOUNDS_CHECK)
+  g.nHits = 0;  // only the bounds-checked build's kernels read it
+#endif
+  const unsigned char* b = reinterpret_cast<const unsigned char*>(&g);
   for (size_t i = 0; i < sizeof(DevConfig); ++i) mix(b[i]);
   return k;
+}
+
+// The uploaded hits fit the buffers and the grid layout the graph was captured with.
+bool graph_fits(trax_ctx* c) {
+  const size_t n = c->nHits;
+  const DevBuf* words[] = {&c->px, &c->py, &c->player, &c->pdet, &c->phid, &c->pevt, &c->porig, &c->sc_cell,
+                           &c->sc_phi, &c->sc_perm};
+  for (const DevBuf* b : words)
+    if (n * 4 > b->cap) return false;
+  if ((n + 4) * 4 > c->pz.cap || n * 16 > c->pxyzp.cap) return false;
+  if (c->cfg.fineRows && n * 16 > c->fineHits.cap) return false;
+  return c->maxLayerHits <= c->capLayerHits;
 }
 
 }  // namespace
@@ -1581,7 +1613,7 @@ int trax_seed_batch(trax_ctx* c, const trax_batch_opts* opts, trax_batch_stats* 
   for (int attempt = 0; attempt < 2; ++attempt) {
     RC(build_config(c));
     const uint64_t key = shape_key(c, linking);
-    if (!c->graphExec || key != c->graphKey) {
+    if (!c->graphExec || key != c->graphKey || !graph_fits(c)) {
       // calibrate the capacities with one host-synced run, then capture
       NvtxRange nvtxCal("trax.calibrate_and_capture");
       ++c->graphCaptures;

@@ -504,6 +504,24 @@ static unsigned grid_threads(uint32_t tasks) {
   return tasks <= sms ? 1024u : tasks <= 4u * sms ? 512u : 256u;
 }
 
+// shared memory of grid_kernel16, or 0 when it cannot take these layers
+static size_t grid16_bytes(const DevConfig& cfg, uint32_t maxLayerHits) {
+  const size_t bytes = (size_t)maxLayerHits * 8 + (size_t)(cfg.C + 1) / 2 * 4;
+  return cfg.C <= GRID_SMEM_CELLS && cfg.C < 65536u && maxLayerHits < 65536u && bytes <= GRID_SMEM_MAX ? bytes : 0;
+}
+
+uint32_t grid_layer_room(const DevConfig& cfg, uint32_t maxLayerHits) {
+  const size_t bytes = grid16_bytes(cfg, maxLayerHits);
+  if (!bytes) return maxLayerHits;
+  const size_t sm = 228u * 1024u, fixed = 1024u + 256u;  // per CTA: the system's share, static arrays
+  const size_t ctas = std::min<size_t>(sm / (bytes + fixed), 2048u / grid_threads(cfg.E * cfg.L));
+  size_t most = GRID_SMEM_MAX;
+  if (ctas > 1) most = std::min(most, sm / ctas - fixed);
+  if (most <= bytes) return maxLayerHits;
+  const size_t more = std::min<size_t>((most - bytes) / 8, maxLayerHits / 4);
+  return (uint32_t)std::min<size_t>(maxLayerHits + more, 65535u);
+}
+
 cudaError_t grid_build(const DevConfig& cfg, const GridInput& in, uint32_t* grid, DevHits out, GridScratch sc,
                        uint32_t maxLayerHits, uint32_t* err, Queue& q) {
   const uint32_t tasks = cfg.E * cfg.L;
@@ -512,8 +530,7 @@ cudaError_t grid_build(const DevConfig& cfg, const GridInput& in, uint32_t* grid
   const size_t counterBytes = useSmem ? (size_t)cfg.C * sizeof(uint32_t) : 0;
   const size_t hitBytes = (size_t)maxLayerHits * 3 * sizeof(uint32_t);
   // 16-bit counters, cells and slots when every index fits
-  const size_t bytes16 = (size_t)maxLayerHits * 8 + (size_t)(cfg.C + 1) / 2 * 4;
-  if (useSmem && cfg.C < 65536u && maxLayerHits < 65536u && bytes16 <= GRID_SMEM_MAX) {
+  if (const size_t bytes16 = grid16_bytes(cfg, maxLayerHits)) {
     launch(q, grid_kernel16, tasks, grid_threads(tasks), bytes16, cfg, in, grid, out, sc, err, maxLayerHits);
     return cudaGetLastError();
   }

@@ -163,6 +163,9 @@ struct GridScratch {
 cudaError_t grid_build(const DevConfig& cfg, const GridInput& in, uint32_t* grid, DevHits out,
                        GridScratch scratch, uint32_t maxLayerHits, uint32_t* err, Queue& q);
 cudaError_t grid_prepare(int device);  // one-time kernel attributes
+// Layer size a grid build captured for layers of up to maxLayerHits hits can
+// be laid out for at no cost: a quarter more, as far as the CTAs per SM stay.
+uint32_t grid_layer_room(const DevConfig& cfg, uint32_t maxLayerHits);
 
 // The fine z grid the prediction count walks when cfg.fineRows > 0: the
 // grid-ordered hits of every (event, layer) sorted again by fine cell (fine
