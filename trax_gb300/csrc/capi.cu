@@ -1946,7 +1946,7 @@ int trax_fit_prepare(trax_ctx* c, const trax_fit_opts* opts, uint64_t* n_fit) {
   }
   if (run > 0xffffffffull) return fail(c, TRAX_ERR_CAPACITY, "too many fit rows");
   c->nFit = run;
-  f.chunk = fit_chunk(run, sm_count());
+  f.chunk = fit_chunk(run, f.nLT, std::max(sm_count(), (int)TRAX_MAX_LT));
   uint64_t base = 0, blk = 0;
   for (uint32_t k = 0; k < f.nLT; ++k) {
     f.ltBase[k] = (uint32_t)base;

@@ -368,16 +368,18 @@ cudaError_t ca_tracks(CABuffers b, const uint32_t* nTDev, uint64_t maxT, uint32_
 // triplet k are [ltBase[k], ltBase[k+1]) and are reduced by the blocks
 // [blkStart[k], blkStart[k+1]), each taking `chunk` rows, so that every
 // sum is taken in a fixed order.
-// Rows per block: TRAX_FIT_CHUNK_MAX, or fewer (a power of two, at least one
-// row per thread) while that leaves fewer than eight blocks per SM -- 66 k
-// rows in blocks of 4096 kept 17 of 152 SMs busy.
+// Rows per block: two blocks of the gradient fit in an SM at a time, and about
+// four blocks per SM give two full waves of equal blocks, each thread with as
+// many rows as possible before the block's sums; at least one row per thread.
+// (Blocks of a fixed 4096 rows kept 17 of 152 SMs busy for 66 k rows, and
+// blocks of 512 spent a seventh of their instructions on the sums.)
 #define TRAX_FIT_CHUNK_MIN 256u
-#define TRAX_FIT_CHUNK_MAX 2048u
-inline uint32_t fit_chunk(uint64_t rows, int sms) {
-  uint32_t c = TRAX_FIT_CHUNK_MAX;
-  while (c > TRAX_FIT_CHUNK_MIN && rows / c < 8u * (uint64_t)sms) c >>= 1;
-  return c;
+inline uint32_t fit_chunk(uint64_t rows, uint32_t nLT, int sms) {
+  const uint64_t blocks = (uint64_t)sms * 4 - nLT;  // a layer triplet's last block is not full
+  const uint64_t c = (rows / blocks + TRAX_FIT_CHUNK_MIN) / TRAX_FIT_CHUNK_MIN * TRAX_FIT_CHUNK_MIN;
+  return (uint32_t)(c > 0x40000000ull ? 0x40000000ull : c);
 }
+
 // per block: chi2, d chi2 / d(dr, dz, dphi) of the three hit layers, and an
 // approximate Gauss-Newton diagonal for the same nine (a preconditioner)
 #define TRAX_FIT_SLOTS 19
