@@ -141,3 +141,37 @@ def test_one_graph_serves_a_stream_of_unequal_batches(trax_lib, oracle_lib):
                 assert np.array_equal(got[name], want[k][name]), (k, name)
     assert captures[0] == 1 and captures[3] == 0 and captures[4] >= 1
     assert captures[5:] == [0, 0, 0]  # the dense group's graph holds the others too
+
+
+@pytest.mark.parametrize("n", [1, 31, 255, 256, 257, 1025])
+def test_fit_block_edges(trax_lib, align_ref, n):
+    """The fit's sums over n rows (lanes, warps and blocks that are partly empty) against the FP64 reference, the error
+    relative to the sum of the rows' magnitudes: 5e-4 (hit gradients of single rows are within 3e-4)."""
+    batch = events.generate(4, n_events=2, seed=11)
+    batch.n_z, batch.n_phi = 50, 128
+    shifts = np.random.default_rng(n).normal(0, 1, (batch.n_layers, 3)) * [0.003, 0.003, 2e-5]
+    sigma_tip = [0.01 + 0.01 * k for k in range(len(batch.lts))]
+    with trax_lib.Context(0) as ctx:
+        ctx.upload(batch)
+        ctx.seed_batch(use_graph=False, run_linking=False)
+        h1, h2, h3, _ = ctx.triplets()
+        perm = ctx.hit_perm().astype(np.int64)
+        ids = batch.hit_id[perm]
+        good = np.nonzero((ids[h1] != 0) & (ids[h1] == ids[h2]) & (ids[h2] == ids[h3]))[0]
+        pick = good[np.linspace(0, good.size - 1, n).astype(np.int64)]
+        a, b, c = (perm[h[pick]] for h in (h1, h2, h3))
+        key = batch.event[a].astype(np.int64) * 16 + batch.layer[a]
+        o = np.argsort(key, kind="stable")
+        a, b, c = a[o], b[o], c[o]
+        ctx.set_tracklets(a, b, c)
+        assert ctx.fit_prepare(sigma_z=0.002, sigma_tip=sigma_tip, truth_only=True) == n
+        chi2, grad, _ = ctx.fit_backward(shifts)
+        chi2_f, params = ctx.fit_forward(shifts, params=True)
+    sig = np.asarray(sigma_tip)[batch.layer[a] - 1]
+    args = (batch.x, batch.y, batch.z, batch.layer)
+    want, want_grad, _ = align_ref.loss_and_grad(*args, a, b, c, np.ones(n), shifts, sig, 0.002)
+    size = sum(np.abs(align_ref.loss_and_grad(*args, a[k:k + 1], b[k:k + 1], c[k:k + 1], np.ones(1), shifts,
+                                              sig[k:k + 1], 0.002)[1]) for k in range(n))
+    assert abs(chi2 - want) <= 1e-4 * want and chi2_f == pytest.approx(chi2, rel=1e-12)
+    assert np.all(np.abs(grad - want_grad) <= 5e-4 * size.max(axis=0))
+    assert params.shape == (n, 4) and np.isfinite(params).all()

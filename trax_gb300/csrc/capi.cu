@@ -147,6 +147,7 @@ struct trax_ctx {
   size_t scanUsed = 0;  // scan scratch taken by the chain being captured
   uint32_t* hSlots = nullptr;  // pinned copy of the slots
   uint32_t maxLayerHits = 0;   // most hits of one (event, layer) in the uploaded batch
+  std::vector<uint64_t> layerTotals;  // hits of each layer in the uploaded batch
   uint32_t capLayerHits = 0;   // the same the captured grid build is laid out for
   // sizes of the last run
   uint64_t nTasks = 0, nPairs = 0, nCands = 0, nT = 0, nLinks = 0, nConn = 0, nNonConn = 0, nTracks = 0;
@@ -523,16 +524,17 @@ int stage_pairs(trax_ctx* c, Mode mode) {
   ENSURE(taskBase, S + 1, 4);
   ENSURE(pairOffsets, S + 1, 4);
   uint32_t* taskBase = ptr<uint32_t>(c->taskBase);
-  const uint64_t capTasks = mode == DEVICE ? c->capTasks : NO_CAP;
-  CK(pair_segments(c->cfg, ptr<uint32_t>(c->grid), ptr<uint32_t>(c->segOuter), taskBase,
-                   scan_total(c, mode, S_TASKS, capTasks), dev_err(c), c->q));
-  if (S > TRAX_SEGMENT_SCAN) RC(scan_publish(c, mode, taskBase, S, nullptr, S, S_TASKS, capTasks));
-  const uint32_t* nTasksDev = slot(c, S_TASKS);
+  // in SYNCED mode the host bounds the outer hits by the supplements' layers
+  // instead of waiting for their number
   uint64_t maxTasks = c->capTasks;
   if (mode == SYNCED) {
-    RC(read_total(c, S_TASKS, &c->nTasks));
-    maxTasks = c->nTasks;
+    maxTasks = 0;
+    for (uint32_t p = 0; p < c->cfg.nLT; ++p) maxTasks += c->layerTotals[c->cfg.layer2[p] - 1];
   }
+  CK(pair_segments(c->cfg, ptr<uint32_t>(c->grid), ptr<uint32_t>(c->segOuter), taskBase,
+                   scan_total(c, mode, S_TASKS, maxTasks), dev_err(c), c->q));
+  if (S > TRAX_SEGMENT_SCAN) RC(scan_publish(c, mode, taskBase, S, nullptr, S, S_TASKS, maxTasks));
+  const uint32_t* nTasksDev = slot(c, S_TASKS);
   ENSURE(taskCount, maxTasks + 1, 4);
   ENSURE(taskState, pair_task_state_bytes(maxTasks) + 16, 1);
   uint32_t* taskCount = ptr<uint32_t>(c->taskCount);
@@ -541,11 +543,11 @@ int stage_pairs(trax_ctx* c, Mode mode) {
   CK(pair_tasks(c->cfg, false, ptr<uint32_t>(c->grid), dev_hits(c), ptr<uint32_t>(c->segOuter), taskBase, nTasksDev,
                 maxTasks, taskCount, taskState, nullptr, 0, nullptr, slot(c, S_PAIR_SENT), dev_err(c), c->q));
   KEND(TK_PAIR_COUNT);
-  RC(scan_publish(c, mode, taskCount, c->nTasks, mode == DEVICE ? nTasksDev : nullptr, maxTasks, S_PAIRS,
-                  mode == DEVICE ? c->capPairs : NO_CAP));
+  RC(scan_publish(c, mode, taskCount, 0, nTasksDev, maxTasks, S_PAIRS, mode == DEVICE ? c->capPairs : NO_CAP));
   uint64_t maxPairs = c->capPairs;
   if (mode == SYNCED) {
     RC(read_total(c, S_PAIRS, &c->nPairs));
+    c->nTasks = c->hSlots[S_TASKS];
     maxPairs = c->nPairs;
   }
   ENSURE(pairs, maxPairs, 8);
@@ -708,10 +710,6 @@ int stage_connectivity(trax_ctx* c, Mode mode) {
                   maxTW, S_CONN, NO_CAP));
   CK(connectable_lists(tv, ptr<uint32_t>(c->connW), ptr<uint32_t>(c->connS), ptr<uint32_t>(c->connIdx),
                        ptr<uint32_t>(c->nonConnIdx), c->q));
-  if (mode == SYNCED) {
-    RC(read_total(c, S_CONN, &c->nConn));
-    c->nNonConn = c->nT - 1 - c->nConn;  // with links there are at least two triplets
-  }
   return TRAX_OK;
 }
 
@@ -810,6 +808,10 @@ int run_stage(trax_ctx* c, int stage) {
   mark(c, MARK_STAGE + stage);  // written by the read-back below, or again as the next stage starts
   c->stageUsed[stage - 1] = true;
   RC(check_device_error(c));
+  if (stage == 5 && !c->noLinks) {  // the lists' lengths came with that read-back
+    c->nConn = c->hSlots[S_CONN];
+    c->nNonConn = c->nT - 1 - c->nConn;  // with links there are at least two triplets
+  }
   c->stage = stage;
   if (stage == 4) ++c->tripGen;
   if (stage == 6) c->ptGen = c->tripGen;
@@ -1236,6 +1238,7 @@ int trax_upload_hits(trax_ctx* c, const trax_hits_soa* h, uint32_t n_hits, const
   // the supplements must describe the hits contiguously (HitCollection.cpp:120-133)
   uint64_t pos = 0;
   uint32_t maxLayer = 0;
+  std::vector<uint64_t> totals(n_layers, 0);
   for (uint32_t e = 0; e < n_events; ++e) {
     if (event_offsets[e] != pos) return fail(c, TRAX_ERR_ARG, "event offsets are not contiguous");
     uint64_t lpos = 0;
@@ -1243,6 +1246,7 @@ int trax_upload_hits(trax_ctx* c, const trax_hits_soa* h, uint32_t n_hits, const
       const size_t k = (size_t)e * n_layers + l;
       if (layer_offsets[k] != lpos) return fail(c, TRAX_ERR_ARG, "layer offsets are not contiguous");
       lpos += layer_hits[k];
+      totals[l] += layer_hits[k];
       maxLayer = std::max(maxLayer, layer_hits[k]);
     }
     pos += lpos;
@@ -1270,6 +1274,7 @@ int trax_upload_hits(trax_ctx* c, const trax_hits_soa* h, uint32_t n_hits, const
   c->L = n_layers;
   c->nHits = n_hits;
   c->maxLayerHits = maxLayer;
+  c->layerTotals = std::move(totals);
   c->haveHits = true;
   c->stage = 0;
   return TRAX_OK;
@@ -1327,6 +1332,8 @@ int trax_events_upload(trax_ctx* c, const trax_event_set* events, uint64_t first
   c->L = L;
   c->nHits = n;
   c->maxLayerHits = raw.maxLayerHits;
+  c->layerTotals.assign(L, 0);
+  for (size_t k = 0; k < raw.layerHits.size(); ++k) c->layerTotals[k % L] += raw.layerHits[k];
   c->haveHits = true;
   c->stage = 0;
   sizes->n_hits = n;
