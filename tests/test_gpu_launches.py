@@ -175,3 +175,28 @@ def test_fit_block_edges(trax_lib, align_ref, n):
     assert abs(chi2 - want) <= 1e-4 * want and chi2_f == pytest.approx(chi2, rel=1e-12)
     assert np.all(np.abs(grad - want_grad) <= 5e-4 * size.max(axis=0))
     assert params.shape == (n, 4) and np.isfinite(params).all()
+
+
+@pytest.mark.parametrize("tasks", [0, 36000, 120000])
+def test_pair_lanes_on_degenerate_windows(trax_lib, oracle_lib, tasks):
+    """The pair kernels with 8, 4 and 1 lanes per outer hit (by the number of outer hits) on the degenerate batch's
+    windows (NaN, infinite, wider than 2 pi, on cell edges), repeated to reach that number: every copy's pairs are the
+    oracle's, sentinels included."""
+    from tests.test_oracle_kats import degenerate_batch
+    few = degenerate_batch()
+    per = sum(int(few.layer_hits[:, lt.layer2 - 1].sum()) for lt in few.lts)
+    copies = tasks // per + 1
+    batch = few.subset(list(range(few.n_events)) * copies)
+    want = oracle_lib.run(few)[0]["pairs"].reshape(-1, 2).astype(np.int64)
+    with trax_lib.Context(0) as ctx:
+        ctx.upload(batch)
+        ctx.grid_build()
+        ctx.pair_gen()
+        p, off = ctx.pairs()
+        st = ctx.stats()
+    assert p.shape[0] == copies * want.shape[0] and off[-1] == p.shape[0]
+    shift = np.repeat(np.arange(copies) * few.n_hits, want.shape[0])[:, None]
+    p = p.astype(np.int64)
+    p[p != 0xFFFFFFFF] -= np.broadcast_to(shift, p.shape)[p != 0xFFFFFFFF]
+    assert np.array_equal(p, np.tile(want, (copies, 1)))
+    assert st.n_pair_sentinels == copies * int((want[:, 0] == 0xFFFFFFFF).sum())

@@ -258,6 +258,24 @@ __global__ void __launch_bounds__(SEG_THREADS)
   }
 }
 
+// The exact slow path of the store pass: every inner index that some visit
+// range of the task contains, up to `limit`; returns how many were written.
+__device__ uint32_t pair_store_unordered(const DevConfig& cfg, const PairWindow& w, const uint32_t* lG1,
+                                         const float4* hits, uint32_t i, uint32_t limit, uint2* out) {
+  const uint32_t C = cfg.C, innerBegin = lG1[0], innerEnd = lG1[C - 1];
+  uint32_t written = 0;
+  for (uint32_t j = innerBegin; j < innerEnd && written < limit; ++j) {
+    bool visited = false;
+    for (uint32_t zs = w.zLowSector; zs < w.zHighSector && !visited; ++zs) {
+      uint32_t a1, b1, a2, b2;
+      pair_row_parts(w, lG1, C, cfg.nP, zs, a1, b1, a2, b2);
+      visited = (a1 <= j && j < b1) || (a2 <= j && j < b2);
+    }
+    if (visited && pair_valid(w, hits[trax_hit(j, cfg)])) out[written++] = make_uint2(j, i);
+  }
+  return written;
+}
+
 template <bool EMIT>
 __global__ void __launch_bounds__(TRAX_MAX_TUNED_THREADS)
     pair_kernel(Stamp stamp, DevConfig cfg, const uint32_t* __restrict__ grid, const float4* __restrict__ hits,
@@ -350,18 +368,163 @@ __global__ void __launch_bounds__(TRAX_MAX_TUNED_THREADS)
         }
         if (written != limit) raise_error(err, TRAX_EBIT_BOUNDS);
       } else {
-        // exact slow path: every inner index that some visit range contains
-        const uint32_t innerBegin = lG1[0], innerEnd = lG1[C - 1];
-        for (uint32_t j = innerBegin; j < innerEnd && written < limit; ++j) {
-          bool visited = false;
-          for (uint32_t zs = w.zLowSector; zs < w.zHighSector && !visited; ++zs) {
-            uint32_t a1, b1, a2, b2;
-            pair_row_parts(w, lG1, C, nP, zs, a1, b1, a2, b2);
-            visited = (a1 <= j && j < b1) || (a2 <= j && j < b2);
-          }
-          if (visited && pair_valid(w, hits[trax_hit(j, cfg)])) out[written++] = make_uint2(j, i);
+        written = pair_store_unordered(cfg, w, lG1, hits, i, limit, out);
+      }
+      if (written < limit) {
+        atomicAdd(sentinels, limit - written);
+        for (uint32_t q = written; q < limit; ++q) out[q] = make_uint2(TRAX_SENTINEL, TRAX_SENTINEL);
+      }
+    }
+  }
+  if (!EMIT && blockIdx.x == 0 && threadIdx.x == 0) taskCount[nTasks] = 0u;  // the scan's +1 slot
+}
+
+// pair_kernel with G lanes per task, a z row each at a time, for batches whose
+// tasks leave the chip idle: there the time is the latency of one task's walk
+// over its rows, one visit after the other.  The count pass adds up the
+// lanes' rows; the store pass counts each row, scans the counts of the G
+// rows over the group and walks them again to write, so the pairs of a task
+// come out in the same order.  All lanes of a warp stay in step (the rounds
+// are those of its longest task), so that the shuffles see every lane.
+template <bool EMIT, int G>
+__global__ void __launch_bounds__(TRAX_MAX_TUNED_THREADS)
+    pair_group_kernel(Stamp stamp, DevConfig cfg, const uint32_t* __restrict__ grid, const float4* __restrict__ hits,
+                      const uint32_t* __restrict__ segOuter, const uint32_t* __restrict__ taskBase,
+                      const uint32_t* __restrict__ nTasksDev, uint32_t* taskCount, PairTaskState state, uint2* pairs,
+                      uint32_t capPairs, uint32_t* pairOffsets, uint32_t* sentinels, uint32_t* err) {
+  stamp_begin(stamp);
+  constexpr uint32_t ALL = 0xffffffffu;
+  const uint32_t S = cfg.E * cfg.nLT;
+  const uint32_t nTasks = *nTasksDev;
+  if (EMIT)  // taskCount is scanned: the first pair of every segment
+    for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s <= S; s += gridDim.x * blockDim.x)
+      pairOffsets[s] = s == 0 ? 0u : taskCount[min(taskBase[s], nTasks)];
+  const uint32_t C = cfg.C, nP = cfg.nP;
+  const uint32_t lane = threadIdx.x & 31u, sub = lane % G;
+  const float2* zphi = reinterpret_cast<const float2*>(hits) + 1;  // (z, phi) of hit j at zphi[2 j]
+  const uint32_t perStep = gridDim.x * (blockDim.x / G);
+  for (uint32_t k0 = (blockIdx.x * blockDim.x + (threadIdx.x & ~31u)) / G; k0 < nTasks; k0 += perStep) {
+    const uint32_t k = k0 + lane / G;
+    const bool task = k < nTasks;
+    uint32_t s = 0, i = 0;
+    PairWindow w;
+    w.zLowSector = w.zHighSector = 0u;
+    bool ordered = true;
+    if (task && !EMIT) {
+      s = find_segment(taskBase, S, k);
+      i = segOuter[s] + (k - taskBase[s]);
+      const float4 ho = hits[trax_hit(i, cfg)];
+      w = pair_window(cfg, s % cfg.nLT, ho.x, ho.y, ho.z, ho.w);
+    } else if (task) {
+      const float4 b = state.bounds[k];
+      const uint4 q = state.secs[k];
+      const uint2 id = state.ids[k];
+      i = id.x;
+      s = id.y;
+      w.zLow = b.x;
+      w.zHigh = b.y;
+      w.phiLow = b.z;
+      w.phiHigh = b.w;
+      w.zLowSector = q.x & 0x7fffffffu;
+      w.zHighSector = q.y & 0x7fffffffu;
+      w.pL = q.z;
+      w.pH = q.w;
+      w.wrap = q.y >> 31;
+      ordered = (q.x >> 31) != 0u;
+    }
+    const uint32_t e = s / cfg.nLT, p = s % cfg.nLT;
+    const uint32_t* lG1 = grid + ((size_t)e * cfg.L + (cfg.layer1[p] - 1)) * C;
+    const uint32_t rows = w.zLowSector < w.zHighSector ? w.zHighSector - w.zLowSector : 0u;
+    const uint32_t walked = EMIT && !ordered ? 0u : rows;  // the store pass's slow path does not walk by rows
+    const uint32_t rounds = (__reduce_max_sync(ALL, walked) + G - 1) / G;
+    uint32_t pos0 = 0, limit = 0;
+    if (EMIT && task) {
+      pos0 = taskCount[k];
+      limit = taskCount[k + 1] - pos0;
+      if (pos0 >= capPairs) limit = 0;
+      else if (limit > capPairs - pos0) limit = capPairs - pos0;
+    }
+    uint2* out = pairs + pos0;
+    uint32_t total = 0;         // of this lane's rows (count), of the task so far (store)
+    uint32_t prevEnd = 0;       // of the rounds before
+    bool inOrder = true;
+    PairTest t;
+    if (EMIT) t = pair_test(w);
+    for (uint32_t round = 0; round < rounds; ++round) {
+      const uint32_t r = round * G + sub;
+      uint32_t a1 = 0, b1 = 0, a2 = 0, b2 = 0;
+      if (r < walked) pair_row_parts(w, lG1, C, nP, w.zLowSector + r, a1, b1, a2, b2);
+      if (!EMIT) {
+        for (uint32_t j = a1; j < b1; ++j) total += pair_count_ok(w, hits[trax_hit(j, cfg)]);
+        for (uint32_t j = a2; j < b2; ++j) total += pair_count_ok(w, hits[trax_hit(j, cfg)]);
+        // The row's ranges disjoint, and starting at or after the end of
+        // every row before: with all rows in order the ends ascend, so the
+        // largest end before is the last one (rows_in_order).
+        const bool n1 = a1 < b1, n2 = a2 < b2;
+        uint32_t start = 0xffffffffu, end = 0;
+        if (n1 && n2) {
+          if (b2 <= a1) start = a2, end = b1;
+          else if (b1 <= a2) start = a1, end = b2;
+          else inOrder = false;
+        } else if (n1) {
+          start = a1, end = b1;
+        } else if (n2) {
+          start = a2, end = b2;
+        }
+        uint32_t before = end;  // inclusive maximum over the group's rows so far
+#pragma unroll
+        for (int d = 1; d < G; d <<= 1) {
+          const uint32_t v = __shfl_up_sync(ALL, before, d, G);
+          if (sub >= (uint32_t)d) before = max(before, v);
+        }
+        const uint32_t upTo = __shfl_up_sync(ALL, before, 1, G);
+        if (start < max(prevEnd, sub ? upTo : 0u)) inOrder = false;
+        prevEnd = max(prevEnd, __shfl_sync(ALL, before, G - 1, G));
+      } else {
+        uint32_t lo0 = a1, hi0 = b1, lo1 = a2, hi1 = b2;
+        if (a2 < b2 && b2 <= a1) {  // P2 precedes P1
+          lo0 = a2; hi0 = b2; lo1 = a1; hi1 = b1;
+        }
+        uint32_t n = 0;
+        for (uint32_t j = lo0; j < hi0; ++j) n += pair_ok(t, __ldg(zphi + 2 * (size_t)trax_hit(j, cfg)));
+        for (uint32_t j = lo1; j < hi1; ++j) n += pair_ok(t, __ldg(zphi + 2 * (size_t)trax_hit(j, cfg)));
+        uint32_t incl = n;
+#pragma unroll
+        for (int d = 1; d < G; d <<= 1) {
+          const uint32_t v = __shfl_up_sync(ALL, incl, d, G);
+          if (sub >= (uint32_t)d) incl += v;
+        }
+        uint32_t written = total + incl - n;
+        total += __shfl_sync(ALL, incl, G - 1, G);
+        if (n) {
+          for (uint32_t j = lo0; j < hi0; ++j)
+            if (pair_ok(t, __ldg(zphi + 2 * (size_t)trax_hit(j, cfg)))) {
+              if (written < limit) out[written] = make_uint2(j, i);
+              ++written;
+            }
+          for (uint32_t j = lo1; j < hi1; ++j)
+            if (pair_ok(t, __ldg(zphi + 2 * (size_t)trax_hit(j, cfg)))) {
+              if (written < limit) out[written] = make_uint2(j, i);
+              ++written;
+            }
         }
       }
+    }
+    if (!EMIT) {
+      for (int d = G / 2; d > 0; d >>= 1) total += __shfl_xor_sync(ALL, total, d, G);
+      const uint32_t bad = __ballot_sync(ALL, !inOrder) >> (lane & ~(uint32_t)(G - 1));
+      if (task && sub == 0) {
+        const bool simple = (bad & (uint32_t)((1ull << G) - 1ull)) == 0u;
+        taskCount[k] = total;
+        state.bounds[k] = make_float4(w.zLow, w.zHigh, w.phiLow, w.phiHigh);
+        state.secs[k] = make_uint4(w.zLowSector | (simple ? 0x80000000u : 0u), w.zHighSector | (w.wrap << 31), w.pL,
+                                   w.pH);
+        state.ids[k] = make_uint2(i, s);
+      }
+    } else if (task && sub == 0) {
+      uint32_t written = total;
+      if (!ordered) written = pair_store_unordered(cfg, w, lG1, hits, i, limit, out);
+      else if (written != limit) raise_error(err, TRAX_EBIT_BOUNDS);
       if (written < limit) {
         atomicAdd(sentinels, limit - written);
         for (uint32_t q = written; q < limit; ++q) out[q] = make_uint2(TRAX_SENTINEL, TRAX_SENTINEL);
@@ -391,6 +554,26 @@ cudaError_t pair_segments(const DevConfig& cfg, const uint32_t* grid, uint32_t* 
   return cudaGetLastError();
 }
 
+// Lanes per outer-hit task.  One lane has the fewest instructions per visit
+// and serves batches that fill the chip; fewer tasks than that leave the time
+// to the latency of one walk, which 8 and then 4 lanes share.  The store pass
+// of dense tasks (40 pairs and more each, `pairs` its capacity) takes 4 lanes
+// at any size: neighbouring lanes then write neighbouring pairs.  Measured on
+// 152 SMs, count / store, us:
+//   tasks (pairs each)      1 lane         4 lanes        8 lanes
+//   5.7 k  (12)          17.5 /  18.4   10.1 /  13.1    8.8 /   9.1
+//   45 k   (12)          23.8 /  25.9   14.9 /  17.8   16.3 /  15.9
+//   75 k  (148)            92 /   132     55 /   123     77 /   127
+//   153 k  (12)          27.5 /  28.2   32.2 /  36.2   41.4 /  43.0
+//   226 k (148)           110 /   382    118 /   298    211 /   377
+//   1.2 M (148)           306 /  1892      - /  1580      - /  1981
+static int pair_lanes(uint64_t tasks, uint64_t pairs) {
+  const uint64_t sms = (uint64_t)sm_count();
+  if (tasks * 8 <= sms * 1792) return 8;
+  if (tasks * 4 <= sms * 2560 || pairs >= 40 * tasks) return 4;
+  return 1;
+}
+
 cudaError_t pair_tasks(const DevConfig& cfg, bool emit, const uint32_t* grid, DevHits hits, const uint32_t* segOuter,
                        const uint32_t* taskBase, const uint32_t* nTasksDev, uint64_t maxTasks, uint32_t* taskCount,
                        PairTaskState state, uint2* pairs, uint64_t capPairs, uint32_t* pairOffsets,
@@ -398,12 +581,24 @@ cudaError_t pair_tasks(const DevConfig& cfg, bool emit, const uint32_t* grid, De
   const uint32_t cap = capPairs > 0xffffffffull ? 0xffffffffu : (uint32_t)capPairs;
   const int threads = (int)cfg.pairThreads;
   const int blocks = grid_for(maxTasks + 1, threads);
-  if (emit)
+  const int lanes = pair_lanes(maxTasks, emit ? capPairs : 0);
+  auto group = [&](auto kernel) {
+    launch(q, kernel, grid_for((maxTasks + 1) * lanes, threads), threads, 0, cfg, grid, hits.xyzp, segOuter, taskBase,
+           nTasksDev, taskCount, state, pairs, cap, pairOffsets, sentinels, err);
+  };
+  if (lanes == 8) {
+    if (emit) group(pair_group_kernel<true, 8>);
+    else group(pair_group_kernel<false, 8>);
+  } else if (lanes == 4) {
+    if (emit) group(pair_group_kernel<true, 4>);
+    else group(pair_group_kernel<false, 4>);
+  } else if (emit) {
     launch(q, pair_kernel<true>, blocks, threads, 0, cfg, grid, hits.xyzp, segOuter, taskBase, nTasksDev, taskCount,
            state, pairs, cap, pairOffsets, sentinels, err);
-  else
-    launch(q, pair_kernel<false>, blocks, threads, 0, cfg, grid, hits.xyzp, segOuter, taskBase, nTasksDev,
-           taskCount, state, pairs, cap, pairOffsets, sentinels, err);
+  } else {
+    launch(q, pair_kernel<false>, blocks, threads, 0, cfg, grid, hits.xyzp, segOuter, taskBase, nTasksDev, taskCount,
+           state, pairs, cap, pairOffsets, sentinels, err);
+  }
   return cudaGetLastError();
 }
 
