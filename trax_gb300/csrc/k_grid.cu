@@ -188,8 +188,8 @@ __global__ void __launch_bounds__(GRID_MAX_THREADS)
 // arrays in global scratch.
 __device__ __forceinline__ uint32_t half_of(uint32_t word, uint32_t c) { return (word >> ((c & 1u) * 16u)) & 0xffffu; }
 
-__global__ void __launch_bounds__(GRID_MAX_THREADS)
-    grid_kernel16(Stamp stamp, DevConfig cfg, GridInput in, uint32_t* __restrict__ grid, DevHits out, GridScratch sc,
+__global__ void __launch_bounds__(GRID_MAX_THREADS, 2)
+    grid_kernel16(Stamp stamp, DevConfig cfg, const __grid_constant__ GridInput in, uint32_t* __restrict__ grid, const __grid_constant__ DevHits out, GridScratch sc,
                   uint32_t* err, uint32_t maxHits) {
   stamp_begin(stamp);
   clear_scan_scratch(sc);
@@ -339,25 +339,16 @@ __global__ void __launch_bounds__(GRID_MAX_THREADS)
     // Through shared memory, where the counters and cells were: columns are
     // read and written in order, and only shared memory is read at random.
     // Reading the columns at random takes a 32-byte sector per 4 bytes.
+    // One column at a time, their pointers taken from the parameters in turn.
     uint32_t* stage = cnt;
-    const uint32_t room = W + maxHits / 2;
-    const uint32_t atOnce = n ? min(room / n, 7u) : 7u;
-    const uint32_t* cols[7] = {reinterpret_cast<const uint32_t*>(in.x), reinterpret_cast<const uint32_t*>(in.y),
-                               reinterpret_cast<const uint32_t*>(in.z), in.layer, in.det, in.hid, in.evt};
-    uint32_t* outs[7] = {reinterpret_cast<uint32_t*>(out.x), reinterpret_cast<uint32_t*>(out.y),
-                         reinterpret_cast<uint32_t*>(out.z), out.layer, out.det, out.hid, out.evt};
-    for (uint32_t c0 = 0; c0 < 7; c0 += atOnce) {
-      for (uint32_t i = tid; i < n; i += blockDim.x)
-#pragma unroll
-        for (uint32_t c = 0; c < 7; ++c)
-          if (c >= c0 && c < c0 + atOnce) stage[(c - c0) * n + i] = cols[c][base + i];
+    const uint32_t* const* cols = reinterpret_cast<const uint32_t* const*>(&in.x);
+    uint32_t* const* outs = reinterpret_cast<uint32_t* const*>(&out.x);
+    for (int c = 0; c < 7; ++c) {
+      const uint32_t* col = cols[c] + base;
+      uint32_t* o = outs[c] + base;
+      for (uint32_t i = tid; i < n; i += blockDim.x) stage[i] = col[i];
       __syncthreads();
-      for (uint32_t s = tid; s < n; s += blockDim.x) {
-        const uint32_t i = permS[s];
-#pragma unroll
-        for (uint32_t c = 0; c < 7; ++c)
-          if (c >= c0 && c < c0 + atOnce) outs[c][base + s] = stage[(c - c0) * n + i];
-      }
+      for (uint32_t s = tid; s < n; s += blockDim.x) o[s] = stage[permS[s]];
       __syncthreads();
     }
     for (uint32_t s = tid; s < n; s += blockDim.x) {  // x, y and z as this thread wrote them
@@ -513,10 +504,17 @@ static size_t grid16_bytes(const DevConfig& cfg, uint32_t maxLayerHits) {
 uint32_t grid_layer_room(const DevConfig& cfg, uint32_t maxLayerHits) {
   const size_t bytes = grid16_bytes(cfg, maxLayerHits);
   if (!bytes) return maxLayerHits;
-  const size_t sm = 228u * 1024u, fixed = 1024u + 256u;  // per CTA: the system's share, static arrays
-  const size_t ctas = std::min<size_t>(sm / (bytes + fixed), 2048u / grid_threads(cfg.E * cfg.L));
+  // The first-level cache has what the SM's shared-memory partition leaves
+  // (partitions of these sizes); a larger one costs the gather its cache.
+  const size_t partitions[] = {8, 16, 32, 64, 100, 132, 164, 196, 228};
+  const size_t fixed = 1024u + 256u;  // per CTA: the system's share, static arrays
+  const size_t ctas = std::min<size_t>(228u * 1024u / (bytes + fixed), 2048u / grid_threads(cfg.E * cfg.L));
   size_t most = GRID_SMEM_MAX;
-  if (ctas > 1) most = std::min(most, sm / ctas - fixed);
+  for (size_t p : partitions)
+    if (ctas * (bytes + fixed) <= p * 1024u) {
+      most = std::min(most, p * 1024u / ctas - fixed);
+      break;
+    }
   if (most <= bytes) return maxLayerHits;
   const size_t more = std::min<size_t>((most - bytes) / 8, maxLayerHits / 4);
   return (uint32_t)std::min<size_t>(maxLayerHits + more, 65535u);

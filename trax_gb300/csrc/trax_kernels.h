@@ -138,7 +138,7 @@ cudaError_t track_greedy(TrackLists t, uint32_t nTracks, unsigned long long* tab
                          unsigned long long* counts, cudaStream_t st);
 
 // ------------------------------------------------------------ grid build
-struct GridInput {
+struct GridInput {  // the seven columns first, in DevHits' order
   const float* x;
   const float* y;
   const float* z;
