@@ -285,9 +285,16 @@ __global__ void __launch_bounds__(GRID_MAX_THREADS, 2)
     run = hi + (v >> 16);
   }
   __syncthreads();
-  // the boundaries, written with consecutive threads on consecutive cells
+  // the boundaries, consecutive threads on consecutive pairs of cells (8-byte
+  // stores, so a pair starts on an even word of the grid)
   uint32_t* gl = grid + (size_t)task * C;
-  for (uint32_t c = tid; c < C; c += blockDim.x) gl[c] = base + half_of(cnt[c >> 1], c);
+  const uint32_t odd = (uint32_t)(((size_t)task * C) & 1u);
+  if (odd && tid == 0) gl[0] = base + half_of(cnt[0], 0u);
+  for (uint32_t c = odd + 2u * tid; c < C; c += 2u * blockDim.x) {
+    const uint32_t v0 = base + half_of(cnt[c >> 1], c);
+    if (c + 1u < C) *reinterpret_cast<uint2*>(gl + c) = make_uint2(v0, base + half_of(cnt[(c + 1u) >> 1], c + 1u));
+    else gl[c] = v0;
+  }
   __syncthreads();
 
   // 3. placement by the cell cursors, then the stable order inside each cell
@@ -306,11 +313,9 @@ __global__ void __launch_bounds__(GRID_MAX_THREADS, 2)
     }
   }
   __syncthreads();
-  for (uint32_t c = tid; c < C; c += blockDim.x) {
-    const uint32_t lo = c ? half_of(cnt[(c - 1) >> 1], c - 1) : 0u, hi = half_of(cnt[c >> 1], c);
-    if (hi - lo < 2) continue;
+  auto sort_cell = [&](uint32_t lo, uint32_t hi) {  // insertion sort: cells hold a few hits
     if (inSmem) {
-      for (uint32_t a = lo + 1; a < hi; ++a) {  // insertion sort: cells hold a few hits
+      for (uint32_t a = lo + 1; a < hi; ++a) {
         const uint16_t v = permS[a];
         uint32_t b = a;
         while (b > lo && permS[b - 1] > v) {
@@ -331,6 +336,13 @@ __global__ void __launch_bounds__(GRID_MAX_THREADS, 2)
         p[b] = v;
       }
     }
+  };
+  // two cells per word, most of them with fewer than two hits
+  for (uint32_t w = tid; w < W; w += blockDim.x) {
+    const uint32_t ends = cnt[w], start = w ? cnt[w - 1] >> 16 : 0u;
+    const uint32_t mid = ends & 0xffffu, end = 2u * w + 1u < C ? ends >> 16 : mid;
+    if (mid - start >= 2u) sort_cell(start, mid);
+    if (end - mid >= 2u) sort_cell(mid, end);
   }
   __syncthreads();
 
