@@ -200,3 +200,21 @@ def test_pair_lanes_on_degenerate_windows(trax_lib, oracle_lib, tasks):
     p[p != 0xFFFFFFFF] -= np.broadcast_to(shift, p.shape)[p != 0xFFFFFFFF]
     assert np.array_equal(p, np.tile(want, (copies, 1)))
     assert st.n_pair_sentinels == copies * int((want[:, 0] == 0xFFFFFFFF).sum())
+
+
+@pytest.mark.parametrize("middle", [(2, 3, 4), (3, 3, 4), (4, 3, 4)])
+def test_links_with_and_without_shared_second_layers(trax_lib, oracle_lib, middle):
+    """Followers are looked up by the run of triplets with their second hit unless a layer is the second of two layer
+    triplets; both give the oracle's links, on a context that had other batches' runs before."""
+    lts = events.layer_triplets([1, 2, 3])
+    lts = [dataclasses.replace(lt, layer2=m, layer3=max(lt.layer3, m + 1)) for lt, m in zip(lts, middle)]
+    batches = [dataclasses.replace(events.generate(2, n_events=n, seed=n), lts=lts) for n in (4, 3)]
+    with trax_lib.Context(0) as ctx:
+        for b in batches:
+            want = oracle_lib.run(b)[0]
+            ctx.upload(b)
+            ctx.seed_batch(use_graph=False)
+            got = ctx.results()
+            assert want["link_basis"].size > 0
+            for name in ("trip_h2", "link_basis", "link_follower", "connectable", "ca_states", "tracks"):
+                assert np.array_equal(got[name], want[name]), name

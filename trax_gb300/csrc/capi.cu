@@ -139,7 +139,7 @@ struct trax_ctx {
   // prediction / filter
   DevBuf candLocal, predWarps, predKeep, cands, candOffsets, flagWords, flagSums, h1, h2, h3, tripOffsets;
   // connectivity / fit / CA
-  DevBuf eta, segOf, segStart, linkCount, linkRun, inDeg, basis, follower, connS, connW, connIdx, nonConnIdx, pt;
+  DevBuf eta, segOf, segStart, linkCount, linkRun, linkRuns, inDeg, basis, follower, connS, connW, connIdx, nonConnIdx, pt;
   DevBuf states, inStart, inCursor, inList, best, isBest, handlers, tracks;
   DevBuf userIdx, caNext;  // caller-provided fit list; second state buffer of the caller-link CA
   // bookkeeping
@@ -611,10 +611,23 @@ int link_buffers(trax_ctx* c, Mode mode, uint64_t maxT) {
   ENSURE(eta, maxT, 4);
   ENSURE(inDeg, maxT + 1, 4);
   ENSURE(inCursor, maxT, 4);
+  ENSURE(linkRuns, c->nHits, 8);
   return TRAX_OK;
 }
+// The runs by second hit are kept for the chain's own triplets, whose second
+// hits lie on their layer triplet's second layer, when no two share one.
+uint2* link_runs(trax_ctx* c) {
+  if (c->identityHits) return nullptr;
+  uint32_t seen = 0;
+  for (uint32_t p = 0; p < c->cfg.nLT; ++p) {
+    const uint32_t bit = 1u << (c->cfg.layer2[p] - 1);
+    if (seen & bit) return nullptr;
+    seen |= bit;
+  }
+  return ptr<uint2>(c->linkRuns);
+}
 LinkStart link_start(trax_ctx* c) {
-  return LinkStart{ptr<float>(c->eta), ptr<uint32_t>(c->inDeg), ptr<uint32_t>(c->inCursor)};
+  return LinkStart{ptr<float>(c->eta), ptr<uint32_t>(c->inDeg), ptr<uint32_t>(c->inCursor), link_runs(c)};
 }
 
 int stage_filter(trax_ctx* c, Mode mode) {
@@ -680,8 +693,8 @@ int stage_connectivity(trax_ctx* c, Mode mode) {
   uint32_t* linkCount = ptr<uint32_t>(c->linkCount);
   KBEG(TK_CONN_COUNT);
   CK(connectivity_count(c->cfg, dev_hits(c), tv, ptr<float>(c->eta), ptr<uint32_t>(c->tripOffsets),
-                        ptr<uint32_t>(c->segStart), linkCount, ptr<uint32_t>(c->inDeg), ptr<uint32_t>(c->linkRun),
-                        c->sortedSegments, c->q));
+                        ptr<uint32_t>(c->segStart), link_runs(c), linkCount, ptr<uint32_t>(c->inDeg),
+                        ptr<uint32_t>(c->linkRun), c->sortedSegments, c->q));
   KEND(TK_CONN_COUNT);
   // the links' places, and the places of the incoming links of every follower
   RC(scan_publish(c, mode, {ScanArray{linkCount, linkCount}, ScanArray{ptr<uint32_t>(c->inDeg), ptr<uint32_t>(c->inStart)}},
@@ -870,6 +883,7 @@ int size_device_buffers(trax_ctx* c) {
   ENSURE(h1, c->capT, 4); ENSURE(h2, c->capT, 4); ENSURE(h3, c->capT, 4);
   ENSURE(eta, c->capT, 4); ENSURE(segStart, S + 1, 4);
   ENSURE(linkCount, c->capT + 1, 4); ENSURE(linkRun, c->capT + 1, 4); ENSURE(inDeg, c->capT + 1, 4);
+  ENSURE(linkRuns, c->nHits, 8);
   ENSURE(connS, (c->capT + 31) / 32 + 1, 4); ENSURE(connW, (c->capT + 31) / 32 + 1, 4);
   ENSURE(connIdx, c->capT, 4); ENSURE(nonConnIdx, c->capT, 4); ENSURE(pt, c->capT, 4);
   ENSURE(basis, c->capLinks, 4); ENSURE(follower, c->capLinks, 4);
@@ -935,7 +949,7 @@ bool graph_fits(trax_ctx* c) {
                            &c->sc_phi, &c->sc_perm};
   for (const DevBuf* b : words)
     if (n * 4 > b->cap) return false;
-  if ((n + 4) * 4 > c->pz.cap || n * 16 > c->pxyzp.cap) return false;
+  if ((n + 4) * 4 > c->pz.cap || n * 16 > c->pxyzp.cap || n * 8 > c->linkRuns.cap) return false;
   if (c->cfg.fineRows && n * 16 > c->fineHits.cap) return false;
   return c->maxLayerHits <= c->capLayerHits;
 }
@@ -1104,7 +1118,7 @@ void trax_destroy(trax_ctx* c) {
                     &c->pevt, &c->porig, &c->pxyzp, &c->sc_cell, &c->sc_phi, &c->sc_perm, &c->sc_counts,
                     &c->fineGrid, &c->fineHits, &c->segOuter, &c->taskBase, &c->taskCount, &c->taskState, &c->pairs, &c->pairOffsets, &c->candLocal, &c->predWarps, &c->predKeep, &c->cands,
                     &c->candOffsets, &c->flagWords, &c->flagSums, &c->h1, &c->h2, &c->h3, &c->tripOffsets, &c->eta, &c->segOf,
-                    &c->segStart, &c->linkCount, &c->linkRun, &c->inDeg, &c->basis, &c->follower, &c->connS, &c->connW,
+                    &c->segStart, &c->linkCount, &c->linkRun, &c->linkRuns, &c->inDeg, &c->basis, &c->follower, &c->connS, &c->connW,
                     &c->connIdx, &c->nonConnIdx, &c->pt, &c->states, &c->inStart, &c->inCursor, &c->inList, &c->best,
                     &c->isBest, &c->handlers, &c->tracks, &c->scanScratch, &c->slots, &c->fitOk, &c->fitSegCnt,
                     &c->fitSegDelta, &c->fitRows, &c->fitPartials, &c->fitOut, &c->fitParams, &c->fitDHits,

@@ -287,6 +287,11 @@ struct LinkStart {
   float* eta;
   uint32_t* inDeg;     // [nT+1]
   uint32_t* inCursor;  // [nT]
+  // [nHits] or null: (first, end) of the triplets whose second hit it is.
+  // Only hits that are some triplet's second hit have theirs written, so an
+  // entry counts when its first triplet is there and has that second hit.
+  // Given where every layer is the second of one layer triplet at most.
+  uint2* runs;
 };
 cudaError_t triplet_segments(const DevConfig& cfg, DevHits hits, TripletView t, uint32_t* segStart, uint32_t* segOf,
                              uint32_t* offsets, const LinkStart* link, Queue& q);
@@ -295,8 +300,9 @@ cudaError_t triplet_link_start(const DevConfig& cfg, DevHits hits, TripletView t
 // links per basis triplet (linkCount, +1 slot zeroed) and per follower
 // (inDeg); runStart[t]: where the store pass starts looking for t's followers
 cudaError_t connectivity_count(const DevConfig& cfg, DevHits hits, TripletView t, const float* eta,
-                               const uint32_t* offsets, const uint32_t* segStart, uint32_t* linkCount,
-                               uint32_t* inDeg, uint32_t* runStart, bool sortedSegments, Queue& q);
+                               const uint32_t* offsets, const uint32_t* segStart, const uint2* runs,
+                               uint32_t* linkCount, uint32_t* inDeg, uint32_t* runStart, bool sortedSegments,
+                               Queue& q);
 // With linkCount and inDeg scanned (the latter into inStart): the links, the
 // bases of each follower's links in inList (any order), and the words of 32
 // connectable flags with the number set per word (+1 slot zeroed, the number
