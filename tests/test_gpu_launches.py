@@ -218,3 +218,24 @@ def test_links_with_and_without_shared_second_layers(trax_lib, oracle_lib, middl
             assert want["link_basis"].size > 0
             for name in ("trip_h2", "link_basis", "link_follower", "connectable", "ca_states", "tracks"):
                 assert np.array_equal(got[name], want[name]), name
+
+
+@pytest.mark.parametrize("fine", [0, 8])
+@pytest.mark.parametrize("slots", [16, 32])
+def test_candidates_copied_by_output(trax_lib, oracle_lib, slots, fine):
+    """The store pass that takes a warp's candidates one per lane: warps whose pairs have from no to far more candidates
+    than slots side by side, and a last warp that is not full."""
+    lts = [dataclasses.replace(lt, sigma_phi=1.0, sigma_z=5.0) for lt in events.layer_triplets([1])]
+    batch = events.generate_workload(dataclasses.replace(events.workload(1, 3), n_tracks=300, lts=lts), seed=8)
+    want = oracle_lib.run(batch, links="none")[0]
+    per = np.bincount(want["cands"].reshape(-1, 2)[:, 0])
+    assert (per == 0).any() and (per > slots).any() and ((per > 0) & (per <= slots)).any()
+    assert (want["pairs"].size // 2) % 32
+    with trax_lib.Context(0) as ctx:
+        ctx.set_candidate_slots(slots)
+        ctx.set_fine_rows(fine)
+        ctx.upload(batch)
+        for graph in (False, True):
+            ctx.seed_batch(use_graph=graph, run_linking=False)
+            assert np.array_equal(ctx.candidates()[0].ravel(), want["cands"]), graph
+            assert ctx.stats().n_candidate_sentinels == want["stats_dict"]["cand_undefined_slots"]

@@ -602,12 +602,11 @@ __global__ void __launch_bounds__(TRAX_MAX_TUNED_THREADS, 4)
 // loads better than the few spilled bytes cost (0.61 -> 0.49 ms).
 // IL: the slots' layout (keep_slots).  FINE: the re-walks go over the fine
 // z grid (fine_walk with the store variant as both variants, its captures
-// written straight to the pair's candidates), with the same candidates; it
-// gets 40 registers, where it spills nothing (pileup batch: 4.03 ms with
-// the grid walk, 4.34 ms fine at 32 registers with 80 B spilled, 3.46 ms
-// at 40).
+// written straight to the pair's candidates), with the same candidates (with
+// the copies by output 2.96 ms at 40 registers, 2.76 ms at 32 with 88 B
+// spilled on the re-walks' side, for the pileup batch's 742 M candidates).
 template <bool IL, bool FINE>
-__global__ void __launch_bounds__(TRAX_MAX_TUNED_THREADS, FINE ? 6 : 8)
+__global__ void __launch_bounds__(TRAX_MAX_TUNED_THREADS, 8)
     predict_store_kernel(Stamp stamp, DevConfig cfg, const uint32_t* __restrict__ grid, const float4* __restrict__ hits,
                          const uint32_t* __restrict__ hitEvt, const uint32_t* __restrict__ hitLayer,
                          const uint2* __restrict__ pairs, const uint32_t* __restrict__ nPairsDev,
@@ -629,42 +628,8 @@ __global__ void __launch_bounds__(TRAX_MAX_TUNED_THREADS, FINE ? 6 : 8)
                                    : warpStart[p >> 5] + local[p];
   }
   uint32_t sent = 0;
-  for (uint32_t gid = blockIdx.x * blockDim.x + threadIdx.x; gid < nPairs; gid += gridDim.x * blockDim.x) {
-    const uint32_t wi = gid >> 5;
-    const uint32_t off = local[gid];
-    const uint32_t pos = warpStart[wi] + off;
-    // the next pair's position: the next warp's start after a warp's last pair
-    uint32_t limit = ((gid & 31u) == 31u || gid + 1 == nPairs) ? warpStart[wi + 1] - pos : local[gid + 1] - off;
-    if (pos >= capCands) limit = 0;
-    else if (limit > capCands - pos) limit = capCands - pos;
-    if (limit == 0) continue;
-    uint2* out = cands + pos;
-    if (limit <= cfg.predKeep) {
-      // the slots are read in groups before any of them is written: one
-      // at a time, every read waited for the one before it
-      const KeepSlots<IL, const uint32_t> slot = keep_slots<IL>(keep, gid, cfg.predKeep);
-      constexpr uint32_t GROUP = IL ? 8u : 4u;
-      for (uint32_t q0 = 0; q0 < limit; q0 += GROUP) {
-        uint32_t h[GROUP];
-        if (IL) {
-#pragma unroll
-          for (uint32_t k = 0; k < GROUP; ++k) h[k] = q0 + k < limit ? slot[q0 + k] : 0u;
-        } else {  // four or eight consecutive slots, 16-byte aligned
-          const uint4 v = __ldg(reinterpret_cast<const uint4*>(slot.p + q0));
-          h[0] = v.x;
-          h[1] = v.y;
-          h[2] = v.z;
-          h[3] = v.w;
-        }
-#pragma unroll
-        for (uint32_t k = 0; k < GROUP; ++k)
-          if (q0 + k < limit) {
-            sent += h[k] == TRAX_SENTINEL;
-            out[q0 + k] = make_uint2(gid, h[k]);
-          }
-      }
-      continue;
-    }
+  // the walk again, for a pair with more candidates than slots
+  auto rewalk = [&](uint32_t gid, uint32_t limit, uint2* out) {
     const uint2 pr = pairs[gid];
     const uint32_t hx = trax_hit(pr.x, cfg), hy = trax_hit(pr.y, cfg);
     const uint32_t event = hitEvt[hx];
@@ -698,6 +663,81 @@ __global__ void __launch_bounds__(TRAX_MAX_TUNED_THREADS, FINE ? 6 : 8)
     }
     sent += limit - n;
     for (; n < limit; ++n) out[n] = make_uint2(gid, TRAX_SENTINEL);
+  };
+  if (IL) {
+    // By output: a warp has its 32 pairs' candidates, and each lane takes one
+    // of them a step, whose pair it finds by a 5-step search over the pairs'
+    // ends.  The lanes then write one piece of memory, in as many steps as
+    // there are candidates to 32, where a pair per lane wrote 32 pieces and
+    // took as many steps as the pair with the most candidates (0.73 -> 0.54 ms
+    // for the 139 M of three pileup events).  With few candidates per pair the
+    // search costs more than it saves (0.465 -> 0.575 ms for the 49 M of
+    // the ttbar-like batch's 96 M pairs): there a pair per lane stays.
+    const uint32_t lane = threadIdx.x & 31u;
+    for (uint32_t base = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); base < nPairs;
+         base += gridDim.x * blockDim.x) {
+      const uint32_t start = warpStart[base >> 5], all = warpStart[(base >> 5) + 1] - start;
+      const uint32_t off = base + lane < nPairs ? local[base + lane] : all;
+      const uint32_t next = __shfl_down_sync(0xffffffffu, off, 1);
+      const uint32_t end = lane == 31u ? all : next;
+      const uint32_t total = start < capCands ? min(all, capCands - start) : 0u;
+      const bool fits = end - off <= cfg.predKeep;
+      const uint32_t fitMask = __ballot_sync(0xffffffffu, fits);
+      for (uint32_t k0 = 0; k0 < total; k0 += 64u) {  // two steps' reads before their writes
+        uint32_t p[2], h[2];
+        bool mine[2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          const uint32_t k = k0 + 32u * u + lane;
+          p[u] = 0;  // the first pair whose candidates end after k
+#pragma unroll
+          for (uint32_t step = 16; step > 0; step >>= 1) {
+            const uint32_t v = __shfl_sync(0xffffffffu, end, p[u] + step - 1u);
+            if (v <= k) p[u] += step;
+          }
+          const uint32_t q = k - __shfl_sync(0xffffffffu, off, p[u]);
+          mine[u] = k < total && ((fitMask >> p[u]) & 1u);
+          h[u] = mine[u] ? keep_slots<IL>(keep, base + p[u], cfg.predKeep)[q] : 0u;
+        }
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+          if (mine[u]) {
+            sent += h[u] == TRAX_SENTINEL;
+            cands[start + k0 + 32u * u + lane] = make_uint2(base + p[u], h[u]);
+          }
+      }
+      if (!fits && off < total) rewalk(base + lane, min(end, total) - off, cands + start + off);
+    }
+  } else {
+    for (uint32_t gid = blockIdx.x * blockDim.x + threadIdx.x; gid < nPairs; gid += gridDim.x * blockDim.x) {
+      const uint32_t wi = gid >> 5;
+      const uint32_t off = local[gid];
+      const uint32_t pos = warpStart[wi] + off;
+      // the next pair's position: the next warp's start after a warp's last pair
+      uint32_t limit = ((gid & 31u) == 31u || gid + 1 == nPairs) ? warpStart[wi + 1] - pos : local[gid + 1] - off;
+      if (pos >= capCands) limit = 0;
+      else if (limit > capCands - pos) limit = capCands - pos;
+      if (limit == 0) continue;
+      uint2* out = cands + pos;
+      if (limit > cfg.predKeep) {
+        rewalk(gid, limit, out);
+        continue;
+      }
+      // four consecutive slots at a time (16-byte aligned), read before any
+      // of their candidates is written: one at a time, every read waited for
+      // the one before it
+      const uint32_t* slot = keep_slots<IL>(keep, gid, cfg.predKeep).p;
+      for (uint32_t q0 = 0; q0 < limit; q0 += 4u) {
+        const uint4 v = __ldg(reinterpret_cast<const uint4*>(slot + q0));
+        const uint32_t h[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (uint32_t k = 0; k < 4u; ++k)
+          if (q0 + k < limit) {
+            sent += h[k] == TRAX_SENTINEL;
+            out[q0 + k] = make_uint2(gid, h[k]);
+          }
+      }
+    }
   }
   for (int d = 16; d > 0; d >>= 1) sent += __shfl_down_sync(0xffffffffu, sent, d);
   if ((threadIdx.x & 31u) == 0 && sent) atomicAdd(sentinels, sent);
