@@ -383,10 +383,11 @@ TRAX_HD void normalize2(float& vx, float& vy) {
 //   u and v: atan2_ is within 3 ulp of each direction (7.2e-7 rad below pi),
 //   the subtraction and the +-2 pi_f wrap round by 2.4e-7 rad each, and
 //   pi_f is 8.7e-8 from pi;
-// - the FP32 cross and dot products, a difference and a sum of two rounded
-//   products, are within 2^-23 |u| |v| of the exact ones, which for angles up
-//   to 1 rad puts the angle they give within 6e-7 rad of the true one, as
-//   long as |u| |v| stays far from the under- and overflow limits.
+// - the FP32 cross and dot products, a difference and a sum of two products
+//   (one of them rounded), are within 2^-23 |u| |v| of the exact ones, which
+//   for angles up to 1 rad puts the angle they give within 6e-7 rad of the
+//   true one, as long as |u| |v| (which |cross| + |dot| lies within a factor
+//   sqrt 2 of) stays far from the under- and overflow limits.
 // With a margin of TRAX_DPHI_MARGIN rad on both sides of the cut,
 // cross <= dot tan(cut - margin) means the cut passes and
 // cross >= dot tan(cut + margin) means it fails.  Candidates in between,
@@ -396,14 +397,12 @@ TRAX_HD void normalize2(float& vx, float& vy) {
 #define TRAX_DPHI_MARGIN 1e-4
 
 TRAX_HD int dphi_decide(float tanLo, float tanHi, float ux, float uy, float vx, float vy) {
-  if (!(tanHi < bits2f(0x7f800000u))) return -1;
-  const float nm = (fabs_(ux) + fabs_(uy)) * (fabs_(vx) + fabs_(vy));
-  if (!(nm >= 1e-30f && nm <= 1e30f)) return -1;
-  const float cr = fabs_(ux * vy - uy * vx), dt = ux * vx + uy * vy;
-  if (dt <= 0.0f) return 0;  // at least pi/2 - 6e-7 rad apart
-  if (cr <= dt * tanLo) return 1;
-  if (cr >= dt * tanHi) return 0;
-  return -1;
+  const float cr = fabs_(fmaf(ux, vy, -(uy * vx))), dt = fmaf(ux, vx, uy * vy);
+  const float nm = cr + fabs_(dt);
+  const bool sure = nm >= 1e-30f && nm <= 1e30f && tanHi < bits2f(0x7f800000u);
+  // a dot product of 0 or less: at least pi/2 - 6e-7 rad apart
+  const bool in = cr <= dt * tanLo, out = dt <= 0.0f || cr >= dt * tanHi;
+  return !sure ? -1 : out ? 0 : in ? 1 : -1;
 }
 
 // tan(cut -+ margin) of a dphi cut, or (-1, inf) for a cut outside [0, 1] rad

@@ -280,13 +280,6 @@ __device__ __forceinline__ bool filter_dphi(float dPhiCut, float4 A, float4 B, f
   return fabs_(delta) <= dPhiCut;
 }
 
-// The dphi part decided from cross and dot products where that is certain
-// (dphi_decide), else by the atan2 evaluation above.
-__device__ __forceinline__ bool filter_dphi_fast(const DevConfig& cfg, uint32_t lt, float4 A, float4 B, float4 Cc) {
-  const int q = dphi_decide(cfg.dPhiTanLo[lt], cfg.dPhiTanHi[lt], B.x - A.x, B.y - A.y, Cc.x - B.x, Cc.y - B.y);
-  return q > 0 || (q < 0 && filter_dphi(cfg.dPhiCut[lt], A, B, Cc));
-}
-
 // The dtheta part (:84-117): the polar angles of the two segments.
 __device__ __forceinline__ bool filter_dtheta(const DevConfig& cfg, uint32_t lt, float4 A, float4 B, float4 Cc) {
   const float theta1 = atan2_(sqrt_((B.x - A.x) * (B.x - A.x) + (B.y - A.y) * (B.y - A.y)), (B.z - A.z));
@@ -315,12 +308,6 @@ __device__ __forceinline__ bool filter_circle(const DevConfig& cfg, uint32_t lt,
   const float tip_squared = pCAx * pCAx + pCAy * pCAy;
   const float tipCut = cfg.tipCut[lt];
   return tip_squared <= (tipCut * tipCut) && cR >= cfg.minRcurv;
-}
-
-// The dtheta, TIP and curvature parts together.
-__device__ __forceinline__ bool filter_rest(const DevConfig& cfg, uint32_t lt, float4 A, float4 B, float4 Cc) {
-  const bool dtheta = filter_dtheta(cfg, lt, A, B, Cc);
-  return filter_circle(cfg, lt, A, B, Cc) && dtheta;
 }
 
 }  // namespace trax
