@@ -101,8 +101,13 @@ __device__ __forceinline__ PairTest pair_test(const PairWindow& w) {
   return t;
 }
 __device__ __forceinline__ bool pair_ok(const PairTest& t, float2 h) {
-  return t.zl <= h.x && h.x <= t.zh && ((t.a1 <= h.y && h.y <= t.b1) || (t.a2 <= h.y && h.y <= t.b2));
+  return (t.zl <= h.x) & (h.x <= t.zh) & (((t.a1 <= h.y) & (h.y <= t.b1)) | ((t.a2 <= h.y) & (h.y <= t.b2)));
 }
+
+// (Both tests combine their comparisons without branches, which lanes with
+// different outcomes would split over: three pileup events' count 109 -> 72 us,
+// store 297 -> 276 us; the ttbar-like batch's 494 and 851 -> 831 us.  The
+// prediction's walks gained nothing from it.)
 
 // The count pass's form of the window test (PairGeneratorBeamspot.h:192,
 // :212-214).  The hits' angles come from atan2_ and lie in [-pi, pi] or are
@@ -112,7 +117,7 @@ __device__ __forceinline__ bool pair_ok(const PairTest& t, float2 h) {
 // faster there.
 __device__ __forceinline__ bool pair_count_ok(const PairWindow& w, float4 h) {
   const bool lo = w.phiLow <= h.w, hi = h.w <= w.phiHigh;
-  return w.zLow <= h.z && h.z <= w.zHigh && (w.wrap ? (lo || hi) : (lo && hi));
+  return (w.zLow <= h.z) & (h.z <= w.zHigh) & (w.wrap ? (lo | hi) : (lo & hi));
 }
 
 __device__ __forceinline__ bool pair_valid(const PairWindow& w, float4 h) {
