@@ -85,7 +85,11 @@ __device__ __forceinline__ PairWindow pair_window(const DevConfig& cfg, uint32_t
 }
 
 // pair_valid on (z, phi) with the phi test as two intervals, the second
-// empty unless the window wraps
+// empty unless the window wraps.  This test and the count pass's below combine
+// their comparisons without branches, which lanes with different outcomes
+// split over: three pileup events' count 109 -> 72 us and store 297 -> 276 us,
+// the ttbar-like batch's 494 and 851 -> 831 us.  (The prediction's walks
+// gained nothing from it.)
 struct PairTest {
   float zl, zh, a1, b1, a2, b2;
 };
@@ -103,11 +107,6 @@ __device__ __forceinline__ PairTest pair_test(const PairWindow& w) {
 __device__ __forceinline__ bool pair_ok(const PairTest& t, float2 h) {
   return (t.zl <= h.x) & (h.x <= t.zh) & (((t.a1 <= h.y) & (h.y <= t.b1)) | ((t.a2 <= h.y) & (h.y <= t.b2)));
 }
-
-// (Both tests combine their comparisons without branches, which lanes with
-// different outcomes would split over: three pileup events' count 109 -> 72 us,
-// store 297 -> 276 us; the ttbar-like batch's 494 and 851 -> 831 us.  The
-// prediction's walks gained nothing from it.)
 
 // The count pass's form of the window test (PairGeneratorBeamspot.h:192,
 // :212-214).  The hits' angles come from atan2_ and lie in [-pi, pi] or are
@@ -564,7 +563,8 @@ cudaError_t pair_segments(const DevConfig& cfg, const uint32_t* grid, uint32_t* 
 // to the latency of one walk, which 8 and then 4 lanes share.  The store pass
 // of dense tasks (40 pairs and more each, `pairs` its capacity) takes 4 lanes
 // at any size: neighbouring lanes then write neighbouring pairs.  Measured on
-// 152 SMs, count / store, us:
+// 152 SMs, count / store, us (with branches in the tests; without, 226 k dense
+// tasks take 72 / 276 with the lanes chosen here, 1.2 M take 245 / 1480):
 //   tasks (pairs each)      1 lane         4 lanes        8 lanes
 //   5.7 k  (12)          17.5 /  18.4   10.1 /  13.1    8.8 /   9.1
 //   45 k   (12)          23.8 /  25.9   14.9 /  17.8   16.3 /  15.9
