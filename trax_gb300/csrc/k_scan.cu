@@ -26,22 +26,17 @@ constexpr int SCAN_THREADS = 256;
 constexpr int SCAN_ITEMS = 16;
 constexpr uint32_t SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
 
-__global__ void __launch_bounds__(SCAN_THREADS)
-    scan_kernel(Stamp stamp, ScanJob job0, ScanJob job1, uint64_t nHost, const uint32_t* nDev, uint32_t nAdd,
-                uint32_t* err, uint32_t overflowBit, WaitCtl ctl) {
-  stamp_begin(stamp);
+__device__ __forceinline__ void scan_tile(const ScanJob& job, uint64_t n, uint32_t* err, uint32_t overflowBit,
+                                          WaitCtl ctl) {
   __shared__ uint32_t s_tile;
   __shared__ uint32_t s_warp[SCAN_THREADS / 32];
   __shared__ unsigned long long s_wide[SCAN_THREADS / 32];
   __shared__ uint32_t s_prefix;
-  // two arrays of one length may share a launch (blockIdx.y), each with its own tickets
-  const ScanJob& job = blockIdx.y ? job1 : job0;
   const uint32_t* __restrict__ in = job.in;
   uint32_t* out = job.out;
   uint32_t* ticket = static_cast<uint32_t*>(job.scratch);
   unsigned long long* status = reinterpret_cast<unsigned long long*>(static_cast<char*>(job.scratch) + 256);
   const ScanTotal total = job.total;
-  const uint64_t n = nDev ? (uint64_t)(*nDev) + nAdd : nHost;
   if (threadIdx.x == 0) s_tile = gridDim.x > 1 ? atomicAdd(ticket, 1u) : 0u;
   __syncthreads();
   const uint32_t tile = s_tile;
@@ -127,6 +122,21 @@ __global__ void __launch_bounds__(SCAN_THREADS)
   }
 }
 
+__global__ void __launch_bounds__(SCAN_THREADS)
+    scan_kernel(Stamp stamp, ScanJob job, uint64_t nHost, const uint32_t* nDev, uint32_t nAdd, uint32_t* err,
+                uint32_t overflowBit, WaitCtl ctl) {
+  stamp_begin(stamp);
+  scan_tile(job, nDev ? (uint64_t)(*nDev) + nAdd : nHost, err, overflowBit, ctl);
+}
+
+// two arrays of one length in one launch (blockIdx.y), each with its own tickets
+__global__ void __launch_bounds__(SCAN_THREADS)
+    scan_pair_kernel(Stamp stamp, ScanJob job0, ScanJob job1, uint64_t nHost, const uint32_t* nDev, uint32_t nAdd,
+                     uint32_t* err, uint32_t overflowBit, WaitCtl ctl) {
+  stamp_begin(stamp);
+  scan_tile(blockIdx.y ? job1 : job0, nDev ? (uint64_t)(*nDev) + nAdd : nHost, err, overflowBit, ctl);
+}
+
 // the context's slots and time marks to page-locked host memory
 __global__ void slots_to_host_kernel(Stamp stamp, const uint32_t* slots, uint32_t* host, uint32_t n) {
   stamp_begin(stamp);
@@ -157,8 +167,12 @@ cudaError_t scan_exclusive(const ScanJob* jobs, int nJobs, uint64_t n, const uin
       if (e != cudaSuccess) return e;
     }
   }
-  launch(q, scan_kernel, dim3((unsigned)tiles, nJobs), SCAN_THREADS, 0, jobs[0], jobs[nJobs - 1], n, nDev, nAdd, err,
-         flagOverflow ? TRAX_EBIT_OVERFLOW : 0u, ctl);
+  const uint32_t overflowBit = flagOverflow ? TRAX_EBIT_OVERFLOW : 0u;
+  if (nJobs == 1)
+    launch(q, scan_kernel, (unsigned)tiles, SCAN_THREADS, 0, jobs[0], n, nDev, nAdd, err, overflowBit, ctl);
+  else
+    launch(q, scan_pair_kernel, dim3((unsigned)tiles, 2), SCAN_THREADS, 0, jobs[0], jobs[1], n, nDev, nAdd, err,
+           overflowBit, ctl);
   return cudaGetLastError();
 }
 
@@ -250,7 +264,7 @@ extern "C" int trax_prefix_sum_noalloc(const uint32_t* d_in, uint32_t* d_out, ui
   e = cudaMemsetAsync(base, 0, NOALLOC_HEADER + tiles * sizeof(unsigned long long), st);
   if (e == cudaSuccess) {
     const trax::ScanJob job{d_in, d_out, base, trax::ScanTotal{}};
-    trax::scan_kernel<<<(unsigned)tiles, trax::SCAN_THREADS, 0, st>>>(trax::Stamp{}, job, job, n, nullptr, 0, err, 0u,
+    trax::scan_kernel<<<(unsigned)tiles, trax::SCAN_THREADS, 0, st>>>(trax::Stamp{}, job, n, nullptr, 0, err, 0u,
                                                                       noalloc_wait());
     e = cudaGetLastError();
   }
