@@ -15,8 +15,8 @@ e2e        the same metric through the C ABI from host buffers: upload of the
            inside the timed region (host wall clock, synchronized)
 plain      the per-event launch structure of the reference (one event per
            stage call, host-synced count/scan/store) over the first events
-roofline   the dominant kernel's algorithmic bytes / its CUDA-event time
-           against the measured HBM copy bandwidth
+roofline   the dominant kernel's algorithmic bytes / its device time (the
+           time marks the kernels write) against the measured HBM copy bandwidth
 cpu_baseline  the reference's own OpenCL kernel text compiled for the CPU
            (oracle/_ref, built where the reference's sources were available;
            "kind": "reference"), else the CPU oracle that restates it
@@ -251,7 +251,7 @@ def kernel_bytes(name, st, n_tasks, n_hits, cells, cells_inner=None, cells_third
 TRAFFIC_PER_UNIT = {  # by grid (nZ x nPhi): the grid changes the cells read and the hits visited
     "150x64": {"predict_count": ("pairs", 32.5), "filter": ("candidates", 27.3), "grid_build": ("hits", 97.0)},
     "200x64": {"predict_count": ("pairs", 32.7), "filter": ("candidates", 27.3), "grid_build": ("hits", 110.9)},
-    "250x48": {"predict_count": ("pairs", 32.2), "filter": ("candidates", 30.5), "grid_build": ("hits", 107.6)},
+    "250x48": {"predict_count": ("pairs", 32.2), "filter": ("candidates", 31.2), "grid_build": ("hits", 107.8)},
     "300x48": {"predict_count": ("pairs", 32.9), "filter": ("candidates", 27.1), "grid_build": ("hits", 118.4)},
     "250x32": {"predict_count": ("pairs", 32.2), "filter": ("candidates", 27.2), "grid_build": ("hits", 90.4)},
     "200x48": {"predict_count": ("pairs", 32.4), "filter": ("candidates", 27.2), "grid_build": ("hits", 97.2)},
@@ -263,7 +263,7 @@ TRAFFIC_PER_UNIT = {  # by grid (nZ x nPhi): the grid changes the cells read and
 # 300-event capture / its units): the dominant kernels are issue-bound, so
 # their position against the SMs' issue rate is reported beside the HBM one.
 # Captured for the current prediction kernel at the workload's grid only.
-INST_PER_UNIT = {"250x48": {"predict_count": ("pairs", 23.55)}}
+INST_PER_UNIT = {"250x48": {"predict_count": ("pairs", 23.47)}}
 
 
 def kernel_issue(name, st, ms, clk, device, grid):
@@ -536,10 +536,10 @@ def run_ours(args, ranks):
     ms_per_step = 1e3 * t_max / args.steps
     launches = st.kernel_launches * args.steps
 
-    # roofline of the dominant kernel (mean CUDA-event time over the steps)
+    # roofline of the dominant kernel (mean device time over the steps)
     kmean = {k: float(np.mean(v)) for k, v in kern.items() if v and min(v) >= 0}
     if not kmean:
-        raise RuntimeError("no per-kernel CUDA-event timings were recorded")
+        raise RuntimeError("no per-kernel timings were recorded")
     dom = max(kmean, key=kmean.get)
     # pair-stage tasks: one per outer-layer hit of every (event, layer triplet)
     n_tasks = int(sum(int(batch.layer_hits[:, lt.layer2 - 1].sum()) for lt in batch.lts))

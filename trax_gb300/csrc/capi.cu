@@ -2,16 +2,17 @@
 // uploads, the stage chain and result downloads.
 //
 // One chain implementation runs in two modes:
-//   * SYNCED: after every compaction scan the host reads the total (one
-//     4-byte device-to-host copy) and sizes the next buffers exactly -- the
-//     launch structure of the reference's run() methods (count, scan,
-//     downloadScalar, allocate, store).  The stage entry points use it.
+//   * SYNCED: after every compaction scan the host waits for the total (which
+//     the scan also writes to page-locked host memory) and sizes the next
+//     buffers exactly -- the launch structure of the reference's run() methods
+//     (count, scan, downloadScalar, allocate, store).  The stage entry points
+//     use it.
 //   * DEVICE: no host reads.  Every kernel takes its item count from a fixed
-//     device slot (written by a one-thread publish kernel after each scan) and
-//     every output has a capacity learnt from an earlier SYNCED run plus
-//     headroom.  A total above its capacity is clamped and reported as
-//     TRAX_ERR_CAPACITY, never silently truncated.  This mode is captured once
-//     into a CUDA graph and replayed by trax_seed_batch.
+//     device slot (written by the scan before it) and every output has a
+//     capacity learnt from earlier SYNCED runs plus headroom.  A total above
+//     its capacity is clamped and reported as TRAX_ERR_CAPACITY, never silently
+//     truncated.  This mode is captured into a CUDA graph, which
+//     trax_seed_batch replays for every batch that fits it.
 #include <cuda_runtime.h>
 #include <nvtx3/nvToolsExt.h>
 
@@ -79,7 +80,7 @@ static_assert(S_N <= 64, "the slot buffers hold 64 words");
 
 enum Mode { SYNCED, DEVICE };
 
-// kernels timed individually with CUDA events (order of trax_get_timings)
+// kernels timed individually by device time marks (order of trax_get_timings)
 enum TimedKernel {
   TK_GRID = 0,
   TK_PAIR_COUNT,
@@ -139,7 +140,8 @@ struct trax_ctx {
   // prediction / filter
   DevBuf candLocal, predWarps, predKeep, cands, candOffsets, flagWords, flagSums, h1, h2, h3, tripOffsets;
   // connectivity / fit / CA
-  DevBuf eta, segOf, segStart, linkCount, linkRun, linkRuns, inDeg, basis, follower, connS, connW, connIdx, nonConnIdx, pt;
+  DevBuf eta, segOf, segStart, linkCount, linkRun, linkRuns, inDeg, basis, follower, connS, connW, connIdx;
+  DevBuf nonConnIdx, pt;
   DevBuf states, inStart, inCursor, inList, best, isBest, handlers, tracks;
   DevBuf userIdx, caNext;  // caller-provided fit list; second state buffer of the caller-link CA
   // bookkeeping
@@ -553,8 +555,8 @@ int stage_pairs(trax_ctx* c, Mode mode) {
   ENSURE(pairs, maxPairs, 8);
   KBEG(TK_PAIR_EMIT);
   CK(pair_tasks(c->cfg, true, ptr<uint32_t>(c->grid), dev_hits(c), ptr<uint32_t>(c->segOuter), taskBase, nTasksDev,
-                maxTasks, taskCount, taskState, ptr<uint2>(c->pairs), maxPairs, ptr<uint32_t>(c->pairOffsets), slot(c, S_PAIR_SENT), dev_err(c),
-                c->q));
+                maxTasks, taskCount, taskState, ptr<uint2>(c->pairs), maxPairs, ptr<uint32_t>(c->pairOffsets),
+                slot(c, S_PAIR_SENT), dev_err(c), c->q));
   KEND(TK_PAIR_EMIT);
   return TRAX_OK;
 }
@@ -697,7 +699,8 @@ int stage_connectivity(trax_ctx* c, Mode mode) {
                         ptr<uint32_t>(c->linkRun), c->sortedSegments, c->q));
   KEND(TK_CONN_COUNT);
   // the links' places, and the places of the incoming links of every follower
-  RC(scan_publish(c, mode, {ScanArray{linkCount, linkCount}, ScanArray{ptr<uint32_t>(c->inDeg), ptr<uint32_t>(c->inStart)}},
+  RC(scan_publish(c, mode,
+                  {ScanArray{linkCount, linkCount}, ScanArray{ptr<uint32_t>(c->inDeg), ptr<uint32_t>(c->inStart)}},
                   c->nT, mode == DEVICE ? nTDev : nullptr, maxT, S_LINKS, mode == DEVICE ? c->capLinks : NO_CAP));
   uint64_t maxLinks = c->capLinks;
   if (mode == SYNCED) {
@@ -1114,11 +1117,14 @@ void trax_destroy(trax_ctx* c) {
                     &c->phys_findIds, &c->phys_flags, &c->phys_counts, &c->trk_isTrack, &c->trk_hitsOf,
                     &c->trk_start, &c->trk_size, &c->trk_real, &c->trk_firstId, &c->trk_parent, &c->trk_compSize,
                     &c->trk_compStart, &c->trk_cursor, &c->trk_members, &c->trk_filtered, &c->trk_hits,
-                    &c->trk_entryTrack, &c->trk_owner, &c->trk_table, &c->trk_counts, &c->grid, &c->px, &c->py, &c->pz, &c->player, &c->pdet, &c->phid,
+                    &c->trk_entryTrack, &c->trk_owner, &c->trk_table, &c->trk_counts, &c->grid, &c->px, &c->py,
+                    &c->pz, &c->player, &c->pdet, &c->phid,
                     &c->pevt, &c->porig, &c->pxyzp, &c->sc_cell, &c->sc_phi, &c->sc_perm, &c->sc_counts,
-                    &c->fineGrid, &c->fineHits, &c->segOuter, &c->taskBase, &c->taskCount, &c->taskState, &c->pairs, &c->pairOffsets, &c->candLocal, &c->predWarps, &c->predKeep, &c->cands,
-                    &c->candOffsets, &c->flagWords, &c->flagSums, &c->h1, &c->h2, &c->h3, &c->tripOffsets, &c->eta, &c->segOf,
-                    &c->segStart, &c->linkCount, &c->linkRun, &c->linkRuns, &c->inDeg, &c->basis, &c->follower, &c->connS, &c->connW,
+                    &c->fineGrid, &c->fineHits, &c->segOuter, &c->taskBase, &c->taskCount, &c->taskState, &c->pairs,
+                    &c->pairOffsets, &c->candLocal, &c->predWarps, &c->predKeep, &c->cands,
+                    &c->candOffsets, &c->flagWords, &c->flagSums, &c->h1, &c->h2, &c->h3, &c->tripOffsets, &c->eta,
+                    &c->segOf, &c->segStart, &c->linkCount, &c->linkRun, &c->linkRuns, &c->inDeg, &c->basis,
+                    &c->follower, &c->connS, &c->connW,
                     &c->connIdx, &c->nonConnIdx, &c->pt, &c->states, &c->inStart, &c->inCursor, &c->inList, &c->best,
                     &c->isBest, &c->handlers, &c->tracks, &c->scanScratch, &c->slots, &c->fitOk, &c->fitSegCnt,
                     &c->fitSegDelta, &c->fitRows, &c->fitPartials, &c->fitOut, &c->fitParams, &c->fitDHits,
@@ -1950,7 +1956,8 @@ int trax_fit_prepare(trax_ctx* c, const trax_fit_opts* opts, uint64_t* n_fit) {
   CK(ensure(c, c->fitSegDelta, (size_t)S * 4));
   CK(cudaMemsetAsync(c->fitSegCnt.p, 0, (size_t)S * 4, c->st));
   uint32_t* ok = ptr<uint32_t>(c->fitOk);
-  CK(fit_select(f, c->cfg, dev_hits(c), fit_triplets(c), nT, truthOnly, ok, ptr<uint32_t>(c->fitSegCnt), c->st, &c->q.launches));
+  CK(fit_select(f, c->cfg, dev_hits(c), fit_triplets(c), nT, truthOnly, ok, ptr<uint32_t>(c->fitSegCnt), c->st,
+                &c->q.launches));
   CK(ensure(c, c->scanScratch, scan_scratch_bytes(nT + 1)));
   CK(scan_exclusive(ok, ok, nT + 1, c->scanScratch.p, dev_err(c), c->q, true, c->wait));
   // 2. rows ordered by layer triplet, then by event (segment order inside a layer triplet)
@@ -2051,7 +2058,8 @@ int trax_fit_backward(trax_ctx* c, const double* align, double* chi2, double* d_
   CK(cudaMemcpyAsync(out.data(), c->fitOut.p, out.size() * sizeof(double), cudaMemcpyDeviceToHost, c->st));
   if (d_hits && c->nHits) {
     CK(ensure(c, c->fitDHitsF, (size_t)c->nHits * 3 * sizeof(float)));
-    CK(fit_hits_out(ptr<double>(c->fitDHits), ptr<uint32_t>(c->porig), c->nHits, ptr<float>(c->fitDHitsF), c->st, &c->q.launches));
+    CK(fit_hits_out(ptr<double>(c->fitDHits), ptr<uint32_t>(c->porig), c->nHits, ptr<float>(c->fitDHitsF), c->st,
+                    &c->q.launches));
     CK(cudaMemcpyAsync(d_hits, c->fitDHitsF.p, (size_t)c->nHits * 3 * sizeof(float), cudaMemcpyDeviceToHost,
                        c->st));
   }

@@ -189,7 +189,8 @@ __global__ void __launch_bounds__(GRID_MAX_THREADS)
 __device__ __forceinline__ uint32_t half_of(uint32_t word, uint32_t c) { return (word >> ((c & 1u) * 16u)) & 0xffffu; }
 
 __global__ void __launch_bounds__(GRID_MAX_THREADS, 2)
-    grid_kernel16(Stamp stamp, DevConfig cfg, const __grid_constant__ GridInput in, uint32_t* __restrict__ grid, const __grid_constant__ DevHits out, GridScratch sc,
+    grid_kernel16(Stamp stamp, DevConfig cfg, const __grid_constant__ GridInput in, uint32_t* __restrict__ grid,
+                  const __grid_constant__ DevHits out, GridScratch sc,
                   uint32_t* err, uint32_t maxHits) {
   stamp_begin(stamp);
   clear_scan_scratch(sc);

@@ -357,7 +357,8 @@ __global__ void circle_fit_kernel(Stamp stamp, const float4* __restrict__ hits, 
   }
 }
 
-__global__ void in_degree_kernel(Stamp stamp, const uint32_t* __restrict__ follower, const uint32_t* nLinksDev, uint32_t* inDeg) {
+__global__ void in_degree_kernel(Stamp stamp, const uint32_t* __restrict__ follower, const uint32_t* nLinksDev,
+                                 uint32_t* inDeg) {
   stamp_begin(stamp);
   const uint32_t n = *nLinksDev;
   GRID_STRIDE(p, n) atomicAdd(&inDeg[follower[p]], 1u);
@@ -437,9 +438,9 @@ __global__ void ca_level_kernel(Stamp stamp, DevConfig cfg, uint32_t level, uint
 // copying (CellularAutomaton.cpp:52-98), until no cell lives.  Used for
 // caller-provided links, which need not go from one layer triplet to the
 // next as the chain's own do.
-__global__ void ca_iteration_kernel(Stamp stamp, const uint32_t* __restrict__ basis, const uint32_t* __restrict__ follower,
-                                    uint32_t nLinks, const uint32_t* __restrict__ cur, uint32_t* next,
-                                    uint32_t* living) {
+__global__ void ca_iteration_kernel(Stamp stamp, const uint32_t* __restrict__ basis,
+                                    const uint32_t* __restrict__ follower, uint32_t nLinks,
+                                    const uint32_t* __restrict__ cur, uint32_t* next, uint32_t* living) {
   stamp_begin(stamp);
   GRID_STRIDE(p, nLinks) {
     const uint32_t f = follower[p];

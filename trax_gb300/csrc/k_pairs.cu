@@ -17,13 +17,13 @@
 // P2 = [max(J0, zEnd) - len, end2 - len).  When all ranges of an outer hit
 // are disjoint and can be ordered, the store pass walks them in ascending
 // order; otherwise (only for NaN/inf or > 2 pi windows) it walks the whole
-// inner layer and keeps the indices that some range contains.
+// inner layer and keeps the indices that some range contains.  One lane walks
+// an outer hit's rows, or a group of lanes one row each (pair_lanes).
 #include "trax_kernels.h"
 
 namespace trax {
 
 namespace {
-
 
 struct PairWindow {
   float zLow, zHigh, phiLow, phiHigh;

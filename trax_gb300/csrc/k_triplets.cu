@@ -22,7 +22,6 @@ namespace trax {
 
 namespace {
 
-
 int grid_for(uint64_t items, int threads) {
   uint64_t blocks = (items + threads - 1) / threads;
   uint64_t cap = (uint64_t)sm_count() * (4096 / threads);  // two waves at full occupancy
@@ -430,11 +429,11 @@ struct PredStage {
 
 template <int K>
 __global__ void __launch_bounds__(TRAX_MAX_TUNED_THREADS, 4)
-    predict_count_k_kernel(Stamp stamp, DevConfig cfg, const uint32_t* __restrict__ grid, const float4* __restrict__ hits,
-                           const uint32_t* __restrict__ hitEvt, const uint32_t* __restrict__ hitLayer,
-                           const uint2* __restrict__ pairs, const uint32_t* __restrict__ nPairsDev,
-                           uint32_t* candCount, uint32_t* keep, uint32_t* warpSums, uint32_t* nWarpsOut,
-                           uint32_t* err) {
+    predict_count_k_kernel(Stamp stamp, DevConfig cfg, const uint32_t* __restrict__ grid,
+                           const float4* __restrict__ hits, const uint32_t* __restrict__ hitEvt,
+                           const uint32_t* __restrict__ hitLayer, const uint2* __restrict__ pairs,
+                           const uint32_t* __restrict__ nPairsDev, uint32_t* candCount, uint32_t* keep,
+                           uint32_t* warpSums, uint32_t* nWarpsOut, uint32_t* err) {
   stamp_begin(stamp);
   extern __shared__ PredStage s_stage[];  // [warp][k][lane]
   const uint32_t nPairs = *nPairsDev;

@@ -5,7 +5,7 @@ this implementation's timings.
 One record per chain run: the batch shape, host<->device transfers and, per
 stage, count / scan / store / wall / kernel milliseconds.  Records with the
 same shape form a class; a row holds the class's means and standard
-deviations over its runs.  Stage split (CUDA-event times of trax_get_timings):
+deviations over its runs.  Stage split (device times of trax_get_timings):
 
   buildGrid            count = the fused grid kernel (count, scan and scatter in one)
   pairGen              count / store kernels; scan = the rest of the stage
