@@ -459,7 +459,7 @@ __global__ void fill_u32_kernel(Stamp stamp, uint32_t* p, uint32_t v, uint32_t n
 // followerBestBasisStore semantics (CellularAutomaton.h:212-263) over the
 // incoming bases in ascending order, which is the order of their links (an
 // insertion sort first; lists are short)
-__device__ __forceinline__ void ca_pick_best(const CABuffers& b, const float* pt, uint32_t t) {
+__device__ __forceinline__ void ca_pick_best(const CABuffers& b, const float* pt, uint32_t t, uint32_t sf) {
   const uint32_t first = b.inStart[t], end = b.inStart[t + 1];
   for (uint32_t i = first + 1; i < end; ++i) {
     const uint32_t v = b.inList[i];
@@ -471,7 +471,6 @@ __device__ __forceinline__ void ca_pick_best(const CABuffers& b, const float* pt
     b.inList[j] = v;
   }
   if (first >= end) return;
-  const uint32_t sf = b.states[t];
   const float ptT = pt[t];
   bool have = false;
   float minPt = 0.0f;
@@ -501,7 +500,7 @@ __global__ void ca_best_kernel(Stamp stamp, const float* pt, CABuffers b, const 
   stamp_begin(stamp);
   if (ca_skip(err)) return;
   const uint32_t nT = *nTDev;
-  GRID_STRIDE(t, nT) ca_pick_best(b, pt, t);
+  GRID_STRIDE(t, nT) ca_pick_best(b, pt, t, b.states[t]);
 }
 
 // Both phases and the handlers of one event per CTA: the chain's links stay
@@ -517,16 +516,20 @@ __global__ void __launch_bounds__(1024)
   if (nT == 0u || ca_skip(cfg.err)) return;
   const uint32_t s0 = blockIdx.x * cfg.nLT;
   const uint32_t t0 = segStart[s0], t1 = segStart[s0 + cfg.nLT];
+  // A triplet's bases lie in earlier levels, so its state and its best basis
+  // come out of one visit (the CA stage of 37 ttbar-like events took 39.5 us
+  // with a pass of its own for the best bases, 35.0 us so; of 1000, 155 and
+  // 146 us).  Taking a single basis without the general case gained nothing.
   for (uint32_t level = 0; level < cfg.nLT; ++level) {
     for (uint32_t t = segStart[s0 + level] + threadIdx.x, end = segStart[s0 + level + 1]; t < end; t += blockDim.x) {
-      b.states[t] = level ? ca_state(b.inStart, b.inList, b.states, t) : 1u;
+      const uint32_t state = level ? ca_state(b.inStart, b.inList, b.states, t) : 1u;
+      b.states[t] = state;
       b.best[t] = TRAX_SENTINEL;
       b.isBest[t] = 0u;
+      if (level) ca_pick_best(b, pt, t, state);
     }
     __syncthreads();
   }
-  for (uint32_t t = t0 + threadIdx.x; t < t1; t += blockDim.x) ca_pick_best(b, pt, t);
-  __syncthreads();
   const bool any = *nLinksDev != 0u;
   for (uint32_t t = t0 + threadIdx.x; t < t1; t += blockDim.x)
     b.handlers[t] = any ? (b.isBest[t] == 0u) * b.states[t] : 0u;
