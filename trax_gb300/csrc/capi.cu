@@ -672,6 +672,10 @@ int stage_filter(trax_ctx* c, Mode mode) {
   return TRAX_OK;
 }
 
+ConnLists conn_lists(trax_ctx* c) {
+  return ConnLists{ptr<uint32_t>(c->connS), ptr<uint32_t>(c->connIdx), ptr<uint32_t>(c->nonConnIdx)};
+}
+
 int stage_connectivity(trax_ctx* c, Mode mode) {
   NvtxRange nvtx("trax.connectivity");
   const uint32_t S = c->cfg.E * c->cfg.nLT;
@@ -724,8 +728,8 @@ int stage_connectivity(trax_ctx* c, Mode mode) {
   // is what the first leaves of the triplets but the last
   RC(scan_publish(c, mode, ptr<uint32_t>(c->connS), (c->nT + 31) / 32, mode == DEVICE ? slot(c, S_CONN_WORDS) : nullptr,
                   maxTW, S_CONN, NO_CAP));
-  CK(connectable_lists(tv, ptr<uint32_t>(c->connW), ptr<uint32_t>(c->connS), ptr<uint32_t>(c->connIdx),
-                       ptr<uint32_t>(c->nonConnIdx), c->q));
+  // (a captured chain writes them with the circle fit, which follows)
+  if (mode == SYNCED) CK(connectable_lists(tv, ptr<uint32_t>(c->connW), conn_lists(c), c->q));
   return TRAX_OK;
 }
 
@@ -737,7 +741,9 @@ int stage_fit(trax_ctx* c, Mode mode) {
     CK(cudaMemsetAsync(c->pt.p, 0, (size_t)std::max<uint64_t>(maxT, 1) * 4, c->st));
     return TRAX_OK;
   }
-  CK(circle_fit_words(dev_hits(c), triplets(c, maxT), ptr<uint32_t>(c->connW), ptr<float>(c->pt), c->q));
+  const ConnLists lists = conn_lists(c);
+  CK(circle_fit_words(dev_hits(c), triplets(c, maxT), ptr<uint32_t>(c->connW), ptr<float>(c->pt),
+                      mode == DEVICE ? &lists : nullptr, c->q));
   return TRAX_OK;
 }
 

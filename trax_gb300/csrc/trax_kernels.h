@@ -324,8 +324,12 @@ struct LinkStore {
 cudaError_t connectivity_store(const DevConfig& cfg, TripletView t, const float* eta, LinkStore ls, Queue& q);
 // With connSums scanned into wordStart: the connectable and non-connectable
 // triplets among the first nT - 1
-cudaError_t connectable_lists(TripletView t, const uint32_t* connWords, const uint32_t* wordStart, uint32_t* connIdx,
-                              uint32_t* nonConnIdx, Queue& q);
+struct ConnLists {
+  const uint32_t* wordStart;
+  uint32_t* conn;
+  uint32_t* nonConn;
+};
+cudaError_t connectable_lists(TripletView t, const uint32_t* connWords, ConnLists lists, Queue& q);
 // the context's slots and the time marks after them to page-locked host memory
 cudaError_t slots_to_host(const uint32_t* slots, uint32_t* host, uint32_t words, Queue& q);
 
@@ -334,7 +338,8 @@ cudaError_t circle_fit(DevHits hits, TripletView t, const uint32_t* connectable,
                        uint64_t maxConn, float* pt, Queue& q);
 
 // pt[t] of every triplet: the circle fit of the connectable ones, 0 for the others
-cudaError_t circle_fit_words(DevHits hits, TripletView t, const uint32_t* connWords, float* pt, Queue& q);
+cudaError_t circle_fit_words(DevHits hits, TripletView t, const uint32_t* connWords, float* pt,
+                             const ConnLists* lists, Queue& q);
 
 struct CABuffers {
   uint32_t* states;    // [nT]
