@@ -159,7 +159,6 @@ struct trax_ctx {
   // triplets of every segment ordered by (second hit, first hit): true for the
   // chain's own filter output; checked for caller-provided triplets
   bool sortedSegments = true;
-  bool chainLinking = false;  // the chain being captured includes the linking stages
   bool inListOwn = false;     // inStart / inList hold the incoming links of the last connectivity run
   bool identityHits = false;  // hit collection taken as uploaded (trax_set_tracklets)
   // DEVICE-mode capacities and the captured graph
@@ -608,7 +607,7 @@ TripletView triplets(trax_ctx* c, uint64_t maxT) {
   return t;
 }
 
-// what the link part of triplet_segments writes
+// what triplet_link_start writes
 int link_buffers(trax_ctx* c, Mode mode, uint64_t maxT) {
   ENSURE(eta, maxT, 4);
   ENSURE(inDeg, maxT + 1, 4);
@@ -661,14 +660,11 @@ int stage_filter(trax_ctx* c, Mode mode) {
   ENSURE(h3, maxT, 4);
   KBEG(TK_FILTER_STORE);
   CK(filter_store(ptr<uint2>(c->pairs), ptr<uint2>(c->cands), nCandsDev, maxCands, words, sums, ptr<uint32_t>(c->h1),
-                  ptr<uint32_t>(c->h2), ptr<uint32_t>(c->h3), maxT, c->q));
+                  ptr<uint32_t>(c->h2), ptr<uint32_t>(c->h3), maxT,
+                  TripletSegments{S, ptr<uint32_t>(c->candOffsets), slot(c, S_TRIPLETS), ptr<uint32_t>(c->segStart),
+                                  ptr<uint32_t>(c->tripOffsets)},
+                  c->q));
   KEND(TK_FILTER_STORE);
-  // a captured chain that goes on to the linking prepares it in the same pass
-  const bool link = mode == DEVICE && c->chainLinking;
-  if (link) RC(link_buffers(c, mode, maxT));
-  const LinkStart ls = link_start(c);
-  CK(triplet_segments(c->cfg, dev_hits(c), triplets(c, maxT), ptr<uint32_t>(c->segStart), nullptr,
-                      ptr<uint32_t>(c->tripOffsets), link ? &ls : nullptr, c->q));
   return TRAX_OK;
 }
 
@@ -695,7 +691,7 @@ int stage_connectivity(trax_ctx* c, Mode mode) {
   ENSURE(connIdx, maxT, 4);
   ENSURE(nonConnIdx, maxT, 4);
   TripletView tv = triplets(c, maxT);
-  if (mode == SYNCED) CK(triplet_link_start(c->cfg, dev_hits(c), tv, link_start(c), c->q));
+  CK(triplet_link_start(c->cfg, dev_hits(c), tv, link_start(c), c->q));
   uint32_t* linkCount = ptr<uint32_t>(c->linkCount);
   KBEG(TK_CONN_COUNT);
   CK(connectivity_count(c->cfg, dev_hits(c), tv, ptr<float>(c->eta), ptr<uint32_t>(c->tripOffsets),
@@ -848,7 +844,6 @@ int chain_device(trax_ctx* c, bool linking) {
   int (*stages[N_STAGES])(trax_ctx*, Mode) = {stage_grid, stage_pairs, stage_predict, stage_filter,
                                               stage_connectivity, stage_fit, stage_ca};
   const int n = linking ? N_STAGES : 4;
-  c->chainLinking = linking;
   mark(c, MARK_STAGE);
   for (int s = 0; s < n; ++s) {
     RC(stages[s](c, DEVICE));
@@ -1427,7 +1422,7 @@ int trax_set_tracklets(trax_ctx* c, const uint32_t* h1, const uint32_t* h2, cons
   c->hSlots[S_TRIPLETS] = (uint32_t)n;
   CK(cudaMemcpyAsync(slot(c, S_TRIPLETS), c->hSlots + S_TRIPLETS, 4, cudaMemcpyHostToDevice, c->st));
   CK(triplet_segments(c->cfg, dev_hits(c), triplets(c, n), ptr<uint32_t>(c->segStart), ptr<uint32_t>(c->segOf),
-                      ptr<uint32_t>(c->tripOffsets), nullptr, c->q));
+                      ptr<uint32_t>(c->tripOffsets), c->q));
   c->nPairs = c->nCands = 0;
   c->nT = n;
   c->identityHits = true;

@@ -43,73 +43,77 @@ int grid_for(uint64_t items, int threads) {
 
 #define GRID_STRIDE(i, n) for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < (n); i += gridDim.x * blockDim.x)
 
-// The triplets' segments: segStart[s] = first triplet of segment s or later.
-// A triplet whose segment differs from its predecessor's starts all segments
-// in between; the warp fills a gap of empty ones together.  LINK: what
-// connectivity starts from as well (TripletConnectivityTight.h:47-74).
-template <bool SEGMENTS, bool LINK>
+// What connectivity starts from (TripletConnectivityTight.h:47-74), in one pass
+// over the triplets.
 __global__ void __launch_bounds__(256)
-    triplet_segments_kernel(Stamp stamp, DevConfig cfg, const float4* __restrict__ hits,
-                            const uint32_t* __restrict__ hitEvt, const uint32_t* __restrict__ hitLayer,
-                            const uint32_t* __restrict__ h1, const uint32_t* __restrict__ h2,
-                            const uint32_t* __restrict__ h3, const uint32_t* nTDev, uint32_t* segStart,
-                            uint32_t* segOf, LinkStart link) {
+    link_start_kernel(Stamp stamp, DevConfig cfg, const float4* __restrict__ hits, const uint32_t* __restrict__ h1,
+                      const uint32_t* __restrict__ h2, const uint32_t* __restrict__ h3, const uint32_t* nTDev,
+                      LinkStart link) {
+  stamp_begin(stamp);
+  const uint32_t nT = *nTDev;
+  GRID_STRIDE(t, nT) {
+    const float4 a = hits[trax_hit(h1[t], cfg)], b = hits[trax_hit(h3[t], cfg)];
+    const float px = b.x - a.x, py = b.y - a.y, pz = b.z - a.z;
+    const float tt = div_(pz, sqrt_(px * px + py * py));
+    link.eta[t] = asinh_(tt);
+    link.inDeg[t] = 0u;
+    link.inCursor[t] = 0u;
+    if (link.runs) {
+      const uint32_t mid = trax_hit(h2[t], cfg);
+      const uint32_t prev = t ? trax_hit(h2[t - 1], cfg) : mid;
+      if (t == 0 || prev != mid) {
+        link.runs[mid].x = t;
+        if (t) link.runs[prev].y = t;
+      }
+      if (t + 1 == nT) link.runs[mid].y = nT;
+    }
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) link.inDeg[nT] = 0u;  // the scan's +1 slot
+}
+
+// The segments of a caller's triplets: segStart[s] = first triplet of segment s
+// or later.  A triplet whose segment differs from its predecessor's starts all
+// segments in between; the warp fills a gap of empty ones together.
+__global__ void __launch_bounds__(256)
+    triplet_segments_kernel(Stamp stamp, DevConfig cfg, const uint32_t* __restrict__ hitEvt,
+                            const uint32_t* __restrict__ hitLayer, const uint32_t* __restrict__ h1,
+                            const uint32_t* nTDev, uint32_t* segStart, uint32_t* segOf) {
   stamp_begin(stamp);
   const uint32_t nT = *nTDev;
   const uint32_t S = cfg.E * cfg.nLT;
   const uint32_t lane = threadIdx.x & 31u;
   for (uint32_t base = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); base < nT; base += gridDim.x * blockDim.x) {
     const uint32_t t = base + lane;
-    uint32_t hi = 0, seg = 0;
+    uint32_t seg = 0;
     if (t < nT) {
-      hi = trax_hit(h1[t], cfg);
-      if (SEGMENTS) seg = hitEvt[hi] * cfg.nLT + (hitLayer[hi] - 1);
+      const uint32_t hi = trax_hit(h1[t], cfg);
+      seg = hitEvt[hi] * cfg.nLT + (hitLayer[hi] - 1);
+      segOf[t] = seg;
     }
-    if (LINK && t < nT) {
-      const float4 a = hits[hi], b = hits[trax_hit(h3[t], cfg)];
-      const float px = b.x - a.x, py = b.y - a.y, pz = b.z - a.z;
-      const float tt = div_(pz, sqrt_(px * px + py * py));
-      link.eta[t] = asinh_(tt);
-      link.inDeg[t] = 0u;
-      link.inCursor[t] = 0u;
-      if (link.runs) {
-        const uint32_t mid = trax_hit(h2[t], cfg);
-        const uint32_t prev = t ? trax_hit(h2[t - 1], cfg) : mid;
-        if (t == 0 || prev != mid) {
-          link.runs[mid].x = t;
-          if (t) link.runs[prev].y = t;
-        }
-        if (t + 1 == nT) link.runs[mid].y = nT;
+    // the first segment this triplet starts: after its predecessor's
+    uint32_t from = __shfl_up_sync(0xffffffffu, seg, 1) + 1u;
+    if (lane == 0) {
+      if (t == 0) {
+        from = 0u;
+      } else {
+        const uint32_t hp = trax_hit(h1[t - 1], cfg);
+        from = hitEvt[hp] * cfg.nLT + (hitLayer[hp] - 1) + 1u;
       }
     }
-    if (SEGMENTS) {
-      if (t < nT && segOf) segOf[t] = seg;
-      // the first segment this triplet starts: after its predecessor's
-      uint32_t from = __shfl_up_sync(0xffffffffu, seg, 1) + 1u;
-      if (lane == 0) {
-        if (t == 0) {
-          from = 0u;
-        } else {
-          const uint32_t hp = trax_hit(h1[t - 1], cfg);
-          from = hitEvt[hp] * cfg.nLT + (hitLayer[hp] - 1) + 1u;
-        }
-      }
-      const bool starts = t < nT && from <= seg;
-      if (starts && seg <= S) segStart[seg] = t;
-      uint32_t gaps = __ballot_sync(0xffffffffu, starts && from < seg);
-      while (gaps) {
-        const int l = __ffs(gaps) - 1;
-        gaps &= gaps - 1u;
-        const uint32_t a = __shfl_sync(0xffffffffu, from, l), b = __shfl_sync(0xffffffffu, seg, l);
-        for (uint32_t s = a + lane; s < b && s <= S; s += 32u) segStart[s] = base + l;
-      }
-      if (base + 32u >= nT) {  // the warp with the last triplet: nothing starts after it
-        const uint32_t last = __shfl_sync(0xffffffffu, seg, (nT - 1u) & 31u);
-        for (uint32_t s = last + 1u + lane; s <= S; s += 32u) segStart[s] = nT;
-      }
+    const bool starts = t < nT && from <= seg;
+    if (starts && seg <= S) segStart[seg] = t;
+    uint32_t gaps = __ballot_sync(0xffffffffu, starts && from < seg);
+    while (gaps) {
+      const int l = __ffs(gaps) - 1;
+      gaps &= gaps - 1u;
+      const uint32_t a = __shfl_sync(0xffffffffu, from, l), b = __shfl_sync(0xffffffffu, seg, l);
+      for (uint32_t s = a + lane; s < b && s <= S; s += 32u) segStart[s] = base + l;
+    }
+    if (base + 32u >= nT) {  // the warp with the last triplet: nothing starts after it
+      const uint32_t last = __shfl_sync(0xffffffffu, seg, (nT - 1u) & 31u);
+      for (uint32_t s = last + 1u + lane; s <= S; s += 32u) segStart[s] = nT;
     }
   }
-  if (LINK && blockIdx.x == 0 && threadIdx.x == 0) link.inDeg[nT] = 0u;  // the scan's +1 slot
 }
 
 // trackletOffsets: filterOffsetStore (TripletThetaPhiFilter.h:221-257) writes
@@ -575,23 +579,16 @@ __global__ void tracks_kernel(Stamp stamp, const uint32_t* __restrict__ handlers
 }  // namespace
 
 cudaError_t triplet_segments(const DevConfig& cfg, DevHits hits, TripletView t, uint32_t* segStart, uint32_t* segOf,
-                             uint32_t* offsets, const LinkStart* link, Queue& q) {
-  const uint32_t S = cfg.E * cfg.nLT;
-  if (t.maxN > 0) {
-    if (link)
-      launch(q, triplet_segments_kernel<true, true>, grid_for(t.maxN, 256), 256, 0, cfg, hits.xyzp, hits.evt,
-             hits.layer, t.h1, t.h2, t.h3, t.nDev, segStart, segOf, *link);
-    else
-      launch(q, triplet_segments_kernel<true, false>, grid_for(t.maxN, 256), 256, 0, cfg, hits.xyzp, hits.evt,
-             hits.layer, t.h1, t.h2, t.h3, t.nDev, segStart, segOf, LinkStart{});
-  }
-  launch(q, triplet_offsets_kernel, 1, OFF_THREADS, 0, S, t.nDev, segStart, offsets);
+                             uint32_t* offsets, Queue& q) {
+  if (t.maxN > 0)
+    launch(q, triplet_segments_kernel, grid_for(t.maxN, 256), 256, 0, cfg, hits.evt, hits.layer, t.h1, t.nDev,
+           segStart, segOf);
+  launch(q, triplet_offsets_kernel, 1, OFF_THREADS, 0, cfg.E * cfg.nLT, t.nDev, segStart, offsets);
   return cudaGetLastError();
 }
 
 cudaError_t triplet_link_start(const DevConfig& cfg, DevHits hits, TripletView t, LinkStart link, Queue& q) {
-  launch(q, triplet_segments_kernel<false, true>, grid_for(t.maxN + 1, 256), 256, 0, cfg, hits.xyzp, hits.evt,
-         hits.layer, t.h1, t.h2, t.h3, t.nDev, nullptr, nullptr, link);
+  launch(q, link_start_kernel, grid_for(t.maxN + 1, 256), 256, 0, cfg, hits.xyzp, t.h1, t.h2, t.h3, t.nDev, link);
   return cudaGetLastError();
 }
 

@@ -892,12 +892,42 @@ __global__ void __launch_bounds__(TRAX_MAX_TUNED_THREADS, 8)
 // step, finding its word by a 5-step search over the words' running counts
 // and its candidate by the rank of the bit in the word (0.21 -> 0.15 ms on
 // the 1000-event batch against one thread per candidate).
+// It also writes the segments (TripletSegments): a segment's first triplet is
+// the number of flags before its first candidate.
 __global__ void filter_store_kernel(Stamp stamp, const uint2* __restrict__ pairs, const uint2* __restrict__ cands,
                                     const uint32_t* nCandsDev, const uint32_t* __restrict__ masks,
                                     const uint32_t* __restrict__ wordStart, uint32_t* h1, uint32_t* h2, uint32_t* h3,
-                                    uint32_t capT, uint32_t residentWarps) {
+                                    uint32_t capT, uint32_t residentWarps, TripletSegments seg) {
   stamp_begin(stamp);
   const uint32_t n = *nCandsDev;
+  const uint32_t S = seg.S, nT = *seg.nTDev;
+  auto first = [&](uint32_t s) {  // triplet of segment s or later
+    if (s == 0u) return 0u;
+    const uint32_t p = s < S ? seg.candOffsets[s] : n;
+    if (p >= n) return nT;
+    return min(nT, wordStart[p >> 5] + (uint32_t)__popc(masks[p >> 5] & ((1u << (p & 31u)) - 1u)));
+  };
+  for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s <= S; s += gridDim.x * blockDim.x) {
+    const uint32_t cur = first(s);
+    seg.segStart[s] = cur;
+    // filterOffsetStore (TripletThetaPhiFilter.h:221-257) and the monotonize
+    // kernel (:267-280): the first triplet of a segment that holds one, of
+    // the last such segment before one that does not, and the last triplet
+    // after them all
+    uint32_t off = cur;
+    if (cur >= nT) {
+      off = nT ? nT - 1u : 0u;
+    } else if (cur && first(s + 1u) == cur) {
+      uint32_t lo = 1u, hi = s;  // the first segment that starts at cur or later
+      while (lo < hi) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (first(mid) < cur) lo = mid + 1u;
+        else hi = mid;
+      }
+      off = first(lo - 1u);
+    }
+    seg.offsets[s] = off;
+  }
   const uint32_t nW = (n + 31u) >> 5;
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t warps = gridDim.x * (blockDim.x >> 5);
@@ -1005,11 +1035,10 @@ cudaError_t filter_candidates(const DevConfig& cfg, DevHits hits, const uint2* p
 
 cudaError_t filter_store(const uint2* pairs, const uint2* cands, const uint32_t* nCandsDev, uint64_t maxCands,
                          const uint32_t* masks, const uint32_t* wordStart, uint32_t* h1, uint32_t* h2, uint32_t* h3,
-                         uint64_t capT, Queue& q) {
-  if (maxCands == 0) return cudaSuccess;
+                         uint64_t capT, TripletSegments seg, Queue& q) {
   const uint32_t cap = capT > 0xffffffffull ? 0xffffffffu : (uint32_t)capT;
-  launch(q, filter_store_kernel, grid_for(maxCands, 256), 256, 0, pairs, cands, nCandsDev, masks, wordStart, h1, h2,
-         h3, cap, (uint32_t)sm_count() * 64u);
+  launch(q, filter_store_kernel, grid_for(maxCands + 1, 256), 256, 0, pairs, cands, nCandsDev, masks, wordStart, h1,
+         h2, h3, cap, (uint32_t)sm_count() * 64u, seg);
   return cudaGetLastError();
 }
 

@@ -265,11 +265,20 @@ cudaError_t predict_pairs(const DevConfig& cfg, bool emit, const uint32_t* grid,
 cudaError_t filter_candidates(const DevConfig& cfg, DevHits hits, const uint2* pairs, const uint2* cands,
                               const uint32_t* nCandsDev, uint64_t maxCands, uint32_t* masks, uint32_t* warpSums,
                               uint32_t* nWordsOut, Queue& q);
+// Segments of the triplets: segStart[s] = first triplet of segment s or later,
+// offsets = trackletOffsets, both S + 1 entries.
+struct TripletSegments {
+  uint32_t S;
+  const uint32_t* candOffsets;  // first candidate of every segment
+  const uint32_t* nTDev;
+  uint32_t* segStart;
+  uint32_t* offsets;
+};
 // with warpSums exclusively scanned into wordStart: the triplets of the
 // flagged candidates at wordStart[g / 32] + (flags below g in its word)
 cudaError_t filter_store(const uint2* pairs, const uint2* cands, const uint32_t* nCandsDev, uint64_t maxCands,
                          const uint32_t* masks, const uint32_t* wordStart, uint32_t* h1, uint32_t* h2, uint32_t* h3,
-                         uint64_t capT, Queue& q);
+                         uint64_t capT, TripletSegments seg, Queue& q);
 // ---------------------------------------------------------- connectivity
 struct TripletView {
   const uint32_t* h1;
@@ -279,10 +288,7 @@ struct TripletView {
   uint64_t maxN;
 };
 
-// Segments of the triplets: segStart[s] = first triplet of segment s or
-// later (S + 1 entries), offsets = trackletOffsets with the reference's
-// filterOffsetStore + monotonize semantics, segOf[t] (unless null).  With
-// `link` also what connectivity starts from: eta, and inDeg / inCursor zeroed.
+// What connectivity starts from: eta, inDeg / inCursor zeroed, and the runs.
 struct LinkStart {
   float* eta;
   uint32_t* inDeg;     // [nT+1]
@@ -293,9 +299,9 @@ struct LinkStart {
   // Given where every layer is the second of one layer triplet at most.
   uint2* runs;
 };
+// A caller's triplets: segStart and offsets as TripletSegments, and segOf[t].
 cudaError_t triplet_segments(const DevConfig& cfg, DevHits hits, TripletView t, uint32_t* segStart, uint32_t* segOf,
-                             uint32_t* offsets, const LinkStart* link, Queue& q);
-// the link part alone
+                             uint32_t* offsets, Queue& q);
 cudaError_t triplet_link_start(const DevConfig& cfg, DevHits hits, TripletView t, LinkStart link, Queue& q);
 // links per basis triplet (linkCount, +1 slot zeroed) and per follower
 // (inDeg); runStart[t]: where the store pass starts looking for t's followers
