@@ -893,7 +893,9 @@ __global__ void __launch_bounds__(TRAX_MAX_TUNED_THREADS, 8)
 // and its candidate by the rank of the bit in the word (0.21 -> 0.15 ms on
 // the 1000-event batch against one thread per candidate).
 // It also writes the segments (TripletSegments): a segment's first triplet is
-// the number of flags before its first candidate.
+// the number of flags before its first candidate.  (A pass over the triplets
+// for the segments and a block for the offsets took two launches more: an event
+// by stages 331 us, 320 us so.)
 __global__ void filter_store_kernel(Stamp stamp, const uint2* __restrict__ pairs, const uint2* __restrict__ cands,
                                     const uint32_t* nCandsDev, const uint32_t* __restrict__ masks,
                                     const uint32_t* __restrict__ wordStart, uint32_t* h1, uint32_t* h2, uint32_t* h3,
