@@ -239,3 +239,12 @@ def test_candidates_copied_by_output(trax_lib, oracle_lib, slots, fine):
             ctx.seed_batch(use_graph=graph, run_linking=False)
             assert np.array_equal(ctx.candidates()[0].ravel(), want["cands"]), graph
             assert ctx.stats().n_candidate_sentinels == want["stats_dict"]["cand_undefined_slots"]
+
+
+@pytest.mark.parametrize("n", [1, 4096, 4097, 8191, 8192, 8193, 16383, 16384, 16385, 20481])
+def test_scan_by_one_block_and_by_tiles(trax_lib, n):
+    """Sizes around one tile, around the tiles one block takes in turn, and past what is left to one block."""
+    x = np.random.default_rng(n).integers(0, 1 << 32, n, dtype=np.uint64).astype(np.uint32)
+    want = (np.cumsum(x, dtype=np.uint64) - x).astype(np.uint32)  # 32-bit sums wrap
+    with trax_lib.Context(0) as ctx:
+        assert np.array_equal(ctx.prefix_sum(x), want)
