@@ -248,3 +248,14 @@ def test_scan_by_one_block_and_by_tiles(trax_lib, n):
     want = (np.cumsum(x, dtype=np.uint64) - x).astype(np.uint32)  # 32-bit sums wrap
     with trax_lib.Context(0) as ctx:
         assert np.array_equal(ctx.prefix_sum(x), want)
+
+
+@pytest.mark.parametrize("graph", [True, False])
+def test_tracks_of_a_batch_without_links(trax_lib, graph):
+    """One layer triplet links nothing: reading the tracks of a fresh context's batch gives none, in both modes."""
+    with trax_lib.Context(0) as ctx:
+        ctx.upload(events.generate(0, n_events=3))
+        st = ctx.seed_batch(use_graph=graph)
+        out = [np.zeros(st.n_triplets + 1, np.uint32) for _ in range(3)]
+        assert st.n_triplets > 0 and st.n_links == 0 and st.n_track_entries == 0
+        assert all(v.size == 0 for v in ctx.tracks(out=out)) and all(v.size == 0 for v in ctx.tracks())

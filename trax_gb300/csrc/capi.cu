@@ -833,7 +833,7 @@ int run_stage(trax_ctx* c, int stage) {
   c->stage = stage;
   if (stage == 4) ++c->tripGen;
   if (stage == 6) c->ptGen = c->tripGen;
-  if (stage == 7) c->caGen = c->tripGen;
+  if (stage == 7 && !c->noLinks) c->caGen = c->tripGen;  // without links the CA does not run
   c->caOnly = false;
   return TRAX_OK;
 }
