@@ -165,7 +165,10 @@ int trax_circle_fit_on(trax_ctx* ctx, const uint32_t* valid_idx, uint64_t n_vali
 int trax_get_pt(trax_ctx* ctx, float* pt);
 
 /* CellularAutomaton::run (CellularAutomaton.h:43-49, .cpp:7-465) on the
- * links and pt of the last trax_connectivity / trax_circle_fit. */
+ * links and pt of the last trax_connectivity / trax_circle_fit; after
+ * trax_cellular_automaton_on on that call's links and pt, swept once over the
+ * layer triplets (links go from one to a later one; for others the result is
+ * the sweep's, not the reference's iteration). */
 int trax_cellular_automaton(trax_ctx* ctx, uint64_t* n_track_entries);
 
 /* CellularAutomaton::run on the caller's inputs (CellularAutomaton.h:43-49:

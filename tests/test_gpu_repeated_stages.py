@@ -1,0 +1,81 @@
+"""Stages run again, out of the chain's order or on nothing: the linking stages after a caller's links, a batch of no
+events, connectivity with another cut, and the times of a stage that runs again by itself."""
+import numpy as np
+import pytest
+
+from trax_gb300 import events
+
+pytestmark = pytest.mark.gpu
+
+
+def _links_between_levels(level, n_links, down, seed):
+    """Links without a cycle (along a random order of the triplets) between triplets of different levels, upwards only
+    or in both directions, by basis, each once."""
+    rng = np.random.default_rng(seed)
+    n = level.size
+    rank = rng.permutation(n)
+    b, f = rng.integers(0, n, (2, 8 * n_links))
+    keep = (rank[b] < rank[f]) & (level[b] != level[f]) if down else level[b] < level[f]
+    return np.unique(np.stack([b[keep], f[keep]], axis=1), axis=0)[:n_links].T
+
+
+def _ca_by_levels(level, b, f, pt):
+    """The automaton swept once over the levels: a triplet's state is one above its highest basis, the best basis the
+    one of the state below with the least pt difference, the lowest index of several.  A link against the levels can
+    leave a state without such a base: the track ends there, its further places (-1 here) hold nothing."""
+    n = level.size
+    bases = [[] for _ in range(n)]
+    for i, j in zip(b, f):
+        bases[j].append(i)
+    state = np.ones(n, np.int64)
+    for lv in range(1, int(level.max()) + 1):
+        new = {t: 1 + max(state[bases[t]]) for t in np.nonzero(level == lv)[0] if bases[t]}
+        for t, s in new.items():
+            state[t] = s
+    best, is_best = np.full(n, -1), np.zeros(n, bool)
+    for t in range(n):
+        ok = [k for k in bases[t] if state[k] + 1 == state[t]]
+        if ok:
+            best[t] = min(ok, key=lambda k: (abs(pt[k] - pt[t]), k))
+            is_best[best[t]] = True
+    tracks, offsets = [], [0]
+    for t in range(n):
+        k, length = t, 0 if is_best[t] else state[t]
+        for _ in range(length):
+            tracks.append(k)
+            k = best[k] if k >= 0 else -1
+        offsets.append(len(tracks))
+    return state, np.array(tracks), np.array(offsets)
+
+
+@pytest.mark.parametrize("down", [False, True])
+@pytest.mark.parametrize("graph", [False, True])
+def test_ca_stage_on_a_callers_links(trax_lib, graph, down):
+    """trax_cellular_automaton right after trax_cellular_automaton_on takes that call's links and pt, which may cross
+    events and go against the levels: one sweep over the levels of all events."""
+    batch = events.generate(2, n_events=4)
+    with trax_lib.Context(0) as ctx:
+        ctx.upload(batch)
+        ctx.seed_batch(use_graph=graph)
+        first = ctx.results()
+        level = batch.layer[first["perm"]][first["trip_h1"]].astype(np.int64) - 1
+        event = batch.event[first["perm"]][first["trip_h1"]]
+        pt = np.random.default_rng(1).choice(np.float32([10.0, 20.0, 33.25, 50.0]), level.size)
+        b, f = _links_between_levels(level, 3 * level.size // 2, down, seed=2)
+        assert (event[b] != event[f]).any() and (not down or (level[b] > level[f]).any())
+        want = _ca_by_levels(level, b, f, pt)
+        by_caller = ctx.cellular_automaton_on(b, f, pt)
+        for run in range(2):
+            ctx.cellular_automaton()
+            got = ctx.tracks()
+            for w, g, name in zip(want, got, ("states", "tracks", "offsets")):
+                assert g.shape == w.shape and np.array_equal(g[w >= 0], w[w >= 0]), (run, name)
+        if not down:  # upwards the sweep is the reference's iteration
+            assert all(np.array_equal(g, w) for g, w in zip(got, by_caller))
+        # the chain's own links again
+        assert ctx.connectivity(batch.d_eta_cut) == first["link_basis"].size
+        ctx.circle_fit()
+        ctx.cellular_automaton()
+        again = ctx.results()
+    for k, v in first.items():
+        assert np.array_equal(v, again[k]), k

@@ -159,7 +159,8 @@ struct trax_ctx {
   // triplets of every segment ordered by (second hit, first hit): true for the
   // chain's own filter output; checked for caller-provided triplets
   bool sortedSegments = true;
-  bool inListOwn = false;     // inStart / inList hold the incoming links of the last connectivity run
+  bool inListOwn = false;     // inStart / inList hold the incoming links of basis / follower, for the chain's CA
+  bool callerLinks = false;   // basis / follower are the links of trax_cellular_automaton_on
   bool identityHits = false;  // hit collection taken as uploaded (trax_set_tracklets)
   // DEVICE-mode capacities and the captured graph
   uint64_t capTasks = 0, capPairs = 0, capCands = 0, capT = 0, capLinks = 0, capTracks = 0;
@@ -720,6 +721,7 @@ int stage_connectivity(trax_ctx* c, Mode mode) {
   CK(connectivity_store(c->cfg, tv, ptr<float>(c->eta), store, c->q));
   KEND(TK_CONN_EMIT);
   c->inListOwn = true;
+  c->callerLinks = false;
   // the Q9 streams: the scan runs over the words' counts; the second stream
   // is what the first leaves of the triplets but the last
   RC(scan_publish(c, mode, ptr<uint32_t>(c->connS), (c->nT + 31) / 32, mode == DEVICE ? slot(c, S_CONN_WORDS) : nullptr,
@@ -771,15 +773,17 @@ int stage_ca(trax_ctx* c, Mode mode) {
   ENSURE(isBest, maxT, 4);
   ENSURE(handlers, maxT + 1, 4);
   CABuffers b = ca_buffers(c);
-  if (!c->inListOwn) {  // a caller's links took the lists (trax_cellular_automaton_on): fill them again
+  if (!c->inListOwn) {  // trax_cellular_automaton_on took links and lists: fill the lists from its links
     CK(ca_in_degree(ptr<uint32_t>(c->follower), nLinksDev, maxLinks, b, nTDev, maxT, c->q));
     RC(scan_publish(c, mode, b.inStart, c->nT, nullptr, maxT, -1, NO_CAP));
     CK(ca_fill(ptr<uint32_t>(c->basis), ptr<uint32_t>(c->follower), nLinksDev, maxLinks, b, c->q));
     c->inListOwn = true;
   }
   // one CTA per event while that fills the CTAs evenly enough; the chain's
-  // own triplets only: a caller's may link across events
-  const bool perEvent = !c->identityHits && c->cfg.E > 0 && maxT <= (uint64_t)c->cfg.E * TRAX_CA_EVENT_TRIPLETS;
+  // own triplets and links only: a caller's may go across events and to
+  // earlier levels, which need the levels swept over all events in turn
+  const bool perEvent = !c->identityHits && !c->callerLinks && c->cfg.E > 0 &&
+                        maxT <= (uint64_t)c->cfg.E * TRAX_CA_EVENT_TRIPLETS;
   CK(ca_chain(c->cfg, ptr<float>(c->pt), b, c->identityHits ? nullptr : ptr<uint32_t>(c->segStart), perEvent, nTDev,
               maxT, nLinksDev, c->q));
   RC(scan_publish(c, mode, b.handlers, c->nT, mode == DEVICE ? nTDev : nullptr, maxT, S_TRACKS,
@@ -1533,6 +1537,8 @@ int trax_cellular_automaton_on(trax_ctx* c, const uint32_t* basis, const uint32_
   ENSURE(isBest, nT, 4);
   ENSURE(handlers, nT + 1, 4);
   CK(ensure(c, c->scanScratch, scan_scratch_bytes(nT + 1)));
+  c->inListOwn = false;
+  c->callerLinks = true;
   CK(cudaMemcpyAsync(c->basis.p, basis, nL * 4, cudaMemcpyHostToDevice, c->st));
   CK(cudaMemcpyAsync(c->follower.p, follower, nL * 4, cudaMemcpyHostToDevice, c->st));
   CK(cudaMemcpyAsync(c->pt.p, pt, nT * 4, cudaMemcpyHostToDevice, c->st));
@@ -1546,7 +1552,6 @@ int trax_cellular_automaton_on(trax_ctx* c, const uint32_t* basis, const uint32_
   // states 1, in-degrees, the incoming bases of every follower (ascending)
   CK(ca_in_degree(ptr<uint32_t>(c->follower), nLinksDev, nL, b, nTDev, nT, c->q));
   CK(scan_exclusive(b.inStart, b.inStart, nT + 1, c->scanScratch.p, dev_err(c), c->q, true, c->wait));
-  c->inListOwn = false;
   CK(ca_fill(ptr<uint32_t>(c->basis), ptr<uint32_t>(c->follower), nLinksDev, nL, b, c->q));
   // forward phase: the reference's iteration (CellularAutomaton.cpp:37-98),
   // both state buffers starting at 1, swapped without copying; a link set
@@ -1699,7 +1704,10 @@ int trax_seed_batch(trax_ctx* c, const trax_batch_opts* opts, trax_batch_stats* 
     c->stage = linking ? 7 : 4;
     ++c->tripGen;
     if (linking) c->ptGen = c->caGen = c->tripGen;
-    if (linking) c->inListOwn = true;
+    if (linking) {
+      c->inListOwn = true;
+      c->callerLinks = false;
+    }
     c->caOnly = false;
     fill_stats(c, stats);
     return TRAX_OK;
