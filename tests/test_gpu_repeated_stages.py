@@ -79,3 +79,24 @@ def test_ca_stage_on_a_callers_links(trax_lib, graph, down):
         again = ctx.results()
     for k, v in first.items():
         assert np.array_equal(v, again[k]), k
+
+
+@pytest.mark.parametrize("linking", [True, False])
+@pytest.mark.parametrize("graph", [False, True])
+def test_batch_of_no_events(trax_lib, graph, linking):
+    """No events (an empty shard) run in both modes and give nothing, before and after a batch that gives something."""
+    some = events.generate(2, n_events=2)
+    none = some.subset([])
+    with trax_lib.Context(0) as ctx:
+        ctx.upload(none)
+        counts = []
+        for batch in (none, none, some, none, some):
+            ctx.upload_hits(batch)
+            st = ctx.seed_batch(use_graph=graph, run_linking=linking)
+            counts.append((st.n_pairs, st.n_candidates, st.n_triplets, st.n_links, st.n_track_entries))
+            h1, _, _, offsets = ctx.triplets()
+            assert h1.size == st.n_triplets and offsets[-1] == max(st.n_triplets, 1) - 1
+            if linking:
+                assert ctx.tracks()[1].size == st.n_track_entries
+    assert counts[0] == counts[1] == counts[3] == (0,) * 5
+    assert counts[2] == counts[4] and counts[2][2] > 0 and (counts[2][3] > 0) == linking

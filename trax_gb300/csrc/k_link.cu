@@ -652,13 +652,13 @@ cudaError_t ca_chain(const DevConfig& cfg, const float* pt, CABuffers b, const u
     return cudaGetLastError();
   }
   launch(q, ca_init_kernel, grid_for(maxT + 1, 256), 256, 0, b, nTDev, false);
-  const uint64_t events = cfg.E ? cfg.E : 1;
+  const uint64_t events = cfg.E ? cfg.E : 1;  // (a launch needs a block; without events it has no triplets)
   uint64_t bpe = maxT / (events * cfg.nLT * 256) + 1;
   const uint64_t most = (uint64_t)sm_count() * 16 / events + 1;
   if (bpe > most) bpe = most;
   for (uint32_t level = 1; level < cfg.nLT; ++level) {
     if (segStart)
-      launch(q, ca_level_kernel<true>, (unsigned)(cfg.E * bpe), 256, 0, cfg, level, (uint32_t)bpe, b, segStart,
+      launch(q, ca_level_kernel<true>, (unsigned)(events * bpe), 256, 0, cfg, level, (uint32_t)bpe, b, segStart,
              nTDev);
     else
       launch(q, ca_level_kernel<false>, grid_for(maxT, 256), 256, 0, cfg, level, 1u, b, segStart, nTDev);
