@@ -100,3 +100,36 @@ def test_batch_of_no_events(trax_lib, graph, linking):
                 assert ctx.tracks()[1].size == st.n_track_entries
     assert counts[0] == counts[1] == counts[3] == (0,) * 5
     assert counts[2] == counts[4] and counts[2][2] > 0 and (counts[2][3] > 0) == linking
+
+
+@pytest.mark.parametrize("graph", [False, True])
+def test_tracks_after_connectivity_again(trax_lib, graph):
+    """Connectivity run again leaves no earlier automaton's tracks: none with a cut that links nothing (the caller's
+    arrays stay as they are), an error until the automaton has run with one that links."""
+    batch = events.generate(2, n_events=3)
+    with trax_lib.Context(0) as ctx:
+        ctx.upload(batch)
+        ctx.seed_batch(use_graph=graph)
+        first = ctx.results()
+        assert first["tracks"].size > 0
+
+        def untouched():
+            n = first["trip_h1"].size
+            out = [np.full(k, 7, np.uint32) for k in (n, first["tracks"].size, n + 1)]
+            ctx.tracks(out=out)
+            return all((v == 7).all() for v in out)
+
+        assert ctx.connectivity(0.0) == 0
+        assert untouched()
+        ctx.circle_fit()
+        assert ctx.cellular_automaton() == 0
+        assert untouched()
+        assert ctx.connectivity(batch.d_eta_cut) == first["link_basis"].size
+        with pytest.raises(trax_lib.TraxError) as e:
+            ctx.tracks()
+        assert e.value.code == 6
+        ctx.circle_fit()
+        ctx.cellular_automaton()
+        again = ctx.results()
+    for k, v in first.items():
+        assert np.array_equal(v, again[k]), k

@@ -815,6 +815,7 @@ int run_stage(trax_ctx* c, int stage) {
     for (bool& u : c->stageUsed) u = false;
     for (bool& u : c->kUsed) u = false;
   }
+  if (stage == 5) c->caGen = 0;  // tracks of the links before
   mark(c, MARK_STAGE + stage - 1);
   switch (stage) {
     case 1: rc = begin_run(c, false); if (!rc) rc = stage_grid(c, SYNCED); break;
