@@ -133,3 +133,17 @@ def test_tracks_after_connectivity_again(trax_lib, graph):
         again = ctx.results()
     for k, v in first.items():
         assert np.array_equal(v, again[k]), k
+
+
+def test_circle_fit_when_connectivity_linked_nothing(trax_lib):
+    """trax_circle_fit fits the connectable triplets of the last connectivity: none, when that linked nothing, also after
+    trax_cellular_automaton_on gave the context links of the caller's."""
+    batch = events.generate(2, n_events=3)
+    with trax_lib.Context(0) as ctx:
+        ctx.upload(batch)
+        n = ctx.seed_batch(use_graph=False).n_triplets
+        assert (ctx.eta_pt()[1] > 0).any()
+        assert ctx.connectivity(0.0) == 0
+        ctx.cellular_automaton_on([0, 1], [n - 1, n - 1], np.ones(n, np.float32))
+        ctx.circle_fit()
+        assert (ctx.eta_pt()[1] == 0).all()

@@ -156,6 +156,7 @@ struct trax_ctx {
   uint64_t pairSent = 0, candSent = 0;
   int stage = 0;  // last completed stage: 1 grid .. 7 CA
   bool noLinks = true;
+  bool noConnectable = true;  // the last connectivity linked nothing and wrote no connectable flags
   // triplets of every segment ordered by (second hit, first hit): true for the
   // chain's own filter output; checked for caller-provided triplets
   bool sortedSegments = true;
@@ -680,7 +681,7 @@ int stage_connectivity(trax_ctx* c, Mode mode) {
   const uint32_t* nTDev = slot(c, S_TRIPLETS);
   if (mode == SYNCED) {
     c->nLinks = c->nConn = c->nNonConn = c->nTracks = 0;
-    c->noLinks = true;
+    c->noLinks = c->noConnectable = true;
   }
   RC(link_buffers(c, mode, maxT));
   ENSURE(linkCount, maxT + 1, 4);
@@ -707,7 +708,7 @@ int stage_connectivity(trax_ctx* c, Mode mode) {
   if (mode == SYNCED) {
     RC(read_total(c, S_LINKS, &c->nLinks));
     maxLinks = c->nLinks;
-    c->noLinks = c->nLinks == 0;
+    c->noLinks = c->noConnectable = c->nLinks == 0;
     if (c->noLinks) return TRAX_OK;  // TripletConnectivityTight.cpp:127-129
   }
   ENSURE(basis, maxLinks, 4);
@@ -735,7 +736,7 @@ int stage_fit(trax_ctx* c, Mode mode) {
   NvtxRange nvtx("trax.circle_fit");
   const uint64_t maxT = mode == SYNCED ? c->nT : c->capT;
   ENSURE(pt, maxT, 4);
-  if (mode == SYNCED && c->noLinks) {
+  if (mode == SYNCED && c->noConnectable) {  // (noLinks may be of trax_cellular_automaton_on's)
     CK(cudaMemsetAsync(c->pt.p, 0, (size_t)std::max<uint64_t>(maxT, 1) * 4, c->st));
     return TRAX_OK;
   }
@@ -1708,6 +1709,7 @@ int trax_seed_batch(trax_ctx* c, const trax_batch_opts* opts, trax_batch_stats* 
     if (linking) {
       c->inListOwn = true;
       c->callerLinks = false;
+      c->noConnectable = false;  // the graph writes the flags in any case
     }
     c->caOnly = false;
     fill_stats(c, stats);
