@@ -147,3 +147,29 @@ def test_circle_fit_when_connectivity_linked_nothing(trax_lib):
         ctx.cellular_automaton_on([0, 1], [n - 1, n - 1], np.ones(n, np.float32))
         ctx.circle_fit()
         assert (ctx.eta_pt()[1] == 0).all()
+
+
+def test_times_of_a_stage_run_again(trax_lib):
+    """A stage that runs again by itself has its new time and leaves the others theirs; every timed kernel lies inside
+    its stage."""
+    inside = {"grid": ["grid_build"], "pairs": ["pair_count", "pair_store"],
+              "predict": ["predict_count", "predict_store"], "filter": ["filter", "filter_store"],
+              "connectivity": ["connectivity_count", "connectivity_store"]}
+    batch = events.generate(2, n_events=3)
+    with trax_lib.Context(0) as ctx:
+        ctx.upload(batch)
+        ctx.seed_batch(use_graph=True)
+        ctx.seed_batch(use_graph=True)
+        stage, kernel = ctx.timings()
+        for s, ks in inside.items():
+            assert 0 < sum(kernel[k] for k in ks) <= stage[s] + 1e-6, s
+        ctx.seed_batch(use_graph=False)
+        before, kernel = ctx.timings()
+        for s, ks in inside.items():
+            assert 0 < sum(kernel[k] for k in ks) <= before[s] + 1e-6, s
+        for again, run in (("connectivity", lambda: ctx.connectivity(batch.d_eta_cut)), ("pairs", ctx.pair_gen)):
+            run()
+            after, _ = ctx.timings()
+            assert 0 < after[again] < 1e3
+            assert {s: t for s, t in after.items() if s != again} == {s: t for s, t in before.items() if s != again}
+            before = after

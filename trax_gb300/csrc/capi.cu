@@ -281,15 +281,16 @@ struct NvtxRange {
   NvtxRange& operator=(const NvtxRange&) = delete;
 };
 
-// Time marks: the stage boundaries, then a begin and an end per timed
-// kernel.  A mark is written by the next kernel launched as it starts.
-enum { MARK_STAGE = 0, MARK_KERNEL = N_STAGES + 1, MARK_N = MARK_KERNEL + 2 * TK_N };
+// Time marks: a begin and an end per stage (its own, so that a stage run again
+// by itself changes no other's time), then per timed kernel.  A mark is
+// written by the next kernel launched as it starts.
+enum { MARK_STAGE = 0, MARK_KERNEL = 2 * N_STAGES, MARK_N = MARK_KERNEL + 2 * TK_N };
 static_assert(MARK_N <= 32, "the marks pending on a queue are one word");
 const size_t SLOT_WORDS = 64;  // the marks follow the slots
 const size_t SLOT_BYTES = SLOT_WORDS * sizeof(uint32_t) + MARK_N * sizeof(unsigned long long);
 
 void mark(trax_ctx* c, int k) { c->q.marks.which |= 1u << k; }
-#define KBEG(k) mark(c, MARK_KERNEL + 2 * (k))
+#define KBEG(k) (mark(c, MARK_KERNEL + 2 * (k)), c->kUsed[k] = false)
 #define KEND(k) (mark(c, MARK_KERNEL + 2 * (k) + 1), c->kUsed[k] = true)
 uint32_t* dev_err(trax_ctx* c) { return slot(c, S_ERR); }
 
@@ -817,7 +818,8 @@ int run_stage(trax_ctx* c, int stage) {
     for (bool& u : c->kUsed) u = false;
   }
   if (stage == 5) c->caGen = 0;  // tracks of the links before
-  mark(c, MARK_STAGE + stage - 1);
+  c->stageUsed[stage - 1] = false;  // until it ends: a stage that fails has no time
+  mark(c, MARK_STAGE + 2 * (stage - 1));
   switch (stage) {
     case 1: rc = begin_run(c, false); if (!rc) rc = stage_grid(c, SYNCED); break;
     case 2: rc = stage_pairs(c, SYNCED); break;
@@ -829,7 +831,7 @@ int run_stage(trax_ctx* c, int stage) {
     default: return fail(c, TRAX_ERR_ARG, "unknown stage");
   }
   if (rc) return rc;
-  mark(c, MARK_STAGE + stage);  // written by the read-back below, or again as the next stage starts
+  mark(c, MARK_STAGE + 2 * (stage - 1) + 1);  // written by the read-back below
   c->stageUsed[stage - 1] = true;
   RC(check_device_error(c));
   if (stage == 5 && !c->noLinks) {  // the lists' lengths came with that read-back
@@ -850,10 +852,10 @@ int chain_device(trax_ctx* c, bool linking) {
   int (*stages[N_STAGES])(trax_ctx*, Mode) = {stage_grid, stage_pairs, stage_predict, stage_filter,
                                               stage_connectivity, stage_fit, stage_ca};
   const int n = linking ? N_STAGES : 4;
-  mark(c, MARK_STAGE);
   for (int s = 0; s < n; ++s) {
+    mark(c, MARK_STAGE + 2 * s);
     RC(stages[s](c, DEVICE));
-    mark(c, MARK_STAGE + s + 1);
+    mark(c, MARK_STAGE + 2 * s + 1);
     c->stageUsed[s] = true;
   }
   // the last node: slots and marks to the host
@@ -1724,7 +1726,7 @@ int trax_get_timings(trax_ctx* c, float* stage_ms, float* kernel_ms) {
   const unsigned long long* at = reinterpret_cast<const unsigned long long*>(c->hSlots + SLOT_WORDS);
   auto between = [at](int a, int b) { return (float)((double)(at[b] - at[a]) * 1e-6); };
   for (int s = 0; s < N_STAGES; ++s)
-    if (stage_ms) stage_ms[s] = c->stageUsed[s] ? between(MARK_STAGE + s, MARK_STAGE + s + 1) : -1.0f;
+    if (stage_ms) stage_ms[s] = c->stageUsed[s] ? between(MARK_STAGE + 2 * s, MARK_STAGE + 2 * s + 1) : -1.0f;
   for (int k = 0; k < TK_N; ++k)
     if (kernel_ms) kernel_ms[k] = c->kUsed[k] ? between(MARK_KERNEL + 2 * k, MARK_KERNEL + 2 * k + 1) : -1.0f;
   return TRAX_OK;
