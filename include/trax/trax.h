@@ -248,8 +248,9 @@ int trax_noalloc_set_wait(uint32_t polls, uint32_t skip_tile);
  * results are the same on every device.  fn: 0 atan2(a, b), 1 acos, 2 atan,
  * 3 asinh, 4 log, 5 a / b, 6 sqrt, 7 floor, 8 saturating float->uint32 and
  * 9 float->int32 (truncation, NaN -> 0; out holds the integer's bits);
- * 10-14 CUDA's own atan2f, acosf, atanf, asinhf, logf for comparison.
- * b may be null unless fn is 0, 5 or 10. */
+ * 10-14 CUDA's own atan2f, acosf, atanf, asinhf, logf for comparison;
+ * 15-17 the fit's reciprocal 1 / a, quotient a / b and root of a.
+ * b may be null unless fn is 0, 5, 10 or 16. */
 int trax_math_eval(int device, int fn, const float* a, const float* b, float* out, uint64_t n);
 
 /* Threads per block of the pair, prediction and filter kernels (multiples of

@@ -28,7 +28,7 @@ CHECKED_LIB_PATH = os.path.join(LIB_DIR, "libtrax_gb300_checked.so")
 
 SOURCES = ["k_scan.cu", "k_grid.cu", "k_pairs.cu", "k_triplets.cu", "k_link.cu", "capi.cu", "tune.cu", "k_fit.cu", "host_events.cpp", "k_events.cu", "k_tracks.cu", "k_math.cu"]
 HEADERS = ["trax_device.cuh", "trax_kernels.h", "trax_math.h", "trax_math_coeffs.h", "trax_stages.cuh",
-           "trax_lookback.cuh", "trax_events.h"]
+           "trax_lookback.cuh", "trax_fit_math.cuh", "trax_events.h"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 NVCC_FLAGS = ARCH + [
     "-O3", "-lineinfo", "-std=c++17",

@@ -184,7 +184,7 @@ def load() -> ctypes.CDLL:
 
 MATH_CODES = {"atan2": 0, "acos": 1, "atan": 2, "asinh": 3, "log": 4, "div": 5, "sqrt": 6, "floor": 7,
               "f2u_sat": 8, "f2i_sat": 9, "cuda_atan2f": 10, "cuda_acosf": 11, "cuda_atanf": 12,
-              "cuda_asinhf": 13, "cuda_logf": 14}
+              "cuda_asinhf": 13, "cuda_logf": 14, "fit_reciprocal": 15, "fit_quotient": 16, "fit_root": 17}
 
 
 def math_eval(fn: str, a: np.ndarray, b: Optional[np.ndarray] = None, device: int = 0) -> np.ndarray:

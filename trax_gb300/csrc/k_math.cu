@@ -1,9 +1,11 @@
 // k_math.cu -- the shared single-precision math (trax_math.h) evaluated on
 // the device, for the tests that hold it to the CPU build bit for bit and
-// to CUDA's own functions within a few ulp.
+// to CUDA's own functions within a few ulp; and the fit's quotients and roots
+// (trax_fit_math.cuh), held to the correctly rounded ones.
 #include <cuda_runtime.h>
 
 #include "trax/trax.h"
+#include "trax_fit_math.cuh"
 #include "trax_math.h"
 
 namespace {
@@ -30,6 +32,10 @@ __global__ void math_eval_kernel(int fn, const float* __restrict__ a, const floa
       case 12: r = atanf(x); break;
       case 13: r = asinhf(x); break;
       case 14: r = logf(x); break;
+      // the fit's
+      case 15: r = trax::Divisor(x).r; break;
+      case 16: r = x / trax::Divisor(y); break;
+      case 17: r = trax::root(x); break;
       default: break;
     }
     out[i] = r;
@@ -39,7 +45,7 @@ __global__ void math_eval_kernel(int fn, const float* __restrict__ a, const floa
 }  // namespace
 
 extern "C" int trax_math_eval(int device, int fn, const float* a, const float* b, float* out, uint64_t n) {
-  if (fn < 0 || fn > 14 || !a || !out || (n && !b && (fn == 0 || fn == 5 || fn == 10))) return TRAX_ERR_ARG;
+  if (fn < 0 || fn > 17 || !a || !out || (n && !b && (fn == 0 || fn == 5 || fn == 10 || fn == 16))) return TRAX_ERR_ARG;
   if (n == 0) return TRAX_OK;
   if (cudaSetDevice(device) != cudaSuccess) return TRAX_ERR_CUDA;
   float *da = nullptr, *db = nullptr, *dout = nullptr;
