@@ -28,9 +28,10 @@ constexpr int SCAN_ITEMS = 16;
 constexpr uint32_t SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
 // Scans of up to this many elements (by capacity) are left to one CTA, which
 // takes tile after tile: no tickets, no cleared scratch (a node or a call of its
-// own in the host-synced stages), no look-back.  37 events 436 -> 432 us, 100
-// events of 200 tracks 158.1 -> 157.5 us; 1024 threads took 2 to 4 us more of
-// the smallest batch's 115.
+// own in the host-synced stages), no look-back.  One event by stages 330.6 ->
+// 326.0 us, 100 events of 200 tracks 159.0 -> 157.8 us, 37 ttbar-like events
+// 436.7 -> 436.5 us, 10 events of 10 muons 117.1 -> 117.8 us; 1024 threads took
+// 2 to 4 us more of those last.
 constexpr int SCAN_ONE_THREADS = 512;
 constexpr uint32_t SCAN_ONE_MAX = 16384;
 
